@@ -225,10 +225,11 @@ struct View {
     int ntiles = 0;
     DevBuf<float4> pts;          // sorted points, .w = loop index (int bits)
     DevBuf<int32_t> tile_start;  // ntiles + 1
+    DevBuf<float4> box;          // tile boxes: lo at 2 t, hi at 2 t + 1
     std::vector<int32_t> h_tile_start;
     std::vector<Box> boxes;
     size_t upload_bytes = 0;  // host-to-device bytes of its construction
-    size_t bytes() const { return pts.bytes() + tile_start.bytes(); }
+    size_t bytes() const { return pts.bytes() + tile_start.bytes() + box.bytes(); }
 };
 
 // One split of order[lo, hi): along the widest axis, so that the left part
@@ -492,46 +493,6 @@ static int three_side_bin_of_d2(float d2, float lo, float hi, float bw, int n) {
     return (int)q;
 }
 
-// The pair code of a squared separation d2 (ref_bin_tp of the pair program,
-// src/2pcf_C_version.cc:57-86, on sqrtf(d2)): 0 below lo, bin + 1 inside,
-// nbins + 2 at or above hi.  IEEE single operations, as on the device.
-static int pair_code_of_d2(float d2, float lo, float hi, float bw, int n) {
-    volatile float d = sqrtf(d2);
-    if (d < lo) return 0;
-    if (d >= hi) return n + 2;
-    volatile float x = d - lo;
-    volatile float q = x / bw;
-    return (int)q + 1;
-}
-
-// Smallest non-negative float d2 whose code (a non-decreasing function of
-// d2) is >= v, by bisection over the ordered bit patterns of floats.
-template <class Code>
-static float smallest_d2_with_code(int v, Code code) {
-    uint32_t lo = 0, hi = 0x7F800000u;  // +0 .. +inf (the largest code)
-    while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        float x;
-        memcpy(&x, &mid, 4);
-        if (code(x) >= v) hi = mid;
-        else lo = mid + 1;
-    }
-    float r;
-    memcpy(&r, &lo, 4);
-    return r;
-}
-
-static bool pair_thresholds(PairParams& p) {
-    if (p.n + 4 > PR_UMAX) return false;
-    if (std::max(fabs((double)p.lo), fabs((double)p.hi)) / (double)p.bw > 16384.0) return false;
-    p.inv_bw = 1.0f / p.bw;
-    p.u[0] = -INFINITY;
-    for (int v = 1; v <= p.n + 2; v++)
-        p.u[v] = smallest_d2_with_code(v, [&](float x) { return pair_code_of_d2(x, p.lo, p.hi, p.bw, p.n); });
-    for (int v = p.n + 3; v < PR_UMAX; v++) p.u[v] = NAN;
-    return true;
-}
-
 // Thresholds u[v] (smallest float d2 >= 0 with bin >= v) by bisection over
 // the ordered bit patterns of non-negative floats; the bin is a
 // non-decreasing function of d2 (sqrt, subtraction, division and truncation
@@ -666,7 +627,7 @@ Binning make_binning(const tpcf_spec& sp) {
         p.lo = sp.axis[0].lo;
         p.hi = sp.axis[0].hi;
         p.bw = ref_bw(p.lo, p.hi, p.n);
-        p.fast = pair_thresholds(p) ? 1 : 0;
+        pair_guard(p);
         b.len = p.n;
         b.lmax = (double)p.hi * (1 + 1e-6) + 1e-6;
     } else {
@@ -675,6 +636,11 @@ Binning make_binning(const tpcf_spec& sp) {
     if (!sp.prune) {
         b.lmax = INFINITY;
         b.tri_prune = false;
+    }
+    if (sp.kind == TPCF_PAIR) {
+        const double r2 = b.lmax * b.lmax;
+        // (no counted separation at all below a negative upper edge)
+        b.pair.reach2 = b.lmax < 0 ? 0.f : r2 < 3e38 ? nextafterf((float)r2, INFINITY) : INFINITY;
     }
     // device copy of the bound, rounded up so that a float side >= it is >= lmax
     if (sp.kind == TPCF_TRIANGLE_JBJ) b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
@@ -793,6 +759,7 @@ struct Lane {
     size_t plan_ngroups = 0;  // task groups of the fast triangle kernel
     size_t plan_ntasks2 = 0, plan_ngroups2 = 0;  // second part of a pipelined plan (0: none)
     uint64_t plan_evaluated = 0;
+    int plan_chunk = 0;  // pairs: tiles B per item
     // the launch sequence of the last batch, captured as a CUDA graph and
     // replayed while the batch and every buffer it touches stay the same
     cudaGraphExec_t graph = nullptr;
@@ -999,8 +966,16 @@ std::shared_ptr<View> build_view(const Catalog& c, int64_t begin, int64_t end, i
     v->tile_start.reserve(v->ntiles + 1);
     CK(cudaMemcpyAsync(v->tile_start.p, v->h_tile_start.data(), (v->ntiles + 1) * sizeof(int32_t),
                        cudaMemcpyHostToDevice, st));
+    std::vector<float4> dbox(2 * std::max<size_t>(v->boxes.size(), 1));
+    for (size_t t = 0; t < v->boxes.size(); t++) {
+        const Box& b = v->boxes[t];
+        dbox[2 * t] = make_float4(b.lo[0], b.lo[1], b.lo[2], 0.f);
+        dbox[2 * t + 1] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.f);
+    }
+    v->box.reserve(dbox.size());
+    CK(cudaMemcpyAsync(v->box.p, dbox.data(), dbox.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
-    v->upload_bytes = pts.size() * sizeof(float4) + (v->ntiles + 1) * sizeof(int32_t);
+    v->upload_bytes = pts.size() * sizeof(float4) + (v->ntiles + 1) * sizeof(int32_t) + dbox.size() * sizeof(float4);
     if (plan_trace()) {
         auto ms = [](std::chrono::steady_clock::time_point a, std::chrono::steady_clock::time_point b) {
             return std::chrono::duration<double, std::milli>(b - a).count();
@@ -1110,11 +1085,6 @@ struct PlannedJob {
         return v[r].get();
     }
 };
-
-inline bool close_enough(const View& a, int ta, const View& b, int tb, double lmax) {
-    if (!(lmax < INFINITY)) return true;
-    return box_lower_bound(a.boxes[ta], b.boxes[tb]) < lmax;
-}
 
 uint64_t task_units3(const View& A, int a, const View& B, int b, const View& C, int c, uint32_t flags) {
     uint64_t na = A.h_tile_start[a + 1] - A.h_tile_start[a];
@@ -1348,29 +1318,6 @@ struct TripletPlan {
     }
 };
 
-// Pair tasks of A tiles [a0, a1).
-void plan_pairs(const tpcf_spec& sp, const PlannedJob& pj, uint32_t slot, double lmax, int a0, int a1,
-                TaskList& tasks, uint64_t& evaluated) {
-    const View &A = *pj.v[0], &B = *pj.v[1];
-    if (A.ntiles == 0 || B.ntiles == 0) return;
-    const bool same = pj.v[0] == pj.v[1] && sp.loop == TPCF_LOOP_SAME;
-    for (int a = a0; a < a1; a++)
-        for (int b = same ? a : 0; b < B.ntiles; b++) {
-            if (!close_enough(A, a, B, b, lmax)) continue;
-            uint64_t na = A.h_tile_start[a + 1] - A.h_tile_start[a], nb = B.h_tile_start[b + 1] - B.h_tile_start[b];
-            uint32_t flags = 0, pred = PRED_NONE;
-            uint64_t u = na * nb;
-            if (same && a == b) {
-                flags = TASK_DIAG_IJ;
-                u = na * (na + 1) / 2;
-            } else if (!same && sp.loop == TPCF_LOOP_SAME) {
-                pred = PRED_SAME;
-            }
-            evaluated += u;
-            tasks.push_back({u, make_uint4(slot | (pred << TASK_PRED_SHIFT) | flags, (uint32_t)a, (uint32_t)b, 0)});
-        }
-}
-
 // Host worker threads for planning, started once per process (thread
 // creation would cost more than the planning work of a small batch).  run()
 // calls fn(i) for i in [0, n) on the workers and the calling thread; a run
@@ -1555,16 +1502,16 @@ std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Bi
         Shape def;
         def.copies = -1;
         for (int cc : {8, 4, 2, 1}) {
-            Shape sh = fit(cc, 8);
+            Shape sh = fit(cc, PAIR_CTAS);
             if (sh.per_sm >= 2) {
                 def = sh;
                 break;
             }
         }
-        if (def.copies < 0) def = fit(1, 8);
+        if (def.copies < 0) def = fit(1, PAIR_CTAS);
         if (def.per_sm < 1) throw InvalidArg{"pair histogram too large"};
         add(def);
-        for (int cc : {8, 4, 2, 1}) add(fit(cc, 8));
+        for (int cc : {8, 4, 2, 1}) add(fit(cc, PAIR_CTAS));
     }
     return out;
 }
@@ -1803,7 +1750,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             const View* rv = pj[g].role(r);
             dj[g].pts[r] = rv->pts.p;
             dj[g].tile_start[r] = rv->tile_start.p;
+            dj[g].box[r] = rv->box.p;
+            dj[g].ntiles[r] = rv->ntiles;
         }
+        if (ncat == 2 && group[g].spec->loop == TPCF_LOOP_SAME)
+            dj[g].mode = pj[g].v[0] == pj[g].v[1] ? JOB_B_FROM_A : (uint32_t)PRED_SAME;
         dj[g].hist = L.d_hist.p + (size_t)bin.len * slot_of[g];
     };
     cudaStream_t st = L.stream;
@@ -1817,6 +1768,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                                                                               t_wall0).count()});
     };
     const bool pairs = sp.kind == TPCF_PAIR;
+    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item
     const bool fast_tri = (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) && guarded_fp32(sp, bin);
     // A newly planned batch of two to eight fast-kernel jobs (an estimator's
     // DDD/DDR/DRR/RRR set) is pipelined: the first job is planned, uploaded and
@@ -1848,10 +1800,26 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     // last two for the fast triangle kernel); returns the evaluated units.
     auto plan_jobs = [&](size_t g0, size_t g1, std::vector<uint4>& h_tasks, std::vector<uint32_t>& h_groups,
                          std::vector<float>& h_gbox) -> uint64_t {
+        if (pairs) {
+            // the pair kernel finds its tile pairs itself: the plan is the
+            // number of (tile A, chunk of tiles B) items of each job
+            long long tile_pairs = 0;
+            for (size_t g = g0; g < g1; g++) tile_pairs += (long long)pj[g].v[0]->ntiles * pj[g].v[1]->ntiles;
+            plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS);
+            h_groups.assign(1, 0);
+            uint64_t items = 0;
+            for (size_t g = g0; g < g1; g++) {
+                const uint64_t nbc = (pj[g].v[1]->ntiles + plan_chunk - 1) / plan_chunk;
+                items += (uint64_t)pj[g].v[0]->ntiles * nbc;
+                if (items > 0xF0000000ull) throw InvalidArg{"too many tile pairs in one batch"};
+                h_groups.push_back((uint32_t)items);
+            }
+            return 0;
+        }
         // plan in parallel: bound tables and neighbour lists by rows, then
-        // tile triples (pairs) by ranges of A tiles
+        // tile triples by ranges of A tiles
         uint64_t ev = 0;
-        if (!pairs) {
+        {
             const size_t t_first = table_list.size();
             const int pass = plan_pass++;
             auto table = [&](const View* x, const View* y, bool nb) {
@@ -1894,8 +1862,8 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         // tiles of a clustered catalog would otherwise each be one long item)
         std::vector<std::array<int, 5>> items;
         for (size_t g = g0; g < g1; g++) {
-            const int na = pj[g].role(0)->ntiles, step = pairs ? 16 : 2;
-            const PairTable* ab = pairs || tp[g].empty ? nullptr : tp[g].AB;
+            const int na = pj[g].role(0)->ntiles, step = 2;
+            const PairTable* ab = tp[g].empty ? nullptr : tp[g].AB;
             for (int a0 = 0; a0 < na;) {
                 const int nb = ab && ab->need_nb ? (int)ab->nb[a0].size() : 0;
                 if (nb > 48) {
@@ -1917,11 +1885,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         parallel_items(items.size(), [&](size_t i) {
             const auto& it = items[i];
             part[i].clear();
-            if (pairs)
-                plan_pairs(*group[it[0]].spec, pj[it[0]], (uint32_t)it[0], bin.lmax, it[1], it[2], part[i],
-                           part_eval[i]);
-            else
-                tp[it[0]].enumerate(it[1], it[2], part[i], part_eval[i], (size_t)it[3], (size_t)it[4]);
+            tp[it[0]].enumerate(it[1], it[2], part[i], part_eval[i], (size_t)it[3], (size_t)it[4]);
         });
         phase("enumerate");
         std::vector<size_t> off(items.size() + 1, 0);  // each item's first task
@@ -1995,10 +1959,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         const size_t ng = h_groups.empty() ? 0 : h_groups.size() - 1;
         if (ng) {
             d_groups.reserve(h_groups.size());
-            d_gbox.reserve(h_gbox.size());
+            d_gbox.reserve(std::max<size_t>(h_gbox.size(), 1));
             CK(cudaMemcpyAsync(d_groups.p, h_groups.data(), h_groups.size() * sizeof(uint32_t),
                                cudaMemcpyHostToDevice, s));
-            CK(cudaMemcpyAsync(d_gbox.p, h_gbox.data(), h_gbox.size() * sizeof(float), cudaMemcpyHostToDevice, s));
+            if (!h_gbox.empty())
+                CK(cudaMemcpyAsync(d_gbox.p, h_gbox.data(), h_gbox.size() * sizeof(float), cudaMemcpyHostToDevice, s));
             L.h2d += h_groups.size() * sizeof(uint32_t) + h_gbox.size() * sizeof(float);
         }
         d_tasks.reserve(std::max<size_t>(h_tasks.size(), 1));
@@ -2022,10 +1987,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         CK(cudaMemcpyAsync(L.d_jobs.p, dj.data(), g_first * sizeof(DevJob), cudaMemcpyHostToDevice, st));
         L.h2d += g_first * sizeof(DevJob);
         ngroups = upload_part(S.tasks, S.groups, S.gbox, L.d_tasks, L.d_groups, L.d_gbox, st);
-        ntasks = S.tasks.size();
+        ntasks = pairs ? (S.groups.empty() ? 0 : S.groups.back()) : S.tasks.size();
         CK(cudaStreamSynchronize(st));
         if (!pipeline) {
             L.plan_sig = sig;
+            L.plan_chunk = plan_chunk;
             L.plan_ntasks = ntasks;
             L.plan_ngroups = ngroups;
             L.plan_ntasks2 = L.plan_ngroups2 = 0;
@@ -2153,7 +2119,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                     if (sp.kind == TPCF_THREE_SIDE)
                         return launch_three_side(L.d_jobs.p, tk, n, L.d_counters.p, bin.three, fp64, grid, copies,
                                                  sh.groups, st);
-                    return launch_pairs(L.d_jobs.p, tk, n, L.d_counters.p, bin.pair, fp64, grid, copies, st);
+                    return launch_pairs(L.d_jobs.p, L.d_groups.p, (int)group.size(), t0, n, plan_chunk, L.d_counters.p,
+                                        reinterpret_cast<unsigned long long*>(L.d_counters.p + 2), bin.pair, fp64, grid,
+                                        copies, st);
                 };
                 if (two_part) {
                     // the first job's groups, then the others' (their own group
@@ -2331,9 +2299,10 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     // contain and counts the triangles it walks; other kernels walk every
     // triangle of their tasks
     const bool fast_kernel = (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) && !fp64;
-    L.stats.evaluated_units = fast_kernel ? dev_evaluated : evaluated;
-    L.stats.binned_units = fast_kernel ? dev_binned : evaluated;
-    L.stats.tasks = ntasks + ntasks2;
+    // (the pair kernel finds its tile pairs itself and counts them beside the pairs)
+    L.stats.evaluated_units = fast_kernel || pairs ? dev_evaluated : evaluated;
+    L.stats.binned_units = fast_kernel ? dev_binned : L.stats.evaluated_units;
+    L.stats.tasks = pairs ? dev_binned : ntasks + ntasks2;
     L.stats.kernel_launches = launches * std::max<uint64_t>(1, tuned_runs);
     L.stats.recheck_regrows = regrows;
     L.stats.total_ms =

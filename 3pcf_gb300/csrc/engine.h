@@ -8,6 +8,9 @@
 
 namespace tpcf {
 
+// Resident CTAs per SM of the pair kernels (their register budget).
+constexpr int PAIR_CTAS = 5;
+
 // Points per spatial tile.  A triangle task covers one tile of each role.
 constexpr int TILE = 64;
 
@@ -71,10 +74,14 @@ constexpr uint32_t CODE3_CLEAN_FAR = 1u << 28;
 struct DevJob {
     const float4* pts[3];        // spatially sorted points of roles A, B, C; .w = loop index (int bits)
     const int32_t* tile_start[3];// tile -> first point, ntiles+1 entries
+    const float4* box[3];        // tile bounding boxes: lo at 2 t, hi at 2 t + 1 (.w unused)
+    int32_t ntiles[3];
+    uint32_t mode;               // JOB_* bits
     unsigned long long* hist;    // global uint64 histogram (hist_len entries)
-    int32_t weight_pred;         // unused by kernels (kept for stats)
-    int32_t pad;
 };
+// the job's tile tuples and the predicate of its points
+constexpr uint32_t JOB_PRED_MASK = 0x7u;  // Pred
+constexpr uint32_t JOB_B_FROM_A = 8u;     // tiles B >= A of one view, positions j >= i in a diagonal pair
 
 // Launch-wide binning constants for the triangle kernels.
 struct TriParams {
@@ -117,18 +124,16 @@ struct ThreeParams {
     int zcode;  // bin of a zero-length side (nbins + 1 at or above hist_max)
 };
 
-constexpr int PR_UMAX = 704;  // squared-length thresholds of up to 700 pair bins
-
 struct PairParams {
     int n;
     float lo, hi, bw;
-    // Bins from squared lengths (guarded FP32 kernel, when fast != 0): the
-    // code of a separation d is 0 below lo, bin + 1 inside (up to nbins + 1
-    // where rounding gives bin nbins), nbins + 2 at or above hi; u[v] is the
-    // smallest float d2 whose code is >= v, u[0] = -inf, u[nbins + 3] = NaN.
+    // Guarded FP32 bins (when fast != 0): the coordinate d * inv_bw + off (bin
+    // coordinate - 0.5) from an approximate square root is within 0.5 - thr
+    // of the reference's; only values closer than that to a bin edge are
+    // recomputed with the reference's formula.
     int fast = 0;
-    float inv_bw = 0.f;
-    float u[PR_UMAX];
+    float inv_bw = 0.f, off = 0.f, thr = 0.f;
+    float reach2 = 0.f;  // tiles at least sqrt(reach2) apart hold no counted pair (rounded up)
 };
 
 // Exact glibc-acosf exception table on the device.
@@ -166,9 +171,12 @@ cudaError_t launch_triangle_fp64(const DevJob* jobs, const uint4* tasks, unsigne
 cudaError_t launch_three_side(const DevJob* jobs, const uint4* tasks, unsigned int ntasks,
                               unsigned int* task_counter, const ThreeParams& p, int fp64, int grid,
                               int hist_copies, int groups, cudaStream_t st);
-cudaError_t launch_pairs(const DevJob* jobs, const uint4* tasks, unsigned int ntasks,
-                         unsigned int* task_counter, const PairParams& p, int fp64, int grid,
-                         int hist_copies, cudaStream_t st);
+// item_off[j] .. item_off[j + 1]: the items (tile A, chunk of `chunk` tiles B)
+// of job j; counts items [item0, item0 + nitems); work[0], work[1] receive the
+// pairs and tile pairs evaluated
+cudaError_t launch_pairs(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
+                         unsigned int nitems, int chunk, unsigned int* counter, unsigned long long* work,
+                         const PairParams& p, int fp64, int grid, int hist_copies, cudaStream_t st);
 cudaError_t launch_acos_check(AcosTable t, uint32_t key_begin, uint32_t count, unsigned int* mismatches,
                               cudaStream_t st);
 cudaError_t launch_radecz_to_xyz(const double* ra, const double* dec, const double* redshift, int64_t n,
@@ -178,6 +186,8 @@ cudaError_t launch_radecz_to_xyz(const double* ra, const double* dec, const doub
 size_t triangle_smem_bytes(int hist_len, int hist_copies);
 size_t three_side_smem_bytes(const ThreeParams& p, int hist_copies, int groups);
 size_t pair_smem_bytes(int hist_len, int hist_copies);
+void pair_guard(PairParams& p);  // from p.n, lo, hi, bw
+int pair_chunk(long long tile_pairs, int ctas);
 
 }  // namespace tpcf
 #endif

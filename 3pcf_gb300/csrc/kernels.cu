@@ -18,6 +18,7 @@
 // exact arithmetic (including glibc's acosf through an exception table).
 #include <stdint.h>
 #include <limits.h>
+#include <math.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1768,103 +1769,230 @@ three_side_grouped_kernel(const DevJob* __restrict__ jobs, const uint4* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Pair counts (src/2pcf_C_version.cc).  Tasks name a tile of each role (w unused).
+// Pair counts (src/2pcf_C_version.cc).
 
 constexpr int PR_WARPS = 8;
 constexpr int PR_THREADS = PR_WARPS * 32;
+constexpr int PR_CHUNK_MAX = 32;  // tiles B of one item at most (one mask word)
 constexpr size_t PR_SMEM_FIXED = 2 * TILE * sizeof(float4);
 
-// Pair bin of the separation a-b, -1 if not counted.  The guarded FP32
-// kernel works on the squared separation: a first guess from an approximate
-// square root (within one step) corrected against the exact thresholds U of
-// the neighbouring steps of the code (0 below lo, bin + 1, nbins + 2 at or
-// above hi); the plain FP64 kernel evaluates the reference's formula.
+// Tile A of an item, by coordinate, so that four points of one coordinate come
+// in one 16-byte load; points past the end are NaN.
+struct PairTile {
+    float x[TILE], y[TILE], z[TILE];
+    int key[TILE];
+};
+static_assert(sizeof(PairTile) <= PR_SMEM_FIXED, "pair tile");
+
+// The reference's pair bin of the separation a-b, -1 if not counted.
 template <bool FP64>
-__device__ __forceinline__ int pair_bin(float4 a, float4 b, const PairParams& p, const float* U) {
-    if (!FP64 && p.fast) {
-        const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y), dz = __fsub_rn(a.z, b.z);
-        float d2 = __fmul_rn(dx, dx);
-        d2 = __fadd_rn(d2, __fmul_rn(dy, dy));
-        d2 = __fadd_rn(d2, __fmul_rn(dz, dz));
-        float da;
-        asm("sqrt.approx.f32 %0, %1;" : "=f"(da) : "f"(d2));
-        // rounded guess (as for the three-side codes: the code jumps over
-        // nbins + 1 where d reaches hi)
-        int v = __float2int_rn(__fmul_rn(__fsub_rn(da, p.lo), p.inv_bw)) + 1;
-        v = min(max(v, 0), p.n + 2);
-        v = v - 1 + (d2 >= U[v] ? 1 : 0) + (d2 >= U[v + 1] ? 1 : 0);
-        return v >= 1 && v <= p.n ? v - 1 : -1;
-    }
+__device__ __forceinline__ int pair_bin(float4 a, float4 b, const PairParams& p) {
     const int bn = ref_bin_tp<FP64>(ref_dist<FP64>(a, b), p.lo, p.hi, p.n, 0);
     return bn >= 0 && bn < p.n ? bn : -1;
 }
 
-template <bool FP64, int PRED>
-__device__ void pair_task(const DevJob& J, uint4 task, const PairParams& p, const float* U, float4* P,
-                          unsigned int* Hw) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int a0 = J.tile_start[0][task.y], nA = J.tile_start[0][task.y + 1] - a0;
-    const int b0 = J.tile_start[1][task.z], nB = J.tile_start[1][task.z + 1] - b0;
-    const bool diag = task.x & TASK_DIAG_IJ;
-    for (int t = threadIdx.x; t < 2 * TILE; t += blockDim.x) {
-        int role = t / TILE, idx = t % TILE;
-        int nn = role == 0 ? nA : nB, base = role == 0 ? a0 : b0;
-        P[t] = idx < nn ? J.pts[role][base + idx] : make_float4(0.f, 0.f, 0.f, 0.f);
+// Which pairs of two tiles count: every one, positions j >= i of one tile
+// (self pairs are counted, as the reference's j >= i), or loop indices j >= i.
+enum PairKind : int { PK_ALL = 0, PK_DIAG = 1, PK_KEY = 2 };
+
+// Counts points [i0, i1) of tile A (i0 a multiple of 4) against tile B, whose
+// points lane and lane + 32 each lane holds.  Guarded FP32: the squared
+// separations of two points i run in packed f32x2 instructions, the bin
+// coordinate comes from rsqrt.approx, and a coordinate inside the guard band
+// around a bin edge -- or NaN: zero separations, padded and NaN points -- goes
+// to the reference's formula.  Issue-bound: about 14 lane-instructions a pair
+// instead of 57 with exact square roots and threshold lookups for every pair.
+template <bool FP64, int KIND>
+__device__ __forceinline__ void pair_tiles(const PairTile& A, int i0, int i1, const float4 (&pj)[2], int nB,
+                                           const PairParams& p, unsigned int* Hw) {
+    const int lane = threadIdx.x & 31;
+    auto counted = [&](int i, int r) -> bool {
+        if (KIND == PK_DIAG) return lane + 32 * r >= i;
+        if (KIND == PK_KEY) return pkey(pj[r]) >= A.key[i];
+        return true;
+    };
+    auto exact = [&](int i, int r) {
+        if (i >= i1 || lane + 32 * r >= nB || !counted(i, r)) return;
+        const int b = pair_bin<FP64>(make_float4(A.x[i], A.y[i], A.z[i], 0.f), pj[r], p);
+        if (b >= 0) atomicAdd(Hw + b, 1u);
+    };
+    if (FP64 || !p.fast) {
+        for (int i = i0; i < i1; i++) {
+            exact(i, 0);
+            exact(i, 1);
+        }
+        return;
     }
-    __syncthreads();
-    // each lane keeps its two points of tile B in registers for the whole task
-    const float4 pj[2] = {P[TILE + lane], P[TILE + lane + 32]};
-    for (int i = warp; i < nA; i += PR_WARPS) {
-        const float4 pi = P[i];
-        const int ki = pkey(pi);
+    const f32x2 X[2] = {splat2(pj[0].x), splat2(pj[1].x)}, Y[2] = {splat2(pj[0].y), splat2(pj[1].y)},
+                Z[2] = {splat2(pj[0].z), splat2(pj[1].z)};
+    const f32x2 scale = splat2(p.inv_bw), off = splat2(p.off);
+    for (int i = i0; i < i1; i += 4) {
+        const float4 x4 = *reinterpret_cast<const float4*>(A.x + i), y4 = *reinterpret_cast<const float4*>(A.y + i),
+                     z4 = *reinterpret_cast<const float4*>(A.z + i);
+        const f32x2 xi[2] = {pk2(x4.x, x4.y), pk2(x4.z, x4.w)}, yi[2] = {pk2(y4.x, y4.y), pk2(y4.z, y4.w)},
+                    zi[2] = {pk2(z4.x, z4.y), pk2(z4.z, z4.w)};
+        unsigned redo = 0;  // bit 4 h + 2 t + r: pair (i + 2 h + t, lane + 32 r) near a bin edge
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const int j = lane + 32 * r;
-            if (j >= nB) continue;
-            if (diag && j < i) continue;  // self pairs (j == i) are counted, as the reference's j >= i
-            if (PRED == PRED_SAME && pkey(pj[r]) < ki) continue;
-            const int b = pair_bin<FP64>(pi, pj[r], p, U);
-            if (b >= 0) atomicAdd(Hw + b, 1u);
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const f32x2 dx = sub2(xi[h], X[r]), dy = sub2(yi[h], Y[r]), dz = sub2(zi[h], Z[r]);
+                const f32x2 d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+                float s0, s1, e[2];
+                int b[2];
+                up2(d2, s0, s1);
+                const f32x2 d = mul2(d2, pk2(rsqrt_approx(s0), rsqrt_approx(s1)));
+                magic_floor2(fma2(d, scale, off), b[0], b[1], e[0], e[1]);
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+                    const bool safe = fabsf(e[t]) <= p.thr;
+                    if (safe && (unsigned)b[t] < (unsigned)p.n && counted(i + 2 * h + t, r)) atomicAdd(Hw + b[t], 1u);
+                    if (!safe) redo |= 1u << (4 * h + 2 * t + r);
+                }
+            }
+        while (redo) {
+            const int q = __ffs(redo) - 1;
+            redo &= redo - 1u;
+            exact(i + (q >> 1), q & 1);
         }
     }
-    __syncthreads();
 }
 
 template <bool FP64>
-__global__ void __launch_bounds__(PR_THREADS)
-pair_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tasks, unsigned int ntasks,
-            unsigned int* task_counter, PairParams p, int copies) {
+__device__ __forceinline__ void pair_tiles_kind(int kind, const PairTile& A, int i0, int i1, const float4 (&pj)[2],
+                                                int nB, const PairParams& p, unsigned int* Hw) {
+    if (kind == PK_DIAG) pair_tiles<FP64, PK_DIAG>(A, i0, i1, pj, nB, p, Hw);
+    else if (kind == PK_KEY) pair_tiles<FP64, PK_KEY>(A, i0, i1, pj, nB, p, Hw);
+    else pair_tiles<FP64, PK_ALL>(A, i0, i1, pj, nB, p, Hw);
+}
+
+// Runs f(q, i0, i1) for this warp's share of n tiles B against nA points of
+// tile A: with few tiles B the points of A are shared out too.
+template <typename F>
+__device__ __forceinline__ void pair_share(int n, int nA, F&& f) {
+    const int warp = threadIdx.x >> 5;
+    const int split = n >= 2 * PR_WARPS ? 1 : (n >= PR_WARPS ? 2 : (n >= 4 ? 4 : 8)), len = TILE / split;
+    for (int u = warp; u < n * split; u += PR_WARPS) {
+        const int i0 = (u % split) * len;
+        if (i0 < nA) f(u / split, i0, min(i0 + len, nA));
+    }
+}
+
+// Last job j of [0, n) with off[j] <= t (off[0] <= t; a job without items is
+// never the last one), searched 32 ways at a time by a whole warp.
+__device__ __forceinline__ int find_job(const uint32_t* __restrict__ off, int n, uint32_t t) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = n;
+    while (len > 1) {
+        const int step = (len + 31) / 32;
+        const bool le = lane * step < len && off[lo + lane * step] <= t;
+        const int k = 31 - __clz(__ballot_sync(0xffffffffu, le) | 1u);
+        lo += k * step;
+        len = min(step, len - k * step);
+    }
+    return lo;
+}
+
+// Squared gap of two tile boxes (reduced by a margin that covers the rounding
+// of the bound and of the reference's separation) below reach2: the tiles can
+// hold a counted pair.
+__device__ __forceinline__ bool boxes_near(const float4* __restrict__ A, const float4* __restrict__ B, float reach2) {
+    const float4 al = A[0], ah = A[1], bl = B[0], bh = B[1];
+    const float gx = fmaxf(0.f, fmaxf(al.x - bh.x, bl.x - ah.x));
+    const float gy = fmaxf(0.f, fmaxf(al.y - bh.y, bl.y - ah.y));
+    const float gz = fmaxf(0.f, fmaxf(al.z - bh.z, bl.z - ah.z));
+    // (an overflowing gap is kept below an infinite reach only)
+    return !((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f) >= reach2);
+}
+
+// Persistent over items (job, tile A, chunk of tiles B); the first warp draws
+// the next item with tiles B in reach, stages its tile A and leaves the mask of
+// those tiles; the warps share the tiles B out, each keeping its tile's points
+// in registers.  No task list: an item is its index, its tiles are tested
+// here against the views' boxes.
+template <bool FP64>
+__global__ void __launch_bounds__(PR_THREADS, PAIR_CTAS)
+pair_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ item_off, int njobs, unsigned int item0,
+            unsigned int nitems, int chunk, unsigned int* counter, unsigned long long* work, PairParams p, int copies) {
     extern __shared__ __align__(16) unsigned char smem[];
-    float4* P = reinterpret_cast<float4*>(smem);
+    PairTile& A = *reinterpret_cast<PairTile*>(smem);
     unsigned int* H = reinterpret_cast<unsigned int*>(smem + PR_SMEM_FIXED);
-    __shared__ uint4 s_task;
-    __shared__ float s_u[PR_UMAX];
-    if (!FP64 && p.fast)
-        for (int v = threadIdx.x; v < PR_UMAX; v += blockDim.x) s_u[v] = p.u[v];
+    __shared__ int4 s_item;  // job (-1: none), first tile B, mask of tiles B, tile A
     for (int b = threadIdx.x; b < copies * p.n; b += blockDim.x) H[b] = 0;
-    unsigned int* Hw = H + ((threadIdx.x >> 5) % copies) * p.n;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned int* Hw = H + (warp % copies) * p.n;
+    unsigned long long pairs = 0;   // lanes of the first warp
+    unsigned int tile_pairs = 0;
     int cur = -1;
     unsigned int since = 0;
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int t = atomicAdd(task_counter, 1u);
-            s_task = t < ntasks ? tasks[t] : make_uint4(TASK_NONE, 0, 0, 0);
+        if (warp == 0) {
+            int4 it = make_int4(-1, 0, 0, 0);
+            for (;;) {
+                unsigned int t = 0;
+                if (lane == 0) t = atomicAdd(counter, 1u);
+                t = __shfl_sync(0xffffffffu, t, 0);
+                if (t >= nitems) break;
+                t += item0;
+                const int slot = find_job(item_off, njobs, t);
+                const DevJob& J = jobs[slot];
+                const unsigned int nbc = (unsigned int)(J.ntiles[1] + chunk - 1) / chunk, l = t - item_off[slot];
+                const int a = (int)(l / nbc), b0 = (int)(l % nbc) * chunk, b = b0 + lane;
+                const bool near = lane < chunk && b < J.ntiles[1] && (!(J.mode & JOB_B_FROM_A) || b >= a) &&
+                                  boxes_near(J.box[0] + 2 * (size_t)a, J.box[1] + 2 * (size_t)b, p.reach2);
+                const unsigned int mask = __ballot_sync(0xffffffffu, near);
+                if (!mask) continue;
+                const int a0 = J.tile_start[0][a], nA = J.tile_start[0][a + 1] - a0;
+                if (near) {
+                    const unsigned int nB = (unsigned int)(J.tile_start[1][b + 1] - J.tile_start[1][b]);
+                    pairs += (J.mode & JOB_B_FROM_A) && b == a ? (unsigned)nA * ((unsigned)nA + 1u) / 2u : (unsigned)nA * nB;
+                    tile_pairs++;
+                }
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const int i = lane + 32 * r;
+                    const float4 v = i < nA ? J.pts[0][a0 + i] : make_float4(NAN, NAN, NAN, 0.f);
+                    A.x[i] = v.x;
+                    A.y[i] = v.y;
+                    A.z[i] = v.z;
+                    A.key[i] = pkey(v);
+                }
+                it = make_int4(slot, b0, (int)mask, a);
+                break;
+            }
+            if (lane == 0) s_item = it;
         }
         __syncthreads();
-        const uint4 task = s_task;
-        const int slot = task.x == TASK_NONE ? -1 : (int)(task.x & TASK_SLOT_MASK);
-        if ((slot != cur || since >= 4096) && cur >= 0) {
+        const int4 it = s_item;
+        // (an item adds at most 32 x 64^2 counts to a bin: 4096 items keep the 32-bit counters below 2^30)
+        if ((it.x != cur || since >= 4096) && cur >= 0) {
             flush_hist(H, copies, p.n, jobs[cur].hist);
             since = 0;
         }
-        cur = slot;
-        if (slot < 0) break;
+        cur = it.x;
+        if (cur < 0) break;
         since++;
-        if (((task.x >> TASK_PRED_SHIFT) & TASK_PRED_MASK) == PRED_SAME)
-            pair_task<FP64, PRED_SAME>(jobs[slot], task, p, s_u, P, Hw);
-        else
-            pair_task<FP64, PRED_NONE>(jobs[slot], task, p, s_u, P, Hw);
+        const DevJob& J = jobs[cur];
+        const int nA = J.tile_start[0][it.w + 1] - J.tile_start[0][it.w];
+        unsigned int left = (unsigned int)it.z;
+        int at = 0;  // tiles of the mask taken from `left`
+        pair_share(__popc((unsigned int)it.z), nA, [&](int q, int i0, int i1) {
+            for (; at < q; at++) left &= left - 1u;
+            const int b = it.y + __ffs(left) - 1;
+            const int b0 = J.tile_start[1][b], nB = J.tile_start[1][b + 1] - b0;
+            float4 pj[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+                pj[r] = lane + 32 * r < nB ? J.pts[1][b0 + lane + 32 * r] : make_float4(NAN, NAN, NAN, 0.f);
+            const int kind = (J.mode & JOB_PRED_MASK) == PRED_SAME ? PK_KEY
+                             : (J.mode & JOB_B_FROM_A) && b == it.w ? PK_DIAG : PK_ALL;
+            pair_tiles_kind<FP64>(kind, A, i0, i1, pj, nB, p, Hw);
+        });
+    }
+    if (warp == 0) {
+        if (pairs) atomicAdd(work, pairs);
+        if (tile_pairs) atomicAdd(work + 1, (unsigned long long)tile_pairs);
     }
 }
 
@@ -1892,6 +2020,31 @@ size_t three_side_smem_bytes(const ThreeParams& p, int copies, int groups) {
     if (groups > 0) return (size_t)groups * pipe + (size_t)words * 4;
     return pipe + (size_t)words * copies * 4;
 }
+// Guard band of the fast pair bins.  With u = 2^-24 the reference's separation
+// is within 2.5 u of the exact one of the same float differences and the fast
+// one (packed FMAs, rsqrt.approx at 2^-22.9, one product) within 4.7 u; the
+// subtraction of lo, the two divisions by bw and the fused coordinate add at
+// most 5.5 u of the coordinate range D = max(|lo|, |hi|) / bw + 1: together
+// below 12.7 u D = 7.6e-7 D bins.  The band is 1e-6 (D + 1).  Finer binnings
+// than 2^16 steps go to the reference's formula pair by pair.
+void pair_guard(PairParams& p) {
+    const double D = std::max(fabs((double)p.lo), fabs((double)p.hi)) / (double)p.bw + 1.0;
+    p.fast = D <= 65536.0 && p.bw >= 1e-30f ? 1 : 0;
+    if (!p.fast) return;
+    p.inv_bw = (float)(1.0 / (double)p.bw);
+    p.off = (float)(-(double)p.lo / (double)p.bw - 0.5);
+    p.thr = (float)(0.5 - 1e-6 * (D + 1.0));
+}
+
+// Tiles B per item of the pair kernels: as many as leave eight items to every
+// resident CTA, at least one for each of its warps (an item's tile A is staged
+// once, but the items are what balances the CTAs).
+int pair_chunk(long long tile_pairs, int ctas) {
+    int chunk = PR_CHUNK_MAX;
+    while (chunk > PR_WARPS && tile_pairs / chunk < 8ll * ctas) chunk /= 2;
+    return chunk;
+}
+
 size_t pair_smem_bytes(int hist_len, int copies) { return PR_SMEM_FIXED + (size_t)hist_len * copies * 4; }
 
 // Every counting kernel may use the device's whole opt-in shared memory per
@@ -2014,13 +2167,17 @@ cudaError_t launch_radecz_to_xyz(const double* ra, const double* dec, const doub
     return cudaGetLastError();
 }
 
-cudaError_t launch_pairs(const DevJob* jobs, const uint4* tasks, unsigned int ntasks, unsigned int* task_counter,
+cudaError_t launch_pairs(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
+                         unsigned int nitems, int chunk, unsigned int* counter, unsigned long long* work,
                          const PairParams& p, int fp64, int grid, int copies, cudaStream_t st) {
+    if (chunk < 1 || chunk > PR_CHUNK_MAX) return cudaErrorInvalidValue;
     size_t smem = pair_smem_bytes(p.n, copies);
     if (fp64)
-        pair_kernel<true><<<grid, PR_THREADS, smem, st>>>(jobs, tasks, ntasks, task_counter, p, copies);
+        pair_kernel<true><<<grid, PR_THREADS, smem, st>>>(jobs, item_off, njobs, item0, nitems, chunk, counter, work, p,
+                                                          copies);
     else
-        pair_kernel<false><<<grid, PR_THREADS, smem, st>>>(jobs, tasks, ntasks, task_counter, p, copies);
+        pair_kernel<false><<<grid, PR_THREADS, smem, st>>>(jobs, item_off, njobs, item0, nitems, chunk, counter, work,
+                                                           p, copies);
     return cudaGetLastError();
 }
 
@@ -2038,91 +2195,70 @@ cudaError_t launch_acos_check(AcosTable t, uint32_t key_begin, uint32_t count, u
 // For callers that cannot call cudaMalloc -- code running inside a framework
 // that owns all device memory through its own pool, or a library that must not
 // grow the process's footprint behind its host application's back.  They pass
-// device pointers to their catalogs and to the output histogram; every other
-// buffer the count needs (packed points, tile table, job descriptor, task
-// counter) is the file-scope array below, which exists on every device that
-// loads this library until the process exits.
-//
-// Limits and sharing: at most NOALLOC_MAX_POINTS points per catalog; all calls
-// on a device share the array, so calls whose work overlaps on the GPU (two
-// streams, or two host threads) race and must be serialised by the caller.
-// The array keeps the previous call's contents; everything that must start
-// from zero (task counter, output histogram) is cleared by the call itself.
+// device pointers to their catalogs and to the output histogram; the kernel
+// reads the coordinates where they are and needs no other buffer, so that
+// calls may overlap.  At most NOALLOC_MAX_POINTS points per catalog.
 // ===========================================================================
 
 namespace tpcf {
 
 constexpr int64_t NOALLOC_MAX_POINTS = 1 << 18;             // per catalog
-constexpr int NOALLOC_MAX_TILES = (int)(NOALLOC_MAX_POINTS / TILE);
 
-struct NoAllocScratch {
-    float4 pts[2][NOALLOC_MAX_POINTS];        // 2 x 4 MiB
-    int32_t tile_start[2][NOALLOC_MAX_TILES + 1];
-    DevJob job;
-    unsigned int task_counter;
-};
-static __device__ __align__(256) NoAllocScratch g_noalloc;  // 8 MiB per device
-
-// packs SoA catalogs into the scratch points (.w = loop index), fills the tile
-// table, resets the task counter
-__global__ void noalloc_prepare(const float* x0, const float* y0, const float* z0, int n0, const float* x1,
-                                const float* y1, const float* z1, int n1, unsigned long long* hist) {
-    NoAllocScratch* S = &g_noalloc;
-    const int stride = gridDim.x * blockDim.x;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int i = tid; i < n0; i += stride) S->pts[0][i] = make_float4(x0[i], y0[i], z0[i], __int_as_float(i));
-    for (int i = tid; i < n1; i += stride) S->pts[1][i] = make_float4(x1[i], y1[i], z1[i], __int_as_float(i));
-    const int t0 = (n0 + TILE - 1) / TILE, t1 = (n1 + TILE - 1) / TILE;
-    for (int t = tid; t <= t0; t += stride) S->tile_start[0][t] = min(t * TILE, n0);
-    for (int t = tid; t <= t1; t += stride) S->tile_start[1][t] = min(t * TILE, n1);
-    if (tid == 0) {
-        S->job.pts[0] = S->pts[0];
-        S->job.pts[1] = S->pts[1];
-        S->job.pts[2] = S->pts[1];
-        S->job.tile_start[0] = S->tile_start[0];
-        S->job.tile_start[1] = S->tile_start[1];
-        S->job.tile_start[2] = S->tile_start[1];
-        S->job.hist = hist;
-        S->task_counter = 0u;
-    }
-}
-
-// pair_kernel with tile-pair tasks computed from the counter value (no task
-// list): task t is tile pair (t / ntB, t % ntB); 'same' enumerates only a <= b
-// of one catalog with j >= i inside the diagonal tile
-template <bool FP64>
-__global__ void __launch_bounds__(PR_THREADS)
-pair_kernel_noalloc(unsigned int* task_counter, int ntA, int ntB, int same, int pred_same, PairParams p, int copies) {
+// Pair counts straight from coordinate arrays: tiles are runs of 64 points,
+// item t is tile A t / nbc with chunk t % nbc of tiles B (from tile A on with
+// 'same': one catalog, j >= i), handed out in grid strides (without spatial
+// order every tile pair costs the same), so that neither a packed copy, a
+// task list nor a counter is needed.
+__global__ void __launch_bounds__(PR_THREADS, PAIR_CTAS)
+pair_kernel_noalloc(const float* __restrict__ x0, const float* __restrict__ y0, const float* __restrict__ z0, int n0,
+                    const float* __restrict__ x1, const float* __restrict__ y1, const float* __restrict__ z1, int n1,
+                    int same, int pred_same, int chunk, PairParams p, int copies, unsigned long long* hist) {
     extern __shared__ __align__(16) unsigned char smem[];
-    float4* P = reinterpret_cast<float4*>(smem);
+    PairTile& A = *reinterpret_cast<PairTile*>(smem);
     unsigned int* H = reinterpret_cast<unsigned int*>(smem + PR_SMEM_FIXED);
-    __shared__ unsigned int s_t;
-    const DevJob& J = g_noalloc.job;
     for (int b = threadIdx.x; b < copies * p.n; b += blockDim.x) H[b] = 0;
+    const int lane = threadIdx.x & 31;
     unsigned int* Hw = H + ((threadIdx.x >> 5) % copies) * p.n;
-    const unsigned int ntasks = (unsigned int)ntA * (unsigned int)ntB;
-    for (;;) {
+    const int ntA = (n0 + TILE - 1) / TILE, ntB = (n1 + TILE - 1) / TILE, nbc = (ntB + chunk - 1) / chunk;
+    // (at most 2^18 points per catalog: a CTA's counters stay below 2^32 unless
+    // one bin of a CTA collects a sixteenth of all 2^36 pairs: flush in between)
+    unsigned int since = 0;
+    for (int t = blockIdx.x; t < ntA * nbc; t += gridDim.x) {
+        const int a = t / nbc, b0 = (same ? a : 0) + (t % nbc) * chunk, nb = min(chunk, ntB - b0);
+        if (nb <= 0) continue;
+        if (++since > 4096) {
+            flush_hist(H, copies, p.n, hist);
+            since = 1;
+        }
+        const int a0 = a * TILE, nA = min(TILE, n0 - a0);
+        __syncthreads();  // the previous item is done with tile A
+        if (threadIdx.x < TILE) {
+            const int i = threadIdx.x;
+            const bool in = i < nA;
+            A.x[i] = in ? x0[a0 + i] : NAN;
+            A.y[i] = in ? y0[a0 + i] : NAN;
+            A.z[i] = in ? z0[a0 + i] : NAN;
+            A.key[i] = a0 + i;
+        }
         __syncthreads();
-        if (threadIdx.x == 0) s_t = atomicAdd(task_counter, 1u);
-        __syncthreads();
-        const unsigned int t = s_t;
-        if (t >= ntasks) break;
-        const unsigned int a = t / (unsigned int)ntB, b = t % (unsigned int)ntB;
-        if (same && b < a) continue;
-        uint4 task = make_uint4((same && a == b ? TASK_DIAG_IJ : 0u), a, b, 0u);
-        if (pred_same) pair_task<FP64, PRED_SAME>(J, task, p, nullptr, P, Hw);
-        else pair_task<FP64, PRED_NONE>(J, task, p, nullptr, P, Hw);
+        pair_share(nb, nA, [&](int q, int i0, int i1) {
+            const int b = b0 + q, j0 = b * TILE, nB = min(TILE, n1 - j0);
+            float4 pj[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int j = lane + 32 * r;
+                pj[r] = j < nB ? make_float4(x1[j0 + j], y1[j0 + j], z1[j0 + j], __int_as_float(j0 + j))
+                               : make_float4(NAN, NAN, NAN, 0.f);
+            }
+            pair_tiles_kind<false>(pred_same ? PK_KEY : same && a == b ? PK_DIAG : PK_ALL, A, i0, i1, pj, nB, p, Hw);
+        });
     }
-    flush_hist(H, copies, p.n, J.hist);
+    flush_hist(H, copies, p.n, hist);
 }
 
 }  // namespace tpcf
 
-// Declared in include/tpcf.h.  Every call looks up the device address of the
-// scratch array (cudaGetSymbolAddress) with the caller's device current: a
-// host call, so the address is never stale (a device reset reloads the
-// module).  The first call on a device may load the library's device code:
-// make it outside any stream capture.
+// Declared in include/tpcf.h.
 extern "C" int32_t tpcf_pair_count_noalloc(const float* x0, const float* y0, const float* z0, int64_t n0,
                                            const float* x1, const float* y1, const float* z1, int64_t n1,
                                            int32_t loop, float lo, float hi, int32_t nbins, uint64_t* hist_out,
@@ -2134,20 +2270,13 @@ extern "C" int32_t tpcf_pair_count_noalloc(const float* x0, const float* y0, con
     if ((n0 > 0 && (!x0 || !y0 || !z0)) || (n1 > 0 && (!x1 || !y1 || !z1))) return TPCF_ERR_INVALID;
     if (loop != TPCF_LOOP_ALL && loop != TPCF_LOOP_SAME && loop != TPCF_LOOP_ONE) return TPCF_ERR_INVALID;
     int copies = 8;
-    while (copies > 1 && pair_smem_bytes(nbins, copies) > 200 * 1024) copies /= 2;
+    while (copies > 1 && pair_smem_bytes(nbins, copies) > 40 * 1024) copies /= 2;
     if (pair_smem_bytes(nbins, copies) > 227 * 1024) return TPCF_ERR_INVALID;
     // an error left by the caller's earlier work is reported, not consumed
     if (cudaPeekAtLastError() != cudaSuccess) return TPCF_ERR_CUDA;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return TPCF_ERR_NO_DEVICE;
-    void* scratch = nullptr;
-    if (cudaGetSymbolAddress(&scratch, g_noalloc) != cudaSuccess || !scratch) {
-        (void)cudaGetLastError();
-        return TPCF_ERR_CUDA;
-    }
     cudaStream_t st = (cudaStream_t)stream;
-    NoAllocScratch* S = (NoAllocScratch*)scratch;
-    unsigned int* counter = &S->task_counter;
     // (an error of this call's own CUDA calls is consumed before returning, so
     // that it does not stay pending for the caller's next CUDA call)
     auto own_error = []() {
@@ -2155,8 +2284,6 @@ extern "C" int32_t tpcf_pair_count_noalloc(const float* x0, const float* y0, con
         return (int32_t)TPCF_ERR_CUDA;
     };
     if (cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * (size_t)nbins, st) != cudaSuccess) return own_error();
-    noalloc_prepare<<<256, 256, 0, st>>>(x0, y0, z0, (int)n0, x1, y1, z1, (int)n1, hist);
-    if (cudaGetLastError() != cudaSuccess) return TPCF_ERR_CUDA;  // (consumed by the check itself)
     const bool same = loop == TPCF_LOOP_SAME && x0 == x1 && y0 == y1 && z0 == z1 && n0 == n1;
     const int pred_same = loop == TPCF_LOOP_SAME && !same;
     const int ntA = (int)((n0 + TILE - 1) / TILE), ntB = (int)((n1 + TILE - 1) / TILE);
@@ -2167,26 +2294,32 @@ extern "C" int32_t tpcf_pair_count_noalloc(const float* x0, const float* y0, con
         p.hi = hi;
         volatile float span = hi - lo;
         p.bw = span / (float)nbins;
-        size_t smem = pair_smem_bytes(nbins, copies);
-        // the kernel's dynamic shared memory limit: always the device's opt-in
-        // maximum, never lowered (a lower per-call value would invalidate
-        // launches recorded earlier with a larger size)
-        // (dynamic plus the kernel's static shared memory within the opt-in limit)
-        int optin = 0, sms = 0;
-        cudaFuncAttributes fa;
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaFuncGetAttributes(&fa, pair_kernel_noalloc<false>) != cudaSuccess)
-            return own_error();
-        const int smem_max = optin - (int)fa.sharedSizeBytes;
-        if ((size_t)smem_max < smem) return TPCF_ERR_INVALID;
-        if (cudaFuncSetAttribute(pair_kernel_noalloc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) !=
-            cudaSuccess)
-            return own_error();
-        long long tasks = (long long)ntA * ntB;
-        int grid = (int)std::min<long long>(tasks, (long long)sms * 4);
-        pair_kernel_noalloc<false><<<grid, PR_THREADS, smem, st>>>(counter, ntA, ntB, same ? 1 : 0, pred_same, p, copies);
-        if (cudaGetLastError() != cudaSuccess) return TPCF_ERR_CUDA;
+        pair_guard(p);
+        const size_t smem = pair_smem_bytes(nbins, copies);
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return own_error();
+        if (smem > 48 * 1024) {
+            // the kernel's dynamic shared memory limit: always the device's opt-in
+            // maximum, never lowered (a lower per-call value would invalidate
+            // launches recorded earlier with a larger size); dynamic plus the
+            // kernel's static shared memory within the opt-in limit
+            int optin = 0;
+            cudaFuncAttributes fa;
+            if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+                cudaFuncGetAttributes(&fa, pair_kernel_noalloc) != cudaSuccess)
+                return own_error();
+            const int smem_max = optin - (int)fa.sharedSizeBytes;
+            if ((size_t)smem_max < smem) return TPCF_ERR_INVALID;
+            if (cudaFuncSetAttribute(pair_kernel_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) !=
+                cudaSuccess)
+                return own_error();
+        }
+        const int slots = sms * PAIR_CTAS, chunk = pair_chunk((long long)ntA * ntB, slots);
+        const int nbc = (ntB + chunk - 1) / chunk;
+        const int grid = (int)std::min<long long>((long long)ntA * nbc, slots);
+        pair_kernel_noalloc<<<grid, PR_THREADS, smem, st>>>(x0, y0, z0, (int)n0, x1, y1, z1, (int)n1, same ? 1 : 0,
+                                                            pred_same, chunk, p, copies, hist);
+        if (cudaGetLastError() != cudaSuccess) return TPCF_ERR_CUDA;  // (consumed by the check itself)
     }
     return TPCF_OK;
 }

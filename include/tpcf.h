@@ -254,18 +254,15 @@ tpcf_status tpcf_convert_radecz(tpcf_ctx* ctx, const double* ra, const double* d
  * host application's device footprint.  It counts the same pair histogram as
  * tpcf_count with TPCF_PAIR (same loop nests, bit-identical counts) from device
  * arrays x0/y0/z0 (n0 points) and x1/y1/z1 (n1 points), writing nbins counts to
- * the device array hist, and calls no cudaMalloc or cudaFree: its working
- * buffers are one 8 MiB array per device, reserved when the library is loaded
- * and held until the process exits.
+ * the device array hist, and calls no cudaMalloc or cudaFree: it reads the
+ * coordinates where they are and needs no buffer of its own.
  *   - at most 262144 points per catalog (TPCF_ERR_INVALID beyond);
  *   - loop TPCF_LOOP_SAME with identical pointers and sizes counts j >= i of
  *     one catalog; with different arrays it compares loop indices;
- *   - each call looks up that array's device address with the caller's device
- *     current (a host call; valid after a device reset too); the first call on
- *     a device may load the library's device code, so make it before any
- *     stream capture;
- *   - calls share the array: calls that overlap on the GPU (other streams or
- *     host threads) race; the call clears the counter and hist it needs;
+ *   - the first call on a device may load the library's device code, so make
+ *     it before any stream capture;
+ *   - calls share nothing: they may overlap on the GPU (other streams or host
+ *     threads) with histograms of their own; the call clears hist;
  *   - returns TPCF_ERR_CUDA without launching when a CUDA error is already
  *     pending on the calling thread (left pending for its owner);
  *   - a NaN separation is not counted (as the x86-64 build of the reference,
