@@ -291,28 +291,6 @@ void kd_order(const float* xyz, std::vector<int32_t>& order, int64_t n, int tile
     }
 }
 
-// Lower bound on the reference's float side length between any point of box
-// a and any point of box b (computed in double, then reduced by a relative
-// margin that covers the float rounding of the reference's distance).
-double box_lower_bound(const Box& a, const Box& b) {
-    double s = 0;
-    for (int k = 0; k < 3; k++) {
-        double g = std::max({0.0, (double)a.lo[k] - (double)b.hi[k], (double)b.lo[k] - (double)a.hi[k]});
-        s += g * g;
-    }
-    return sqrt(s) * (1.0 - 1e-5);
-}
-
-// Upper bound on the reference's float side length between box a and box b.
-double box_upper_bound(const Box& a, const Box& b) {
-    double s = 0;
-    for (int k = 0; k < 3; k++) {
-        double g = std::max((double)a.hi[k] - (double)b.lo[k], (double)b.hi[k] - (double)a.lo[k]);
-        s += g * g;
-    }
-    return sqrt(s) * (1.0 + 1e-5) + 1e-30;
-}
-
 // ---------------------------------------------------------------------------
 // exact glibc acosf exception table
 
@@ -674,55 +652,27 @@ bool same_binning(const tpcf_spec& a, const tpcf_spec& b) {
 // loop units (the reference's numcalc / fake_tot)
 
 uint64_t loop_units(int kind, int loop, const int64_t n[3]) {
+    typedef unsigned __int128 u128;  // sums of the loops' bounds in closed form, modulo 2^64
     if (kind == TPCF_THREE_SIDE) return (uint64_t)n[0] * n[1] * n[2];
     if (kind == TPCF_PAIR) {
-        if (loop == TPCF_LOOP_SAME) {
-            uint64_t u = 0;
-            for (int64_t i = 0; i < n[0]; i++) u += i < n[1] ? (uint64_t)(n[1] - i) : 0;
-            return u;
-        }
-        return (uint64_t)n[0] * n[1];
+        if (loop != TPCF_LOOP_SAME) return (uint64_t)n[0] * n[1];
+        const u128 m = std::min(n[0], n[1]);  // sum over i < m of n1 - i
+        return m ? (uint64_t)(m * (u128)n[1] - m * (m - 1) / 2) : 0;
     }
     if (loop == TPCF_LOOP_ALL) return (uint64_t)n[0] * n[1] * n[2];
-    uint64_t u = 0;
-    for (int64_t j = 0; j < n[1]; j++) {
-        uint64_t ks = j < n[2] ? (uint64_t)(n[2] - j) : 0;
-        uint64_t is = loop == TPCF_LOOP_SAME ? (uint64_t)std::min<int64_t>(n[0], j + 1) : (uint64_t)n[0];
-        u += is * ks;
-    }
-    return u;
+    const u128 n0 = n[0], n2 = n[2], m = std::min(n[1], n[2]);
+    if (m == 0 || n0 == 0) return 0;
+    const u128 tail = m * n2 - m * (m - 1) / 2;  // sum over j < m of n2 - j
+    if (loop == TPCF_LOOP_ONE) return (uint64_t)(n0 * tail);
+    // LOOP_SAME: min(n0, j + 1) points i for each j
+    const u128 p = std::min(m, n0);
+    const u128 sq = (p - 1) * p * (2 * p - 1) / 6, lin = p * (p - 1) / 2;  // sums of j^2 and j over j < p
+    const u128 head = p * n2 + n2 * lin - lin - sq;                        // (j + 1) (n2 - j)
+    return (uint64_t)(head + n0 * (tail - (p * n2 - lin)));
 }
 
 // ---------------------------------------------------------------------------
 // context
-
-// tile triples (pairs) with their unit estimates, in enumeration order
-typedef std::vector<std::pair<uint64_t, uint4>> TaskList;
-
-// one window's task groups of the fast triangle kernel: sizes, boxes (lo, hi)
-// of their A tiles and summed unit estimates; keys: radix-sort scratch
-struct GroupedPart {
-    std::vector<uint32_t> sizes;
-    std::vector<float> boxes;
-    std::vector<uint64_t> units;
-    std::vector<uint64_t> keys[2];
-};
-
-// host buffers of the planner, kept from batch to batch so that they are not
-// allocated (and paged in) again for every batch
-struct PlanScratch {
-    std::vector<TaskList> part;
-    std::vector<GroupedPart> gpart;
-    std::vector<uint4> tasks;
-    std::vector<uint32_t> groups;
-    std::vector<float> gbox;
-    std::vector<uint4> tasks2;  // the second part of a pipelined plan
-    std::vector<uint32_t> groups2;
-    std::vector<float> gbox2;
-    std::vector<uint4> tasks3;  // both parts in one (the merged plan)
-    std::vector<uint32_t> groups3;
-    std::vector<float> gbox3;
-};
 
 // One lane = one stream with its own scratch buffers.  The synchronous API uses
 // lane 0; every serving worker owns one further lane, so batches of different
@@ -732,34 +682,21 @@ struct Lane {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_mid = nullptr;
     uint64_t h2d = 0, d2h = 0;  // bytes copied since the last stats read
     DevBuf<DevJob> d_jobs;
-    DevBuf<uint4> d_tasks;
-    DevBuf<uint32_t> d_groups;  // fast triangle kernel: first task of each group (+ end)
-    DevBuf<float> d_gbox;       // ... and the box of each group's A tiles
-    // second part of a pipelined plan (the jobs after the first, planned while
-    // the first job counts): its tasks, groups and boxes
-    DevBuf<uint4> d_tasks2;
-    DevBuf<uint32_t> d_groups2;
-    DevBuf<float> d_gbox2;
-    // the whole plan in one part, uploaded while the parts count, for the
-    // repeats of the batch
-    DevBuf<uint4> d_tasks3;
-    DevBuf<uint32_t> d_groups3;
-    DevBuf<float> d_gbox3;
-    cudaStream_t side = nullptr;   // the second part: its upload and its launch
-    cudaStream_t side2 = nullptr;  // the upload of the merged plan
-    cudaEvent_t ev_side = nullptr;
-    DevBuf<unsigned int> d_counters;  // [0] task counter, [1] recheck count, [2..5] evaluated/binned
+    PinnedBuf<DevJob> h_jobs;         // device jobs of the batch being planned
+    PinnedBuf<uint32_t> h_rows;
+    DevBuf<uint32_t> d_rows;          // first row (pairs: item) of each job, and the end
+    DevBuf<uint2> d_row_cnt, d_block_sum;
+    DevBuf<uint4> d_units;            // the plan: units and their A tiles
+    DevBuf<uint32_t> d_masks;
+    DevBuf<unsigned int> d_counters;  // see CTR_*
     DevBuf<uint4> d_queue;
     DevBuf<unsigned long long> d_hist;
     PinnedBuf<unsigned long long> h_hist;
     PinnedBuf<unsigned int> h_counters;
     // last planned batch (see run_group)
     std::vector<uint64_t> plan_sig;
-    size_t plan_ntasks = 0;
-    size_t plan_ngroups = 0;  // task groups of the fast triangle kernel
-    size_t plan_ntasks2 = 0, plan_ngroups2 = 0;  // second part of a pipelined plan (0: none)
-    uint64_t plan_evaluated = 0;
-    int plan_chunk = 0;  // pairs: tiles B per item
+    uint32_t plan_rows = 0;  // rows (pairs: items) of the plan
+    int plan_chunk = 0;      // pairs: tiles B per item
     // the launch sequence of the last batch, captured as a CUDA graph and
     // replayed while the batch and every buffer it touches stay the same
     cudaGraphExec_t graph = nullptr;
@@ -770,7 +707,6 @@ struct Lane {
     int sm_cap = 0;
     // count in slices of the task list (heavy serving batches)
     bool slice_batches = false;
-    PlanScratch scratch;
     tpcf_stats stats{};
     void drop_graph() {
         if (graph) cudaGraphExecDestroy(graph);
@@ -782,24 +718,16 @@ struct Lane {
         h_hist.release();
         h_counters.release();
         d_jobs.release();
-        d_tasks.release();
-        d_groups.release();
-        d_gbox.release();
-        d_tasks2.release();
-        d_groups2.release();
-        d_gbox2.release();
-        d_tasks3.release();
-        d_groups3.release();
-        d_gbox3.release();
-        if (ev_side) cudaEventDestroy(ev_side);
-        if (side) cudaStreamDestroy(side);
-        if (side2) cudaStreamDestroy(side2);
-        ev_side = nullptr;
-        side = side2 = nullptr;
+        h_jobs.release();
+        h_rows.release();
+        d_rows.release();
+        d_row_cnt.release();
+        d_block_sum.release();
+        d_units.release();
+        d_masks.release();
         d_counters.release();
         d_queue.release();
         d_hist.release();
-        scratch = PlanScratch();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (ev_mid) cudaEventDestroy(ev_mid);
@@ -808,6 +736,14 @@ struct Lane {
         stream = nullptr;
     }
 };
+
+// d_counters: words zeroed before every count, then the header of the plan
+constexpr int CTR_WORK = 0;     // units (items) handed out
+constexpr int CTR_RECHECK = 1;  // queued guard-band triangles
+constexpr int CTR_EVAL = 2;     // evaluated (two words), binned (pairs: tile pairs; two words)
+constexpr int CTR_ZEROED = 8;
+constexpr int CTR_HEADER = 8;
+constexpr int CTR_WORDS = CTR_HEADER + (int)(sizeof(PlanHeader) / sizeof(unsigned int));
 
 struct Pending {
     uint64_t ticket;
@@ -885,7 +821,7 @@ struct tpcf_ctx {
     int reserve_sms = 0;       // SMs a heavy serving batch leaves free for light jobs
     bool slice_heavy = true;   // heavy serving batches count in slices (light lanes run between them)
     int slice_tasks = 0;       // tasks per slice (0: at least 8 per CTA and at most 64 slices)
-    int group_tasks = 0;       // fast triangle kernel: most tasks sharing one j-k table (0: by the batch)
+    int group_tasks = 0;       // A tiles per row of the planner, sharing one j-k table (0: by the batch)
     int64_t inflight_bytes = 0;  // device bytes of batches running on serving lanes
     // autotuner: launch shape per batch signature
     std::mutex tune_mu;
@@ -1083,238 +1019,6 @@ struct PlannedJob {
         if (swap == 1) return r == 0 ? v[2].get() : v[0].get();
         if (swap == 2) return r == 2 ? v[0].get() : v[1].get();
         return v[r].get();
-    }
-};
-
-uint64_t task_units3(const View& A, int a, const View& B, int b, const View& C, int c, uint32_t flags) {
-    uint64_t na = A.h_tile_start[a + 1] - A.h_tile_start[a];
-    uint64_t nb = B.h_tile_start[b + 1] - B.h_tile_start[b];
-    uint64_t nc = C.h_tile_start[c + 1] - C.h_tile_start[c];
-    bool dij = flags & TASK_DIAG_IJ, djk = flags & TASK_DIAG_JK;
-    if (dij && djk) return na * (na - 1) * (na - 2) / 6;
-    if (dij) return na * (na - 1) / 2 * nc;
-    if (djk) return na * (nb * (nb - 1) / 2);
-    return na * nb * nc;
-}
-
-// Tile tasks of one triangle/three-side job.
-// Lower/upper side bounds of every tile pair of two views, held densely when
-// small enough (else computed on demand).
-struct PairBounds {
-    const View* a = nullptr;
-    const View* b = nullptr;
-    bool dense = false;
-    std::vector<float> lb, ub;
-    // sizes the table; fill_rows(i0, i1) then fills rows independently (threads)
-    void alloc(const View& A, const View& B) {
-        a = &A;
-        b = &B;
-        dense = (int64_t)A.ntiles * B.ntiles <= ((int64_t)1 << 24);
-        if (!dense) return;
-        lb.resize((size_t)A.ntiles * B.ntiles);
-        ub.resize(lb.size());
-    }
-    void fill_rows(int i0, int i1) {
-        if (!dense) return;
-        for (int i = i0; i < i1; i++)
-            for (int j = 0; j < b->ntiles; j++) {
-                // float copies rounded outwards so they stay conservative
-                lb[(size_t)i * b->ntiles + j] = nextafterf((float)box_lower_bound(a->boxes[i], b->boxes[j]), 0.f);
-                ub[(size_t)i * b->ntiles + j] = nextafterf((float)box_upper_bound(a->boxes[i], b->boxes[j]), INFINITY);
-            }
-    }
-    double L(int i, int j) const {
-        return dense ? (double)lb[(size_t)i * b->ntiles + j] : box_lower_bound(a->boxes[i], b->boxes[j]);
-    }
-    double U(int i, int j) const {
-        return dense ? (double)ub[(size_t)i * b->ntiles + j] : box_upper_bound(a->boxes[i], b->boxes[j]);
-    }
-};
-
-// Whether a tile triple can hold a counted triangle-parametrization triangle:
-// with the three pair bounds sorted (L1<=L2<=L3 lower, U1<=U2<=U3 upper) the
-// shortest side lies in [L1,U1], the middle in [L2,U2], the longest in [L3,U3];
-// permutations 0/2 need s_lo <= shortest < s_hi and middle < q_hi*shortest,
-// permutation 1 needs s_lo <= middle < s_hi and longest < q_hi*middle.
-bool tri_triple_possible(const Binning& bin, double l0, double l1, double l2, double u0, double u1, double u2) {
-    double L[3] = {l0, l1, l2}, U[3] = {u0, u1, u2};
-    if (L[0] > L[1]) std::swap(L[0], L[1]);
-    if (L[1] > L[2]) std::swap(L[1], L[2]);
-    if (L[0] > L[1]) std::swap(L[0], L[1]);
-    if (U[0] > U[1]) std::swap(U[0], U[1]);
-    if (U[1] > U[2]) std::swap(U[1], U[2]);
-    if (U[0] > U[1]) std::swap(U[0], U[1]);
-    bool p0 = L[0] < bin.s_hi && U[0] >= bin.s_lo && L[1] < bin.q_hi * U[0];
-    bool p1 = L[1] < bin.s_hi && U[1] >= bin.s_lo && L[2] < bin.q_hi * U[1];
-    return p0 || p1;
-}
-
-
-// Lower/upper side bounds and neighbour lists (tile pairs whose lower bound is
-// below lmax) of one pair of views, shared by every job of a launch that
-// pairs those views; rows() fills a range of rows (parallel planning).
-struct PairTable {
-    const View* x = nullptr;
-    const View* y = nullptr;
-    bool prune = false, need_nb = false;
-    int listed = -1;  // the planning pass whose row list holds it
-    double lmax = INFINITY;
-    PairBounds pb;
-    std::vector<std::vector<int>> nb;
-    void init(const View& X, const View& Y, double lmax_) {
-        x = &X;
-        y = &Y;
-        lmax = lmax_;
-        prune = lmax < INFINITY;
-        if (prune) pb.alloc(X, Y);
-    }
-    void rows(int r0, int r1) {
-        if (prune) pb.fill_rows(r0, r1);
-        if (!need_nb) return;
-        for (int i = r0; i < r1; i++) {
-            nb[i].clear();
-            for (int j = 0; j < y->ntiles; j++)
-                if (!prune || pb.L(i, j) < lmax) nb[i].push_back(j);
-        }
-    }
-};
-
-// Tile tasks of one triangle/three-side job: enumerate() lists the tile
-// triples of a range of A tiles from the pair tables of (A,B), (A,C), (B,C).
-struct TripletPlan {
-    const tpcf_spec* sp = nullptr;
-    const PlannedJob* pj = nullptr;
-    const Binning* bin = nullptr;
-    uint32_t slot = 0;
-    bool empty = true, prune = false, tri = false, sameAB = false, sameBC = false;
-    bool sym_three = true;  // TPCF_SYM3=0: ordered three-side tasks
-    const PairTable *AB = nullptr, *AC = nullptr, *BC = nullptr;
-
-    void init(const tpcf_spec& s, const PlannedJob& p, uint32_t sl, const Binning& b, const PairTable* ab,
-              const PairTable* ac, const PairTable* bc) {
-        sp = &s;
-        pj = &p;
-        bin = &b;
-        slot = sl;
-        const View &A = *p.role(0), &B = *p.role(1), &C = *p.role(2);
-        empty = A.ntiles == 0 || B.ntiles == 0 || C.ntiles == 0;
-        prune = b.lmax < INFINITY;
-        tri = s.kind == TPCF_TRIANGLE || s.kind == TPCF_TRIANGLE_JBJ;
-        sameAB = p.role(0) == p.role(1);
-        sameBC = p.role(1) == p.role(2);
-        const char* e3 = getenv("TPCF_SYM3");
-        sym_three = !(e3 && e3[0] == '0');
-        AB = ab;
-        AC = ac;
-        BC = bc;
-    }
-    // Tile triples of A tiles [a0, a1); with one A tile, only its neighbour-list
-    // entries [blo, bhi) as tile B (a heavy tile's triples in several parts).
-    void enumerate(int a0, int a1, TaskList& tasks, uint64_t& evaluated, size_t blo = 0,
-                   size_t bhi = SIZE_MAX) const {
-        if (empty) return;  // a role without tiles: no triple (and no neighbour lists)
-        const View &A = *pj->role(0), &B = *pj->role(1), &C = *pj->role(2);
-        const double lmax = bin->lmax;
-        // bounds of the pair (a, b), looked up once for all its c
-        struct AB_ {
-            double l = 0, u = 0;
-        };
-        auto ab_bounds = [&](int a, int b) {
-            AB_ r;
-            if (prune) {
-                r.l = AB->pb.L(a, b);
-                r.u = AB->pb.U(a, b);
-            }
-            return r;
-        };
-        auto add = [&](int a, int b, int c, const AB_& ab, uint32_t pred, uint32_t flags) {
-            if (prune) {
-                const double lbc = BC->pb.L(b, c);
-                if (!(lbc < lmax)) return;
-                const double lac = AC->pb.L(a, c), uac = AC->pb.U(a, c);
-                if (bin->tri_prune && !tri_triple_possible(*bin, ab.l, lac, lbc, ab.u, uac, BC->pb.U(b, c))) return;
-                if (ab.u >= lmax) flags |= TASK_CHECK_B;
-                if (uac >= lmax) flags |= TASK_CHECK_C;
-            }
-            uint64_t u = task_units3(A, a, B, b, C, c, flags);
-            if (u == 0) return;
-            evaluated += u;
-            tasks.push_back({u, make_uint4(slot | (pred << TASK_PRED_SHIFT) | flags, (uint32_t)a, (uint32_t)b,
-                                           (uint32_t)c)});
-        };
-        // the entries >= from of an ascending neighbour list
-        auto from = [](const std::vector<int>& l, int v) { return std::lower_bound(l.begin(), l.end(), v); };
-        // tile B's entries of the list: positions [blo, bhi), at least v
-        struct Span {
-            std::vector<int>::const_iterator b, e;
-            std::vector<int>::const_iterator begin() const { return b; }
-            std::vector<int>::const_iterator end() const { return e; }
-        };
-        auto bspan = [&](const std::vector<int>& l, int v) {
-            auto lo = l.begin() + (ptrdiff_t)std::min(blo, l.size());
-            auto hi = l.begin() + (ptrdiff_t)std::min(bhi, l.size());
-            auto f = from(l, v);
-            if (f > lo) lo = f;
-            return Span{lo, std::max(lo, hi)};
-        };
-        const tpcf_spec& s = *sp;
-        // three-side histogram of one catalog in all roles: the kernel counts
-        // each multiset {i, j, k} once for all its orderings
-        const bool sym3 = s.kind == TPCF_THREE_SIDE && s.loop == TPCF_LOOP_ALL && sym_three && sameAB && sameBC;
-        if (pj->swap == 1) {
-            // roles (C, A, A) of a D-D-R job: each point of C with every
-            // unordered pair of the single array, weight [k_c >= j] + [k_c >= k]
-            for (int a = a0; a < a1; a++)
-                for (int b : bspan(AB->nb[a], INT_MIN)) {
-                    const AB_ ab = ab_bounds(a, b);
-                    for (auto c = from(AC->nb[a], b); c != AC->nb[a].end(); ++c)
-                        add(a, b, *c, ab, PRED_RDD, b == *c ? TASK_DIAG_JK : 0);
-                }
-        } else if (pj->swap == 2) {
-            // roles (B, B, A) of a D-R-R job: every unordered pair of the pair
-            // array with each point of the other
-            for (int a = a0; a < a1; a++)
-                for (int b : bspan(AB->nb[a], a)) {
-                    const AB_ ab = ab_bounds(a, b);
-                    for (int c : AC->nb[a]) add(a, b, c, ab, PRED_NONE, a == b ? TASK_DIAG_IJ : 0);
-                }
-        } else if ((tri && s.loop == TPCF_LOOP_SAME || sym3) && sameAB && sameBC) {
-            // i <= j <= k over one array: unordered distinct triples (triangle
-            // programs), or every multiset of three points counted for each of
-            // its orderings (three-side: PRED_SAME marks the task)
-            for (int a = a0; a < a1; a++)
-                for (int b : bspan(AB->nb[a], a)) {
-                    const AB_ ab = ab_bounds(a, b);
-                    for (auto c = from(AC->nb[a], b); c != AC->nb[a].end(); ++c) {
-                        uint32_t f = (a == b ? TASK_DIAG_IJ : 0) | (b == *c ? TASK_DIAG_JK : 0);
-                        add(a, b, *c, ab, sym3 ? PRED_SAME : PRED_NONE, f);
-                    }
-                }
-        } else if (tri && s.loop == TPCF_LOOP_ONE && sameBC) {
-            // j <= k over one array (j == k has a zero side): unordered pairs
-            for (int a = a0; a < a1; a++)
-                for (int b : bspan(AB->nb[a], INT_MIN)) {
-                    const AB_ ab = ab_bounds(a, b);
-                    for (auto c = from(AC->nb[a], b); c != AC->nb[a].end(); ++c)
-                        add(a, b, *c, ab, PRED_NONE, b == *c ? TASK_DIAG_JK : 0);
-                }
-        } else if (tri && s.loop == TPCF_LOOP_ONE && sameAB) {
-            // every ordered (i, j) of one array, k >= j: unordered {i, j} with
-            // weight [k >= i] + [k >= j]
-            for (int a = a0; a < a1; a++)
-                for (int b : bspan(AB->nb[a], a)) {
-                    const AB_ ab = ab_bounds(a, b);
-                    for (int c : AC->nb[a]) add(a, b, c, ab, PRED_DDR, a == b ? TASK_DIAG_IJ : 0);
-                }
-        } else {
-            uint32_t pred = PRED_NONE;
-            if (tri) pred = s.loop == TPCF_LOOP_SAME ? PRED_SAME : s.loop == TPCF_LOOP_ONE ? PRED_ONE : PRED_NONE;
-            for (int a = a0; a < a1; a++)
-                for (int b : bspan(AB->nb[a], INT_MIN)) {
-                    const AB_ ab = ab_bounds(a, b);
-                    for (int c : AC->nb[a]) add(a, b, c, ab, pred, 0);
-                }
-        }
     }
 };
 
@@ -1523,125 +1227,6 @@ int grid_for(tpcf_ctx* ctx, const Shape& sh, uint64_t ntasks, int sm_cap) {
     return (int)g;
 }
 
-// Task groups of the fast triangle kernel: tasks of one job with the same
-// tiles B and C run one after another in one CTA, which builds their j-k
-// table once.  Each window of planning parts (one job, a run of consecutive A
-// tiles) groups its own tasks, in parallel with the others: a sort on (b, c)
-// that keeps the order of A tiles, runs of equal (b, c) cut into groups of at
-// most max_group tasks (a group is the unit a CTA takes, so large ones would
-// leave a long tail at the end of the launch).  boxes: lo/hi of the union of each
-// group's A tiles, for the j-k rows that no point of the group can reach;
-// units: the group's summed task estimates.
-
-void group_parts(const TaskList* parts, size_t nparts, const PlannedJob& J, size_t max_group, uint4* dst,
-                 GroupedPart& out) {
-    const uint64_t nc = (uint64_t)J.role(2)->ntiles;
-    size_t n = 0;
-    for (size_t i = 0; i < nparts; i++) n += parts[i].size();
-    // (b, c) key above the task's index in the window, sorted by an LSD
-    // radix sort on the key (stable: ties stay in the order of A tiles)
-    std::vector<uint64_t>&ka = out.keys[0], &kb = out.keys[1];
-    ka.resize(n);
-    kb.resize(n);
-    uint64_t kmax = 0;
-    for (size_t i = 0, t = 0; i < nparts; i++)
-        for (const auto& pr : parts[i]) {
-            const uint64_t k = (uint64_t)pr.second.z * nc + pr.second.w;
-            kmax = std::max(kmax, k);
-            ka[t] = k << 32 | t;
-            t++;
-        }
-    for (int shift = 32; shift < 64 && (kmax >> (shift - 32)) != 0; shift += 8) {
-        uint32_t cnt[257] = {0};
-        for (size_t t = 0; t < n; t++) cnt[((ka[t] >> shift) & 255) + 1]++;
-        for (int d = 0; d < 256; d++) cnt[d + 1] += cnt[d];
-        for (size_t t = 0; t < n; t++) kb[cnt[(ka[t] >> shift) & 255]++] = ka[t];
-        ka.swap(kb);
-    }
-    // the window's tasks by index
-    std::vector<const std::pair<uint64_t, uint4>*> src(n);
-    for (size_t i = 0, t = 0; i < nparts; i++)
-        for (const auto& pr : parts[i]) src[t++] = &pr;
-    const View& A = *J.role(0);
-    out.sizes.resize(n);
-    out.boxes.resize(6 * n);
-    out.units.resize(n);
-    size_t ng = 0;
-    for (size_t t = 0; t < n;) {
-        const uint64_t k = ka[t] >> 32;
-        size_t e = t + 1;
-        while (e < n && e - t < max_group && (ka[e] >> 32) == k) e++;
-        float* bx = &out.boxes[6 * ng];
-        bx[0] = bx[1] = bx[2] = INFINITY;
-        bx[3] = bx[4] = bx[5] = -INFINITY;
-        uint64_t u = 0;
-        for (size_t q = t; q < e; q++) {
-            const auto& pr = *src[(uint32_t)ka[q]];
-            dst[q] = pr.second;
-            u += pr.first;
-            const Box& b = A.boxes[pr.second.y];
-            for (int d = 0; d < 3; d++) {
-                bx[d] = std::min(bx[d], b.lo[d]);
-                bx[3 + d] = std::max(bx[3 + d], b.hi[d]);
-            }
-        }
-        out.sizes[ng] = (uint32_t)(e - t);
-        out.units[ng++] = u;
-        t = e;
-    }
-    out.sizes.resize(ng);
-    out.boxes.resize(6 * ng);
-    out.units.resize(ng);
-}
-
-// Group starts (ngroups + 1 entries) and boxes of the grouped windows, whose
-// tasks are in place in `tasks` (window w from toff[w]).  With few tasks per
-// CTA the groups go largest first (summed estimates), so that the dynamic
-// fetch balances the tail; else in window order (job order).
-void assemble_groups(const std::vector<GroupedPart>& gp, size_t nw, const std::vector<size_t>& toff,
-                     bool largest_first, std::vector<uint4>& tasks, std::vector<uint32_t>& starts,
-                     std::vector<float>& boxes) {
-    std::vector<size_t> goff(nw + 1, 0);
-    for (size_t i = 0; i < nw; i++) goff[i + 1] = goff[i] + gp[i].sizes.size();
-    const size_t total = toff[nw], ng = goff[nw];
-    starts.resize(ng + 1);
-    boxes.resize(6 * ng);
-    starts[ng] = (uint32_t)total;
-    if (largest_first) {
-        std::vector<std::array<uint32_t, 2>> ref;  // window, group in window
-        std::vector<uint32_t> first;                // its first task
-        std::vector<uint64_t> units;
-        for (size_t i = 0; i < nw; i++)
-            for (uint32_t g = 0, t = (uint32_t)toff[i]; g < gp[i].sizes.size(); t += gp[i].sizes[g], g++) {
-                ref.push_back({(uint32_t)i, g});
-                first.push_back(t);
-                units.push_back(gp[i].units[g]);
-            }
-        std::vector<uint32_t> order(ng);
-        for (size_t g = 0; g < ng; g++) order[g] = (uint32_t)g;
-        std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return units[a] > units[b]; });
-        const std::vector<uint4> in(tasks.begin(), tasks.begin() + total);
-        size_t w = 0;
-        for (size_t o = 0; o < ng; o++) {
-            const auto& r = ref[order[o]];
-            const GroupedPart& P = gp[r[0]];
-            starts[o] = (uint32_t)w;
-            for (uint32_t t = 0; t < P.sizes[r[1]]; t++) tasks[w++] = in[first[order[o]] + t];
-            std::copy(&P.boxes[6 * r[1]], &P.boxes[6 * r[1]] + 6, &boxes[6 * o]);
-        }
-        return;
-    }
-    parallel_items(nw, [&](size_t i) {
-        const GroupedPart& P = gp[i];
-        std::copy(P.boxes.begin(), P.boxes.end(), boxes.begin() + 6 * goff[i]);
-        uint32_t s = (uint32_t)toff[i];
-        for (size_t g = 0; g < P.sizes.size(); g++) {
-            starts[goff[i] + g] = s;
-            s += P.sizes[g];
-        }
-    });
-}
-
 // Runs one group of jobs that share kind, binning and precision in a single
 // persistent launch.  outs[i] receives hist_len counts.
 void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
@@ -1649,24 +1234,29 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     const tpcf_spec& sp = *group[0].spec;
     Binning bin = make_binning(sp);
     const int ncat = sp.kind == TPCF_PAIR ? 2 : 3;
+    const bool pairs = sp.kind == TPCF_PAIR;
+    const bool fp64 = !guarded_fp32(sp, bin);
+    const bool tri_kind = sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ;
+    const bool fast_tri = tri_kind && !fp64;
+    const bool fast_jbj = sp.kind == TPCF_TRIANGLE_JBJ && !fp64;  // the fast kernel's JBJ binning
     if (group.size() > MAX_BATCH_JOBS) throw InvalidArg{"too many jobs in one batch"};
-    std::vector<PlannedJob> pj(group.size());
-    std::vector<DevJob> dj(group.size());
-    uint64_t evaluated = 0, units = 0;
+    std::vector<std::pair<const char*, double>> phases;
+    auto phase = [&](const char* name) {
+        if (plan_trace())
+            phases.push_back({name, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
+                                                                              t_wall0).count()});
+    };
     // device histogram slots: one per job, or one per distinct output for
     // accumulating jobs
     std::vector<size_t> slot_of(group.size());
     std::vector<size_t> slot_job;  // first job of each slot
     {
-        std::map<uint64_t*, size_t> by_out;
+        std::unordered_map<uint64_t*, size_t> by_out;
         for (size_t g = 0; g < group.size(); g++) {
             if (group[g].accumulate) {
-                auto it = by_out.find(group[g].out);
-                if (it != by_out.end()) {
-                    slot_of[g] = it->second;
-                    continue;
-                }
-                by_out[group[g].out] = slot_job.size();
+                auto ins = by_out.emplace(group[g].out, slot_job.size());
+                slot_of[g] = ins.first->second;
+                if (!ins.second) continue;
             }
             slot_of[g] = slot_job.size();
             slot_job.push_back(g);
@@ -1675,16 +1265,13 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     const size_t nslots = slot_job.size();
     size_t hist_total = (size_t)bin.len * nslots;
     L.d_hist.reserve(hist_total);
-    // signature of the batch: a repeated batch over the same resident views
-    // reuses its task list and device upload
-    std::vector<uint64_t> sig;
-    sig.push_back((uint64_t)(uintptr_t)L.d_hist.p);
     const char* rdd_env = getenv("TPCF_RDD");
-    const bool rdd = !(rdd_env && rdd_env[0] == '0');
-    // The batch signature takes the jobs' view ids; views still being built
-    // (new catalogs) are waited for only when a job's planning needs them.
-    // (A batch of many jobs names few distinct catalog ranges: each is looked
-    // up once.)
+    const bool rdd = fast_tri && !(rdd_env && rdd_env[0] == '0');
+    const char* sym_env = getenv("TPCF_SYM3");
+    const bool sym_three = !(sym_env && sym_env[0] == '0');
+    // The distinct catalog ranges of the batch (a batch of many jobs names
+    // few): each is looked up once, and its view -- which may still be being
+    // built (new catalogs) -- is waited for only when the batch is planned.
     struct RangeKey {
         uint64_t h;
         int64_t b, e;
@@ -1698,400 +1285,253 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             return (size_t)(x ^ (x >> 29));
         }
     };
-    std::unordered_map<RangeKey, ViewRef, RangeHash> refs;
-    sig.reserve(1 + group.size() * 22);
+    struct Range {
+        RangeKey key;
+        ViewRef ref;
+        std::shared_ptr<View> view;
+    };
+    std::vector<Range> ranges;
+    std::unordered_map<RangeKey, uint32_t, RangeHash> range_at;
+    auto range_of = [&](const RangeKey& k) -> uint32_t {
+        auto ins = range_at.emplace(k, (uint32_t)ranges.size());
+        if (ins.second) {
+            Range r{k, {}, nullptr};
+            get_view(ctx, L, k.h, k.b, k.e, k.gl, &r.ref);
+            ranges.push_back(std::move(r));
+        }
+        return ins.first->second;
+    };
+    // Signature of the batch (its binning, and each job's views, slot and loop
+    // nest): a repeated batch over the same resident views reuses its plan.
+    std::vector<uint64_t> sig;
+    sig.reserve(16 + group.size() * 4);
+    sig.push_back((uint64_t)(uintptr_t)L.d_hist.p);
+    {
+        const uint64_t f[6] = {(uint64_t)sp.kind, (uint64_t)sp.prune, (uint64_t)sp.precision, (uint64_t)sp.nan_policy,
+                               (uint64_t)sp.overflow, (uint64_t)rdd << 1 | (uint64_t)sym_three};
+        sig.insert(sig.end(), f, f + 6);
+        for (int a = 0; a < 3; a++) {
+            sig.push_back((uint64_t)fbits(sp.axis[a].lo) << 32 | fbits(sp.axis[a].hi));
+            sig.push_back((uint64_t)(uint32_t)sp.axis[a].nbins);
+        }
+        sig.push_back((uint64_t)bin.len);
+        sig.push_back((uint64_t)group.size());
+    }
+    // each job: its ranges in the kernel's role order, and how its tiles and
+    // points are enumerated (JOB_*)
+    struct RoleJob {
+        uint32_t range[3];
+        uint32_t mode;
+    };
+    std::vector<RoleJob> roles(group.size());
+    uint64_t units = 0;
+    // reference loop size of job g
+    auto job_units = [&](size_t g) {
+        const tpcf_job& job = *group[g].job;
+        int64_t n[3] = {0, 0, 0};
+        for (int r = 0; r < ncat; r++)
+            n[r] = ranges[range_of({job.catalog[r], job.begin[r], job.end[r],
+                                    (job.flags & TPCF_JOB_GLOBAL_INDEX) != 0})].ref.n;
+        return loop_units(group[g].spec->kind, group[g].spec->loop, n);
+    };
+    // a role's range is often the previous job's
+    RangeKey last_key[3] = {};
+    uint32_t last_at[3] = {};
+    bool last_ok[3] = {};
     for (size_t g = 0; g < group.size(); g++) {
         const tpcf_job& job = *group[g].job;
         const tpcf_spec& jsp = *group[g].spec;  // same binning as sp; the loop nest may differ
         int64_t n[3] = {0, 0, 0};
-        uint64_t vid[3] = {0, 0, 0};
+        uint32_t rg[3] = {0, 0, 0};
         for (int r = 0; r < ncat; r++) {
             const RangeKey k{job.catalog[r], job.begin[r], job.end[r], (job.flags & TPCF_JOB_GLOBAL_INDEX) != 0};
-            auto it = refs.find(k);
-            if (it == refs.end()) {
-                ViewRef ref{};
-                get_view(ctx, L, k.h, k.b, k.e, k.gl, &ref);
-                it = refs.emplace(k, ref).first;
+            if (!last_ok[r] || !(last_key[r] == k)) {
+                last_at[r] = range_of(k);
+                last_key[r] = k;
+                last_ok[r] = true;
             }
-            vid[r] = it->second.id;
-            n[r] = it->second.n;
+            rg[r] = last_at[r];
+            n[r] = ranges[rg[r]].ref.n;
         }
-        if (ncat == 2) vid[2] = vid[1];
-        pj[g].loop_units = loop_units(jsp.kind, jsp.loop, n);
-        units += pj[g].loop_units;
-        pj[g].swap = 0;
-        if (rdd && (jsp.kind == TPCF_TRIANGLE || jsp.kind == TPCF_TRIANGLE_JBJ) &&
-            guarded_fp32(jsp, bin) && jsp.loop == TPCF_LOOP_ONE) {
-            if (vid[0] == vid[1] && vid[1] != vid[2]) pj[g].swap = 1;
-            else if (vid[1] == vid[2] && vid[0] != vid[1]) pj[g].swap = 2;
-        }
-        for (int r = 0; r < 3; r++) {  // role r's view (PlannedJob::role)
-            const int v = pj[g].swap == 1 ? (r == 0 ? 2 : 0) : pj[g].swap == 2 ? (r == 2 ? 0 : 1) : r;
-            sig.push_back(vid[v]);
-        }
-        sig.push_back(pj[g].swap);
-        sig.push_back(slot_of[g]);
-        uint64_t f[6] = {(uint64_t)jsp.kind, (uint64_t)jsp.loop, (uint64_t)jsp.prune, (uint64_t)jsp.precision,
-                         (uint64_t)jsp.nan_policy, (uint64_t)jsp.overflow};
-        sig.insert(sig.end(), f, f + 6);
-        for (int a = 0; a < 3; a++) {
-            sig.push_back((uint64_t)fbits(jsp.axis[a].lo) << 32 | fbits(jsp.axis[a].hi));
-            sig.push_back((uint64_t)(uint32_t)jsp.axis[a].nbins);
-        }
-    }
-    // the views of job g (waiting for any still being built) and its device job
-    auto attach = [&](size_t g) {
-        const tpcf_job& job = *group[g].job;
-        for (int r = 0; r < ncat; r++)
-            pj[g].v[r] = get_view(ctx, L, job.catalog[r], job.begin[r], job.end[r],
-                                  (job.flags & TPCF_JOB_GLOBAL_INDEX) != 0);
-        if (ncat == 2) pj[g].v[2] = pj[g].v[1];
-        for (int r = 0; r < 3; r++) {
-            const View* rv = pj[g].role(r);
-            dj[g].pts[r] = rv->pts.p;
-            dj[g].tile_start[r] = rv->tile_start.p;
-            dj[g].box[r] = rv->box.p;
-            dj[g].ntiles[r] = rv->ntiles;
-        }
-        if (ncat == 2 && group[g].spec->loop == TPCF_LOOP_SAME)
-            dj[g].mode = pj[g].v[0] == pj[g].v[1] ? JOB_B_FROM_A : (uint32_t)PRED_SAME;
-        dj[g].hist = L.d_hist.p + (size_t)bin.len * slot_of[g];
-    };
-    cudaStream_t st = L.stream;
-    L.d_counters.reserve(8);
-    size_t ntasks = 0, ngroups = 0;
-    const bool plan_hit = sig == L.plan_sig;
-    std::vector<std::pair<const char*, double>> phases;
-    auto phase = [&](const char* name) {
-        if (plan_trace())
-            phases.push_back({name, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
-                                                                              t_wall0).count()});
-    };
-    const bool pairs = sp.kind == TPCF_PAIR;
-    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item
-    const bool fast_tri = (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) && guarded_fp32(sp, bin);
-    // A newly planned batch of two to eight fast-kernel jobs (an estimator's
-    // DDD/DDR/DRR/RRR set) is pipelined: the first job is planned, uploaded and
-    // launched, and the others are planned while it counts (a second launch
-    // follows on the same stream).  Larger batches -- voxel and jackknife sets
-    // of many similar jobs, whose first job is a small share -- keep one launch.
-    const char* pl_env = getenv("TPCF_PIPELINE");
-    const bool pipeline = !plan_hit && fast_tri && group.size() >= 2 && group.size() <= 8 && !L.slice_batches &&
-                          !(pl_env && pl_env[0] == '0');
-    // a pipelined batch waits here for the first job's views only (a planned
-    // batch needs none: its device jobs are in place)
-    if (!plan_hit)
-        for (size_t g = 0; g < (pipeline ? 1 : group.size()); g++) attach(g);
-    phase("views");
-    size_t ntasks2 = 0, ngroups2 = 0;
-    uint64_t evaluated2 = 0;
-    // planning state shared by the parts of a plan: bound tables by view pair
-    std::vector<TripletPlan> tp(pairs ? 0 : group.size());
-    struct ViewPairHash {
-        size_t operator()(const std::pair<const View*, const View*>& k) const {
-            const uint64_t x = (uint64_t)(uintptr_t)k.first * 0x9E3779B97F4A7C15ull ^ (uint64_t)(uintptr_t)k.second;
-            return (size_t)(x ^ (x >> 31));
-        }
-    };
-    std::unordered_map<std::pair<const View*, const View*>, std::unique_ptr<PairTable>, ViewPairHash> tables;
-    std::vector<PairTable*> table_list;
-    int plan_pass = 0;
-    // Plans jobs [g0, g1) into task list, group starts and group boxes (the
-    // last two for the fast triangle kernel); returns the evaluated units.
-    auto plan_jobs = [&](size_t g0, size_t g1, std::vector<uint4>& h_tasks, std::vector<uint32_t>& h_groups,
-                         std::vector<float>& h_gbox) -> uint64_t {
+        if (ncat == 2) rg[2] = rg[1];
+        units += loop_units(jsp.kind, jsp.loop, n);
+        // (two ranges with one view, e.g. [0, n) and [0, -1), are the same array)
+        auto id = [&](int r) { return ranges[rg[r]].ref.id; };
+        const bool ab = id(0) == id(1), bc = id(1) == id(2);
+        uint32_t mode = PRED_NONE, v[3] = {rg[0], rg[1], rg[2]};
         if (pairs) {
-            // the pair kernel finds its tile pairs itself: the plan is the
-            // number of (tile A, chunk of tiles B) items of each job
-            long long tile_pairs = 0;
-            for (size_t g = g0; g < g1; g++) tile_pairs += (long long)pj[g].v[0]->ntiles * pj[g].v[1]->ntiles;
-            plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS);
-            h_groups.assign(1, 0);
-            uint64_t items = 0;
-            for (size_t g = g0; g < g1; g++) {
-                const uint64_t nbc = (pj[g].v[1]->ntiles + plan_chunk - 1) / plan_chunk;
-                items += (uint64_t)pj[g].v[0]->ntiles * nbc;
-                if (items > 0xF0000000ull) throw InvalidArg{"too many tile pairs in one batch"};
-                h_groups.push_back((uint32_t)items);
-            }
-            return 0;
+            if (jsp.loop == TPCF_LOOP_SAME) mode = ab ? JOB_B_FROM_A : (uint32_t)PRED_SAME;
+        } else if (tri_kind && jsp.loop == TPCF_LOOP_ONE && ab && !bc && rdd) {
+            // Loop ONE jobs of two arrays are counted with the point of the
+            // array that appears once in role B or C and the pair array
+            // first, so that points out of reach of a tile are skipped whole:
+            // D-D-R (A == B) in the roles (C, A, A), each point of C with
+            // every unordered pair of the single array ...
+            v[0] = rg[2], v[1] = v[2] = rg[0];
+            mode = PRED_RDD | JOB_C_FROM_B;
+        } else if (tri_kind && jsp.loop == TPCF_LOOP_ONE && bc && !ab && rdd) {
+            // ... and D-R-R (B == C) in the roles (B, B, A), every unordered
+            // pair of the pair array with each point of the other
+            v[0] = v[1] = rg[1], v[2] = rg[0];
+            mode = PRED_NONE | JOB_B_FROM_A;
+        } else if (ab && bc && tri_kind && jsp.loop == TPCF_LOOP_SAME) {
+            // i <= j <= k over one array: unordered distinct triples
+            mode = PRED_NONE | JOB_B_FROM_A | JOB_C_FROM_B;
+        } else if (ab && bc && sp.kind == TPCF_THREE_SIDE && jsp.loop == TPCF_LOOP_ALL && sym_three) {
+            // three-side histogram of one catalog in all roles: the kernel
+            // counts each multiset {i, j, k} once for all its orderings
+            mode = PRED_SAME | JOB_B_FROM_A | JOB_C_FROM_B;
+        } else if (tri_kind && jsp.loop == TPCF_LOOP_ONE && bc) {
+            // j <= k over one array (j == k has a zero side): unordered pairs
+            mode = PRED_NONE | JOB_C_FROM_B;
+        } else if (tri_kind && jsp.loop == TPCF_LOOP_ONE && ab) {
+            // every ordered (i, j) of one array, k >= j: unordered {i, j} with
+            // weight [k >= i] + [k >= j]
+            mode = PRED_DDR | JOB_B_FROM_A;
+        } else if (tri_kind) {
+            mode = jsp.loop == TPCF_LOOP_SAME ? PRED_SAME : jsp.loop == TPCF_LOOP_ONE ? PRED_ONE : PRED_NONE;
         }
-        // plan in parallel: bound tables and neighbour lists by rows, then
-        // tile triples by ranges of A tiles
-        uint64_t ev = 0;
-        {
-            const size_t t_first = table_list.size();
-            const int pass = plan_pass++;
-            auto table = [&](const View* x, const View* y, bool nb) {
-                auto& t = tables[std::make_pair(x, y)];
-                if (!t) {
-                    t.reset(new PairTable());
-                    t->init(*x, *y, bin.lmax);
-                    t->listed = pass;
-                    table_list.push_back(t.get());
-                }
-                if (nb && !t->need_nb) {
-                    if (t->listed != pass) {  // filled by an earlier pass without neighbour lists: fill again
-                        t->listed = pass;
-                        table_list.push_back(t.get());
-                    }
-                    t->need_nb = true;
-                    t->nb.assign(x->ntiles, {});
-                }
-                return t.get();
-            };
-            for (size_t g = g0; g < g1; g++) {
-                const View *A = pj[g].role(0), *B = pj[g].role(1), *C = pj[g].role(2);
-                const bool empty = A->ntiles == 0 || B->ntiles == 0 || C->ntiles == 0;
-                tp[g].init(*group[g].spec, pj[g], (uint32_t)g, bin, empty ? nullptr : table(A, B, true),
-                           empty ? nullptr : table(A, C, true), empty ? nullptr : table(B, C, false));
-            }
-            std::vector<std::array<int, 3>> items;  // table, row begin, row end
-            for (size_t t = t_first; t < table_list.size(); t++)
-                for (int r = 0; r < table_list[t]->x->ntiles; r += 16)
-                    items.push_back({(int)t, r, std::min(r + 16, table_list[t]->x->ntiles)});
-            parallel_items(items.size(), [&](size_t i) {
-                const auto& it = items[i];
-                table_list[it[0]]->rows(it[1], it[2]);
-            });
-        }
-        phase("tables");
-        // items: job, A-tile begin, end, and for a heavy single tile the
-        // part [lo, hi) of its neighbour list taken as tile B (the work of a
-        // tile grows with the square of its neighbour count: the densest
-        // tiles of a clustered catalog would otherwise each be one long item)
-        std::vector<std::array<int, 5>> items;
-        for (size_t g = g0; g < g1; g++) {
-            const int na = pj[g].role(0)->ntiles, step = 2;
-            const PairTable* ab = tp[g].empty ? nullptr : tp[g].AB;
-            for (int a0 = 0; a0 < na;) {
-                const int nb = ab && ab->need_nb ? (int)ab->nb[a0].size() : 0;
-                if (nb > 48) {
-                    for (int lo = 0; lo < nb; lo += 24) items.push_back({(int)g, a0, a0 + 1, lo, lo + 24});
-                    a0++;
-                } else {
-                    const int a1 = std::min(a0 + step, na);
-                    items.push_back({(int)g, a0, a1, 0, INT_MAX});
-                    a0 = a1;
-                }
-            }
-        }
-        // one task list per item, so that the concatenation keeps job order
-        // (a CTA flushes its shared histogram whenever the job changes)
-        PlanScratch& S = L.scratch;
-        std::vector<TaskList>& part = S.part;
-        if (part.size() < items.size()) part.resize(items.size());
-        std::vector<uint64_t> part_eval(items.size(), 0);
-        parallel_items(items.size(), [&](size_t i) {
-            const auto& it = items[i];
-            part[i].clear();
-            tp[it[0]].enumerate(it[1], it[2], part[i], part_eval[i], (size_t)it[3], (size_t)it[4]);
-        });
-        phase("enumerate");
-        std::vector<size_t> off(items.size() + 1, 0);  // each item's first task
-        for (size_t i = 0; i < items.size(); i++) {
-            ev += part_eval[i];
-            off[i + 1] = off[i] + part[i].size();
-        }
-        const size_t total = off[items.size()];
-        // tasks per group of the fast triangle kernel: 4, or 64 for sets of
-        // many jobs with thousands of tasks per CTA (voxel and jackknife sets
-        // of light tasks: the j-k tables are the larger share there, and the
-        // tail of a few large groups a small one; tp10k 12.91 ms with 4, 13.00
-        // with 8; voxel100k 267 ms with 4, 236 with 16, 230 with 32, 226 with
-        // 64; a heavy serving batch of a few dense jobs keeps 4)
-        const size_t group_max =
-            ctx->group_tasks > 0 ? (size_t)ctx->group_tasks
-                                 : (g1 - g0 > 64 && total >= (size_t)ctx->num_sms * 4 * 4096 ? MAX_GROUP_TASKS : 4);
-        // fast triangle kernel: groups form in windows of consecutive items of
-        // one job whose first A tiles lie in one aligned span of twice the
-        // group size
-        std::vector<std::array<size_t, 2>> windows;  // first item, item count
-        if (fast_tri) {
-            const int span = 2 * (int)group_max;
-            for (size_t i = 0; i < items.size();) {
-                size_t e = i + 1;
-                while (e < items.size() && items[e][0] == items[i][0] && items[e][1] / span == items[i][1] / span) e++;
-                windows.push_back({i, e - i});
-                i = e;
-            }
-        }
-        h_tasks.resize(total);
-        h_groups.clear();
-        h_gbox.clear();
-        if (fast_tri) {
-            if (S.gpart.size() < windows.size()) S.gpart.resize(windows.size());
-            std::vector<size_t> toff(windows.size() + 1);
-            for (size_t w = 0; w < windows.size(); w++) toff[w] = off[windows[w][0]];
-            toff[windows.size()] = total;
-            parallel_items(windows.size(), [&](size_t w) {
-                group_parts(&part[windows[w][0]], windows[w][1], pj[items[windows[w][0]][0]],
-                            group_max, h_tasks.data() + toff[w], S.gpart[w]);
-            });
-            assemble_groups(S.gpart, windows.size(), toff, total <= (size_t)ctx->num_sms * 3 * 64, h_tasks, h_groups,
-                            h_gbox);
-        } else if (total <= (size_t)ctx->num_sms * 3 * 64 && !(sp.kind == TPCF_THREE_SIDE && bin.len > 8192)) {
-            // (three-side histograms above 8192 bins keep job order: their CTAs
-            // flush, and the task pipelines of one CTA meet, at every job change)
-            // few tasks per CTA: largest first, so that the dynamic fetch
-            // balances the tail (a stable counting pass over 64 size classes)
-            auto cls = [](uint64_t u) { return 63 - (u ? 63 - __builtin_clzll(u) : 0); };
-            std::vector<size_t> start(65, 0);
-            for (size_t i = 0; i < items.size(); i++)
-                for (auto& e : part[i]) start[cls(e.first) + 1]++;
-            for (int c = 0; c < 64; c++) start[c + 1] += start[c];
-            for (size_t i = 0; i < items.size(); i++)
-                for (auto& e : part[i]) h_tasks[start[cls(e.first)]++] = e.second;
-        } else {
-            // many tasks per CTA: the tail is a small share; job order
-            parallel_items(items.size(), [&](size_t i) {
-                for (size_t e = 0; e < part[i].size(); e++) h_tasks[off[i] + e] = part[i][e].second;
-            });
-        }
-        phase("order");
-        return ev;
-    };
-    // Uploads a planned part on stream s into the given buffers; returns the
-    // group count.
-    auto upload_part = [&](const std::vector<uint4>& h_tasks, const std::vector<uint32_t>& h_groups,
-                           const std::vector<float>& h_gbox, DevBuf<uint4>& d_tasks, DevBuf<uint32_t>& d_groups,
-                           DevBuf<float>& d_gbox, cudaStream_t s) -> size_t {
-        const size_t ng = h_groups.empty() ? 0 : h_groups.size() - 1;
-        if (ng) {
-            d_groups.reserve(h_groups.size());
-            d_gbox.reserve(std::max<size_t>(h_gbox.size(), 1));
-            CK(cudaMemcpyAsync(d_groups.p, h_groups.data(), h_groups.size() * sizeof(uint32_t),
-                               cudaMemcpyHostToDevice, s));
-            if (!h_gbox.empty())
-                CK(cudaMemcpyAsync(d_gbox.p, h_gbox.data(), h_gbox.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-            L.h2d += h_groups.size() * sizeof(uint32_t) + h_gbox.size() * sizeof(float);
-        }
-        d_tasks.reserve(std::max<size_t>(h_tasks.size(), 1));
-        L.h2d += h_tasks.size() * sizeof(uint4);
-        if (!h_tasks.empty())
-            CK(cudaMemcpyAsync(d_tasks.p, h_tasks.data(), h_tasks.size() * sizeof(uint4), cudaMemcpyHostToDevice, s));
-        return ng;
-    };
-    if (plan_hit) {
-        ntasks = L.plan_ntasks;
-        ngroups = L.plan_ngroups;
-        ntasks2 = L.plan_ntasks2;
-        ngroups2 = L.plan_ngroups2;
-        evaluated = L.plan_evaluated;
-    } else {
-        L.plan_sig.clear();  // (set again once the whole plan is on the device)
-        PlanScratch& S = L.scratch;
-        const size_t g_first = pipeline ? 1 : group.size();
-        evaluated = plan_jobs(0, g_first, S.tasks, S.groups, S.gbox);
-        L.d_jobs.reserve(dj.size());
-        CK(cudaMemcpyAsync(L.d_jobs.p, dj.data(), g_first * sizeof(DevJob), cudaMemcpyHostToDevice, st));
-        L.h2d += g_first * sizeof(DevJob);
-        ngroups = upload_part(S.tasks, S.groups, S.gbox, L.d_tasks, L.d_groups, L.d_gbox, st);
-        ntasks = pairs ? (S.groups.empty() ? 0 : S.groups.back()) : S.tasks.size();
-        CK(cudaStreamSynchronize(st));
-        if (!pipeline) {
-            L.plan_sig = sig;
-            L.plan_chunk = plan_chunk;
-            L.plan_ntasks = ntasks;
-            L.plan_ngroups = ngroups;
-            L.plan_ntasks2 = L.plan_ngroups2 = 0;
-            L.plan_evaluated = evaluated;
-        }
-        phase("upload");
+        roles[g] = {{v[0], v[1], v[2]}, mode};
+        sig.push_back(ranges[v[0]].ref.id);
+        sig.push_back(ranges[v[1]].ref.id);
+        sig.push_back(ranges[v[2]].ref.id);
+        sig.push_back((uint64_t)slot_of[g] << 32 | (uint64_t)mode << 8 | (uint64_t)jsp.loop);
     }
-    // the second part of a pipelined plan, planned and uploaded (on the side
-    // stream) while the first part counts; the counting stream waits for it
-    bool second_pending = pipeline;
-    auto plan_second = [&]() {
-        PlanScratch& S = L.scratch;
-        for (size_t g = 1; g < group.size(); g++) attach(g);
-        evaluated2 = plan_jobs(1, group.size(), S.tasks2, S.groups2, S.gbox2);
-        if (!L.side) {
-            // (the lane's priority: a light serving lane's second part must
-            // not queue behind a heavy batch's CTAs)
-            int prio = 0;
-            CK(cudaStreamGetPriority(st, &prio));
-            CK(cudaStreamCreateWithPriority(&L.side, cudaStreamNonBlocking, prio));
-            CK(cudaEventCreateWithFlags(&L.ev_side, cudaEventDisableTiming));
+    cudaStream_t st = L.stream;
+    L.d_counters.reserve(CTR_WORDS);
+    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64);
+    const bool plan_hit = sig == L.plan_sig;
+    phase("batch");
+    const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
+    uint32_t nrows = L.plan_rows;   // pairs: items
+    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item
+    PlanHeader* d_header = nullptr;
+    // Finds the units of the batch on the device (see plan_rows): the host
+    // gives each job's number of rows.
+    auto plan_units = [&](size_t capacity) {
+        L.d_units.reserve(capacity);
+        L.d_masks.reserve(capacity);
+        PlanParams pp{};
+        pp.window = window;
+        pp.per_tile = fast_tri ? 0 : 1;
+        pp.tri = bin.tri_prune ? 1 : 0;
+        pp.slots = grid_for(ctx, cands[0], UINT64_MAX, L.sm_cap) * std::max(1, cands[0].groups);
+        const double l2 = bin.lmax * bin.lmax;
+        pp.lmax2 = l2 < 3e38 ? nextafterf((float)l2, INFINITY) : INFINITY;
+        auto sq_up = [](double v) { return v > 0 ? (v * v < 3e38 ? nextafterf((float)(v * v), INFINITY) : INFINITY) : 0.f; };
+        pp.s_hi2 = sq_up(bin.s_hi);
+        pp.q_hi2 = sq_up(bin.q_hi);
+        pp.s_lo2 = bin.s_lo > 0 ? nextafterf((float)std::min(bin.s_lo * bin.s_lo, 3e38), 0.f) : 0.f;
+        // heavy: what takes a CTA that has its SM to itself some 15 us (a line
+        // at 6000 or 8192 instead cost 1 % on 10k points and 2 % on 1k)
+        pp.r = (float)(bin.lmax < 3e38 ? (sp.kind == TPCF_TRIANGLE ? std::max(0.0, bin.s_hi * bin.q_hi) : bin.lmax) : 3e38);
+        pp.heavy = fast_tri ? 3000.f : 0.f;
+        int rpb = 0;
+        const int blocks = plan_blocks(nrows, &rpb);
+        L.d_row_cnt.reserve(std::max<size_t>(nrows, 1));
+        L.d_block_sum.reserve((size_t)blocks + 1);
+        CK(launch_plan(L.d_jobs.p, L.d_rows.p, (int)group.size(), nrows, pp, L.d_row_cnt.p, L.d_block_sum.p, d_header,
+                       L.d_units.p, L.d_masks.p, (uint32_t)capacity, st));
+    };
+    d_header = reinterpret_cast<PlanHeader*>(L.d_counters.p + CTR_HEADER);
+    if (!plan_hit) {
+        L.plan_sig.clear();  // (set again once the plan is on the device)
+        for (Range& r : ranges) r.view = get_view(ctx, L, r.key.h, r.key.b, r.key.e, r.key.gl);
+        phase("views");
+        CK(cudaStreamSynchronize(st));  // (a failed batch may still read the pinned buffers)
+        L.h_jobs.reserve(group.size());
+        L.h_rows.reserve(group.size() + 1);
+        uint64_t rows = 0;
+        plan_chunk = 0;
+        if (pairs) {
+            long long tile_pairs = 0;
+            for (const RoleJob& r : roles)
+                tile_pairs += (long long)ranges[r.range[0]].view->ntiles * ranges[r.range[1]].view->ntiles;
+            plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS);
         }
-        CK(cudaMemcpyAsync(L.d_jobs.p + 1, dj.data() + 1, (group.size() - 1) * sizeof(DevJob),
-                           cudaMemcpyHostToDevice, L.side));
-        L.h2d += (group.size() - 1) * sizeof(DevJob);
-        ngroups2 = upload_part(S.tasks2, S.groups2, S.gbox2, L.d_tasks2, L.d_groups2, L.d_gbox2, L.side);
-        ntasks2 = S.tasks2.size();
-        evaluated += evaluated2;
-        second_pending = false;
-        phase("second part");
-    };
-    // The merged plan (the first part's groups, then the second's, its task
-    // indices shifted), uploaded on a stream of its own while the parts count;
-    // it replaces the two parts once they are done.
-    bool merge_pending = pipeline;
-    auto merge_plan = [&]() {
-        PlanScratch& S = L.scratch;
-        S.tasks3.resize(ntasks + ntasks2);
-        std::copy(S.tasks.begin(), S.tasks.end(), S.tasks3.begin());
-        std::copy(S.tasks2.begin(), S.tasks2.end(), S.tasks3.begin() + ntasks);
-        S.groups3.resize(ngroups + ngroups2 + 1);
-        for (size_t g = 0; g < ngroups; g++) S.groups3[g] = S.groups[g];
-        for (size_t g = 0; g <= ngroups2; g++)
-            S.groups3[ngroups + g] = (uint32_t)ntasks + (ngroups2 ? S.groups2[g] : 0u);
-        S.gbox3.resize(6 * (ngroups + ngroups2));
-        std::copy(S.gbox.begin(), S.gbox.begin() + 6 * ngroups, S.gbox3.begin());
-        std::copy(S.gbox2.begin(), S.gbox2.begin() + 6 * ngroups2, S.gbox3.begin() + 6 * ngroups);
-        if (!L.side2) CK(cudaStreamCreateWithFlags(&L.side2, cudaStreamNonBlocking));
-        const uint64_t h2d0 = L.h2d;
-        upload_part(S.tasks3, S.groups3, S.gbox3, L.d_tasks3, L.d_groups3, L.d_gbox3, L.side2);
-        L.h2d = h2d0;  // (a copy for later calls: not this count's input)
-        merge_pending = false;
-    };
+        for (size_t g = 0; g < group.size(); g++) {
+            DevJob d{};
+            for (int r = 0; r < 3; r++) {
+                const View& v = *ranges[roles[g].range[r]].view;
+                d.pts[r] = v.pts.p;
+                d.tile_start[r] = v.tile_start.p;
+                d.box[r] = v.box.p;
+                d.ntiles[r] = v.ntiles;
+            }
+            d.mode = roles[g].mode;
+            d.hist = L.d_hist.p + (size_t)bin.len * slot_of[g];
+            L.h_jobs.p[g] = d;
+            L.h_rows.p[g] = (uint32_t)rows;
+            if (pairs) rows += (uint64_t)d.ntiles[0] * ((d.ntiles[1] + plan_chunk - 1) / plan_chunk);
+            else if (d.ntiles[2] > 0) rows += (uint64_t)((d.ntiles[0] + window - 1) / window) * d.ntiles[1];
+            if (rows > 0xF0000000ull) throw InvalidArg{"too many tile pairs in one batch"};
+        }
+        L.h_rows.p[group.size()] = (uint32_t)rows;
+        nrows = (uint32_t)rows;
+        L.d_jobs.reserve(group.size());
+        L.d_rows.reserve(group.size() + 1);
+        CK(cudaMemcpyAsync(L.d_jobs.p, L.h_jobs.p, group.size() * sizeof(DevJob), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(L.d_rows.p, L.h_rows.p, (group.size() + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        L.h2d += group.size() * sizeof(DevJob) + (group.size() + 1) * sizeof(uint32_t);
+        if (!pairs) plan_units(std::max<size_t>(L.d_units.n, (size_t)1 << 20));
+        L.plan_sig = sig;
+        L.plan_rows = nrows;
+        L.plan_chunk = plan_chunk;
+        phase("plan");
+    }
     L.stats.plan_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_wall0).count();
-    const bool fp64 = !guarded_fp32(sp, bin);
-    const bool fast_jbj = sp.kind == TPCF_TRIANGLE_JBJ && !fp64;  // the fast kernel's JBJ binning
     if (sp.kind == TPCF_TRIANGLE) ensure_acos(ctx);
     const AcosTable acos_t = sp.kind == TPCF_TRIANGLE ? acos_table(ctx) : AcosTable{};
-    const unsigned int nt = (unsigned int)ntasks;
     uint64_t launches = (sp.kind == TPCF_TRIANGLE && !fp64) ? 2 : 1;  // counting (+ recheck)
     const char* genv = getenv("TPCF_GRAPHS");
     const bool graphs = L.graphs_ok && !(genv && genv[0] == '0');
     L.h_hist.reserve(hist_total);
-    L.h_counters.reserve(8);
+    L.h_counters.reserve(CTR_WORDS);
     // recheck queue: at least 4M entries; TPCF_RECHECK_CAP lowers the floor
     // (tests use it to run the overflow path: grow the queue, count again)
     size_t queue_floor = (size_t)1 << 22;
     if (const char* qc = getenv("TPCF_RECHECK_CAP")) queue_floor = (size_t)std::max(1L, std::atol(qc));
     unsigned int queue_cap = (unsigned int)std::max<size_t>(L.d_queue.n, queue_floor);
     uint64_t dev_evaluated = 0, dev_binned = 0, replays = 0, regrows = 0;
+    PlanHeader header{};
+    // units (pairs: items) known on the host: needed where a batch is counted in slices
+    bool sized = pairs;
+    uint32_t nwork = pairs ? nrows : 0xffffffffu;
 
     // One complete count of the group with launch shape sh: zero, count,
     // recheck, copy back (replayed from a captured graph when allowed and
     // the batch repeats).  Returns the device time in ms.
     auto count_with = [&](const Shape& sh, bool allow_graph) -> float {
         const int copies = sh.copies;
-        // units the persistent CTAs pull: task groups (fast triangle kernel) or tasks
-        const unsigned int nwork = fast_tri ? (unsigned int)ngroups : nt;
-        const int grid = grid_for(ctx, sh, nwork, L.sm_cap);
-        // slices of at least 8 units per CTA, at most 64 of them
-        unsigned int slice = L.slice_batches ? std::max<unsigned int>((unsigned int)grid * 8u, (nwork + 63u) / 64u)
-                                             : std::max(nwork, 1u);
-        if (L.slice_batches && ctx->slice_tasks > 0) slice = (unsigned int)ctx->slice_tasks;
-        // a pipelined plan: two launches, one per part
-        const bool two_part = fast_tri && (ngroups2 > 0 || second_pending);
-        launches = (two_part ? 2 : (nwork > slice ? (nwork + slice - 1) / slice : 1)) +
-                   ((sp.kind == TPCF_TRIANGLE && !fp64) ? 1 : 0);
-        for (int attempt = 0; attempt < 3; attempt++) {
+        const int grid = grid_for(ctx, sh, pairs ? nrows : UINT64_MAX, L.sm_cap);
+        for (int attempt = 0; attempt < 4; attempt++) {
+            if (L.slice_batches && !sized) {
+                // (the header of a plan that overflowed the unit list asks for a
+                // larger one: the count below finds no units and regrows it)
+                CK(cudaMemcpyAsync(L.h_counters.p, L.d_counters.p, CTR_WORDS * sizeof(unsigned int),
+                                   cudaMemcpyDeviceToHost, st));
+                CK(cudaStreamSynchronize(st));
+                memcpy(&header, L.h_counters.p + CTR_HEADER, sizeof(header));
+                nwork = header.nunits;
+                sized = true;
+            }
+            // slices of at least 8 units per CTA, at most 64 of them
+            unsigned int slice = L.slice_batches ? std::max<unsigned int>((unsigned int)grid * 8u, (nwork + 63u) / 64u)
+                                                 : std::max(nwork, 1u);
+            if (L.slice_batches && ctx->slice_tasks > 0) slice = (unsigned int)ctx->slice_tasks;
+            launches = (nwork > slice ? (nwork + slice - 1) / slice : 1) + ((sp.kind == TPCF_TRIANGLE && !fp64) ? 1 : 0);
             RecheckQueue q{};
             if (sp.kind == TPCF_TRIANGLE && !fp64) {
                 if (L.d_queue.n < queue_cap) L.drop_graph();
                 L.d_queue.reserve(queue_cap);
                 q.items = L.d_queue.p;
-                q.count = L.d_counters.p + 1;
+                q.count = L.d_counters.p + CTR_RECHECK;
                 q.cap = queue_cap;
-                q.evaluated = reinterpret_cast<unsigned long long*>(L.d_counters.p + 2);
+                q.evaluated = reinterpret_cast<unsigned long long*>(L.d_counters.p + CTR_EVAL);
             } else if (fast_jbj) {
-                q.count = L.d_counters.p + 1;  // no item is ever queued (cap 0)
-                q.evaluated = reinterpret_cast<unsigned long long*>(L.d_counters.p + 2);
+                q.count = L.d_counters.p + CTR_RECHECK;  // no item is ever queued (cap 0)
+                q.evaluated = reinterpret_cast<unsigned long long*>(L.d_counters.p + CTR_EVAL);
             }
             auto enqueue = [&](bool capturing) -> cudaError_t {
                 const unsigned int ev_flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -2101,63 +1541,38 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         if ((e = (x)) != cudaSuccess) return e; \
     } while (0)
                 EQ(cudaMemsetAsync(L.d_hist.p, 0, hist_total * sizeof(unsigned long long), st));
-                EQ(cudaMemsetAsync(L.d_counters.p, 0, 8 * sizeof(unsigned int), st));
+                EQ(cudaMemsetAsync(L.d_counters.p, 0, CTR_ZEROED * sizeof(unsigned int), st));
                 EQ(cudaEventRecordWithFlags(L.ev0, st, ev_flags));
-                // the counting kernel over tasks [t0, t0 + n) (groups [t0, t0 + n)
-                // for the fast triangle kernel)
+                // the counting kernel over units (items) [t0, t0 + n)
                 auto launch_main = [&](unsigned int t0, unsigned int n) -> cudaError_t {
-                    const uint4* tk = L.d_tasks.p + t0;
-                    if (sp.kind == TPCF_TRIANGLE && fp64)
-                        return launch_triangle_fp64(L.d_jobs.p, tk, n, L.d_counters.p, bin.tri, acos_t, grid, copies,
-                                                    sp.precision == TPCF_GEOMETRY_FP64 ? 1 : 0, st);
-                    if (sp.kind == TPCF_TRIANGLE || fast_jbj)  // JBJ in FP32: exact without a recheck
-                        return launch_triangle_fast(L.d_jobs.p, L.d_tasks.p, L.d_groups.p + t0, L.d_gbox.p + 6 * (size_t)t0,
-                                                    n, L.d_counters.p, bin.tri, q, grid, copies, fast_jbj ? 1 : 0, st);
-                    if (sp.kind == TPCF_TRIANGLE_JBJ)
-                        return launch_triangle_fp64(L.d_jobs.p, tk, n, L.d_counters.p, bin.tri, acos_t, grid, copies, 2,
-                                                    st);
+                    unsigned int* counter = L.d_counters.p + CTR_WORK;
+                    const UnitList ul{d_header, L.d_units.p, L.d_masks.p, t0, n};
+                    if (fast_tri)  // (JBJ: exact without a recheck)
+                        return launch_triangle_fast(L.d_jobs.p, ul, counter, bin.tri, q, grid, copies, fast_jbj ? 1 : 0, st);
+                    if (tri_kind)
+                        return launch_triangle_fp64(L.d_jobs.p, ul, counter, bin.tri, acos_t, grid, copies,
+                                                    sp.kind == TPCF_TRIANGLE_JBJ ? 2
+                                                    : sp.precision == TPCF_GEOMETRY_FP64 ? 1 : 0, st);
                     if (sp.kind == TPCF_THREE_SIDE)
-                        return launch_three_side(L.d_jobs.p, tk, n, L.d_counters.p, bin.three, fp64, grid, copies,
-                                                 sh.groups, st);
-                    return launch_pairs(L.d_jobs.p, L.d_groups.p, (int)group.size(), t0, n, plan_chunk, L.d_counters.p,
-                                        reinterpret_cast<unsigned long long*>(L.d_counters.p + 2), bin.pair, fp64, grid,
-                                        copies, st);
+                        return launch_three_side(L.d_jobs.p, ul, counter, bin.three, fp64, grid, copies, sh.groups, st);
+                    return launch_pairs(L.d_jobs.p, L.d_rows.p, (int)group.size(), t0, n, plan_chunk, counter,
+                                        reinterpret_cast<unsigned long long*>(L.d_counters.p + CTR_EVAL), bin.pair, fp64,
+                                        grid, copies, st);
                 };
-                if (two_part) {
-                    // the first job's groups, then the others' (their own group
-                    // counter, d_counters[6]); on the first count of a pipelined
-                    // plan the second part is planned between the two launches
-                    EQ(launch_main(0, (unsigned int)ngroups));
-                    if (second_pending) plan_second();
-                    if (ngroups2) {
-                        // on the side stream, behind its upload and the zeroing of
-                        // the histograms and counters: its CTAs take the SMs the
-                        // first part's CTAs leave at its end
-                        EQ(cudaStreamWaitEvent(L.side, L.ev0, 0));
-                        EQ(launch_triangle_fast(L.d_jobs.p, L.d_tasks2.p, L.d_groups2.p, L.d_gbox2.p,
-                                                (unsigned int)ngroups2, L.d_counters.p + 6, bin.tri, q,
-                                                grid_for(ctx, sh, ngroups2, L.sm_cap), copies, fast_jbj ? 1 : 0,
-                                                L.side));
-                        EQ(cudaEventRecord(L.ev_side, L.side));
-                        EQ(cudaStreamWaitEvent(st, L.ev_side, 0));
-                    }
-                    if (merge_pending) merge_plan();
-                } else {
-                    // one launch over all tasks, or (a heavy serving batch) slices of
-                    // them, between which the device can start the kernels that
-                    // higher-priority streams (the light serving lanes) have queued
-                    EQ(launch_main(0, std::min(nwork, slice)));
-                    for (unsigned int t0 = slice; t0 < nwork; t0 += slice) {
-                        EQ(cudaMemsetAsync(L.d_counters.p, 0, sizeof(unsigned int), st));  // the slice's task counter
-                        EQ(launch_main(t0, std::min(slice, nwork - t0)));
-                    }
+                // one launch over all units, or (a heavy serving batch) slices of
+                // them, between which the device can start the kernels that
+                // higher-priority streams (the light serving lanes) have queued
+                EQ(launch_main(0, std::min(nwork, slice)));
+                for (unsigned int t0 = slice; t0 < nwork; t0 += slice) {
+                    EQ(cudaMemsetAsync(L.d_counters.p + CTR_WORK, 0, sizeof(unsigned int), st));  // the slice's counter
+                    EQ(launch_main(t0, std::min(slice, nwork - t0)));
                 }
                 EQ(cudaEventRecordWithFlags(L.ev_mid, st, ev_flags));
                 if (sp.kind == TPCF_TRIANGLE && !fp64)
                     EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, ctx->num_sms * 8, st));
                 EQ(cudaEventRecordWithFlags(L.ev1, st, ev_flags));
-                EQ(cudaMemcpyAsync(L.h_counters.p, L.d_counters.p, 8 * sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                                   st));
+                EQ(cudaMemcpyAsync(L.h_counters.p, L.d_counters.p, CTR_WORDS * sizeof(unsigned int),
+                                   cudaMemcpyDeviceToHost, st));
                 EQ(cudaMemcpyAsync(L.h_hist.p, L.d_hist.p, hist_total * sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost, st));
 #undef EQ
@@ -2167,16 +1582,14 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             if (allow_graph) {
                 // everything the captured launches read: the batch, its buffers, the shape
                 std::vector<uint64_t> gsig = sig;
-                const uint64_t extra[] = {(uint64_t)(uintptr_t)L.d_jobs.p, (uint64_t)(uintptr_t)L.d_tasks.p,
+                const uint64_t extra[] = {(uint64_t)(uintptr_t)L.d_jobs.p, (uint64_t)(uintptr_t)L.d_units.p,
                                           (uint64_t)(uintptr_t)L.d_counters.p, (uint64_t)(uintptr_t)L.d_queue.p,
                                           (uint64_t)(uintptr_t)L.h_hist.p, (uint64_t)(uintptr_t)L.h_counters.p,
                                           (uint64_t)(uintptr_t)acos_t.keys, (uint64_t)(uintptr_t)acos_t.vals,
                                           (uint64_t)(uintptr_t)acos_t.bucket, (uint64_t)acos_t.n, queue_cap,
-                                          (uint64_t)grid, (uint64_t)copies, (uint64_t)sh.groups, hist_total, ntasks,
-                                          (uint64_t)slice, (uint64_t)(uintptr_t)L.d_groups.p,
-                                          (uint64_t)(uintptr_t)L.d_gbox.p, (uint64_t)ngroups,
-                                          (uint64_t)(uintptr_t)L.d_tasks2.p, (uint64_t)(uintptr_t)L.d_groups2.p,
-                                          (uint64_t)(uintptr_t)L.d_gbox2.p, (uint64_t)ngroups2};
+                                          (uint64_t)grid, (uint64_t)copies, (uint64_t)sh.groups, hist_total,
+                                          (uint64_t)nwork, (uint64_t)slice, (uint64_t)(uintptr_t)L.d_rows.p,
+                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk};
                 gsig.insert(gsig.end(), extra, extra + sizeof(extra) / sizeof(extra[0]));
                 if (!L.graph || gsig != L.graph_sig) {
                     L.drop_graph();
@@ -2207,14 +1620,22 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             CK(cudaStreamSynchronize(st));
             replays = replayed ? 1 : 0;
             const unsigned int* counters = L.h_counters.p;
-            L.d2h += 8 * sizeof(unsigned int) + hist_total * sizeof(unsigned long long);
-            L.stats.recheck_units = counters[1];
-            memcpy(&dev_evaluated, &counters[2], sizeof(dev_evaluated));
-            memcpy(&dev_binned, &counters[4], sizeof(dev_binned));
-            if (sp.kind == TPCF_TRIANGLE && !fp64 && counters[1] > queue_cap) {
+            L.d2h += CTR_WORDS * sizeof(unsigned int) + hist_total * sizeof(unsigned long long);
+            memcpy(&header, counters + CTR_HEADER, sizeof(header));
+            if (!pairs && header.nunits == 0 && header.needed > 0) {
+                // the unit list overflowed: nothing was counted; plan again into a larger one
+                L.drop_graph();
+                plan_units((size_t)header.needed + (header.needed >> 3));
+                sized = false;
+                continue;
+            }
+            L.stats.recheck_units = counters[CTR_RECHECK];
+            memcpy(&dev_evaluated, &counters[CTR_EVAL], sizeof(dev_evaluated));
+            memcpy(&dev_binned, &counters[CTR_EVAL + 2], sizeof(dev_binned));
+            if (sp.kind == TPCF_TRIANGLE && !fp64 && counters[CTR_RECHECK] > queue_cap) {
                 // the recheck queue overflowed: grow it and count again
-                queue_cap =
-                    (unsigned int)std::min<uint64_t>((uint64_t)counters[1] + (counters[1] >> 2) + 1024, 0xF0000000ull);
+                queue_cap = (unsigned int)std::min<uint64_t>(
+                    (uint64_t)counters[CTR_RECHECK] + (counters[CTR_RECHECK] >> 2) + 1024, 0xF0000000ull);
                 regrows++;
                 continue;
             }
@@ -2229,7 +1650,6 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     // else the default.  A batch that repeats (its plan was cached) and has no
     // tuned shape yet is counted once with every candidate shape -- each count
     // is exact -- and the fastest is kept for the next calls.
-    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64);
     uint64_t key = 1469598103934665603ull;
     for (uint64_t v : sig) key = (key ^ v) * 1099511628211ull;
     const char* tenv = getenv("TPCF_AUTOTUNE");
@@ -2259,19 +1679,10 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         std::lock_guard<std::mutex> tlk(ctx->tune_mu);
         ctx->tuned[key] = shape;
     } else {
-        count_with(shape, graphs && !pipeline);  // (the first count of a pipelined plan is not captured)
-    }
-    if (pipeline) {
-        // the parts are done: later counts of the batch use the merged plan
-        CK(cudaStreamSynchronize(L.side2));
-        L.d_tasks.swap(L.d_tasks3);
-        L.d_groups.swap(L.d_groups3);
-        L.d_gbox.swap(L.d_gbox3);
-        L.plan_sig = sig;
-        L.plan_ntasks = ntasks + ntasks2;
-        L.plan_ngroups = ngroups + ngroups2;
-        L.plan_ntasks2 = L.plan_ngroups2 = 0;
-        L.plan_evaluated = evaluated;
+        // a batch's first count is launched directly (capturing costs more than
+        // one replay gains); TPCF_PIPELINE=0 captures it at once
+        const char* pl_env = getenv("TPCF_PIPELINE");
+        count_with(shape, graphs && (plan_hit || (pl_env && pl_env[0] == '0')));
     }
     L.stats.tuned_shapes = tuned_runs;
     L.stats.hist_copies = (uint64_t)shape.copies;
@@ -2282,7 +1693,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     L.stats.main_kernel_ms = ms_main;
     // JBJ compat: the reference's two extra counts in bin 0 per visited triangle
     if (sp.kind == TPCF_TRIANGLE_JBJ && sp.overflow == TPCF_OVERFLOW_COMPAT && bin.len > 0)
-        for (size_t g = 0; g < group.size(); g++) L.h_hist.p[(size_t)bin.len * slot_of[g]] += 2 * pj[g].loop_units;
+        for (size_t g = 0; g < group.size(); g++) L.h_hist.p[(size_t)bin.len * slot_of[g]] += 2 * job_units(g);
     for (size_t k = 0; k < nslots; k++) {
         const GroupJob& gj = group[slot_job[k]];
         const unsigned long long* src = L.h_hist.p + (size_t)bin.len * k;
@@ -2296,20 +1707,20 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     L.stats.kernel_ms = ms;
     L.stats.loop_units = units;
     // the fast triangle kernel skips (i,j) pairs that no counted triangle can
-    // contain and counts the triangles it walks; other kernels walk every
-    // triangle of their tasks
-    const bool fast_kernel = (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) && !fp64;
-    // (the pair kernel finds its tile pairs itself and counts them beside the pairs)
-    L.stats.evaluated_units = fast_kernel || pairs ? dev_evaluated : evaluated;
-    L.stats.binned_units = fast_kernel ? dev_binned : L.stats.evaluated_units;
-    L.stats.tasks = pairs ? dev_binned : ntasks + ntasks2;
+    // contain and counts the triangles it walks; the pair kernel counts the
+    // pairs and tile pairs it finds; other kernels walk every triangle of
+    // their units
+    L.stats.evaluated_units = fast_tri || pairs ? dev_evaluated : header.evaluated;
+    L.stats.binned_units = fast_tri ? dev_binned : L.stats.evaluated_units;
+    L.stats.tasks = pairs ? dev_binned : header.tiles;
     L.stats.kernel_launches = launches * std::max<uint64_t>(1, tuned_runs);
     L.stats.recheck_regrows = regrows;
     L.stats.total_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_wall0).count();
     if (plan_trace()) {
-        std::string line = "tpcf plan: tasks " + std::to_string(ntasks + ntasks2) + " groups " +
-                           std::to_string(ngroups + ngroups2) + (pipeline ? " (two parts)" : "");
+        std::string line = "tpcf plan: jobs " + std::to_string(group.size()) + " rows " + std::to_string(nrows) +
+                           " tiles " + std::to_string(L.stats.tasks) + " units " + std::to_string(header.nunits) +
+                           " parts " + std::to_string(header.parts);
         double prev = 0;
         for (auto& ph : phases) {
             line += std::string(" ") + ph.first + " " + std::to_string(ph.second - prev);
@@ -2584,7 +1995,7 @@ tpcf_status tpcf_create(tpcf_ctx** out, int32_t device) {
         const char* hc = getenv("TPCF_HEAVY_COST");
         if (hc) ctx->heavy_cost = atof(hc);
         if (const char* tr = getenv("TPCF_SERVING_TRACE")) ctx->trace_path = tr;
-        if (const char* gt = getenv("TPCF_GROUP_TASKS")) ctx->group_tasks = std::min(MAX_GROUP_TASKS, std::max(1, atoi(gt)));
+        if (const char* gt = getenv("TPCF_GROUP_TASKS")) ctx->group_tasks = std::min(MAX_WINDOW, std::max(1, atoi(gt)));
         const char* shv = getenv("TPCF_SLICE_HEAVY");
         if (shv) ctx->slice_heavy = shv[0] != '0';
         const char* stk = getenv("TPCF_SLICE_TASKS");
@@ -2615,11 +2026,17 @@ tpcf_status tpcf_create(tpcf_ctx** out, int32_t device) {
                 // runs keeps this lane's next kernel from running beside it
                 // (implicit synchronisation), so light batches must not allocate.
                 L->h_hist.reserve((size_t)1 << 20);
-                L->h_counters.reserve(8);
+                L->h_counters.reserve(CTR_WORDS);
                 L->d_hist.reserve((size_t)1 << 22);
-                L->d_counters.reserve(8);
+                L->d_counters.reserve(CTR_WORDS);
                 L->d_jobs.reserve((size_t)1 << 16);
-                L->d_tasks.reserve((size_t)1 << 21);
+                L->h_jobs.reserve(4096);
+                L->h_rows.reserve(4097);
+                L->d_rows.reserve((size_t)1 << 16);
+                L->d_row_cnt.reserve((size_t)1 << 20);
+                L->d_block_sum.reserve((size_t)1 << 15);
+                L->d_units.reserve((size_t)1 << 20);
+                L->d_masks.reserve((size_t)1 << 20);
                 L->d_queue.reserve((size_t)1 << 22);
             }
             ctx->lanes.push_back(std::move(L));

@@ -24,17 +24,12 @@ enum Pred : uint32_t {
     PRED_RDD = 4     // weight [key_i >= key_j] + [key_i >= key_k]   (loop ONE, roles A == B, in the
                      // role order (C, A, A): the single-array point first; guarded kernel only)
 };
-// task.x: bits 0..21 job slot, 22..24 Pred, 28/29 diagonal flags, 30/31 reach checks
-constexpr uint32_t TASK_SLOT_MASK = 0x3FFFFFu;
-constexpr uint32_t MAX_BATCH_JOBS = TASK_SLOT_MASK;  // jobs of one launch
-constexpr int TASK_PRED_SHIFT = 22;
-constexpr uint32_t TASK_PRED_MASK = 0x7u;
-constexpr uint32_t TASK_DIAG_IJ = 1u << 28;  // tiles I and J are the same tile of one view: j > i
-constexpr uint32_t TASK_DIAG_JK = 1u << 29;  // tiles J and K are the same tile of one view: k > j
-// points of tile A may lie out of reach (>= lmax) of tile B / C: worth
-// testing point by point (the guarded triangle kernel; others ignore them)
-constexpr uint32_t TASK_CHECK_B = 1u << 30;
-constexpr uint32_t TASK_CHECK_C = 1u << 31;
+// unit.x: bits 0..21 job slot, 22/23 quarter of the A tile's points, 24 whether
+// the unit is that quarter only
+constexpr uint32_t UNIT_SLOT_MASK = 0x3FFFFFu;
+constexpr uint32_t MAX_BATCH_JOBS = UNIT_SLOT_MASK;  // jobs of one launch
+constexpr int UNIT_QUARTER_SHIFT = 22;
+constexpr uint32_t UNIT_QUARTER = 1u << 24;
 // recheck queue item .x: job slot | weight << 22
 constexpr int RECHECK_WEIGHT_SHIFT = 22;
 
@@ -59,9 +54,8 @@ constexpr int MAX_TRI_BINS = (1 << 22) - 1;  // S*Q*T limit of the triangle kern
 // CODE16_ABOVE).
 constexpr int CODE16_ZERO = -2, CODE16_BELOW = -1, CODE16_ABOVE = 255;
 constexpr int MAX_FAST_S = 254;
-// most tasks in one group of the fast triangle kernel (its shared histogram is
-// flushed between groups, at most every 256 tasks)
-constexpr int MAX_GROUP_TASKS = 64;
+// most A tiles in one window of the planner (one mask word)
+constexpr int MAX_WINDOW = 32;
 // weight sum (4*nBelow + nAbove, >= 32 if rejected) -> permutation validity
 constexpr unsigned VALID_ANY = 0x37u;   // shortest or middle side in range
 constexpr unsigned VALID_02 = 0x07u;    // shortest side in range (permutations 0 and 2)
@@ -80,8 +74,9 @@ struct DevJob {
     unsigned long long* hist;    // global uint64 histogram (hist_len entries)
 };
 // the job's tile tuples and the predicate of its points
-constexpr uint32_t JOB_PRED_MASK = 0x7u;  // Pred
-constexpr uint32_t JOB_B_FROM_A = 8u;     // tiles B >= A of one view, positions j >= i in a diagonal pair
+constexpr uint32_t JOB_PRED_MASK = 0x7u;   // Pred
+constexpr uint32_t JOB_B_FROM_A = 8u;      // tiles B >= A of one view, positions j >= i (triangles: j > i) in a diagonal pair
+constexpr uint32_t JOB_C_FROM_B = 16u;     // the same of tiles C and B, positions k and j
 
 // Launch-wide binning constants for the triangle kernels.
 struct TriParams {
@@ -156,21 +151,49 @@ struct LaunchStats {
     unsigned int* error_flag;    // set by kernels on an internal invariant failure
 };
 
+// Planner: which tile triples of a launch can hold a counted triple.
+struct PlanParams {
+    int window;        // A tiles per row (at most MAX_WINDOW)
+    int per_tile;      // 1: a unit per A tile; 0: a unit per row and tile C, its A tiles as a mask
+    int tri;           // test the s and q ranges on the triple's side bounds
+    int slots;         // CTAs (pipelines) that will share the units
+    float lmax2;       // squared: no counted triple has a side at or above it (infinite: no pruning)
+    float s_lo2, s_hi2, q_hi2;
+    float r, heavy;    // typical longest side of a counted triple; estimated triples above which a unit is heavy
+};
+// The plan of a launch, found on the device and kept while its batch repeats.
+struct PlanHeader {
+    uint32_t nunits;   // units to count (0 where they overflow the unit list)
+    uint32_t needed;   // units found
+    uint32_t parts;    // units each heavy one was cut into
+    uint32_t pad;
+    unsigned long long evaluated, tiles;  // triples and tile triples of the units
+};
+// row_off[j] .. row_off[j + 1]: rows (window of A tiles, tile B) of job j;
+// row_cnt: two words per row; block_sum: plan_blocks(nrows) + 1 pairs of words
+int plan_blocks(uint64_t nrows, int* rows_per_block);
+cudaError_t launch_plan(const DevJob* jobs, const uint32_t* row_off, int njobs, uint32_t nrows, const PlanParams& pp,
+                        uint2* row_cnt, uint2* block_sum, PlanHeader* header, uint4* units, uint32_t* masks,
+                        uint32_t capacity, cudaStream_t st);
+
 // ---- kernel launchers (kernels.cu) ----
 cudaError_t prepare_kernels(int device);  // once per device before any launch
-// groups[g] .. groups[g + 1]: the tasks of group g (same job, tiles B and C);
-// gbox[6 g ..]: lo/hi of the union of their A tiles; jbj: JBJ binning
-cudaError_t launch_triangle_fast(const DevJob* jobs, const uint4* tasks, const uint32_t* groups, const float* gbox,
-                                 unsigned int ngroups, unsigned int* group_counter, const TriParams& p,
+// The counting kernels take units [u0, u0 + n) of a plan; jbj: JBJ binning
+struct UnitList {
+    const PlanHeader* header;
+    const uint4* units;
+    const uint32_t* masks;
+    uint32_t u0, n;
+};
+cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
                                  RecheckQueue q, int grid, int hist_copies, int jbj, cudaStream_t st);
 cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t,
                                     int grid, cudaStream_t st);
-cudaError_t launch_triangle_fp64(const DevJob* jobs, const uint4* tasks, unsigned int ntasks,
-                                 unsigned int* task_counter, const TriParams& p, AcosTable t, int grid,
-                                 int hist_copies, int mode, cudaStream_t st);  // mode: 0 FP64, 1 geometry, 2 JBJ
-cudaError_t launch_three_side(const DevJob* jobs, const uint4* tasks, unsigned int ntasks,
-                              unsigned int* task_counter, const ThreeParams& p, int fp64, int grid,
-                              int hist_copies, int groups, cudaStream_t st);
+cudaError_t launch_triangle_fp64(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
+                                 AcosTable t, int grid, int hist_copies, int mode,
+                                 cudaStream_t st);  // mode: 0 FP64, 1 geometry, 2 JBJ
+cudaError_t launch_three_side(const DevJob* jobs, UnitList ul, unsigned int* counter, const ThreeParams& p, int fp64,
+                              int grid, int hist_copies, int groups, cudaStream_t st);
 // item_off[j] .. item_off[j + 1]: the items (tile A, chunk of `chunk` tiles B)
 // of job j; counts items [item0, item0 + nitems); work[0], work[1] receive the
 // pairs and tile pairs evaluated

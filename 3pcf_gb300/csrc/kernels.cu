@@ -233,6 +233,21 @@ __device__ void tp_geom(double d0, double d1, double d2, const TriParams& p, int
 constexpr unsigned int FLUSH_EVERY = 256;  // tasks between histogram flushes (u32 safety)
 constexpr uint32_t TASK_NONE = 0xFFFFFFFFu;
 
+// A single-tile unit as {slot, tile A, tile B, tile C} (slot TASK_NONE past
+// the end) and the points [i0, i1) of tile A it covers; drawn by one thread.
+__device__ __forceinline__ uint4 draw_unit(const UnitList& ul, unsigned int* counter, int& i0, int& i1) {
+    const unsigned int t = atomicAdd(counter, 1u);
+    i0 = 0;
+    i1 = TILE;
+    if (t >= ul.n || ul.u0 + t >= ul.header->nunits) return make_uint4(TASK_NONE, 0, 0, 0);
+    uint4 u = ul.units[ul.u0 + t];
+    if (u.x & UNIT_QUARTER) {
+        i0 = (int)((u.x >> UNIT_QUARTER_SHIFT) & 3u) * (TILE / 4);
+        i1 = i0 + TILE / 4;
+    }
+    return make_uint4(u.x & UNIT_SLOT_MASK, u.y + (uint32_t)__ffs(ul.masks[ul.u0 + t]) - 1u, u.z, u.w);
+}
+
 // Swizzled shared histograms (three-side kernels): bin b of a copy lives at
 // word hist_pos(b), its low five bits (the bank) XORed with the next two 5-bit
 // groups, so that the lanes of one atomic instruction whose bins differ only
@@ -266,6 +281,349 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+
+// ---------------------------------------------------------------------------
+// Planning.  A launch's units of work -- tile triples (or, for the fast
+// triangle kernel, a tile pair (B, C) with a mask of up to `window` A tiles)
+// that can hold a counted triple -- are found on the device from the views'
+// tile boxes: row (job, window of A tiles, tile B) tests every tile C.
+//   plan_count  units of each row, those of each block of rows, and totals;
+//   plan_scan   (one CTA) exclusive scan of the blocks' sums, the number of
+//               parts heavy units are cut into, the header;
+//   plan_fill   the same tests again, writing each unit to its place.
+// Heavy units (an estimate of their triples above PlanParams::heavy) come
+// first, in job order, then the light ones in job order: a CTA flushes its
+// histogram when the job changes, and the long units are not left to the end.
+// With few of them for the CTAs, each is cut into its A tiles or the quarters
+// of those.  (The 40,000 voxel jobs of a 20k-point cone took 22 ms to plan on
+// 16 host cores, 0.95M tile triples of 150k points 9.3 ms; both are below 1 ms
+// here.)
+
+constexpr int PLAN_WARPS = 8;
+
+// Last job j of [0, n) with off[j] <= t (off[0] <= t; a job without items is
+// never the last one), searched 32 ways at a time by a whole warp.
+__device__ __forceinline__ int find_job(const uint32_t* __restrict__ off, int n, uint32_t t) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = n;
+    while (len > 1) {
+        const int step = (len + 31) / 32;
+        const bool le = lane * step < len && off[lo + lane * step] <= t;
+        const int k = 31 - __clz(__ballot_sync(0xffffffffu, le) | 1u);
+        lo += k * step;
+        len = min(step, len - k * step);
+    }
+    return lo;
+}
+
+int plan_blocks(uint64_t nrows, int* rows_per_block) {
+    // one row per warp while that leaves the scan few sums, else eight
+    const int r = nrows <= 32768 ? PLAN_WARPS : PLAN_WARPS * 8;
+    if (rows_per_block) *rows_per_block = r;
+    return (int)((nrows + r - 1) / r);
+}
+
+// Lower and upper bounds of the squared side between two tile boxes; the
+// margins cover the rounding of the bounds and of the reference's sides.  A
+// lower bound that overflows stays below an infinite limit.
+__device__ __forceinline__ float2 box_bounds2(float4 al, float4 ah, float4 bl, float4 bh) {
+    const float gx = fmaxf(0.f, fmaxf(al.x - bh.x, bl.x - ah.x)), ux = fmaxf(ah.x - bl.x, bh.x - al.x);
+    const float gy = fmaxf(0.f, fmaxf(al.y - bh.y, bl.y - ah.y)), uy = fmaxf(ah.y - bl.y, bh.y - al.y);
+    const float gz = fmaxf(0.f, fmaxf(al.z - bh.z, bl.z - ah.z)), uz = fmaxf(ah.z - bl.z, bh.z - al.z);
+    return make_float2(fminf((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f), 3.4028235e38f),
+                       (ux * ux + uy * uy + uz * uz) * (1.0f + 4e-5f) + 1e-37f);
+}
+
+// Whether a tile triple can hold a counted triangle-parametrization triangle:
+// with the three pair bounds sorted (L1<=L2<=L3 lower, U1<=U2<=U3 upper) the
+// shortest side lies in [L1,U1], the middle in [L2,U2], the longest in
+// [L3,U3]; permutations 0/2 need s_lo <= shortest < s_hi and
+// middle < q_hi*shortest, permutation 1 needs s_lo <= middle < s_hi and
+// longest < q_hi*middle.  All squared.
+__device__ __forceinline__ bool tri_possible(float2 x, float2 y, float2 z, const PlanParams& pp) {
+    const float l0 = fminf(fminf(x.x, y.x), z.x), l2 = fmaxf(fmaxf(x.x, y.x), z.x);
+    const float l1 = fmaxf(fminf(x.x, y.x), fminf(fmaxf(x.x, y.x), z.x));
+    const float u0 = fminf(fminf(x.y, y.y), z.y);
+    const float u1 = fmaxf(fminf(x.y, y.y), fminf(fmaxf(x.y, y.y), z.y));
+    return (l0 < pp.s_hi2 && u0 >= pp.s_lo2 && l1 < pp.q_hi2 * u0) ||
+           (l1 < pp.s_hi2 && u1 >= pp.s_lo2 && l2 < pp.q_hi2 * u1);
+}
+
+// Rough share of the pairs of two tiles that are within r of one another.
+__device__ __forceinline__ float near_share(float2 b, float r) {
+    const float lo = sqrtf(b.x), hi = sqrtf(fminf(b.y, 3e38f));
+    if (hi <= r) return 1.f;
+    const float f = fmaxf(r - lo, 0.f) / fmaxf(hi - lo, 1e-30f);
+    return f * f;
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(PLAN_WARPS * 32)
+plan_rows(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ row_off, int njobs, uint32_t nrows,
+          int rows_per_block, PlanParams pp, uint2* row_cnt, uint2* block_sum, PlanHeader* header, uint4* units,
+          uint32_t* masks) {
+    __shared__ float4 s_box[PLAN_WARPS][2 * MAX_WINDOW];
+    __shared__ float2 s_ab[PLAN_WARPS][MAX_WINDOW];
+    __shared__ int s_na[PLAN_WARPS][MAX_WINDOW];
+    __shared__ uint2 s_sum[PLAN_WARPS];
+    __shared__ unsigned long long s_eval, s_tiles;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    if (!FILL && threadIdx.x == 0) s_eval = s_tiles = 0ull;
+    uint32_t nunits = 0, nheavy = 0, parts = 0;
+    if (FILL) {
+        nunits = header->nunits;
+        if (nunits == 0) return;  // nothing found, or more than the list holds
+        parts = header->parts;
+        nheavy = block_sum[gridDim.x].x;
+    }
+    __syncthreads();
+    const uint32_t row0 = blockIdx.x * (uint32_t)rows_per_block;
+    // consecutive rows of the block go to one warp
+    const int per_warp = rows_per_block / PLAN_WARPS;
+    uint2 place = make_uint2(0, 0);  // FILL: heavy and light units before this warp's rows
+    if (FILL) {
+        for (int r = lane; r < warp * per_warp; r += 32)
+            if (row0 + r < nrows) {
+                const uint2 c = row_cnt[row0 + r];
+                place.x += c.x;
+                place.y += c.y;
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            place.x += __shfl_xor_sync(full, place.x, o);
+            place.y += __shfl_xor_sync(full, place.y, o);
+        }
+        place.x += block_sum[blockIdx.x].x;
+        place.y += block_sum[blockIdx.x].y;
+    }
+    uint2 warp_sum = make_uint2(0, 0);
+    unsigned long long eval = 0, tiles = 0;
+    for (int rr = 0; rr < per_warp; rr++) {
+        const uint32_t row = row0 + (uint32_t)(warp * per_warp + rr);
+        if (row >= nrows) break;
+        if (FILL) {
+            const uint2 c = row_cnt[row];
+            if (c.x + c.y == 0u) continue;
+        }
+        const int slot = find_job(row_off, njobs, row);
+        const DevJob& J = jobs[slot];
+        const uint32_t l = row - row_off[slot];
+        const int ntA = J.ntiles[0], ntB = J.ntiles[1], ntC = J.ntiles[2];
+        const int a0 = (int)(l / (uint32_t)ntB) * pp.window, b = (int)(l % (uint32_t)ntB);
+        const bool from_a = J.mode & JOB_B_FROM_A, from_b = J.mode & JOB_C_FROM_B;
+        const float4 bl = J.box[1][2 * (size_t)b], bh = J.box[1][2 * (size_t)b + 1];
+        const int nb = J.tile_start[1][b + 1] - J.tile_start[1][b];
+        bool ok = false;
+        __syncwarp();
+        if (lane < pp.window && a0 + lane < ntA && (!from_a || b >= a0 + lane)) {
+            const float4 al = J.box[0][2 * (size_t)(a0 + lane)], ah = J.box[0][2 * (size_t)(a0 + lane) + 1];
+            const float2 ab = box_bounds2(al, ah, bl, bh);
+            ok = !(ab.x >= pp.lmax2);
+            s_box[warp][2 * lane] = al;
+            s_box[warp][2 * lane + 1] = ah;
+            s_ab[warp][lane] = ab;
+            s_na[warp][lane] = J.tile_start[0][a0 + lane + 1] - J.tile_start[0][a0 + lane];
+        }
+        const unsigned amask = __ballot_sync(full, ok);
+        __syncwarp();
+        uint2 cnt = make_uint2(0, 0);  // this lane's units of the row
+        if (amask) {
+            for (int c0 = from_b ? b & ~31 : 0; c0 < ntC; c0 += 32) {
+                const int c = c0 + lane;
+                const bool in = c < ntC && (!from_b || c >= b);
+                float4 cl = make_float4(0.f, 0.f, 0.f, 0.f), ch = cl;
+                float2 bc = make_float2(0.f, 0.f);
+                bool cand = in;
+                if (in) {
+                    cl = J.box[2][2 * (size_t)c];
+                    ch = J.box[2][2 * (size_t)c + 1];
+                    bc = box_bounds2(bl, bh, cl, ch);
+                    cand = !(bc.x >= pp.lmax2);
+                }
+                if (!__any_sync(full, cand)) continue;
+                unsigned mask = 0;
+                float est = 0.f;
+                unsigned n_heavy = 0, n_light = 0;
+                if (cand) {
+                    const int nc = J.tile_start[2][c + 1] - J.tile_start[2][c];
+                    for (unsigned m = amask; m; m &= m - 1u) {
+                        const int t = __ffs(m) - 1;
+                        const float2 ab = s_ab[warp][t], ac = box_bounds2(s_box[warp][2 * t], s_box[warp][2 * t + 1], cl, ch);
+                        if (ac.x >= pp.lmax2 || (pp.tri && !tri_possible(ab, ac, bc, pp))) continue;
+                        mask |= 1u << t;
+                        if (pp.heavy > 0.f) {
+                            // triangles within reach, and what walking the points i and
+                            // the j's in their reach costs in the same unit
+                            const float na = (float)s_na[warp][t], nj = (float)nb * near_share(ab, pp.r);
+                            est += na * (25.f + nj * (2.5f + (float)nc * near_share(ac, pp.r) * near_share(bc, pp.r)));
+                        }
+                        if (!FILL) {
+                            const unsigned long long na = (unsigned)s_na[warp][t], n = (unsigned)nb, k = (unsigned)nc;
+                            const bool dij = from_a && a0 + t == b, djk = from_b && b == c;
+                            eval += dij && djk ? na * (na - 1) * (na - 2) / 6
+                                    : dij      ? na * (na - 1) / 2 * k
+                                    : djk      ? na * (n * (n - 1) / 2)
+                                               : na * n * k;
+                        }
+                    }
+                    const unsigned n = pp.per_tile ? __popc(mask) : (mask ? 1u : 0u);
+                    tiles += __popc(mask);
+                    // (without estimates every unit is a heavy one)
+                    if (!(pp.heavy > 0.f) || est > pp.heavy) n_heavy = n;
+                    else n_light = n;
+                }
+                if (!FILL) {
+                    cnt.x += n_heavy;
+                    cnt.y += n_light;
+                    continue;
+                }
+                // this lane's place among the warp's units
+                uint32_t inc = n_heavy | n_light << 16;  // at most 32 x 32 units of a step
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(full, inc, o);
+                    if (lane >= o) inc += v;
+                }
+                const uint32_t total = __shfl_sync(full, inc, 31);
+                uint32_t h = place.x + (inc & 0xffffu) - n_heavy;
+                uint32_t u = nheavy * parts + place.y + (inc >> 16) - n_light;
+                for (unsigned m = mask; m;) {
+                    // one A tile, or all of the row's
+                    const unsigned sub = pp.per_tile ? m & (0u - m) : m;
+                    m &= ~sub;
+                    if (n_light) {
+                        units[u] = make_uint4((uint32_t)slot, (uint32_t)a0, (uint32_t)b, (uint32_t)c);
+                        masks[u++] = sub;
+                        continue;
+                    }
+                    for (uint32_t q = 0; q < parts; q++) {
+                        // a heavy unit's parts: its A tiles, or quarters of them
+                        // (of a single tile: quarters)
+                        uint32_t x = (uint32_t)slot, pm = sub;
+                        if (parts > 1) {
+                            if (pp.per_tile) {
+                                x |= UNIT_QUARTER | q << UNIT_QUARTER_SHIFT;
+                            } else {
+                                const uint32_t w = parts == 4 ? q : q >> 2;
+                                // every fourth set A tile from the w-th (windows of four: one)
+                                uint32_t keep = 0, n = 0;
+                                for (unsigned mm = sub; mm; mm &= mm - 1u, n++)
+                                    if ((n & 3u) == w) keep |= mm & (0u - mm);
+                                pm = keep;
+                                if (parts == 16) x |= UNIT_QUARTER | (q & 3u) << UNIT_QUARTER_SHIFT;
+                            }
+                        }
+                        units[h * parts + q] = make_uint4(x, (uint32_t)a0, (uint32_t)b, (uint32_t)c);
+                        masks[h * parts + q] = pm;
+                    }
+                    h++;
+                }
+                place.x += total & 0xffffu;
+                place.y += total >> 16;
+            }
+        }
+        if (!FILL) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                cnt.x += __shfl_xor_sync(full, cnt.x, o);
+                cnt.y += __shfl_xor_sync(full, cnt.y, o);
+            }
+            if (lane == 0) row_cnt[row] = cnt;
+            warp_sum.x += cnt.x;
+            warp_sum.y += cnt.y;
+        }
+    }
+    if (FILL) return;
+    if (lane == 0) s_sum[warp] = warp_sum;
+    if (eval) atomicAdd(&s_eval, eval);
+    if (tiles) atomicAdd(&s_tiles, tiles);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint2 t = make_uint2(0, 0);
+        for (int w = 0; w < PLAN_WARPS; w++) {
+            t.x += s_sum[w].x;
+            t.y += s_sum[w].y;
+        }
+        block_sum[blockIdx.x] = t;
+        if (s_eval) atomicAdd(&header->evaluated, s_eval);
+        if (s_tiles) atomicAdd(&header->tiles, s_tiles);
+    }
+}
+
+constexpr int PLAN_SCAN_THREADS = 1024;
+
+// Exclusive scan of the block sums in place, totals at [nblocks].
+__global__ void __launch_bounds__(PLAN_SCAN_THREADS)
+plan_scan(uint2* block_sum, int nblocks, PlanParams pp, PlanHeader* header, uint32_t capacity) {
+    __shared__ uint2 s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long th = 0, tl = 0;  // running totals (all threads alike)
+    for (int base = 0; base < nblocks; base += PLAN_SCAN_THREADS) {
+        const int i = base + (int)threadIdx.x;
+        const uint2 v = i < nblocks ? block_sum[i] : make_uint2(0, 0);
+        uint2 x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xffffffffu, x.x, o), b = __shfl_up_sync(0xffffffffu, x.y, o);
+            if (lane >= o) {
+                x.x += a;
+                x.y += b;
+            }
+        }
+        if (lane == 31) s_warp[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            uint2 w = s_warp[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t a = __shfl_up_sync(0xffffffffu, w.x, o), b = __shfl_up_sync(0xffffffffu, w.y, o);
+                if (lane >= o) {
+                    w.x += a;
+                    w.y += b;
+                }
+            }
+            s_warp[lane] = w;
+        }
+        __syncthreads();
+        const uint2 before = warp ? s_warp[warp - 1] : make_uint2(0, 0), all = s_warp[31];
+        if (i < nblocks) block_sum[i] = make_uint2((uint32_t)th + before.x + x.x - v.x, (uint32_t)tl + before.y + x.y - v.y);
+        th += all.x;
+        tl += all.y;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        block_sum[nblocks] = make_uint2((uint32_t)th, (uint32_t)tl);
+        // Few heavy units for the CTAs: cut each, so that the last ones are a
+        // small share of the launch.  (DDD+DDR+DRR+RRR of 1k points: 1.50 ms
+        // with whole units, 0.71 ms with sixteen units per CTA cut once,
+        // 0.51 ms cut to them; 10k points have enough whole units.)
+        // (single tile triples cost alike: two per CTA are enough)
+        const unsigned long long want = (pp.per_tile ? 2ull : 16ull) * (unsigned)pp.slots;
+        const uint32_t top = pp.per_tile ? 4u : 16u;
+        uint32_t parts = 1;
+        while (parts < top && th > 0 && th * parts < want) parts *= 4;
+        const unsigned long long n = th * parts + tl;
+        header->parts = parts;
+        header->needed = (uint32_t)(n < 0xffffffffull ? n : 0xffffffffull);
+        header->nunits = n <= capacity ? (uint32_t)n : 0u;
+    }
+}
+
+cudaError_t launch_plan(const DevJob* jobs, const uint32_t* row_off, int njobs, uint32_t nrows, const PlanParams& pp,
+                        uint2* row_cnt, uint2* block_sum, PlanHeader* header, uint4* units, uint32_t* masks,
+                        uint32_t capacity, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(header, 0, sizeof(PlanHeader), st);
+    if (e != cudaSuccess || nrows == 0) return e;
+    int rpb = 0;
+    const int blocks = plan_blocks(nrows, &rpb);
+    plan_rows<false><<<blocks, PLAN_WARPS * 32, 0, st>>>(jobs, row_off, njobs, nrows, rpb, pp, row_cnt, block_sum,
+                                                         header, units, masks);
+    plan_scan<<<1, PLAN_SCAN_THREADS, 0, st>>>(block_sum, blocks, pp, header, capacity);
+    plan_rows<true><<<blocks, PLAN_WARPS * 32, 0, st>>>(jobs, row_off, njobs, nrows, rpb, pp, row_cnt, block_sum, header,
+                                                        units, masks);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -601,6 +959,20 @@ __device__ __forceinline__ void load_points(float4* P, const DevJob& J, const Ta
 
 __device__ __forceinline__ int pkey(float4 p) { return __float_as_int(p.w); }
 
+// What a unit's CTA shares beside the tiles: boxes (lo, hi) of tiles B and C
+// and of all A tiles of the unit, and the resident A tiles (first point,
+// points, TRI_* flags, position of the first point in its tile).
+struct TriShared {
+    uint4 unit;
+    uint32_t mask;
+    int b0, c0;          // first points of tiles B and C
+    int next_i, end_i;  // points of the resident A tiles handed out, and their number
+    float box[2][6];
+    float abox[6];
+    int4 meta[TRI_GROUP_A];
+};
+constexpr int TRI_DIAG_IJ = 1, TRI_CHECK_B = 2, TRI_CHECK_C = 4;
+
 // Queued candidate triangle of the current i: j (bits 0-5), k (bits 6-11) and
 // its weight (bits 12-13).
 
@@ -609,7 +981,7 @@ __device__ __forceinline__ int pkey(float4 p) { return __float_as_int(p.w); }
 template <bool THETA_FULL, bool JBJ>
 __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, const int2* row_ij, const int2* row_ik,
                                                const float* JKd, const short* JKw, const TriParams& p, unsigned int* Hw,
-                                               RecheckQueue& q, uint32_t slot, uint32_t ia, int b0, int c0) {
+                                               RecheckQueue& q, const TriShared& S, uint32_t ia) {
     const int lane = threadIdx.x & 31;
     const uint32_t e0 = lane < n ? cand[lane] : 0u;
     const uint32_t e1 = lane + 32 < n ? cand[lane + 32] : 0u;
@@ -630,8 +1002,9 @@ __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, cons
     bool guard[2];
     triangle_full2<THETA_FULL>(fa, wa, fb, wb, fc, wc, ww, p, Hw, guard);
     const bool g0 = guard[0], g1 = guard[1];
-    if (g0) push_recheck(q, slot, w0, ia, (uint32_t)(b0 + j0), (uint32_t)(c0 + k0));
-    if (g1) push_recheck(q, slot, w1, ia, (uint32_t)(b0 + j1), (uint32_t)(c0 + k1));
+    const uint32_t slot = S.unit.x & UNIT_SLOT_MASK;
+    if (g0) push_recheck(q, slot, w0, ia, (uint32_t)(S.b0 + j0), (uint32_t)(S.c0 + k0));
+    if (g1) push_recheck(q, slot, w1, ia, (uint32_t)(S.b0 + j1), (uint32_t)(S.c0 + k1));
 }
 
 // Side class for candidate filtering: 0 none (zero length or too long),
@@ -676,54 +1049,53 @@ __device__ __forceinline__ unsigned long long candidate_mask_jbj(int cij, unsign
 }
 
 template <int PRED, bool THETA_FULL, bool JBJ>
-__device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ gt, int nt, const TriParams& p,
-                                    float4* P, float* JKd, short* JKw, int2* IJ, int2* IK, uint32_t* Q,
-                                    unsigned long long* JM, float* BX, int4* s_meta, unsigned int* Hw,
-                                    RecheckQueue& q, unsigned long long& evaluated, unsigned long long& binned,
-                                    int* next_i, const float* abox) {
+__device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriParams& p, float4* P, float* JKd, short* JKw, int2* IJ,
+                                    int2* IK, uint32_t* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
+                                    RecheckQueue& q, unsigned long long& evaluated, unsigned long long& binned) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float4 *PB = P, *PC = P + TILE, *PA = P + 2 * TILE;
-    // every task of the group has the same job and tiles B and C
-    const uint4 t0 = gt[0];
-    const uint32_t slot = t0.x & TASK_SLOT_MASK;
-    const bool diag_jk = t0.x & TASK_DIAG_JK;
-    const int tb0 = J.tile_start[1][t0.z], numB = J.tile_start[1][t0.z + 1] - tb0;  // first point, points of B
-    const int tc0 = J.tile_start[2][t0.w], numC = J.tile_start[2][t0.w + 1] - tc0;  // ... of C
+    // every triple of the unit has the same job and tiles B and C
+    bool diag_jk;
+    int numB, numC;  // points of B and C
+    {
+        const DevJob& J = jobs[S.unit.x & UNIT_SLOT_MASK];
+        diag_jk = (J.mode & JOB_C_FROM_B) && S.unit.z == S.unit.w;
+        numB = J.tile_start[1][S.unit.z + 1] - J.tile_start[1][S.unit.z];
+        numC = J.tile_start[2][S.unit.w + 1] - J.tile_start[2][S.unit.w];
+    }
     // a side that provably reaches lmax is rejected whatever its exact value:
     // points farther than that from a whole tile take no part in the task
     // (the 1e-5 margin covers the rounding of the bound and of the distance)
     const float reach = p.lmax * (1.0f + 1e-5f);
     const float reach2 = reach * reach;
-    auto far_from = [&](float4 pt, int role) -> bool {
-        const float* bx = BX + role * 12;
-        float s2 = 0.f;
-        {
-            const float lo = fminf(bx[0], bx[6]), hi = fmaxf(bx[3], bx[9]);
-            const float gap = fmaxf(0.f, fmaxf(lo - pt.x, pt.x - hi));
-            s2 = fmaf(gap, gap, s2);
-        }
-        {
-            const float lo = fminf(bx[1], bx[7]), hi = fmaxf(bx[4], bx[10]);
-            const float gap = fmaxf(0.f, fmaxf(lo - pt.y, pt.y - hi));
-            s2 = fmaf(gap, gap, s2);
-        }
-        {
-            const float lo = fminf(bx[2], bx[8]), hi = fmaxf(bx[5], bx[11]);
-            const float gap = fmaxf(0.f, fmaxf(lo - pt.z, pt.z - hi));
-            s2 = fmaf(gap, gap, s2);
-        }
-        return s2 >= reach2;
+    auto far_from = [&](float4 pt, const float* bx) -> bool {
+        const float gx = fmaxf(0.f, fmaxf(bx[0] - pt.x, pt.x - bx[3]));
+        const float gy = fmaxf(0.f, fmaxf(bx[1] - pt.y, pt.y - bx[4]));
+        const float gz = fmaxf(0.f, fmaxf(bx[2] - pt.z, pt.z - bx[5]));
+        return fmaf(gz, gz, fmaf(gy, gy, gx * gx)) >= reach2;
     };
     int2* row_ij = IJ + warp * TILE;
     int2* row_ik = IK + warp * TILE;
     uint32_t* cand = Q + warp * TRI_QCAP;
     int key_k0 = 0, key_k1 = 0;
     unsigned ev = 0, bn = 0;
-    for (int ch = 0; ch < nt; ch += TRI_GROUP_A) {
-        const int nr = min(TRI_GROUP_A, nt - ch);
-        if (ch > 0) __syncthreads();  // the previous chunk's i loops are done with its A tiles
-        // tiles B and C (first chunk) and the chunk's A tiles; A tile r of
-        // the chunk at PA + r * TILE
+    // A tiles of the unit, up to TRI_GROUP_A at a time
+    for (int ch = 0; ch < __popc(S.mask); ch += TRI_GROUP_A) {
+        // (read again for every chunk: no registers held across the i loop)
+        const uint4 unit = S.unit;
+        const DevJob& J = jobs[unit.x & UNIT_SLOT_MASK];
+        const int tb0 = J.tile_start[1][unit.z], tc0 = J.tile_start[2][unit.w];
+        const int nr = min(TRI_GROUP_A, __popc(S.mask) - ch);
+        // points of each A tile the unit covers: all, or a quarter
+        const int ifrom = unit.x & UNIT_QUARTER ? (int)((unit.x >> UNIT_QUARTER_SHIFT) & 3u) * (TILE / 4) : 0;
+        const int ilen = unit.x & UNIT_QUARTER ? TILE / 4 : TILE;
+        auto tile_of = [&](int r) {  // the (ch + r)-th A tile of the mask
+            uint32_t m = S.mask;
+            for (int x = 0; x < ch + r; x++) m &= m - 1u;
+            return (int)unit.y + __ffs(m) - 1;
+        };
+        if (ch > 0) __syncthreads();  // the previous tiles' i loops are done
+        // tiles B and C (once) and the A tiles, tile r at PA + r * TILE
         for (int tt = (ch == 0 ? 0 : 2 * TILE) + threadIdx.x; tt < (2 + nr) * TILE; tt += blockDim.x) {
             const int idx = tt % TILE;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -732,55 +1104,71 @@ __device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ g
             } else if (tt < 2 * TILE) {
                 if (idx < numC) v = J.pts[2][tc0 + idx];
             } else {
-                const uint32_t at = gt[ch + tt / TILE - 2].y;
-                const int a0 = J.tile_start[0][at];
-                if (idx < J.tile_start[0][at + 1] - a0) v = J.pts[0][a0 + idx];
+                const int a = tile_of(tt / TILE - 2), a0 = J.tile_start[0][a] + ifrom;
+                if (idx < ilen && a0 + idx < J.tile_start[0][a + 1]) v = J.pts[0][a0 + idx];
             }
             P[tt] = v;
         }
         if (threadIdx.x < nr) {
-            const uint4 t = gt[ch + threadIdx.x];
-            const int a0 = J.tile_start[0][t.y];
-            s_meta[threadIdx.x] = make_int4(a0, J.tile_start[0][t.y + 1] - a0, (int)t.x, 0);
+            const int a = tile_of(threadIdx.x), a0 = J.tile_start[0][a];
+            const int n = min(ilen, J.tile_start[0][a + 1] - a0 - ifrom);
+            // only points of a tile that is not wholly within reach are tested one by one
+            const float4 al = J.box[0][2 * (size_t)a], ah = J.box[0][2 * (size_t)a + 1];
+            int f = (J.mode & JOB_B_FROM_A) && a == (int)unit.z ? TRI_DIAG_IJ : 0;
+            if (p.lmax < 3e38f) {
+                const float lmax2 = p.lmax * p.lmax;
+                if (box_bounds2(al, ah, J.box[1][2 * (size_t)unit.z], J.box[1][2 * (size_t)unit.z + 1]).y >= lmax2)
+                    f |= TRI_CHECK_B;
+                if (box_bounds2(al, ah, J.box[2][2 * (size_t)unit.w], J.box[2][2 * (size_t)unit.w + 1]).y >= lmax2)
+                    f |= TRI_CHECK_C;
+            }
+            S.meta[threadIdx.x] = make_int4(a0 + ifrom, n, f, ifrom);
+            if (threadIdx.x == nr - 1) S.end_i = (nr - 1) * TILE + max(n, 0);
         }
-        if (threadIdx.x == 0) *next_i = 0;
-        __syncthreads();
-        if (ch == 0) {
-            // bounding boxes of tiles B and C (two 32-point halves each), for
-            // the points of A out of reach of a whole tile
-            if (warp >= 2 && warp < 6) {
-                const int role = warp >> 1, idx = (warp & 1) * 32 + lane;
-                const int n = role == 1 ? numB : numC;
-                const float4 pt = P[(role - 1) * TILE + idx];
-                const bool valid = idx < n;
-                float lo[3] = {valid ? pt.x : INFINITY, valid ? pt.y : INFINITY, valid ? pt.z : INFINITY};
-                float hi[3] = {valid ? pt.x : -INFINITY, valid ? pt.y : -INFINITY, valid ? pt.z : -INFINITY};
+        if (ch == 0 && warp == 1) {  // boxes of tiles B, C and of all A tiles
+            if (lane < 12) {
+                const int role = lane < 6 ? 1 : 2, f = lane % 6;
+                const float4 v = J.box[role][2 * (size_t)(role == 1 ? unit.z : unit.w) + f / 3];
+                S.box[role - 1][f] = f % 3 == 0 ? v.x : (f % 3 == 1 ? v.y : v.z);
+            }
+            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+            if ((S.mask >> lane) & 1u) {
+                const float4 al = J.box[0][2 * (size_t)(unit.y + lane)], ah = J.box[0][2 * (size_t)(unit.y + lane) + 1];
+                lo[0] = al.x, lo[1] = al.y, lo[2] = al.z;
+                hi[0] = ah.x, hi[1] = ah.y, hi[2] = ah.z;
+            }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
+            for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-                        hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-                    }
-                if (lane == 0) {
+                for (int a = 0; a < 3; a++) {
+                    lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+                    hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+                }
+            if (lane == 0) {
 #pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        BX[warp * 6 + a] = lo[a];
-                        BX[warp * 6 + 3 + a] = hi[a];
-                    }
+                for (int a = 0; a < 3; a++) {
+                    S.abox[a] = lo[a];
+                    S.abox[3 + a] = hi[a];
                 }
             }
+        }
+        if (threadIdx.x == 0) {
+            S.next_i = 0;
+            S.b0 = tb0;
+            S.c0 = tc0;
+        }
+        __syncthreads();
+        if (ch == 0) {
             key_k0 = pkey(PC[lane]);
             key_k1 = pkey(PC[lane + 32]);
-            // rows j of the j-k side table and their class masks, one warp per row;
-            // abox: the box of every A tile of the group
+            // rows j of the j-k side table and their class masks, one warp per row
             for (int j = warp; j < numB; j += TRI_WARPS) {
                 const float4 pj = PB[j];
                 float a2 = 0.f;
 #pragma unroll
                 for (int a = 0; a < 3; a++) {
                     const float v = a == 0 ? pj.x : (a == 1 ? pj.y : pj.z);
-                    const float gap = fmaxf(0.f, fmaxf(abox[a] - v, v - abox[3 + a]));
+                    const float gap = fmaxf(0.f, fmaxf(S.abox[a] - v, v - S.abox[3 + a]));
                     a2 = fmaf(gap, gap, a2);
                 }
                 if (a2 >= reach2) {  // no i of the group reaches j: empty masks, the row is never read
@@ -819,16 +1207,17 @@ __device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ g
             // points of the chunk's A tiles are handed out to warps
             // dynamically (balances the very uneven work per point)
             int ii = 0;
-            if (lane == 0) ii = atomicAdd(next_i, 1);
+            if (lane == 0) ii = atomicAdd(&S.next_i, 1);
             ii = __shfl_sync(0xffffffffu, ii, 0);
-            if (ii >= nr * TILE) break;
-            const int4 meta = s_meta[ii / TILE];  // first point, points, task flags
+            if (ii >= S.end_i) break;
+            const int4 meta = S.meta[ii / TILE];
             const int i = ii % TILE;
             if (i >= meta.y) continue;
-            const bool diag_ij = meta.z & TASK_DIAG_IJ;
-            const bool chk_b = meta.z & TASK_CHECK_B, chk_c = meta.z & TASK_CHECK_C;
+            // in a diagonal tile pair j > i; else every j
+            const int j_after = meta.z & TRI_DIAG_IJ ? i + meta.w : -1;
             const float4 pi = PA[ii];
-            if ((chk_b && far_from(pi, 1)) || (chk_c && far_from(pi, 2))) continue;
+            if (((meta.z & TRI_CHECK_B) && far_from(pi, S.box[0])) || ((meta.z & TRI_CHECK_C) && far_from(pi, S.box[1])))
+                continue;
             const int ki = pkey(pi);
             // i-k sides: words for the binning path, class masks for the filter
             int c0 = 0, c1 = 0;
@@ -862,7 +1251,7 @@ __device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ g
                 int w = tri_side_word(d, p);
                 row_ij[j] = make_int2(__float_as_int(d), w);
                 const int c = side_class(w, d, p);
-                bool ok = c != 0 && any_k && (!diag_ij || j > i);
+                bool ok = c != 0 && any_k && j > j_after;
                 if (PRED == PRED_SAME) ok = ok && ki <= pkey(PB[j]);
                 if (!ok) return false;
                 cm = JBJ ? candidate_mask_jbj(c, nI, nM, nH, JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j])
@@ -928,7 +1317,7 @@ __device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ g
                     if (qn >= 64) {
                         __syncwarp();
                         qn -= 64;
-                        run_candidates<THETA_FULL, JBJ>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, slot, ia, tb0, tc0);
+                        run_candidates<THETA_FULL, JBJ>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
                         bn += 64;
                         __syncwarp();
                     }
@@ -936,7 +1325,7 @@ __device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ g
             }
             __syncwarp();
             if (qn > 0) {
-                run_candidates<THETA_FULL, JBJ>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, slot, ia, tb0, tc0);
+                run_candidates<THETA_FULL, JBJ>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
                 bn += qn;
             }
             __syncwarp();
@@ -950,34 +1339,26 @@ __device__ void triangle_group_fast(const DevJob& J, const uint4* __restrict__ g
     }
 }
 
-template <bool THETA_FULL, bool JBJ>
-__device__ __forceinline__ void triangle_dispatch(const DevJob& J, const uint4* gt, int nt, const TriParams& p,
-                                                  float4* P, float* JKd, short* JKw, int2* IJ, int2* IK, uint32_t* Q,
-                                                  unsigned long long* JM, float* BX, int4* s_meta, unsigned int* Hw,
-                                                  RecheckQueue& q, unsigned long long& ev, unsigned long long& bn,
-                                                  int* next_i, const float* abox) {
-#define TRI_GROUP_ARGS J, gt, nt, p, P, JKd, JKw, IJ, IK, Q, JM, BX, s_meta, Hw, q, ev, bn, next_i, abox
-    switch ((gt[0].x >> TASK_PRED_SHIFT) & TASK_PRED_MASK) {
-        case PRED_NONE: triangle_group_fast<PRED_NONE, THETA_FULL, JBJ>(TRI_GROUP_ARGS); break;
-        case PRED_DDR: triangle_group_fast<PRED_DDR, THETA_FULL, JBJ>(TRI_GROUP_ARGS); break;
-        case PRED_RDD: triangle_group_fast<PRED_RDD, THETA_FULL, JBJ>(TRI_GROUP_ARGS); break;
-        case PRED_SAME: triangle_group_fast<PRED_SAME, THETA_FULL, JBJ>(TRI_GROUP_ARGS); break;
-        default: triangle_group_fast<PRED_ONE, THETA_FULL, JBJ>(TRI_GROUP_ARGS); break;
+template <bool THETA_FULL, bool JBJ, typename... Args>
+__device__ __forceinline__ void triangle_dispatch(uint32_t pred, Args&&... args) {
+    switch (pred) {
+        case PRED_NONE: triangle_group_fast<PRED_NONE, THETA_FULL, JBJ>(args...); break;
+        case PRED_DDR: triangle_group_fast<PRED_DDR, THETA_FULL, JBJ>(args...); break;
+        case PRED_RDD: triangle_group_fast<PRED_RDD, THETA_FULL, JBJ>(args...); break;
+        case PRED_SAME: triangle_group_fast<PRED_SAME, THETA_FULL, JBJ>(args...); break;
+        default: triangle_group_fast<PRED_ONE, THETA_FULL, JBJ>(args...); break;
     }
-#undef TRI_GROUP_ARGS
 }
 
 #ifndef TRI_MIN_BLOCKS
 #define TRI_MIN_BLOCKS 4
 #endif
-// Persistent over groups of tasks: group g is tasks [groups[g], groups[g+1]),
-// which share the job, tile B and tile C; gbox[6 g ..] is the box (lo, hi) of
-// all their A tiles.
+// Persistent over the plan's units: tiles B and C of a job with a mask of A
+// tiles.
 template <bool THETA_FULL, bool JBJ>
 __global__ void __launch_bounds__(TRI_THREADS, TRI_MIN_BLOCKS)
-triangle_fast_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tasks, const uint32_t* __restrict__ groups,
-                     const float* __restrict__ gbox, unsigned int ngroups, unsigned int* group_counter, TriParams p,
-                     RecheckQueue q, int copies) {
+triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int* counter, TriParams p, RecheckQueue q,
+                     int copies) {
     extern __shared__ __align__(16) unsigned char smem[];
     float4* P = reinterpret_cast<float4*>(smem);
     unsigned long long* JM = reinterpret_cast<unsigned long long*>(P + (2 + TRI_GROUP_A) * TILE);
@@ -987,11 +1368,7 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ 
     uint32_t* Q = reinterpret_cast<uint32_t*>(JKd + TILE * TILE);
     short* JKw = reinterpret_cast<short*>(Q + TRI_WARPS * TRI_QCAP);
     unsigned int* H = reinterpret_cast<unsigned int*>(JKw + TILE * TILE);
-    __shared__ unsigned int s_group;
-    __shared__ int s_next_i;
-    __shared__ float s_box[6 * 6];  // tile bounding boxes: 6 half-tiles x {lo, hi}
-    __shared__ float s_abox[6];
-    __shared__ int4 s_meta[TRI_GROUP_A];  // A tiles of the chunk: first point, points, task flags
+    __shared__ TriShared S;
     for (int b = threadIdx.x; b < copies * p.len; b += blockDim.x) H[b] = 0;
     unsigned int* Hw = H + ((threadIdx.x >> 5) % copies) * p.len;
     int cur = -1;
@@ -1000,22 +1377,25 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ 
     if (threadIdx.x == 0) ev = bn = 0;
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) s_group = atomicAdd(group_counter, 1u);
+        if (threadIdx.x == 0) {
+            const unsigned int t = atomicAdd(counter, 1u);
+            const bool any = t < ul.n && ul.u0 + t < ul.header->nunits;
+            S.unit = any ? ul.units[ul.u0 + t] : make_uint4(TASK_NONE, 0, 0, 0);
+            S.mask = any ? ul.masks[ul.u0 + t] : 0u;
+        }
         __syncthreads();
-        const unsigned int gi = s_group;
-        if (gi >= ngroups) break;
-        if (threadIdx.x < 6) s_abox[threadIdx.x] = gbox[6 * (size_t)gi + threadIdx.x];
-        const uint32_t t0 = groups[gi], t1 = groups[gi + 1];
-        const int slot = (int)(tasks[t0].x & TASK_SLOT_MASK);
-        // (groups hold at most MAX_GROUP_TASKS <= FLUSH_EVERY tasks)
-        if ((slot != cur || since + (t1 - t0) > FLUSH_EVERY) && cur >= 0) {
+        if (S.unit.x == TASK_NONE) break;
+        const int slot = (int)(S.unit.x & UNIT_SLOT_MASK);
+        // (a unit holds at most MAX_WINDOW <= FLUSH_EVERY tile triples)
+        const unsigned int n = __popc(S.mask);
+        if ((slot != cur || since + n > FLUSH_EVERY) && cur >= 0) {
             flush_hist(H, copies, p.len, jobs[cur].hist);
             since = 0;
         }
         cur = slot;
-        since += t1 - t0;
-        triangle_dispatch<THETA_FULL, JBJ>(jobs[slot], tasks + t0, (int)(t1 - t0), p, P, JKd, JKw, IJ, IK, Q, JM,
-                                           s_box, s_meta, Hw, q, ev, bn, &s_next_i, s_abox);
+        since += n;
+        if (n == 0) continue;  // a part without A tiles
+        triangle_dispatch<THETA_FULL, JBJ>(jobs[slot].mode & JOB_PRED_MASK, jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
     }
     if (cur >= 0) flush_hist(H, copies, p.len, jobs[cur].hist);
     __syncthreads();
@@ -1031,7 +1411,7 @@ __global__ void triangle_recheck_kernel(const DevJob* __restrict__ jobs, Recheck
     if (n > q.cap) n = q.cap;
     for (unsigned int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         uint4 it = q.items[e];
-        const DevJob& J = jobs[it.x & TASK_SLOT_MASK];
+        const DevJob& J = jobs[it.x & UNIT_SLOT_MASK];
         unsigned w = it.x >> RECHECK_WEIGHT_SHIFT;
         float4 pa = J.pts[0][it.y], pb = J.pts[1][it.z], pc = J.pts[2][it.w];
         int out[3];
@@ -1099,12 +1479,12 @@ __device__ __forceinline__ typename SideReal<MODE>::type side_fp64(float4 a, flo
 }
 
 template <int PRED, int MODE>
-__device__ void triangle_task_fp64(const DevJob& J, uint4 task, const TriParams& p, const AcosTable& t,
+__device__ void triangle_task_fp64(const DevJob& J, uint4 task, int i0, int i1, const TriParams& p, const AcosTable& t,
                                    float4* P, int2* JK, int2* IJ, unsigned int* Hw) {
     typedef typename SideReal<MODE>::type R;  // at most 8 bytes: fits the int2 slots
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const TaskGeom g = task_geom(J, task);
-    const bool diag_ij = task.x & TASK_DIAG_IJ, diag_jk = task.x & TASK_DIAG_JK;
+    const bool diag_ij = (J.mode & JOB_B_FROM_A) && task.y == task.z, diag_jk = (J.mode & JOB_C_FROM_B) && task.z == task.w;
     R* jk = reinterpret_cast<R*>(JK);
     load_points(P, J, g);
     __syncthreads();
@@ -1114,7 +1494,7 @@ __device__ void triangle_task_fp64(const DevJob& J, uint4 task, const TriParams&
     }
     __syncthreads();
     R* row = reinterpret_cast<R*>(IJ + warp * TILE);
-    for (int i = warp; i < g.nA; i += TRI_WARPS) {
+    for (int i = i0 + warp; i < min(i1, g.nA); i += TRI_WARPS) {
         const float4 pi = P[i];
         R dik[2];
 #pragma unroll
@@ -1156,27 +1536,25 @@ __device__ void triangle_task_fp64(const DevJob& J, uint4 task, const TriParams&
 
 template <int MODE>
 __global__ void __launch_bounds__(TRI_THREADS, 1)
-triangle_fp64_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tasks, unsigned int ntasks,
-                     unsigned int* task_counter, TriParams p, AcosTable t, int copies) {
+triangle_fp64_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int* counter, TriParams p, AcosTable t,
+                     int copies) {
     extern __shared__ __align__(16) unsigned char smem[];
     float4* P = reinterpret_cast<float4*>(smem);
     int2* JK = reinterpret_cast<int2*>(smem + 3 * TILE * sizeof(float4));
     int2* IJ = JK + TILE * TILE;
     unsigned int* H = reinterpret_cast<unsigned int*>(IJ + TRI_WARPS * TILE);
     __shared__ uint4 s_task;
+    __shared__ int s_i0, s_i1;
     for (int b = threadIdx.x; b < copies * p.len; b += blockDim.x) H[b] = 0;
     unsigned int* Hw = H + ((threadIdx.x >> 5) % copies) * p.len;
     int cur = -1;
     unsigned int since = 0;
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int tt = atomicAdd(task_counter, 1u);
-            s_task = tt < ntasks ? tasks[tt] : make_uint4(TASK_NONE, 0, 0, 0);
-        }
+        if (threadIdx.x == 0) s_task = draw_unit(ul, counter, s_i0, s_i1);
         __syncthreads();
         const uint4 task = s_task;
-        const int slot = task.x == TASK_NONE ? -1 : (int)(task.x & TASK_SLOT_MASK);
+        const int slot = task.x == TASK_NONE ? -1 : (int)task.x;
         if ((slot != cur || since >= FLUSH_EVERY) && cur >= 0) {
             flush_hist(H, copies, p.len, jobs[cur].hist);
             since = 0;
@@ -1185,11 +1563,11 @@ triangle_fp64_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ 
         if (slot < 0) break;
         since++;
         const DevJob& J = jobs[slot];
-        switch ((task.x >> TASK_PRED_SHIFT) & TASK_PRED_MASK) {
-            case PRED_NONE: triangle_task_fp64<PRED_NONE, MODE>(J, task, p, t, P, JK, IJ, Hw); break;
-            case PRED_DDR: triangle_task_fp64<PRED_DDR, MODE>(J, task, p, t, P, JK, IJ, Hw); break;
-            case PRED_SAME: triangle_task_fp64<PRED_SAME, MODE>(J, task, p, t, P, JK, IJ, Hw); break;
-            default: triangle_task_fp64<PRED_ONE, MODE>(J, task, p, t, P, JK, IJ, Hw); break;
+        switch (J.mode & JOB_PRED_MASK) {
+            case PRED_NONE: triangle_task_fp64<PRED_NONE, MODE>(J, task, s_i0, s_i1, p, t, P, JK, IJ, Hw); break;
+            case PRED_DDR: triangle_task_fp64<PRED_DDR, MODE>(J, task, s_i0, s_i1, p, t, P, JK, IJ, Hw); break;
+            case PRED_SAME: triangle_task_fp64<PRED_SAME, MODE>(J, task, s_i0, s_i1, p, t, P, JK, IJ, Hw); break;
+            default: triangle_task_fp64<PRED_ONE, MODE>(J, task, s_i0, s_i1, p, t, P, JK, IJ, Hw); break;
         }
     }
 }
@@ -1399,7 +1777,7 @@ __device__ __forceinline__ bool far_from_box(const float* BX, float4 pt, int b, 
 // shared memory starts at 'base'; counts go to the shared copy Hw (swizzled)
 // or, with GLOBAL_HIST, straight to the job's 64-bit histogram.
 template <bool FP64, bool GLOBAL_HIST>
-__device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& p, const float* U,
+__device__ void three_side_task(const DevJob& J, uint4 task, int i0, int i1, const ThreeParams& p, const float* U,
                                 unsigned char* base, unsigned int* Hw, const TsPipe& pp) {
     float4* P = reinterpret_cast<float4*>(base);
     const bool byte_jk = ts_byte_jk(p);
@@ -1419,23 +1797,21 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
     // Symmetric tasks (one catalog in all three roles): tiles a <= b <= c and,
     // on diagonal tile pairs, positions i <= j <= k, so that every multiset
     // {i, j, k} is visited once and counted for all its orderings.
-    const bool sym = ((task.x >> TASK_PRED_SHIFT) & TASK_PRED_MASK) == PRED_SAME;
-    const bool diag_ij = task.x & TASK_DIAG_IJ, diag_jk = task.x & TASK_DIAG_JK;
+    const bool sym = (J.mode & JOB_PRED_MASK) == PRED_SAME;
+    const bool diag_ij = (J.mode & JOB_B_FROM_A) && task.y == task.z, diag_jk = (J.mode & JOB_C_FROM_B) && task.z == task.w;
+    i1 = min(i1, g.nA);  // the unit's points of tile A
     for (int t = pp.tid; t < 3 * TILE; t += TS_GROUP_THREADS) {
         const int role = t / TILE, idx = t % TILE;
         const int nr = role == 0 ? g.nA : (role == 1 ? g.nB : g.nC);
         const int b0 = role == 0 ? g.a0 : (role == 1 ? g.b0 : g.c0);
         P[t] = idx < nr ? J.pts[role][b0 + idx] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (pp.tid == 0) *next_i = 0;
+    if (pp.tid == 0) *next_i = i0;
     pp.sync();
     if (p.clean) {
         // Clean mode drops every triple with a side >= hist_max, so a point
         // farther than that from a whole tile takes no part in the task (the
         // 1e-5 margin covers the rounding of the bound and of the distance).
-        // (The planner flags tile pairs A-B and A-C that are not wholly within
-        // reach; B-C pairs are checked here on the half-tile boxes.)
-        const bool chk_b = task.x & TASK_CHECK_B, chk_c = task.x & TASK_CHECK_C;
         tile_boxes(P, g, BX, warp, lane);
         pp.sync();
         const float reach = p.hi * (1.0f + 1e-5f), reach2 = reach * reach;
@@ -1446,7 +1822,7 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
                 const int j = lane + 32 * r;
                 const float4 pj = P[TILE + j];
                 unsigned f = 0;
-                if (!chk_b || !far_from_box(BX, pj, 0, reach2) || !far_from_box(BX, pj, 1, reach2)) f |= 1u;
+                if (!far_from_box(BX, pj, 0, reach2) || !far_from_box(BX, pj, 1, reach2)) f |= 1u;
                 if (!far_from_box(BX, pj, 4, reach2)) f |= 2u;
                 if (!far_from_box(BX, pj, 5, reach2)) f |= 4u;
                 FJ[j] = (uint8_t)f;
@@ -1457,10 +1833,10 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
                 const int i = lane + 32 * r;
                 const float4 pi = P[i];
                 unsigned f = 0;
-                if (!chk_b || !far_from_box(BX, pi, 2, reach2)) f |= 1u;
-                if (!chk_b || !far_from_box(BX, pi, 3, reach2)) f |= 2u;
-                if (!chk_c || !far_from_box(BX, pi, 4, reach2)) f |= 4u;
-                if (!chk_c || !far_from_box(BX, pi, 5, reach2)) f |= 8u;
+                if (!far_from_box(BX, pi, 2, reach2)) f |= 1u;
+                if (!far_from_box(BX, pi, 3, reach2)) f |= 2u;
+                if (!far_from_box(BX, pi, 4, reach2)) f |= 4u;
+                if (!far_from_box(BX, pi, 5, reach2)) f |= 8u;
                 FI[i] = (uint8_t)f;
             }
         }
@@ -1521,7 +1897,7 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
             i = 0;
             if (lane == 0) i = atomicAdd(next_i, 1);
             i = __shfl_sync(0xffffffffu, i, 0);
-            if (i >= g.nA) break;
+            if (i >= i1) break;
             const float4 pi = P[i];
             const unsigned fi = FI[i];
             if (!(fi & 3u) || !(fi & 12u)) continue;  // out of reach of tile B or tile C (warp-uniform)
@@ -1583,7 +1959,7 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
         }
         pp.sync();
         uint32_t* row = ROWS + warp * TS_ROW;
-        for (int i = warp; i < g.nA; i += TS_WARPS) {
+        for (int i = i0 + warp; i < i1; i += TS_WARPS) {
             const float4 pi = P[i];
             uint32_t vik[2];
 #pragma unroll
@@ -1631,7 +2007,7 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
     }
     pp.sync();
     uint32_t* row = ROWS + warp * TS_ROW;
-    for (int i = warp; i < g.nA; i += TS_WARPS) {
+    for (int i = i0 + warp; i < i1; i += TS_WARPS) {
         const float4 pi = P[i];
         uint32_t cik[2];
 #pragma unroll
@@ -1666,11 +2042,11 @@ __device__ void three_side_task(const DevJob& J, uint4 task, const ThreeParams& 
 // > 0) or the global histogram.
 template <bool FP64, bool GLOBAL_HIST>
 __global__ void __launch_bounds__(TS_GROUP_THREADS, 4)
-three_side_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tasks, unsigned int ntasks,
-                  unsigned int* task_counter, ThreeParams p, int copies) {
+three_side_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int* counter, ThreeParams p, int copies) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned int* H = reinterpret_cast<unsigned int*>(smem + ts_layout(ts_byte_jk(p)).bytes);
     __shared__ uint4 s_task;
+    __shared__ int s_i0, s_i1;
     __shared__ float s_u[TS_UMAX];
     for (int v = threadIdx.x; v < TS_UMAX; v += blockDim.x) s_u[v] = p.u[v];
     const int stride = hist_stride(ts_acc_words(p));
@@ -1683,22 +2059,19 @@ three_side_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tas
     unsigned int since = 0;
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int t = atomicAdd(task_counter, 1u);
-            s_task = t < ntasks ? tasks[t] : make_uint4(TASK_NONE, 0, 0, 0);
-        }
+        if (threadIdx.x == 0) s_task = draw_unit(ul, counter, s_i0, s_i1);
         __syncthreads();
         const uint4 task = s_task;
-        const int slot = task.x == TASK_NONE ? -1 : (int)(task.x & TASK_SLOT_MASK);
+        const int slot = task.x == TASK_NONE ? -1 : (int)task.x;
         if (!GLOBAL_HIST && (slot != cur || since >= TS_FLUSH_EVERY) && cur >= 0) {
             ts_flush(H, copies, p, jobs[cur].hist, cur_sym);
             since = 0;
         }
         cur = slot;
-        cur_sym = ((task.x >> TASK_PRED_SHIFT) & TASK_PRED_MASK) == PRED_SAME;
         if (slot < 0) break;
+        cur_sym = (jobs[slot].mode & JOB_PRED_MASK) == PRED_SAME;
         since++;
-        three_side_task<FP64, GLOBAL_HIST>(jobs[slot], task, p, s_u, smem, Hw, pp);
+        three_side_task<FP64, GLOBAL_HIST>(jobs[slot], task, s_i0, s_i1, p, s_u, smem, Hw, pp);
     }
 }
 
@@ -1713,12 +2086,13 @@ three_side_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tas
 // two flushes, each at most 2^18 per bin, so the 32-bit counters cannot wrap.
 template <bool FP64>
 __global__ void __launch_bounds__(TS_GROUPS_MAX * TS_GROUP_THREADS, 1)
-three_side_grouped_kernel(const DevJob* __restrict__ jobs, const uint4* __restrict__ tasks, unsigned int ntasks,
-                          unsigned int* task_counter, ThreeParams p, int groups) {
+three_side_grouped_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int* counter, ThreeParams p,
+                          int groups) {
     extern __shared__ __align__(16) unsigned char smem[];
     const size_t pipe_bytes = ts_layout(ts_byte_jk(p)).bytes;
     unsigned int* H = reinterpret_cast<unsigned int*>(smem + (size_t)groups * pipe_bytes);
     __shared__ uint4 s_task[TS_GROUPS_MAX];
+    __shared__ int2 s_i[TS_GROUPS_MAX];  // its points of tile A
     __shared__ unsigned int s_stop[TS_GROUPS_MAX];  // the pipeline leaves the job to flush
     __shared__ unsigned int s_since;                // tasks run since the last flush
     __shared__ float s_u[TS_UMAX];
@@ -1729,10 +2103,7 @@ three_side_grouped_kernel(const DevJob* __restrict__ jobs, const uint4* __restri
     for (int b = threadIdx.x; b < hist_stride(ts_acc_words(p)); b += blockDim.x) H[b] = 0;
     if (threadIdx.x == 0) s_since = 0;
     auto draw = [&]() {
-        if (gt == 0) {
-            unsigned int t = atomicAdd(task_counter, 1u);
-            s_task[gi] = t < ntasks ? tasks[t] : make_uint4(TASK_NONE, 0, 0, 0);
-        }
+        if (gt == 0) s_task[gi] = draw_unit(ul, counter, s_i[gi].x, s_i[gi].y);
     };
     draw();
     int cur = -1;
@@ -1743,14 +2114,10 @@ three_side_grouped_kernel(const DevJob* __restrict__ jobs, const uint4* __restri
         uint32_t next = TASK_NONE;
         for (int g2 = 0; g2 < groups; g2++) {
             const uint32_t x = s_task[g2].x;
-            if (x != TASK_NONE) next = min(next, x & TASK_SLOT_MASK);
+            if (x != TASK_NONE) next = min(next, x);
         }
         if (next == TASK_NONE) break;  // uniform: every thread read the same words
-        for (int g2 = 0; g2 < groups; g2++) {  // all tasks of a job are alike
-            const uint32_t x = s_task[g2].x;
-            if (x != TASK_NONE && (x & TASK_SLOT_MASK) == next)
-                cur_sym = ((x >> TASK_PRED_SHIFT) & TASK_PRED_MASK) == PRED_SAME;
-        }
+        cur_sym = (jobs[next].mode & JOB_PRED_MASK) == PRED_SAME;
         if (threadIdx.x < TS_GROUPS_MAX) s_stop[threadIdx.x] = 0;
         if (threadIdx.x == 0) s_since = 0;
         __syncthreads();
@@ -1758,8 +2125,8 @@ three_side_grouped_kernel(const DevJob* __restrict__ jobs, const uint4* __restri
         for (;;) {
             // s_task[gi] and s_stop[gi] change only between this pipeline's barriers
             const uint4 task = s_task[gi];
-            if (task.x == TASK_NONE || (int)(task.x & TASK_SLOT_MASK) != cur || s_stop[gi]) break;
-            three_side_task<FP64, false>(jobs[cur], task, p, s_u, base, H, pp);
+            if (task.x == TASK_NONE || (int)task.x != cur || s_stop[gi]) break;
+            three_side_task<FP64, false>(jobs[cur], task, s_i[gi].x, s_i[gi].y, p, s_u, base, H, pp);
             pp.sync();  // the pipeline is done with s_task[gi] and its buffers
             if (gt == 0) s_stop[gi] = atomicAdd(&s_since, 1u) + 1 >= TS_FLUSH_EVERY;
             draw();
@@ -1876,21 +2243,6 @@ __device__ __forceinline__ void pair_share(int n, int nA, F&& f) {
         const int i0 = (u % split) * len;
         if (i0 < nA) f(u / split, i0, min(i0 + len, nA));
     }
-}
-
-// Last job j of [0, n) with off[j] <= t (off[0] <= t; a job without items is
-// never the last one), searched 32 ways at a time by a whole warp.
-__device__ __forceinline__ int find_job(const uint32_t* __restrict__ off, int n, uint32_t t) {
-    const int lane = threadIdx.x & 31;
-    int lo = 0, len = n;
-    while (len > 1) {
-        const int step = (len + 31) / 32;
-        const bool le = lane * step < len && off[lo + lane * step] <= t;
-        const int k = 31 - __clz(__ballot_sync(0xffffffffu, le) | 1u);
-        lo += k * step;
-        len = min(step, len - k * step);
-    }
-    return lo;
 }
 
 // Squared gap of two tile boxes (reduced by a margin that covers the rounding
@@ -2074,19 +2426,12 @@ cudaError_t prepare_kernels(int device) {
     return cudaSuccess;
 }
 
-cudaError_t launch_triangle_fast(const DevJob* jobs, const uint4* tasks, const uint32_t* groups, const float* gbox,
-                                 unsigned int ngroups, unsigned int* group_counter, const TriParams& p, RecheckQueue q,
-                                 int grid, int copies, int jbj, cudaStream_t st) {
+cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
+                                 RecheckQueue q, int grid, int copies, int jbj, cudaStream_t st) {
     size_t smem = triangle_smem_bytes(p.len, copies);
-    if (jbj)
-        triangle_fast_kernel<false, true><<<grid, TRI_THREADS, smem, st>>>(jobs, tasks, groups, gbox, ngroups,
-                                                                           group_counter, p, q, copies);
-    else if (p.theta_full)
-        triangle_fast_kernel<true, false><<<grid, TRI_THREADS, smem, st>>>(jobs, tasks, groups, gbox, ngroups,
-                                                                           group_counter, p, q, copies);
-    else
-        triangle_fast_kernel<false, false><<<grid, TRI_THREADS, smem, st>>>(jobs, tasks, groups, gbox, ngroups,
-                                                                            group_counter, p, q, copies);
+    if (jbj) triangle_fast_kernel<false, true><<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
+    else if (p.theta_full) triangle_fast_kernel<true, false><<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
+    else triangle_fast_kernel<false, false><<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
     return cudaGetLastError();
 }
 
@@ -2096,34 +2441,32 @@ cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const Tr
     return cudaGetLastError();
 }
 
-cudaError_t launch_triangle_fp64(const DevJob* jobs, const uint4* tasks, unsigned int ntasks,
-                                 unsigned int* task_counter, const TriParams& p, AcosTable t, int grid, int copies,
-                                 int mode, cudaStream_t st) {
+cudaError_t launch_triangle_fp64(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
+                                 AcosTable t, int grid, int copies, int mode, cudaStream_t st) {
     size_t smem = triangle_smem_bytes(p.len, copies);
     auto kern = mode == MODE_GEOM ? triangle_fp64_kernel<MODE_GEOM>
                 : mode == MODE_JBJ  ? triangle_fp64_kernel<MODE_JBJ>
                                     : triangle_fp64_kernel<MODE_FP64>;
-    kern<<<grid, TRI_THREADS, smem, st>>>(jobs, tasks, ntasks, task_counter, p, t, copies);
+    kern<<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, t, copies);
     return cudaGetLastError();
 }
 
-cudaError_t launch_three_side(const DevJob* jobs, const uint4* tasks, unsigned int ntasks,
-                              unsigned int* task_counter, const ThreeParams& p, int fp64, int grid, int copies,
-                              int groups, cudaStream_t st) {
+cudaError_t launch_three_side(const DevJob* jobs, UnitList ul, unsigned int* counter, const ThreeParams& p, int fp64,
+                              int grid, int copies, int groups, cudaStream_t st) {
     if (groups > 0) {
         if (groups > TS_GROUPS_MAX) return cudaErrorInvalidValue;
         const size_t smem = three_side_smem_bytes(p, 1, groups);
         const int threads = groups * TS_GROUP_THREADS;
         if (fp64)
-            three_side_grouped_kernel<true><<<grid, threads, smem, st>>>(jobs, tasks, ntasks, task_counter, p, groups);
+            three_side_grouped_kernel<true><<<grid, threads, smem, st>>>(jobs, ul, counter, p, groups);
         else
-            three_side_grouped_kernel<false><<<grid, threads, smem, st>>>(jobs, tasks, ntasks, task_counter, p, groups);
+            three_side_grouped_kernel<false><<<grid, threads, smem, st>>>(jobs, ul, counter, p, groups);
         return cudaGetLastError();
     }
     const bool global = copies == 0;
     const size_t smem = three_side_smem_bytes(p, global ? 0 : copies, 0);
 #define TS_LAUNCH(FP, GL) \
-    three_side_kernel<FP, GL><<<grid, TS_GROUP_THREADS, smem, st>>>(jobs, tasks, ntasks, task_counter, p, copies > 0 ? copies : 1);
+    three_side_kernel<FP, GL><<<grid, TS_GROUP_THREADS, smem, st>>>(jobs, ul, counter, p, copies > 0 ? copies : 1);
     if (fp64) {
         if (global) { TS_LAUNCH(true, true) } else { TS_LAUNCH(true, false) }
     } else {
