@@ -217,6 +217,7 @@ struct Box {
 struct Catalog {
     std::vector<float> x, y, z;
     int64_t n = 0;
+    bool tame = true;  // every coordinate a number of magnitude at most 1e15
 };
 
 struct View {
@@ -445,7 +446,13 @@ struct Binning {
 // Whether a job of this spec runs in the guarded FP32 kernels.  The fast
 // triangle kernel keeps side words of 16 bits (s-bin below 255): binnings with
 // more s bins are counted by the plain FP64 kernel, with the same histograms.
-bool guarded_fp32(const tpcf_spec& sp, const Binning& bin) {
+// The double-precision geometry takes the fast kernel where float sides and the
+// guard bands tell its bins: coordinates of ordinary size (`tame`), a lower edge
+// that a float separation cannot miss, bands well inside the bins.
+bool guarded_fp32(const tpcf_spec& sp, const Binning& bin, bool tame) {
+    if (sp.precision == TPCF_GEOMETRY_FP64)
+        return tame && bin.tri.S <= MAX_FAST_S && (bin.tri.s_lo <= 0 || bin.tri.s_lo >= 1e-12f) &&
+               bin.tri.geo_s_thr > 0.25f && bin.tri.q_thr > 0.25f && bin.tri.t_thrA > 0.25f;
     if (sp.precision != TPCF_GUARDED_FP32) return false;
     if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) return bin.tri.S <= MAX_FAST_S;
     return true;
@@ -566,6 +573,19 @@ Binning make_binning(const tpcf_spec& sp) {
         p.t_thrB = (float)(5e-7 * K);
         p.t2_off = (float)((1.0 - 3.0 * (double)p.t_lo) / (double)p.t_bw - 1.5);
         p.theta_full = (p.t_lo <= 0.f && p.t_hi >= 1.f);
+        if (sp.precision == TPCF_GEOMETRY_FP64) {
+            // the guard bands of the geometry (triangle_full2): relative errors of
+            // 4e-7 of a side, 3e-6 of a ratio, and of the coordinates themselves
+            p.geo_s_below = p.s_lo > 0 ? (float)std::max(1e-15, (double)p.s_lo * (1 - 1e-6)) : -1.f;
+            p.geo_s_above = (float)((double)p.s_hi * (p.s_hi > 0 ? 1 + 1e-6 : 1 - 1e-6));
+            const double smax = std::max(fabs((double)p.s_lo), fabs((double)p.s_hi)) / (double)p.s_bw;
+            p.geo_s_inv = (float)(1.0 / (double)p.s_bw);
+            p.geo_s_off = (float)(-(double)p.s_lo / (double)p.s_bw - 0.5);
+            p.geo_s_thr = (float)(0.5 - (2e-6 * smax + 1e-5));
+            p.q_thr = (float)(0.5 - (3e-6 * qmax * qs + 1e-5));
+            p.t_thrA = (float)(0.5 - (4e-6 * K + 2e-6 * tmax + 1e-5));
+            p.geo_t = (float)(6e-6 * K);
+        }
         b.len = p.len;
         // every counted permutation needs shortest or middle side < s_hi and a
         // ratio < q_hi; all sides are then below s_hi (1 + q_hi)
@@ -626,13 +646,6 @@ Binning make_binning(const tpcf_spec& sp) {
         b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
         double mid = (double)b.tri.s_hi * (double)b.tri.q_hi * (1 + 1e-5) + 1e-6;
         b.tri.mid_hi = sp.prune && b.tri.q_hi > 0 ? nextafterf((float)mid, INFINITY) : INFINITY;
-        // a permutation whose side ratio is at least q_rej (computed as a float
-        // product with the shorter side) lies past q_hi by more than 1e-4 of
-        // the q range, which no rounding of the reference's q = l/s and
-        // (q - q_lo)/q_bw brings back into the last bin
-        const double qr = (double)b.tri.q_hi + 1e-4 * ((double)b.tri.q_hi - (double)b.tri.q_lo) +
-                          1e-5 * fabs((double)b.tri.q_hi);
-        b.tri.q_rej = sp.prune ? nextafterf((float)qr, INFINITY) : INFINITY;
     }
     return b;
 }
@@ -1235,10 +1248,20 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     Binning bin = make_binning(sp);
     const int ncat = sp.kind == TPCF_PAIR ? 2 : 3;
     const bool pairs = sp.kind == TPCF_PAIR;
-    const bool fp64 = !guarded_fp32(sp, bin);
+    bool tame = true;  // (asked by the double-precision geometry only)
+    if (sp.precision == TPCF_GEOMETRY_FP64) {
+        std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
+        for (const GroupJob& g : group)
+            for (int r = 0; r < ncat; r++) {
+                auto it = ctx->catalogs.find(g.job->catalog[r]);
+                if (it != ctx->catalogs.end()) tame = tame && it->second->tame;
+            }
+    }
+    const bool fp64 = !guarded_fp32(sp, bin, tame);
     const bool tri_kind = sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ;
     const bool fast_tri = tri_kind && !fp64;
     const bool fast_jbj = sp.kind == TPCF_TRIANGLE_JBJ && !fp64;  // the fast kernel's JBJ binning
+    const bool geom = sp.precision == TPCF_GEOMETRY_FP64;
     if (group.size() > MAX_BATCH_JOBS) throw InvalidArg{"too many jobs in one batch"};
     std::vector<std::pair<const char*, double>> phases;
     auto phase = [&](const char* name) {
@@ -1548,11 +1571,12 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                     unsigned int* counter = L.d_counters.p + CTR_WORK;
                     const UnitList ul{d_header, L.d_units.p, L.d_masks.p, t0, n};
                     if (fast_tri)  // (JBJ: exact without a recheck)
-                        return launch_triangle_fast(L.d_jobs.p, ul, counter, bin.tri, q, grid, copies, fast_jbj ? 1 : 0, st);
+                        return launch_triangle_fast(L.d_jobs.p, ul, counter, bin.tri, q, grid, copies,
+                                                    fast_jbj ? 1 : geom ? 2 : 0, st);
                     if (tri_kind)
                         return launch_triangle_fp64(L.d_jobs.p, ul, counter, bin.tri, acos_t, grid, copies,
                                                     sp.kind == TPCF_TRIANGLE_JBJ ? 2
-                                                    : sp.precision == TPCF_GEOMETRY_FP64 ? 1 : 0, st);
+                                                    : geom ? 1 : 0, st);
                     if (sp.kind == TPCF_THREE_SIDE)
                         return launch_three_side(L.d_jobs.p, ul, counter, bin.three, fp64, grid, copies, sh.groups, st);
                     return launch_pairs(L.d_jobs.p, L.d_rows.p, (int)group.size(), t0, n, plan_chunk, counter,
@@ -1569,7 +1593,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                 }
                 EQ(cudaEventRecordWithFlags(L.ev_mid, st, ev_flags));
                 if (sp.kind == TPCF_TRIANGLE && !fp64)
-                    EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, ctx->num_sms * 8, st));
+                    EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, geom ? 1 : 0, ctx->num_sms * 8, st));
                 EQ(cudaEventRecordWithFlags(L.ev1, st, ev_flags));
                 EQ(cudaMemcpyAsync(L.h_counters.p, L.d_counters.p, CTR_WORDS * sizeof(unsigned int),
                                    cudaMemcpyDeviceToHost, st));
@@ -2096,6 +2120,11 @@ tpcf_status tpcf_catalog_create(tpcf_ctx* ctx, const float* x, const float* y, c
         c->x.assign(x, x + n);
         c->y.assign(y, y + n);
         c->z.assign(z, z + n);
+        for (const std::vector<float>* v : {&c->x, &c->y, &c->z}) {
+            bool ok = true;
+            for (float f : *v) ok &= fabsf(f) <= 1e15f;
+            c->tame = c->tame && ok;
+        }
         std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
         uint64_t h = ctx->next_handle++;
         ctx->catalogs[h] = c;

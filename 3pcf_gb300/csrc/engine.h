@@ -99,7 +99,9 @@ struct TriParams {
     float lmax;                  // sides >= lmax cannot belong to a counted triangle
     float mid_hi;                // s_hi * q_hi (rounded up): permutation 0 needs two sides below it,
                                  // permutation 1 needs all three below it
-    float q_rej;                 // a side ratio at or above it is out of the q range whatever the rounding
+    // double-precision geometry: sides that are surely below s_lo / at or above
+    // s_hi, the s coordinate (minus 0.5) and its guard, slope of the angle's
+    float geo_s_below, geo_s_above, geo_s_inv, geo_s_off, geo_s_thr, geo_t;
 };
 
 constexpr int TS_UMAX = 68;  // squared-length thresholds of up to 64 bins
@@ -178,7 +180,8 @@ cudaError_t launch_plan(const DevJob* jobs, const uint32_t* row_off, int njobs, 
 
 // ---- kernel launchers (kernels.cu) ----
 cudaError_t prepare_kernels(int device);  // once per device before any launch
-// The counting kernels take units [u0, u0 + n) of a plan; jbj: JBJ binning
+// The counting kernels take units [u0, u0 + n) of a plan; the fast triangle
+// kernel's mode: 0 reference, 1 JBJ, 2 double-precision geometry
 struct UnitList {
     const PlanHeader* header;
     const uint4* units;
@@ -186,9 +189,9 @@ struct UnitList {
     uint32_t u0, n;
 };
 cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
-                                 RecheckQueue q, int grid, int hist_copies, int jbj, cudaStream_t st);
+                                 RecheckQueue q, int grid, int hist_copies, int mode, cudaStream_t st);
 cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t,
-                                    int grid, cudaStream_t st);
+                                    int geom, int grid, cudaStream_t st);
 cudaError_t launch_triangle_fp64(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
                                  AcosTable t, int grid, int hist_copies, int mode,
                                  cudaStream_t st);  // mode: 0 FP64, 1 geometry, 2 JBJ

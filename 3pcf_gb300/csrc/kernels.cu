@@ -629,6 +629,12 @@ cudaError_t launch_plan(const DevJob* jobs, const uint32_t* row_off, int njobs, 
 // ---------------------------------------------------------------------------
 // Triangle parametrization, guarded FP32.
 
+// What the fast triangle kernel bins: the reference's triangle
+// parametrization, JBJ, or the triangle parametrization of the double-precision
+// geometry (same histogram as evaluating tp_geom for every triangle: only what
+// lies in wider guard bands is).
+enum FastMode : int { FAST_TP = 0, FAST_JBJ = 1, FAST_GEOM = 2 };
+
 constexpr int TRI_WARPS = 8;
 constexpr int TRI_THREADS = TRI_WARPS * 32;
 constexpr int TRI_QCAP = 128;  // per-warp candidate queue: up to 63 pending + 64 new
@@ -676,8 +682,19 @@ __device__ __forceinline__ int tri_side_code(float d, const TriParams& p) {
 // (A division-free s-bin -- a guess corrected against exact thresholds
 // staged in shared memory -- measured slower: 14.19 vs 13.95 ms on the
 // default workload.)
+template <int MODE>
 __device__ __forceinline__ int tri_side_word(float d, const TriParams& p) {
     int code, w;
+    if (MODE == FAST_GEOM) {
+        // a side whose double length may fall on the other side of s_lo or
+        // s_hi counts as in range (the class that rejects least); the guard
+        // band of its s coordinate sends its triangles to the recheck.  A zero
+        // side is no reason to reject: its double length may not be zero.
+        if (d < p.geo_s_below) return CODE16_BELOW * 128 + (d >= p.lmax ? CW_REJECT : CW_BELOW);
+        if (d >= p.geo_s_above) return CODE16_ABOVE * 128 + (d >= p.lmax ? CW_REJECT : CW_ABOVE);
+        code = __float2int_rz(__fdiv_rn(__fsub_rn(d, p.s_lo), p.s_bw));
+        return min(max(code, 0), p.S - 1) * 128 + CW_IN;
+    }
     if (d == 0.f) {
         code = CODE16_ZERO;
         w = CW_REJECT;
@@ -713,24 +730,6 @@ __device__ __forceinline__ GuardedBin magic_floor(float f_m) {
     g.bin = __float_as_int(tm) - MAGIC_BITS;
     g.err = __fsub_rn(f_m, dd);
     return g;
-}
-
-// theta coordinate of a cosine (approximate) and its guard threshold
-__device__ __forceinline__ void theta_fast(float c, const TriParams& p, float& f_m, float& thr) {
-    float x = fabsf(c);
-    float t = __fsub_rn(1.0f, x);
-    float y = rsqrt_approx(t);
-    float sq = __fmul_rn(t, y);
-    float P = p.t_coef[5];
-    P = __fmaf_rn(P, x, p.t_coef[4]);
-    P = __fmaf_rn(P, x, p.t_coef[3]);
-    P = __fmaf_rn(P, x, p.t_coef[2]);
-    P = __fmaf_rn(P, x, p.t_coef[1]);
-    P = __fmaf_rn(P, x, p.t_coef[0]);
-    float a = __fmaf_rn(sq, P, -p.t_half);                                     // K*acos(|c|) - K*pi/2
-    a = __int_as_float(__float_as_int(a) ^ (__float_as_int(c) & 0x80000000));  // acos(-x) = pi - acos(x)
-    f_m = __fadd_rn(a, p.t_off0);
-    thr = __fmaf_rn(-p.t_thrB, y, p.t_thrA);
 }
 
 __device__ __forceinline__ unsigned weight_index(int wa, int wb, int wc) { return (unsigned)(wa + wb + wc) & 127u; }
@@ -784,15 +783,15 @@ __device__ __forceinline__ void magic_floor2(f32x2 f_m, int& b0, int& b1, float&
     b1 = __float_as_int(t1) - MAGIC_BITS;
 }
 
-// theta_fast of two cosines
-__device__ __forceinline__ void theta_fast2(f32x2 c, const TriParams& p, f32x2& f_m, f32x2& thr) {
+// theta_fast of two cosines; t: 1 - |c|, y: its reciprocal square root
+__device__ __forceinline__ void theta_fast2(f32x2 c, const TriParams& p, f32x2& f_m, f32x2& thr, f32x2& t, f32x2& y) {
     float c0, c1;
     up2(c, c0, c1);
     const f32x2 x = pk2(fabsf(c0), fabsf(c1));
-    const f32x2 t = sub2(splat2(1.0f), x);
+    t = sub2(splat2(1.0f), x);
     float t0, t1;
     up2(t, t0, t1);
-    const f32x2 y = pk2(rsqrt_approx(t0), rsqrt_approx(t1));
+    y = pk2(rsqrt_approx(t0), rsqrt_approx(t1));
     const f32x2 sq = mul2(t, y);
     f32x2 P = splat2(p.t_coef[5]);
     P = fma2(P, x, splat2(p.t_coef[4]));
@@ -814,7 +813,18 @@ __device__ __forceinline__ void theta_fast2(f32x2 c, const TriParams& p, f32x2& 
 // weight index says some permutation may count is binned into Hw, unless a
 // permutation that could count has a coordinate inside its guard band: then
 // guard[t] is set and the triangle must be recomputed exactly.
-template <bool THETA_FULL>
+//
+// GEOM: the double-precision geometry is approximated instead of the
+// reference's floats.  With u = 2^-24 a float side is within 3.5 u of its double
+// length, so a ratio is within 11 u (twice that where two sides within rounding
+// change places), and a cosine within 4e-6 E, E = (s^2 + m^2 + l^2) / (2 s m) the
+// amplification of its cancelling numerator (12 u E for the sides and
+// roundings, doubled for changed places, and a margin).  An angle moves by at
+// most 1.42 dc / sqrt(1 - |c|), and a cosine within 2 dc of +-1 is always
+// recomputed.  (Every triangle in double is bound by the FP64 pipe, two lanes a
+// clock and SM: DDD+DDR+DRR+RRR of 1k points 251 ms; so 0.65 ms, 0.2 % of the
+// binned triangles recomputed.)
+template <bool THETA_FULL, bool GEOM>
 __device__ __forceinline__ void triangle_full2(const float (&a)[2], const int (&wa)[2], const float (&b)[2],
                                                const int (&wb)[2], const float (&c)[2], const int (&wc)[2],
                                                const unsigned (&w)[2], const TriParams& p, unsigned int* Hw,
@@ -860,9 +870,34 @@ __device__ __forceinline__ void triangle_full2(const float (&a)[2], const int (&
     const f32x2 half = splat2(0.5f);
     const f32x2 c0 = mul2(mul2(num0, pk2(rcp_approx(sm0), rcp_approx(sm1))), half);
     const f32x2 c1 = mul2(mul2(num1, pk2(rcp_approx(ml0), rcp_approx(ml1))), half);
-    f32x2 f0m, thr0, f1m, thr1;
-    theta_fast2(c0, p, f0m, thr0);
-    theta_fast2(c1, p, f1m, thr1);
+    f32x2 f0m, thr0, f1m, thr1, tc0, tc1, y0, y1;
+    theta_fast2(c0, p, f0m, thr0, tc0, y0);
+    theta_fast2(c1, p, f1m, thr1, tc1, y1);
+    bool gs[2] = {false, false}, gm[2] = {false, false};
+    if (GEOM) {
+        const f32x2 sum2 = add2(add2(S2, M2), L2);
+        const f32x2 E0 = mul2(mul2(sum2, pk2(rcp_approx(sm0), rcp_approx(sm1))), half);
+        const f32x2 E1 = mul2(mul2(sum2, pk2(rcp_approx(ml0), rcp_approx(ml1))), half);
+        float e0[2], e1[2], t0[2], t1[2], h0[2], h1[2], x0[2], x1[2], sv[2], mv[2];
+        up2(E0, e0[0], e0[1]);
+        up2(E1, e1[0], e1[1]);
+        up2(tc0, t0[0], t0[1]);
+        up2(tc1, t1[0], t1[1]);
+        up2(fma2(splat2(-p.geo_t), mul2(E0, y0), splat2(p.t_thrA)), h0[0], h0[1]);
+        up2(fma2(splat2(-p.geo_t), mul2(E1, y1), splat2(p.t_thrA)), h1[0], h1[1]);
+        int b0, b1;
+        magic_floor2(fma2(S, splat2(p.geo_s_inv), splat2(p.geo_s_off)), b0, b1, sv[0], sv[1]);
+        magic_floor2(fma2(M, splat2(p.geo_s_inv), splat2(p.geo_s_off)), b0, b1, mv[0], mv[1]);
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            x0[t] = t0[t] > 8e-6f * e0[t] ? h0[t] : -1.f;
+            x1[t] = t1[t] > 8e-6f * e1[t] ? h1[t] : -1.f;
+            gs[t] = !(fabsf(sv[t]) <= p.geo_s_thr);
+            gm[t] = !(fabsf(mv[t]) <= p.geo_s_thr);
+        }
+        thr0 = pk2(x0[0], x0[1]);
+        thr1 = pk2(x1[0], x1[1]);
+    }
     const f32x2 f2m = sub2(sub2(splat2(p.t2_off), f0m), f1m);
     float thr0v[2], thr1v[2], thr2v[2];
     up2(thr0, thr0v[0], thr0v[1]);
@@ -878,7 +913,7 @@ __device__ __forceinline__ void triangle_full2(const float (&a)[2], const int (&
                    gq2 = !(fabsf(q2e[t]) <= p.q_thr);
         const bool gt0 = !(fabsf(t0e[t]) <= thr0v[t]), gt1 = !(fabsf(t1e[t]) <= thr1v[t]),
                    gt2 = !(fabsf(t2e[t]) <= thr2v[t]);
-        const bool g = (v02[t] && (gq0 || gt0 || gq2 || gt2)) || (v1[t] && (gq1 || gt1));
+        const bool g = (v02[t] && (gq0 || gt0 || gq2 || gt2 || gs[t])) || (v1[t] && (gq1 || gt1 || gm[t]));
         bool ok0 = v02[t] && !g && (unsigned)q0b[t] < (unsigned)p.Q;
         bool ok1 = v1[t] && !g && (unsigned)q1b[t] < (unsigned)p.Q;
         bool ok2 = v02[t] && !g && (unsigned)q2b[t] < (unsigned)p.Q;
@@ -978,7 +1013,7 @@ constexpr int TRI_DIAG_IJ = 1, TRI_CHECK_B = 2, TRI_CHECK_C = 4;
 
 // Runs the full binning path on n (<= 64) queued candidates, two per lane
 // (packed into the f32x2 instructions of one binning path).
-template <bool THETA_FULL, bool JBJ>
+template <bool THETA_FULL, int MODE>
 __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, const int2* row_ij, const int2* row_ik,
                                                const float* JKd, const short* JKw, const TriParams& p, unsigned int* Hw,
                                                RecheckQueue& q, const TriShared& S, uint32_t ia) {
@@ -995,12 +1030,12 @@ __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, cons
     const int wa[2] = {ij0.y, ij1.y}, wb[2] = {ik0.y, ik1.y};
     const int wc[2] = {JKw[j0 * TILE + k0], JKw[j1 * TILE + k1]};
     const unsigned ww[2] = {w0, w1};
-    if (JBJ) {
+    if (MODE == FAST_JBJ) {
         jbj_full2(fa, wa, fb, wb, fc, wc, ww, p, Hw);
         return;
     }
     bool guard[2];
-    triangle_full2<THETA_FULL>(fa, wa, fb, wb, fc, wc, ww, p, Hw, guard);
+    triangle_full2<THETA_FULL, MODE == FAST_GEOM>(fa, wa, fb, wb, fc, wc, ww, p, Hw, guard);
     const bool g0 = guard[0], g1 = guard[1];
     const uint32_t slot = S.unit.x & UNIT_SLOT_MASK;
     if (g0) push_recheck(q, slot, w0, ia, (uint32_t)(S.b0 + j0), (uint32_t)(S.c0 + k0));
@@ -1048,7 +1083,7 @@ __device__ __forceinline__ unsigned long long candidate_mask_jbj(int cij, unsign
     return (nI & (mI | mM | mH)) | ((nM | nH) & mI);
 }
 
-template <int PRED, bool THETA_FULL, bool JBJ>
+template <int PRED, bool THETA_FULL, int MODE>
 __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriParams& p, float4* P, float* JKd, short* JKw, int2* IJ,
                                     int2* IK, uint32_t* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
                                     RecheckQueue& q, unsigned long long& evaluated, unsigned long long& binned) {
@@ -1178,14 +1213,14 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 int c0 = 0, c1 = 0;
                 if (lane < numC) {
                     float d = ref_dist<false>(pj, PC[lane]);
-                    int w = tri_side_word(d, p);
+                    int w = tri_side_word<MODE>(d, p);
                     JKd[j * TILE + lane] = d;
                     JKw[j * TILE + lane] = (short)w;
                     c0 = side_class(w, d, p);
                 }
                 if (lane + 32 < numC) {
                     float d = ref_dist<false>(pj, PC[lane + 32]);
-                    int w = tri_side_word(d, p);
+                    int w = tri_side_word<MODE>(d, p);
                     JKd[j * TILE + lane + 32] = d;
                     JKw[j * TILE + lane + 32] = (short)w;
                     c1 = side_class(w, d, p);
@@ -1223,13 +1258,13 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             int c0 = 0, c1 = 0;
             if (lane < numC) {
                 float d = ref_dist<false>(pi, PC[lane]);
-                int w = tri_side_word(d, p);
+                int w = tri_side_word<MODE>(d, p);
                 row_ik[lane] = make_int2(__float_as_int(d), w);
                 c0 = side_class(w, d, p);
             }
             if (lane + 32 < numC) {
                 float d = ref_dist<false>(pi, PC[lane + 32]);
-                int w = tri_side_word(d, p);
+                int w = tri_side_word<MODE>(d, p);
                 row_ik[lane + 32] = make_int2(__float_as_int(d), w);
                 c1 = side_class(w, d, p);
             }
@@ -1248,13 +1283,13 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 w2 = 0;
                 if (j >= numB) return false;
                 float d = ref_dist<false>(pi, PB[j]);
-                int w = tri_side_word(d, p);
+                int w = tri_side_word<MODE>(d, p);
                 row_ij[j] = make_int2(__float_as_int(d), w);
                 const int c = side_class(w, d, p);
                 bool ok = c != 0 && any_k && j > j_after;
                 if (PRED == PRED_SAME) ok = ok && ki <= pkey(PB[j]);
                 if (!ok) return false;
-                cm = JBJ ? candidate_mask_jbj(c, nI, nM, nH, JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j])
+                cm = MODE == FAST_JBJ ? candidate_mask_jbj(c, nI, nM, nH, JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j])
                          : candidate_mask(c, nB, nI, nM, nH, JM[j], JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j]);
                 if (diag_jk) cm &= j >= 63 ? 0ull : (~0ull << (j + 1));
                 if (PRED == PRED_RDD) {
@@ -1317,7 +1352,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                     if (qn >= 64) {
                         __syncwarp();
                         qn -= 64;
-                        run_candidates<THETA_FULL, JBJ>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
+                        run_candidates<THETA_FULL, MODE>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
                         bn += 64;
                         __syncwarp();
                     }
@@ -1325,7 +1360,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             }
             __syncwarp();
             if (qn > 0) {
-                run_candidates<THETA_FULL, JBJ>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
+                run_candidates<THETA_FULL, MODE>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
                 bn += qn;
             }
             __syncwarp();
@@ -1339,14 +1374,14 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
     }
 }
 
-template <bool THETA_FULL, bool JBJ, typename... Args>
+template <bool THETA_FULL, int MODE, typename... Args>
 __device__ __forceinline__ void triangle_dispatch(uint32_t pred, Args&&... args) {
     switch (pred) {
-        case PRED_NONE: triangle_group_fast<PRED_NONE, THETA_FULL, JBJ>(args...); break;
-        case PRED_DDR: triangle_group_fast<PRED_DDR, THETA_FULL, JBJ>(args...); break;
-        case PRED_RDD: triangle_group_fast<PRED_RDD, THETA_FULL, JBJ>(args...); break;
-        case PRED_SAME: triangle_group_fast<PRED_SAME, THETA_FULL, JBJ>(args...); break;
-        default: triangle_group_fast<PRED_ONE, THETA_FULL, JBJ>(args...); break;
+        case PRED_NONE: triangle_group_fast<PRED_NONE, THETA_FULL, MODE>(args...); break;
+        case PRED_DDR: triangle_group_fast<PRED_DDR, THETA_FULL, MODE>(args...); break;
+        case PRED_RDD: triangle_group_fast<PRED_RDD, THETA_FULL, MODE>(args...); break;
+        case PRED_SAME: triangle_group_fast<PRED_SAME, THETA_FULL, MODE>(args...); break;
+        default: triangle_group_fast<PRED_ONE, THETA_FULL, MODE>(args...); break;
     }
 }
 
@@ -1355,7 +1390,7 @@ __device__ __forceinline__ void triangle_dispatch(uint32_t pred, Args&&... args)
 #endif
 // Persistent over the plan's units: tiles B and C of a job with a mask of A
 // tiles.
-template <bool THETA_FULL, bool JBJ>
+template <bool THETA_FULL, int MODE>
 __global__ void __launch_bounds__(TRI_THREADS, TRI_MIN_BLOCKS)
 triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int* counter, TriParams p, RecheckQueue q,
                      int copies) {
@@ -1395,7 +1430,7 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
         cur = slot;
         since += n;
         if (n == 0) continue;  // a part without A tiles
-        triangle_dispatch<THETA_FULL, JBJ>(jobs[slot].mode & JOB_PRED_MASK, jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
+        triangle_dispatch<THETA_FULL, MODE>(jobs[slot].mode & JOB_PRED_MASK, jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
     }
     if (cur >= 0) flush_hist(H, copies, p.len, jobs[cur].hist);
     __syncthreads();
@@ -1405,7 +1440,9 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
     }
 }
 
-// Exact recomputation of queued guard-band triangles.
+// Exact recomputation of queued guard-band triangles (GEOM: of the
+// double-precision geometry).
+template <bool GEOM>
 __global__ void triangle_recheck_kernel(const DevJob* __restrict__ jobs, RecheckQueue q, TriParams p, AcosTable t) {
     unsigned int n = *q.count;
     if (n > q.cap) n = q.cap;
@@ -1415,7 +1452,8 @@ __global__ void triangle_recheck_kernel(const DevJob* __restrict__ jobs, Recheck
         unsigned w = it.x >> RECHECK_WEIGHT_SHIFT;
         float4 pa = J.pts[0][it.y], pb = J.pts[1][it.z], pc = J.pts[2][it.w];
         int out[3];
-        tp_exact<false>(ref_dist<false>(pa, pb), ref_dist<false>(pa, pc), ref_dist<false>(pb, pc), p, t, out);
+        if (GEOM) tp_geom(geo_dist(pa, pb), geo_dist(pa, pc), geo_dist(pb, pc), p, out);
+        else tp_exact<false>(ref_dist<false>(pa, pb), ref_dist<false>(pa, pc), ref_dist<false>(pb, pc), p, t, out);
         for (int k = 0; k < 3; k++)
             if (out[k] >= 0) atomicAdd(J.hist + out[k], (unsigned long long)w);
     }
@@ -2407,8 +2445,8 @@ cudaError_t prepare_kernels(int device) {
     int optin = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (e != cudaSuccess) return e;
-    const void* fns[] = {(const void*)triangle_fast_kernel<true, false>, (const void*)triangle_fast_kernel<false, false>,
-                         (const void*)triangle_fast_kernel<false, true>,
+    const void* fns[] = {(const void*)triangle_fast_kernel<true, FAST_TP>, (const void*)triangle_fast_kernel<false, FAST_TP>,
+                         (const void*)triangle_fast_kernel<false, FAST_JBJ>, (const void*)triangle_fast_kernel<false, FAST_GEOM>,
                          (const void*)triangle_fp64_kernel<MODE_FP64>, (const void*)triangle_fp64_kernel<MODE_GEOM>,
                          (const void*)triangle_fp64_kernel<MODE_JBJ>, (const void*)three_side_kernel<true, true>,
                          (const void*)three_side_kernel<true, false>, (const void*)three_side_kernel<false, true>,
@@ -2427,17 +2465,20 @@ cudaError_t prepare_kernels(int device) {
 }
 
 cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
-                                 RecheckQueue q, int grid, int copies, int jbj, cudaStream_t st) {
+                                 RecheckQueue q, int grid, int copies, int mode, cudaStream_t st) {
     size_t smem = triangle_smem_bytes(p.len, copies);
-    if (jbj) triangle_fast_kernel<false, true><<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
-    else if (p.theta_full) triangle_fast_kernel<true, false><<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
-    else triangle_fast_kernel<false, false><<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
+    auto kern = mode == FAST_JBJ    ? triangle_fast_kernel<false, FAST_JBJ>
+                : mode == FAST_GEOM ? triangle_fast_kernel<false, FAST_GEOM>
+                : p.theta_full      ? triangle_fast_kernel<true, FAST_TP>
+                                    : triangle_fast_kernel<false, FAST_TP>;
+    kern<<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
     return cudaGetLastError();
 }
 
-cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t, int grid,
-                                    cudaStream_t st) {
-    triangle_recheck_kernel<<<grid, 128, 0, st>>>(jobs, q, p, t);
+cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t, int geom,
+                                    int grid, cudaStream_t st) {
+    if (geom) triangle_recheck_kernel<true><<<grid, 128, 0, st>>>(jobs, q, p, t);
+    else triangle_recheck_kernel<false><<<grid, 128, 0, st>>>(jobs, q, p, t);
     return cudaGetLastError();
 }
 
