@@ -435,6 +435,8 @@ struct Binning {
     int kind = 0;
     TriParams tri{};
     ThreeParams three{};
+    NearParams near{};
+    bool near_ok = false;     // three-side: the binning suits the neighbour lists
     PairParams pair{};
     int len = 0;
     double lmax = INFINITY;   // no counted triangle/pair has a side >= lmax
@@ -526,6 +528,16 @@ Binning make_binning(const tpcf_spec& sp) {
         // (compat mode counts every triple: the side codes are a small part of its work)
         p.fast = p.clean && three_side_thresholds(p) ? 1 : 0;
         p.zcode = three_side_bin_of_d2(0.0f, p.lo, p.hi, p.bw, p.n);
+        PairParams g{};  // the same bins below hist_max
+        g.n = p.n;
+        g.lo = p.lo;
+        g.hi = p.hi;
+        g.bw = p.bw;
+        pair_guard(g);
+        const double r2 = (double)p.hi * (1 + 1e-6) * (double)p.hi;
+        b.near = {p.n, p.len, p.clean, p.zcode, p.lo, p.hi, p.bw, g.inv_bw, g.off, g.thr,
+                  nextafterf((float)std::min(r2, 3e38), INFINITY)};
+        b.near_ok = sp.prune && sp.precision == TPCF_GUARDED_FP32 && g.fast && g.thr > 0.25f && p.hi > 0 && p.hi <= 1e15f;
     } else if (sp.kind == TPCF_TRIANGLE) {
         for (int a = 0; a < 3; a++) check_axis(sp.axis[a], "triangle axis");
         TriParams& p = b.tri;
@@ -704,12 +716,14 @@ struct Lane {
     DevBuf<unsigned int> d_counters;  // see CTR_*
     DevBuf<uint4> d_queue;
     DevBuf<unsigned long long> d_hist;
+    DevBuf<unsigned long long> d_acc;  // three-side accumulators of the neighbour lists
     PinnedBuf<unsigned long long> h_hist;
     PinnedBuf<unsigned int> h_counters;
     // last planned batch (see run_group)
     std::vector<uint64_t> plan_sig;
     uint32_t plan_rows = 0;  // rows (pairs: items) of the plan
-    int plan_chunk = 0;      // pairs: tiles B per item
+    int plan_chunk = 0;      // pairs: tiles B per item; neighbour lists: centres per item
+    uint32_t plan_wedges = 0;  // neighbour lists: items of the wedge kernel
     // the launch sequence of the last batch, captured as a CUDA graph and
     // replayed while the batch and every buffer it touches stay the same
     cudaGraphExec_t graph = nullptr;
@@ -741,6 +755,7 @@ struct Lane {
         d_counters.release();
         d_queue.release();
         d_hist.release();
+        d_acc.release();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (ev_mid) cudaEventDestroy(ev_mid);
@@ -754,6 +769,7 @@ struct Lane {
 constexpr int CTR_WORK = 0;     // units (items) handed out
 constexpr int CTR_RECHECK = 1;  // queued guard-band triangles
 constexpr int CTR_EVAL = 2;     // evaluated (two words), binned (pairs: tile pairs; two words)
+constexpr int CTR_DENSE = 6;    // neighbour lists: a centre has too many near tiles
 constexpr int CTR_ZEROED = 8;
 constexpr int CTR_HEADER = 8;
 constexpr int CTR_WORDS = CTR_HEADER + (int)(sizeof(PlanHeader) / sizeof(unsigned int));
@@ -1159,7 +1175,7 @@ size_t shape_smem(const tpcf_spec& sp, const Binning& bin, int copies, int group
 // Launch shapes worth trying for a group, the default first.  The guarded
 // triangle kernel is compiled for four CTAs per SM (its register budget);
 // the others take as many CTAs as shared memory allows, up to 8.
-std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Binning& bin, bool fp64) {
+std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Binning& bin, bool fp64, bool near) {
     int max_smem_sm = 0, max_smem_block = 0;
     cudaDeviceGetAttribute(&max_smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
     cudaDeviceGetAttribute(&max_smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
@@ -1180,6 +1196,16 @@ std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Bi
             if (o.copies == sh.copies && o.per_sm == sh.per_sm && o.groups == sh.groups) return;
         out.push_back(sh);
     };
+    if (near) {  // one CTA per SM of up to four pipelines
+        for (int g : {4, 2, 1}) {
+            Shape sh;
+            sh.groups = g;
+            sh.smem = three_near_smem_bytes(bin.three.n, g);
+            sh.per_sm = sh.smem + 1024 <= (size_t)max_smem_block ? 1 : 0;
+            add(sh);
+        }
+        return out;
+    }
     if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) {
         const char* bps = getenv("TPCF_TRI_BLOCKS_PER_SM");
         const int tri_per_sm = fp64 ? 2 : (bps ? std::max(1, atoi(bps)) : 4);
@@ -1242,14 +1268,14 @@ int grid_for(tpcf_ctx* ctx, const Shape& sh, uint64_t ntasks, int sm_cap) {
 
 // Runs one group of jobs that share kind, binning and precision in a single
 // persistent launch.  outs[i] receives hist_len counts.
-void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
+void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool lists = true) {
     auto t_wall0 = std::chrono::steady_clock::now();
     const tpcf_spec& sp = *group[0].spec;
     Binning bin = make_binning(sp);
     const int ncat = sp.kind == TPCF_PAIR ? 2 : 3;
     const bool pairs = sp.kind == TPCF_PAIR;
-    bool tame = true;  // (asked by the double-precision geometry only)
-    if (sp.precision == TPCF_GEOMETRY_FP64) {
+    bool tame = true;  // (asked by the double-precision geometry and the neighbour lists only)
+    if (sp.precision == TPCF_GEOMETRY_FP64 || bin.near_ok) {
         std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
         for (const GroupJob& g : group)
             for (int r = 0; r < ncat; r++) {
@@ -1258,6 +1284,12 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             }
     }
     const bool fp64 = !guarded_fp32(sp, bin, tame);
+    // three-side counts from neighbour lists (see three_near_kernel)
+    const char* near_env = getenv("TPCF_NEAR");
+    const bool near = lists && bin.near_ok && tame && !(near_env && near_env[0] == '0') &&
+                      !shape_candidates(ctx, sp, bin, fp64, true).empty() &&
+                      three_near_acc_words(bin.three.n) * group.size() <= ((size_t)1 << 27);
+    const bool items = pairs || near;  // kernels that find their tiles themselves
     const bool tri_kind = sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ;
     const bool fast_tri = tri_kind && !fp64;
     const bool fast_jbj = sp.kind == TPCF_TRIANGLE_JBJ && !fp64;  // the fast kernel's JBJ binning
@@ -1331,7 +1363,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     sig.push_back((uint64_t)(uintptr_t)L.d_hist.p);
     {
         const uint64_t f[6] = {(uint64_t)sp.kind, (uint64_t)sp.prune, (uint64_t)sp.precision, (uint64_t)sp.nan_policy,
-                               (uint64_t)sp.overflow, (uint64_t)rdd << 1 | (uint64_t)sym_three};
+                               (uint64_t)sp.overflow, (uint64_t)near << 2 | (uint64_t)rdd << 1 | (uint64_t)sym_three};
         sig.insert(sig.end(), f, f + 6);
         for (int a = 0; a < 3; a++) {
             sig.push_back((uint64_t)fbits(sp.axis[a].lo) << 32 | fbits(sp.axis[a].hi));
@@ -1382,7 +1414,23 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         auto id = [&](int r) { return ranges[rg[r]].ref.id; };
         const bool ab = id(0) == id(1), bc = id(1) == id(2);
         uint32_t mode = PRED_NONE, v[3] = {rg[0], rg[1], rg[2]};
-        if (pairs) {
+        if (near) {
+            // the centre: the point of the view that appears once, or any
+            const bool ac = id(0) == id(2);
+            if (ab && bc && sym_three) {
+                mode = NEAR_SYM;
+            } else if (bc) {
+                mode = NEAR_PAIR;
+            } else if (ac) {
+                v[0] = rg[1], v[1] = v[2] = rg[0];
+                mode = NEAR_PAIR | 1u << NEAR_CENTRE_SHIFT;
+            } else if (ab) {
+                v[0] = rg[2], v[1] = v[2] = rg[0];
+                mode = NEAR_PAIR | 2u << NEAR_CENTRE_SHIFT;
+            } else {
+                mode = NEAR_ORDERED;
+            }
+        } else if (pairs) {
             if (jsp.loop == TPCF_LOOP_SAME) mode = ab ? JOB_B_FROM_A : (uint32_t)PRED_SAME;
         } else if (tri_kind && jsp.loop == TPCF_LOOP_ONE && ab && !bc && rdd) {
             // Loop ONE jobs of two arrays are counted with the point of the
@@ -1422,12 +1470,29 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     }
     cudaStream_t st = L.stream;
     L.d_counters.reserve(CTR_WORDS);
-    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64);
+    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near);
     const bool plan_hit = sig == L.plan_sig;
     phase("batch");
     const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
-    uint32_t nrows = L.plan_rows;   // pairs: items
-    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item
+    uint32_t nrows = L.plan_rows;   // pairs and neighbour lists: items
+    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item; neighbour lists: centres per item
+    // neighbour lists: an accumulator per output slot and class of job, and the
+    // wedge jobs of the reference's mode (two per job, one for a single catalog)
+    std::vector<uint32_t> acc_of;
+    std::vector<std::pair<size_t, uint32_t>> accs;  // slot, mode
+    const size_t acc_words = near ? three_near_acc_words(bin.three.n) : 0;
+    size_t nwedge_jobs = 0;
+    if (near) {
+        std::map<std::pair<size_t, uint32_t>, uint32_t> at;
+        for (size_t g = 0; g < group.size(); g++) {
+            auto ins = at.emplace(std::make_pair(slot_of[g], roles[g].mode), (uint32_t)accs.size());
+            if (ins.second) accs.push_back(ins.first->first);
+            acc_of.push_back(ins.first->second);
+            if (!bin.three.clean) nwedge_jobs += roles[g].mode == NEAR_SYM ? 1 : 2;
+        }
+        L.d_acc.reserve(acc_words * accs.size());
+    }
+    uint32_t nwedges = L.plan_wedges;
     PlanHeader* d_header = nullptr;
     // Finds the units of the batch on the device (see plan_rows): the host
     // gives each job's number of rows.
@@ -1462,8 +1527,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         for (Range& r : ranges) r.view = get_view(ctx, L, r.key.h, r.key.b, r.key.e, r.key.gl);
         phase("views");
         CK(cudaStreamSynchronize(st));  // (a failed batch may still read the pinned buffers)
-        L.h_jobs.reserve(group.size());
-        L.h_rows.reserve(group.size() + 1);
+        const size_t njobs = group.size() + nwedge_jobs + accs.size();
+        L.h_jobs.reserve(njobs);
+        L.h_rows.reserve(group.size() + nwedge_jobs + 2);
         uint64_t rows = 0;
         plan_chunk = 0;
         if (pairs) {
@@ -1471,6 +1537,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             for (const RoleJob& r : roles)
                 tile_pairs += (long long)ranges[r.range[0]].view->ntiles * ranges[r.range[1]].view->ntiles;
             plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS);
+        } else if (near) {
+            // one centre per item where that balances the pipelines, else four
+            uint64_t centres = 0;
+            for (const RoleJob& r : roles) centres += ranges[r.range[0]].view->n;
+            plan_chunk = centres < 64ull * ctx->num_sms * 4 ? 1 : 4;
         }
         for (size_t g = 0; g < group.size(); g++) {
             DevJob d{};
@@ -1485,21 +1556,70 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             d.hist = L.d_hist.p + (size_t)bin.len * slot_of[g];
             L.h_jobs.p[g] = d;
             L.h_rows.p[g] = (uint32_t)rows;
-            if (pairs) rows += (uint64_t)d.ntiles[0] * ((d.ntiles[1] + plan_chunk - 1) / plan_chunk);
+            if (near) {
+                L.h_jobs.p[g].hist = L.d_acc.p + acc_words * acc_of[g];
+                rows += (uint64_t)d.ntiles[0] * ((TILE + plan_chunk - 1) / plan_chunk);
+            } else if (pairs) rows += (uint64_t)d.ntiles[0] * ((d.ntiles[1] + plan_chunk - 1) / plan_chunk);
             else if (d.ntiles[2] > 0) rows += (uint64_t)((d.ntiles[0] + window - 1) / window) * d.ntiles[1];
             if (rows > 0xF0000000ull) throw InvalidArg{"too many tile pairs in one batch"};
         }
         L.h_rows.p[group.size()] = (uint32_t)rows;
         nrows = (uint32_t)rows;
-        L.d_jobs.reserve(group.size());
-        L.d_rows.reserve(group.size() + 1);
-        CK(cudaMemcpyAsync(L.d_jobs.p, L.h_jobs.p, group.size() * sizeof(DevJob), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(L.d_rows.p, L.h_rows.p, (group.size() + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-        L.h2d += group.size() * sizeof(DevJob) + (group.size() + 1) * sizeof(uint32_t);
-        if (!pairs) plan_units(std::max<size_t>(L.d_units.n, (size_t)1 << 20));
+        size_t nr = group.size() + 1;
+        if (near) {
+            // wedge jobs: pairs of sides at a point of role B (lists A, C; the
+            // pairs B-C weigh the points of A) and of role C (lists A, B)
+            const size_t m = bin.three.n + 1;
+            uint64_t w = 0;
+            size_t at = group.size();
+            for (size_t g = 0; nwedge_jobs && g < group.size(); g++) {
+                const uint32_t centre = roles[g].mode >> NEAR_CENTRE_SHIFT;
+                // the views of the reference's roles
+                const int of[3][3] = {{0, 1, 2}, {1, 0, 2}, {1, 2, 0}};
+                const View* v[3];
+                for (int r = 0; r < 3; r++) v[r] = ranges[roles[g].range[of[centre][r]]].view.get();
+                const bool sym = roles[g].mode == NEAR_SYM;
+                unsigned long long* acc = L.d_acc.p + acc_words * acc_of[g] + m * m * m + m + 1;
+                for (int k = 0; k < (sym ? 1 : 2); k++) {
+                    const View* role[3] = {v[1 + k], v[0], v[2 - k]};
+                    DevJob d{};
+                    for (int r = 0; r < 3; r++) {
+                        d.pts[r] = role[r]->pts.p;
+                        d.tile_start[r] = role[r]->tile_start.p;
+                        d.box[r] = role[r]->box.p;
+                        d.ntiles[r] = role[r]->ntiles;
+                    }
+                    d.mode = sym ? NEAR_SYM : NEAR_ORDERED;
+                    d.hist = acc + k * m * m;
+                    d.aux = k == 0 ? acc + 2 * m * m : nullptr;
+                    d.weight = (unsigned long long)v[0]->n;
+                    L.h_jobs.p[at] = d;
+                    L.h_rows.p[nr++] = (uint32_t)w;
+                    w += (uint64_t)d.ntiles[0] * 8;
+                    if (w > 0xF0000000ull) throw InvalidArg{"too many points in one batch"};
+                    at++;
+                }
+            }
+            L.h_rows.p[nr++] = (uint32_t)w;
+            nwedges = (uint32_t)w;
+            for (const auto& a : accs) {
+                DevJob d{};
+                d.mode = a.second;
+                d.hist = L.d_acc.p + acc_words * (size_t)(&a - accs.data());
+                d.aux = L.d_hist.p + (size_t)bin.len * a.first;
+                L.h_jobs.p[at++] = d;
+            }
+        }
+        L.d_jobs.reserve(njobs);
+        L.d_rows.reserve(nr);
+        CK(cudaMemcpyAsync(L.d_jobs.p, L.h_jobs.p, njobs * sizeof(DevJob), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(L.d_rows.p, L.h_rows.p, nr * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        L.h2d += njobs * sizeof(DevJob) + nr * sizeof(uint32_t);
+        if (!items) plan_units(std::max<size_t>(L.d_units.n, (size_t)1 << 20));
         L.plan_sig = sig;
         L.plan_rows = nrows;
         L.plan_chunk = plan_chunk;
+        L.plan_wedges = nwedges;
         phase("plan");
     }
     L.stats.plan_ms =
@@ -1519,15 +1639,15 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     uint64_t dev_evaluated = 0, dev_binned = 0, replays = 0, regrows = 0;
     PlanHeader header{};
     // units (pairs: items) known on the host: needed where a batch is counted in slices
-    bool sized = pairs;
-    uint32_t nwork = pairs ? nrows : 0xffffffffu;
+    bool sized = items;
+    uint32_t nwork = items ? nrows : 0xffffffffu;
 
     // One complete count of the group with launch shape sh: zero, count,
     // recheck, copy back (replayed from a captured graph when allowed and
     // the batch repeats).  Returns the device time in ms.
     auto count_with = [&](const Shape& sh, bool allow_graph) -> float {
         const int copies = sh.copies;
-        const int grid = grid_for(ctx, sh, pairs ? nrows : UINT64_MAX, L.sm_cap);
+        const int grid = grid_for(ctx, sh, items ? (nrows + std::max(1, sh.groups) - 1) / std::max(1, sh.groups) : UINT64_MAX, L.sm_cap);
         for (int attempt = 0; attempt < 4; attempt++) {
             if (L.slice_batches && !sized) {
                 // (the header of a plan that overflowed the unit list asks for a
@@ -1543,7 +1663,8 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             unsigned int slice = L.slice_batches ? std::max<unsigned int>((unsigned int)grid * 8u, (nwork + 63u) / 64u)
                                                  : std::max(nwork, 1u);
             if (L.slice_batches && ctx->slice_tasks > 0) slice = (unsigned int)ctx->slice_tasks;
-            launches = (nwork > slice ? (nwork + slice - 1) / slice : 1) + ((sp.kind == TPCF_TRIANGLE && !fp64) ? 1 : 0);
+            launches = (nwork > slice ? (nwork + slice - 1) / slice : 1) +
+                       (sp.kind == TPCF_TRIANGLE && !fp64 ? 1 : near ? (nwedges ? 2 : 1) : 0);
             RecheckQueue q{};
             if (sp.kind == TPCF_TRIANGLE && !fp64) {
                 if (L.d_queue.n < queue_cap) L.drop_graph();
@@ -1565,6 +1686,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     } while (0)
                 EQ(cudaMemsetAsync(L.d_hist.p, 0, hist_total * sizeof(unsigned long long), st));
                 EQ(cudaMemsetAsync(L.d_counters.p, 0, CTR_ZEROED * sizeof(unsigned int), st));
+                if (near) EQ(cudaMemsetAsync(L.d_acc.p, 0, acc_words * accs.size() * sizeof(unsigned long long), st));
                 EQ(cudaEventRecordWithFlags(L.ev0, st, ev_flags));
                 // the counting kernel over units (items) [t0, t0 + n)
                 auto launch_main = [&](unsigned int t0, unsigned int n) -> cudaError_t {
@@ -1577,6 +1699,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                         return launch_triangle_fp64(L.d_jobs.p, ul, counter, bin.tri, acos_t, grid, copies,
                                                     sp.kind == TPCF_TRIANGLE_JBJ ? 2
                                                     : geom ? 1 : 0, st);
+                    if (near)
+                        return launch_three_near(L.d_jobs.p, L.d_rows.p, (int)group.size(), t0, n, plan_chunk, counter,
+                                                 L.d_counters.p + CTR_DENSE,
+                                                 reinterpret_cast<unsigned long long*>(L.d_counters.p + CTR_EVAL),
+                                                 bin.near, grid, sh.groups, st);
                     if (sp.kind == TPCF_THREE_SIDE)
                         return launch_three_side(L.d_jobs.p, ul, counter, bin.three, fp64, grid, copies, sh.groups, st);
                     return launch_pairs(L.d_jobs.p, L.d_rows.p, (int)group.size(), t0, n, plan_chunk, counter,
@@ -1592,6 +1719,12 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                     EQ(launch_main(t0, std::min(slice, nwork - t0)));
                 }
                 EQ(cudaEventRecordWithFlags(L.ev_mid, st, ev_flags));
+                if (near) {
+                    const DevJob* after = L.d_jobs.p + group.size();
+                    EQ(launch_three_wedges(after, L.d_rows.p + group.size() + 1, (int)nwedge_jobs, nwedges, bin.near,
+                                           ctx->num_sms * 8, st));
+                    EQ(launch_three_expand(after + nwedge_jobs, (int)accs.size(), bin.near, st));
+                }
                 if (sp.kind == TPCF_TRIANGLE && !fp64)
                     EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, geom ? 1 : 0, ctx->num_sms * 8, st));
                 EQ(cudaEventRecordWithFlags(L.ev1, st, ev_flags));
@@ -1613,7 +1746,8 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
                                           (uint64_t)(uintptr_t)acos_t.bucket, (uint64_t)acos_t.n, queue_cap,
                                           (uint64_t)grid, (uint64_t)copies, (uint64_t)sh.groups, hist_total,
                                           (uint64_t)nwork, (uint64_t)slice, (uint64_t)(uintptr_t)L.d_rows.p,
-                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk};
+                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk,
+                                          (uint64_t)(uintptr_t)L.d_acc.p};
                 gsig.insert(gsig.end(), extra, extra + sizeof(extra) / sizeof(extra[0]));
                 if (!L.graph || gsig != L.graph_sig) {
                     L.drop_graph();
@@ -1646,7 +1780,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
             const unsigned int* counters = L.h_counters.p;
             L.d2h += CTR_WORDS * sizeof(unsigned int) + hist_total * sizeof(unsigned long long);
             memcpy(&header, counters + CTR_HEADER, sizeof(header));
-            if (!pairs && header.nunits == 0 && header.needed > 0) {
+            if (!items && header.nunits == 0 && header.needed > 0) {
                 // the unit list overflowed: nothing was counted; plan again into a larger one
                 L.drop_graph();
                 plan_units((size_t)header.needed + (header.needed >> 3));
@@ -1708,6 +1842,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
         const char* pl_env = getenv("TPCF_PIPELINE");
         count_with(shape, graphs && (plan_hit || (pl_env && pl_env[0] == '0')));
     }
+    if (near && L.h_counters.p[CTR_DENSE]) {
+        // a centre with more near tiles than a list holds: by tile triples
+        run_group(ctx, L, group, false);
+        return;
+    }
     L.stats.tuned_shapes = tuned_runs;
     L.stats.hist_copies = (uint64_t)shape.copies;
     L.stats.ctas_per_sm = (uint64_t)shape.per_sm;
@@ -1734,9 +1873,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group) {
     // contain and counts the triangles it walks; the pair kernel counts the
     // pairs and tile pairs it finds; other kernels walk every triangle of
     // their units
-    L.stats.evaluated_units = fast_tri || pairs ? dev_evaluated : header.evaluated;
+    L.stats.evaluated_units = fast_tri || items ? dev_evaluated : header.evaluated;
     L.stats.binned_units = fast_tri ? dev_binned : L.stats.evaluated_units;
-    L.stats.tasks = pairs ? dev_binned : header.tiles;
+    L.stats.tasks = pairs ? dev_binned : near ? nrows : header.tiles;
     L.stats.kernel_launches = launches * std::max<uint64_t>(1, tuned_runs);
     L.stats.recheck_regrows = regrows;
     L.stats.total_ms =

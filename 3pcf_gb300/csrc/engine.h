@@ -72,6 +72,8 @@ struct DevJob {
     int32_t ntiles[3];
     uint32_t mode;               // JOB_* bits
     unsigned long long* hist;    // global uint64 histogram (hist_len entries)
+    unsigned long long* aux;     // three-side lists: see three_wedge_kernel, three_expand_kernel
+    unsigned long long weight;
 };
 // the job's tile tuples and the predicate of its points
 constexpr uint32_t JOB_PRED_MASK = 0x7u;   // Pred
@@ -132,6 +134,23 @@ struct PairParams {
     float inv_bw = 0.f, off = 0.f, thr = 0.f;
     float reach2 = 0.f;  // tiles at least sqrt(reach2) apart hold no counted pair (rounded up)
 };
+
+// Three-side histogram from neighbour lists: the guard band of pair bins
+// (PairParams), codes 0 .. n below hist_max.
+struct NearParams {
+    int n, len, clean, zcode;    // as ThreeParams
+    float lo, hi, bw, inv_bw, off, thr;
+    float reach2;                // squared: sides at or above it are at or above hist_max
+};
+// DevJob::mode of its jobs (roles: centre, first list, second list): which
+// pairs of the lists make a triple, and the reference's role of the centre.
+enum NearClass : uint32_t {
+    NEAR_SYM = 0,      // one catalog: positions centre < j < k, every ordering
+    NEAR_PAIR = 1,     // both lists of one catalog: unordered pairs, both orderings
+    NEAR_ORDERED = 2   // every pair
+};
+constexpr uint32_t NEAR_CLASS_MASK = 3u;
+constexpr int NEAR_CENTRE_SHIFT = 2;
 
 // Exact glibc-acosf exception table on the device.
 struct AcosTable {
@@ -207,6 +226,17 @@ cudaError_t launch_acos_check(AcosTable t, uint32_t key_begin, uint32_t count, u
                               cudaStream_t st);
 cudaError_t launch_radecz_to_xyz(const double* ra, const double* dec, const double* redshift, int64_t n,
                                  const double poly[3], float* x, float* y, float* z, cudaStream_t st);
+
+// The three launches of a neighbour-list count; *dense is set where the near
+// tiles of a centre are too many (count with launch_three_side instead).
+cudaError_t launch_three_near(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
+                              unsigned int nitems, int centres, unsigned int* counter, unsigned int* dense,
+                              unsigned long long* work, const NearParams& p, int grid, int pipes, cudaStream_t st);
+cudaError_t launch_three_wedges(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int nitems,
+                                const NearParams& p, int grid, cudaStream_t st);
+cudaError_t launch_three_expand(const DevJob* accs, int naccs, const NearParams& p, cudaStream_t st);
+size_t three_near_acc_words(int n);
+size_t three_near_smem_bytes(int n, int pipes);
 
 // shared-memory bytes of a launch (for occupancy / admission)
 size_t triangle_smem_bytes(int hist_len, int hist_copies);

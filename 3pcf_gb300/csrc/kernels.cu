@@ -2173,6 +2173,504 @@ three_side_grouped_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned
     }
 }
 
+// Squared gap of two tile boxes (reduced by a margin that covers the rounding
+// of the bound and of the reference's separation) below reach2: the tiles can
+// hold a counted pair.
+__device__ __forceinline__ bool boxes_near(const float4* __restrict__ A, const float4* __restrict__ B, float reach2) {
+    const float4 al = A[0], ah = A[1], bl = B[0], bh = B[1];
+    const float gx = fmaxf(0.f, fmaxf(al.x - bh.x, bl.x - ah.x));
+    const float gy = fmaxf(0.f, fmaxf(al.y - bh.y, bl.y - ah.y));
+    const float gz = fmaxf(0.f, fmaxf(al.z - bh.z, bl.z - ah.z));
+    // (an overflowing gap is kept below an infinite reach only)
+    return !((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f) >= reach2);
+}
+
+// ---------------------------------------------------------------------------
+// Three-side histogram from neighbour lists.
+//
+// Only triples with all three sides below hist_max are enumerated: for each
+// point of the centre role, the points of the other two roles below hist_max
+// from it go into a list in shared memory (coordinates and side code), and
+// every pair of the list gets its third side.  The reference's mode also
+// counts triples with sides at or above hist_max (code F = n + 1); an index
+// with F in its last place (n^2 F > n^3) is past the array's end, and the rest
+// follow from the near triples T and from pairs of near sides at one point:
+//   T(a,F,c) = WB(a,c) - sum_b T(a,b,c),  WB(a,c) = sum over j of hA_j(a) hC_j(c)
+//   T(F,b,c) = WC(b,c) - sum_a T(a,b,c),  WC(b,c) = sum over k of hA_k(b) hB_k(c)
+//   T(F,F,c) = nA PBC(c) - sum_ab T(a,b,c) - sum_a T(a,F,c) - sum_b T(F,b,c)
+// with hX_p(v) the number of points of role X at code v from p and PBC the
+// pairs of B and C at code c.  All linear in counts, so near counts and the
+// sums W and P are collected per accumulator (three_near_kernel,
+// three_wedge_kernel) and expanded once (three_expand_kernel).
+//
+// Bound by the issue rate and the shared-memory atomics of the pairs of the
+// lists.  (Against tiles of 64^3 triples with class masks, whose rows and
+// candidate queues were most of the work: 150k lattice points, 32 bins,
+// 25.8 ms; D-D-D to R-R-R of 3k points, 16 bins, 23.4 ms.)
+
+constexpr int NEAR_CAP = 1024;        // list entries of a pipeline (halves of 512 for two lists)
+constexpr int NEAR_TILES = 256;       // near tiles of a centre's tile, per list
+constexpr int NEAR_CHUNK = 8;         // tiles of a half list where the lists overflow
+constexpr int NEAR_MAX_POINTS = NEAR_TILES * TILE;
+constexpr float NEAR_PAD = 1e18f;     // coordinate of padding entries: out of every range
+
+struct NearPipe {
+    float x[NEAR_CAP], y[NEAR_CAP], z[NEAR_CAP];
+    uint32_t code[NEAR_CAP];
+    uint32_t tiles[2][NEAR_TILES];
+    int ntiles[2], count[2];
+    uint4 item;  // job, tile, first centre, (unused)
+    unsigned int stop;
+};
+
+// Accumulator words (64 bits each): near triples, two equal indices, three
+// equal, then the wedges and pairs.
+__host__ __device__ inline int near_words3(int n) { return (n + 1) * (n + 1) * (n + 1); }
+size_t three_near_acc_words(int n) {
+    const size_t m = n + 1;
+    return m * m * m + m + 1 + 2 * m * m + m;
+}
+// Shared words of the near triples: strides that spread the banks (odd, and
+// different modulo 32), then the codes of two equal indices, then one word.
+struct NearStride {
+    int q, r, u2, words;
+};
+__host__ __device__ inline NearStride near_stride(int n) {
+    NearStride s;
+    const int m = n + 1;
+    s.q = m | 1;
+    s.r = (m * s.q) | 1;
+    if ((s.r & 31) == (s.q & 31)) s.r += 2;
+    s.u2 = m * s.r;
+    s.words = (s.u2 + m + 1 + 31) & ~31;
+    return s;
+}
+size_t three_near_smem_bytes(int n, int pipes) { return (size_t)pipes * sizeof(NearPipe) + (size_t)near_stride(n).words * 4; }
+
+// Exact three-side code, or -1 at or above hist_max.
+__device__ __forceinline__ int near_exact(float4 a, float4 b, const NearParams& p) {
+    const float d = ref_dist<false>(a, b);
+    if (d < p.lo) return 0;
+    if (d >= p.hi) return -1;
+    return __float2int_rz(__fdiv_rn(__fsub_rn(d, p.lo), p.bw));
+}
+
+// The same from rsqrt.approx outside the guard band (see pair_guard).
+__device__ __forceinline__ int near_code(float4 a, float4 b, const NearParams& p) {
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    const GuardedBin g = magic_floor(fmaf(d2 * rsqrt_approx(d2), p.inv_bw, p.off));
+    if (!(fabsf(g.err) <= p.thr)) return near_exact(a, b, p);
+    return g.bin < p.n ? max(g.bin, 0) : -1;
+}
+
+// Every pair (entry j of [j0, j1), this lane's entry k) of two lists; with
+// DIAG of one list, j < k.
+template <bool DIAG>
+__device__ __forceinline__ void near_block(const NearPipe& N, int j0, int j1, int k, float kx, float ky, float kz,
+                                           unsigned int* Uq, int rs, const NearParams& p) {
+    const f32x2 X = splat2(kx), Y = splat2(ky), Z = splat2(kz), scale = splat2(p.inv_bw), off = splat2(p.off);
+    for (int j = j0; j < j1; j += 4) {
+        const float4 x4 = *reinterpret_cast<const float4*>(N.x + j), y4 = *reinterpret_cast<const float4*>(N.y + j),
+                     z4 = *reinterpret_cast<const float4*>(N.z + j);
+        const uint4 c4 = *reinterpret_cast<const uint4*>(N.code + j);
+        const f32x2 xj[2] = {pk2(x4.x, x4.y), pk2(x4.z, x4.w)}, yj[2] = {pk2(y4.x, y4.y), pk2(y4.z, y4.w)},
+                    zj[2] = {pk2(z4.x, z4.y), pk2(z4.z, z4.w)};
+        const uint32_t cj[4] = {c4.x, c4.y, c4.z, c4.w};
+        unsigned redo = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const f32x2 dx = sub2(xj[h], X), dy = sub2(yj[h], Y), dz = sub2(zj[h], Z);
+            const f32x2 d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+            float s0, s1, e[2];
+            int b[2];
+            up2(d2, s0, s1);
+            const f32x2 d = mul2(d2, pk2(rsqrt_approx(s0), rsqrt_approx(s1)));
+            magic_floor2(fma2(d, scale, off), b[0], b[1], e[0], e[1]);
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const bool safe = fabsf(e[t]) <= p.thr;
+                if (safe && b[t] < p.n && (!DIAG || j + 2 * h + t < k))
+                    atomicAdd(Uq + (max(b[t], 0) * rs + (int)cj[2 * h + t]), 1u);
+                if (!safe) redo |= 1u << (2 * h + t);
+            }
+        }
+        while (redo) {
+            const int q = __ffs(redo) - 1, jj = j + q;
+            redo &= redo - 1u;
+            if (jj >= j1 || kx == -NEAR_PAD || (DIAG && jj >= k)) continue;
+            const int r = near_exact(make_float4(N.x[jj], N.y[jj], N.z[jj], 0.f), make_float4(kx, ky, kz, 0.f), p);
+            if (r >= 0) atomicAdd(Uq + (r * rs + (int)N.code[jj]), 1u);
+        }
+    }
+}
+
+// One CTA per SM of `pipes` 8-warp pipelines around one shared accumulator.  A
+// pipeline takes an item (a few centres of one tile), and waits for the others
+// at a CTA barrier when its item belongs to another job, when there is none
+// left, or when the 32-bit counters have taken 2^30 pairs; there the counters
+// are added to the job's accumulator.  An item adds at most
+// NEAR_ITEM * NEAR_MAX_POINTS^2 / 2 = 2^29 pairs, so that four pipelines stay
+// below 2^32.
+constexpr int NEAR_ITEM = 4;  // centres per item at most
+static_assert((unsigned long long)NEAR_ITEM * NEAR_MAX_POINTS * NEAR_MAX_POINTS / 2 <= (1ull << 29), "near counters");
+
+__global__ void __launch_bounds__(TS_GROUPS_MAX * TS_GROUP_THREADS, 1)
+three_near_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ item_off, int njobs, unsigned int item0,
+                  unsigned int nitems, int centres, unsigned int* counter, unsigned int* dense, unsigned long long* work,
+                  NearParams p, int pipes) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    NearPipe* const pipe = reinterpret_cast<NearPipe*>(smem);
+    unsigned int* const U = reinterpret_cast<unsigned int*>(pipe + pipes);
+    __shared__ unsigned long long s_since, s_pairs;
+    const NearStride st = near_stride(p.n);
+    const int gi = threadIdx.x / TS_GROUP_THREADS, gt = threadIdx.x % TS_GROUP_THREADS, warp = gt >> 5, lane = gt & 31;
+    const TsPipe pp{gt, warp, lane, 1 + gi};
+    NearPipe& N = pipe[gi];
+    const int parts = (TILE + centres - 1) / centres;  // items of a tile
+    for (int b = threadIdx.x; b < st.words; b += blockDim.x) U[b] = 0;
+    if (threadIdx.x == 0) s_since = s_pairs = 0;
+    auto draw = [&]() {  // by the pipeline's first warp
+        if (warp != 0) return;
+        unsigned int t = 0;
+        if (lane == 0) t = atomicAdd(counter, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        uint4 it = make_uint4(TASK_NONE, 0, 0, 0);
+        if (t < nitems) {
+            t += item0;
+            const int slot = find_job(item_off, njobs, t);
+            const unsigned int l = t - item_off[slot];
+            it = make_uint4((unsigned)slot, l / parts, (l % parts) * centres, 0);
+        }
+        if (lane == 0) {
+            N.item = it;
+            N.stop = s_since >= (1ull << 30);
+        }
+    };
+    draw();
+    int cur = -1;
+    const unsigned lt = (1u << lane) - 1u;
+    for (;;) {
+        __syncthreads();  // every pipeline waits here with an item of another job, or none
+        if (cur >= 0) {
+            unsigned long long* g = jobs[cur].hist;
+            const int m = p.n + 1, m3 = near_words3(p.n);
+            for (int b = threadIdx.x; b < m3 + m + 1; b += blockDim.x) {
+                const int at = b < m3 ? (b / (m * m)) * st.r + (b / m % m) * st.q + b % m : st.u2 + (b - m3);
+                const unsigned int u = U[at];
+                if (u) {
+                    U[at] = 0;
+                    atomicAdd(g + b, (unsigned long long)u);
+                }
+            }
+        }
+        uint32_t next = TASK_NONE;
+        for (int g2 = 0; g2 < pipes; g2++) next = min(next, pipe[g2].item.x);  // (TASK_NONE is the largest)
+        if (next == TASK_NONE) break;  // uniform: every thread read the same words
+        __syncthreads();
+        if (threadIdx.x == 0) s_since = 0;
+        if (gt == 0) N.stop = 0;
+        __syncthreads();
+        cur = (int)next;
+        const DevJob& J = jobs[cur];
+        const uint32_t cls = J.mode & NEAR_CLASS_MASK;
+        const int nlists = cls == NEAR_ORDERED ? 2 : 1;
+        for (;;) {
+            const uint4 item = N.item;
+            if (item.x != next || N.stop) break;
+            const int tile = (int)item.y, a0 = J.tile_start[0][tile], nA = J.tile_start[0][tile + 1] - a0;
+            // tiles of each list within reach of the centre's tile
+            if (gt < 2) N.ntiles[gt] = 0;
+            pp.sync();
+            const float4 *abox = J.box[0] + 2 * (size_t)tile;
+            for (int l = 0; l < nlists; l++)
+                for (int t = (cls == NEAR_SYM ? tile : 0) + gt; t < J.ntiles[1 + l]; t += TS_GROUP_THREADS)
+                    if (boxes_near(abox, J.box[1 + l] + 2 * (size_t)t, p.reach2)) {
+                        const int at = atomicAdd(&N.ntiles[l], 1);
+                        if (at < NEAR_TILES) N.tiles[l][at] = (uint32_t)t;
+                    }
+            pp.sync();
+            if (N.ntiles[0] > NEAR_TILES || N.ntiles[nlists - 1] > NEAR_TILES) {
+                if (gt == 0) *dense = 1u;  // too many: the launch is counted by the tile kernel instead
+            } else {
+                // Entries of list l from its near tiles [t0, t1) at N[base ..),
+                // at most cap of them; returns how many there are.  The codes
+                // are scaled by `scale`; w: weight of the equal-index triples.
+                auto build = [&](int l, int t0, int t1, int base, int cap, float4 c, int ci, unsigned w) -> int {
+                    pp.sync();  // the pipeline is done with the list
+                    if (gt == 0) N.count[l] = 0;
+                    pp.sync();
+                    for (int q = t0 + warp; q < t1; q += TS_WARPS) {
+                        const int t = (int)N.tiles[l][q];
+                        const float4 *bx = J.box[1 + l] + 2 * (size_t)t, lo = bx[0], hi = bx[1];
+                        const float gx = fmaxf(0.f, fmaxf(lo.x - c.x, c.x - hi.x)), gy = fmaxf(0.f, fmaxf(lo.y - c.y, c.y - hi.y)),
+                                    gz = fmaxf(0.f, fmaxf(lo.z - c.z, c.z - hi.z));
+                        if ((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f) >= p.reach2) continue;  // warp-uniform
+                        const int b0 = J.tile_start[1 + l][t], nb = J.tile_start[1 + l][t + 1] - b0;
+#pragma unroll
+                        for (int r = 0; r < 2; r++) {
+                            const int i = lane + 32 * r;
+                            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                            int code = -1;
+                            if (i < nb && !(cls == NEAR_SYM && t == tile && i <= ci)) {
+                                v = J.pts[1 + l][b0 + i];
+                                code = near_code(c, v, p);
+                            }
+                            const unsigned in = __ballot_sync(0xffffffffu, code >= 0);
+                            if (!in) continue;
+                            int at = 0;
+                            if (lane == 0) at = atomicAdd(&N.count[l], __popc(in));
+                            at = __shfl_sync(0xffffffffu, at, 0) + __popc(in & lt);
+                            if (code >= 0) {
+                                if (w) atomicAdd(U + st.u2 + code, w);
+                                if (at < cap) {
+                                    N.x[base + at] = v.x;
+                                    N.y[base + at] = v.y;
+                                    N.z[base + at] = v.z;
+                                    N.code[base + at] = (uint32_t)code;
+                                }
+                            }
+                        }
+                    }
+                    pp.sync();
+                    const int n = N.count[l];
+                    // padding to whole groups of four
+                    if (gt < 4 && n + gt < cap && n + gt < ((n + 3) & ~3)) {
+                        N.x[base + n + gt] = N.y[base + n + gt] = N.z[base + n + gt] = NEAR_PAD;
+                        N.code[base + n + gt] = 0;
+                    }
+                    pp.sync();
+                    return n;
+                };
+                // Every pair of entries j at [jb, jb + nj) and k at [kb, kb + nk);
+                // tri: one list, j < k.  Blocks of 32 x 32 shared by the warps.
+                auto pairs = [&](int jb, int nj, int kb, int nk, bool tri) {
+                    const int bj = (nj + 31) / 32, bk = (nk + 31) / 32;
+                    const int total = tri ? bk * (bk + 1) / 2 : bj * bk;
+                    int kx = 0, jx = warp;  // block (jx, kx); tri: jx <= kx
+                    for (int t = warp; t < total; t += TS_WARPS) {
+                        while (jx >= (tri ? kx + 1 : bj)) {
+                            jx -= tri ? kx + 1 : bj;
+                            kx++;
+                        }
+                        const int k = kx * 32 + lane;
+                        const bool in = k < nk;
+                        const float x = in ? N.x[kb + k] : -NEAR_PAD, y = in ? N.y[kb + k] : -NEAR_PAD,
+                                    z = in ? N.z[kb + k] : -NEAR_PAD;
+                        unsigned int* Uq = U + (in ? (int)N.code[kb + k] * st.q : 0);
+                        const int j0 = jb + jx * 32, j1 = jb + min(nj, jx * 32 + 32);
+                        if (tri && jx == kx) near_block<true>(N, j0, j1, kb + k, x, y, z, Uq, st.r, p);
+                        else near_block<false>(N, j0, j1, 0, x, y, z, Uq, st.r, p);
+                        jx += TS_WARPS;
+                    }
+                };
+                unsigned long long done = 0;  // pairs of this item (all threads alike)
+                for (int i = (int)item.z; i < min((int)item.z + centres, nA); i++) {
+                    const float4 c = J.pts[0][a0 + i];
+                    const unsigned w = cls == NEAR_SYM ? 2u : cls == NEAR_PAIR ? 1u : 0u;
+                    if (cls == NEAR_SYM && gt == 0) atomicAdd(U + st.u2 + p.n + 1, 1u);
+                    if (cls != NEAR_ORDERED) {
+                        const int n = build(0, 0, N.ntiles[0], 0, NEAR_CAP, c, i, w);
+                        done += (unsigned long long)n * (unsigned)max(n - 1, 0) / 2;
+                        if (n <= NEAR_CAP) {
+                            pairs(0, n, 0, n, true);
+                        } else {
+                            for (int u = 0; u < N.ntiles[0]; u += NEAR_CHUNK) {
+                                const int nu = build(0, u, min(u + NEAR_CHUNK, N.ntiles[0]), 0, NEAR_CAP / 2, c, i, 0u);
+                                pairs(0, nu, 0, nu, true);
+                                for (int v = u + NEAR_CHUNK; v < N.ntiles[0]; v += NEAR_CHUNK) {
+                                    const int nv = build(0, v, min(v + NEAR_CHUNK, N.ntiles[0]), NEAR_CAP / 2, NEAR_CAP / 2, c, i, 0u);
+                                    pairs(0, nu, NEAR_CAP / 2, nv, false);
+                                }
+                            }
+                        }
+                    } else {
+                        const int n0 = build(0, 0, N.ntiles[0], 0, NEAR_CAP / 2, c, i, 0u);
+                        const int n1 = build(1, 0, N.ntiles[1], NEAR_CAP / 2, NEAR_CAP / 2, c, i, 0u);
+                        done += (unsigned long long)n0 * (unsigned)n1;
+                        if (n0 <= NEAR_CAP / 2 && n1 <= NEAR_CAP / 2) {
+                            pairs(0, n0, NEAR_CAP / 2, n1, false);
+                        } else {
+                            for (int u = 0; u < N.ntiles[0]; u += NEAR_CHUNK) {
+                                const int nu = build(0, u, min(u + NEAR_CHUNK, N.ntiles[0]), 0, NEAR_CAP / 2, c, i, 0u);
+                                for (int v = 0; v < N.ntiles[1]; v += NEAR_CHUNK) {
+                                    const int nv = build(1, v, min(v + NEAR_CHUNK, N.ntiles[1]), NEAR_CAP / 2, NEAR_CAP / 2, c, i, 0u);
+                                    pairs(0, nu, NEAR_CAP / 2, nv, false);
+                                }
+                            }
+                        }
+                    }
+                }
+                if (gt == 0 && done) {
+                    atomicAdd(&s_since, done);
+                    atomicAdd(&s_pairs, done);
+                }
+            }
+            pp.sync();  // the pipeline is done with the item and its list
+            draw();
+            pp.sync();
+        }
+    }
+    if (threadIdx.x == 0 && s_pairs) atomicAdd(work, s_pairs);
+}
+
+// Sums over centres of products of their near counts, WB or WC, and the pair
+// counts PBC: one warp per centre makes the two histograms, the CTA adds up the
+// products.  hist: the sums (m x m, row: first list), aux: the pairs (m),
+// weighted; with NEAR_SYM both lists are the same.
+constexpr int WEDGE_ITEMS = TILE / TS_WARPS;  // items (TS_WARPS centres) of a tile
+
+size_t three_wedge_smem_bytes(int n) { return (size_t)TS_WARPS * 2 * (n + 1) * sizeof(unsigned int); }
+
+__global__ void __launch_bounds__(TS_GROUP_THREADS)
+three_wedge_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ item_off, int njobs,
+                   unsigned int nitems, NearParams p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned int* const H = reinterpret_cast<unsigned int*>(smem);  // [warp][list][code]
+    __shared__ int s_job;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = p.n + 1;
+    for (unsigned int t = blockIdx.x; t < nitems; t += gridDim.x) {
+        __syncthreads();
+        if (warp == 0) {
+            const int slot = find_job(item_off, njobs, t);
+            if (lane == 0) s_job = slot;
+        }
+        for (int b = threadIdx.x; b < TS_WARPS * 2 * m; b += blockDim.x) H[b] = 0;
+        __syncthreads();
+        const DevJob& J = jobs[s_job];
+        const unsigned int l = t - item_off[s_job];
+        const int tile = (int)(l / WEDGE_ITEMS), a0 = J.tile_start[0][tile], nA = J.tile_start[0][tile + 1] - a0;
+        const int i = (int)(l % WEDGE_ITEMS) * TS_WARPS + warp;
+        const bool sym = (J.mode & NEAR_CLASS_MASK) == NEAR_SYM;
+        if (i < nA) {
+            const float4 c = J.pts[0][a0 + i];
+            for (int x = 0; x < (sym ? 1 : 2); x++) {
+                unsigned int* h = H + (warp * 2 + x) * m;
+                for (int q0 = 0; q0 < J.ntiles[1 + x]; q0 += 32) {
+                    bool near = false;
+                    if (q0 + lane < J.ntiles[1 + x]) {
+                        const float4 *bx = J.box[1 + x] + 2 * (size_t)(q0 + lane), lo = bx[0], hi = bx[1];
+                        const float gx = fmaxf(0.f, fmaxf(lo.x - c.x, c.x - hi.x)), gy = fmaxf(0.f, fmaxf(lo.y - c.y, c.y - hi.y)),
+                                    gz = fmaxf(0.f, fmaxf(lo.z - c.z, c.z - hi.z));
+                        near = !((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f) >= p.reach2);
+                    }
+                    for (unsigned mask = __ballot_sync(0xffffffffu, near); mask; mask &= mask - 1u) {
+                        const int q = q0 + __ffs(mask) - 1, b0 = J.tile_start[1 + x][q], nb = J.tile_start[1 + x][q + 1] - b0;
+#pragma unroll
+                        for (int r = 0; r < 2; r++)
+                            if (lane + 32 * r < nb) {
+                                const int code = near_code(c, J.pts[1 + x][b0 + lane + 32 * r], p);
+                                if (code >= 0) atomicAdd(h + code, 1u);
+                            }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        const int y = sym ? 0 : m;
+        for (int e = threadIdx.x; e < m * m + m; e += blockDim.x) {
+            unsigned long long s = 0;
+            if (e < m * m) {
+                for (int w = 0; w < TS_WARPS; w++)
+                    s += (unsigned long long)H[w * 2 * m + e / m] * H[w * 2 * m + y + e % m];
+                if (s) atomicAdd(J.hist + e, s);
+            } else if (J.aux) {
+                for (int w = 0; w < TS_WARPS; w++) s += H[w * 2 * m + y + (e - m * m)];
+                if (s) atomicAdd(J.aux + (e - m * m), s * J.weight);
+            }
+        }
+    }
+}
+
+// Expands accumulators (job: its hist) into the histograms (its aux): the
+// orderings of each multiset, and in the reference's mode the triples with
+// sides at or above hist_max.
+__global__ void __launch_bounds__(256) three_expand_kernel(const DevJob* __restrict__ accs, NearParams p) {
+    const DevJob& A = accs[blockIdx.y];
+    const uint32_t cls = A.mode & NEAR_CLASS_MASK, centre = A.mode >> NEAR_CENTRE_SHIFT;
+    const int n = p.n, m = n + 1, m3 = m * m * m, z = p.zcode, F = n + 1;
+    const unsigned long long *U = A.hist, *U2 = U + m3, *WB = U2 + m + 1, *WC = WB + m * m, *P = WC + m * m;
+    auto at = [&](int pp, int q, int r) { return U[(r * m + q) * m + pp]; };
+    auto put = [&](int v0, int v1, int v2, unsigned long long u) {
+        const long long x = ((long long)v2 * n + v1) * n + v0;
+        if (x < p.len) atomicAdd(A.aux + x, u);
+    };
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m3 + 2 * m * m + m; e += gridDim.x * blockDim.x) {
+        if (e < m3) {
+            const int a = e % m, b = e / m % m, c = e / (m * m);
+            unsigned long long u;
+            if (cls == NEAR_SYM) {
+                u = at(a, b, c) + at(a, c, b) + at(b, a, c) + at(b, c, a) + at(c, a, b) + at(c, b, a);
+                if (a == z && b == c) u += U2[b];
+                if (b == z && a == c) u += U2[a];
+                if (c == z && a == b) u += U2[a];
+                if (a == z && b == z && c == z) u += U2[m];
+            } else if (cls == NEAR_PAIR) {
+                if (centre == 0) u = at(a, b, c) + at(b, a, c) + (c == z && a == b ? U2[a] : 0ull);
+                else if (centre == 1) u = at(a, c, b) + at(c, a, b) + (b == z && a == c ? U2[a] : 0ull);
+                else u = at(b, c, a) + at(c, b, a) + (a == z && b == c ? U2[b] : 0ull);
+            } else {
+                u = at(a, b, c);
+            }
+            if (!u) continue;
+            put(a, b, c, u);
+            if (!p.clean) {
+                put(a, F, c, 0ull - u);
+                put(F, b, c, 0ull - u);
+                put(F, F, c, u);
+            }
+        } else if (!p.clean) {
+            const int k = e - m3;
+            if (k < m * m) {
+                const unsigned long long w = WB[k];
+                if (w) {
+                    put(k / m, F, k % m, w);
+                    put(F, F, k % m, 0ull - w);
+                    if (cls == NEAR_SYM) {
+                        put(F, k / m, k % m, w);
+                        put(F, F, k % m, 0ull - w);
+                    }
+                }
+            } else if (k < 2 * m * m) {
+                const unsigned long long w = WC[k - m * m];
+                if (w) {
+                    put(F, (k - m * m) / m, (k - m * m) % m, w);
+                    put(F, F, (k - m * m) % m, 0ull - w);
+                }
+            } else if (P[k - 2 * m * m]) {
+                put(F, F, k - 2 * m * m, P[k - 2 * m * m]);
+            }
+        }
+    }
+}
+
+cudaError_t launch_three_near(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
+                              unsigned int nitems, int centres, unsigned int* counter, unsigned int* dense,
+                              unsigned long long* work, const NearParams& p, int grid, int pipes, cudaStream_t st) {
+    if (pipes < 1 || pipes > TS_GROUPS_MAX || centres < 1 || centres > NEAR_ITEM) return cudaErrorInvalidValue;
+    three_near_kernel<<<grid, pipes * TS_GROUP_THREADS, three_near_smem_bytes(p.n, pipes), st>>>(
+        jobs, item_off, njobs, item0, nitems, centres, counter, dense, work, p, pipes);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_three_wedges(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int nitems,
+                                const NearParams& p, int grid, cudaStream_t st) {
+    if (nitems == 0) return cudaSuccess;
+    three_wedge_kernel<<<std::min<unsigned int>(nitems, grid), TS_GROUP_THREADS, three_wedge_smem_bytes(p.n), st>>>(
+        jobs, item_off, njobs, nitems, p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_three_expand(const DevJob* accs, int naccs, const NearParams& p, cudaStream_t st) {
+    const int m = p.n + 1, words = m * m * m + 2 * m * m + m;
+    // (at most 65535 accumulators a launch)
+    for (int a = 0; a < naccs; a += 65535) {
+        const dim3 grid(std::min(32, (words + 255) / 256), std::min(65535, naccs - a));
+        three_expand_kernel<<<grid, 256, 0, st>>>(accs + a, p);
+    }
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // Pair counts (src/2pcf_C_version.cc).
 
@@ -2281,18 +2779,6 @@ __device__ __forceinline__ void pair_share(int n, int nA, F&& f) {
         const int i0 = (u % split) * len;
         if (i0 < nA) f(u / split, i0, min(i0 + len, nA));
     }
-}
-
-// Squared gap of two tile boxes (reduced by a margin that covers the rounding
-// of the bound and of the reference's separation) below reach2: the tiles can
-// hold a counted pair.
-__device__ __forceinline__ bool boxes_near(const float4* __restrict__ A, const float4* __restrict__ B, float reach2) {
-    const float4 al = A[0], ah = A[1], bl = B[0], bh = B[1];
-    const float gx = fmaxf(0.f, fmaxf(al.x - bh.x, bl.x - ah.x));
-    const float gy = fmaxf(0.f, fmaxf(al.y - bh.y, bl.y - ah.y));
-    const float gz = fmaxf(0.f, fmaxf(al.z - bh.z, bl.z - ah.z));
-    // (an overflowing gap is kept below an infinite reach only)
-    return !((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f) >= reach2);
 }
 
 // Persistent over items (job, tile A, chunk of tiles B); the first warp draws
@@ -2452,7 +2938,7 @@ cudaError_t prepare_kernels(int device) {
                          (const void*)three_side_kernel<true, false>, (const void*)three_side_kernel<false, true>,
                          (const void*)three_side_kernel<false, false>, (const void*)three_side_grouped_kernel<true>,
                          (const void*)three_side_grouped_kernel<false>, (const void*)pair_kernel<true>,
-                         (const void*)pair_kernel<false>};
+                         (const void*)pair_kernel<false>, (const void*)three_near_kernel, (const void*)three_wedge_kernel};
     for (const void* f : fns) {
         cudaFuncAttributes fa;
         e = cudaFuncGetAttributes(&fa, f);
