@@ -803,6 +803,12 @@ __device__ __forceinline__ void magic_bits2(f32x2 f_m, uint32_t& b0, uint32_t& b
 // points: 24 -> 18 instructions a pair).
 __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void count_at(uint32_t addr) { asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr)); }
+// UNIT: every weight is one
+template <bool UNIT>
+__device__ __forceinline__ void count_at(uint32_t addr, unsigned w) {
+    if (UNIT) count_at(addr);
+    else asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(w));
+}
 
 // theta_fast of two cosines; t: 1 - |c|, y: its reciprocal square root
 __device__ __forceinline__ void theta_fast2(f32x2 c, const TriParams& p, f32x2& f_m, f32x2& thr, f32x2& t, f32x2& y) {
@@ -845,11 +851,11 @@ __device__ __forceinline__ void theta_fast2(f32x2 c, const TriParams& p, f32x2& 
 // recomputed.  (Every triangle in double is bound by the FP64 pipe, two lanes a
 // clock and SM: DDD+DDR+DRR+RRR of 1k points 251 ms; so 0.65 ms, 0.2 % of the
 // binned triangles recomputed.)
-template <bool THETA_FULL, bool GEOM>
+template <bool THETA_FULL, bool GEOM, bool UNIT>
 __device__ __forceinline__ void triangle_full2(const float (&a)[2], const int (&wa)[2], const float (&b)[2],
                                                const int (&wb)[2], const float (&c)[2], const int (&wc)[2],
                                                const unsigned (&w)[2], const TriParams& p, unsigned int* Hw,
-                                               bool (&guard)[2]) {
+                                               unsigned int* dump, bool (&guard)[2]) {
     float s[2], m[2], l[2];
     int off_s[2], off_m[2];
     bool v02[2], v1[2];
@@ -943,9 +949,11 @@ __device__ __forceinline__ void triangle_full2(const float (&a)[2], const int (&
             ok1 = ok1 && (unsigned)t1b[t] < (unsigned)p.T;
             ok2 = ok2 && (unsigned)t2b[t] < (unsigned)p.T;
         }
-        if (ok0) atomicAdd(Hw + (off_s[t] + q0b[t]) * p.T + t0b[t], w[t]);
-        if (ok1) atomicAdd(Hw + (off_m[t] + q1b[t]) * p.T + t1b[t], w[t]);
-        if (ok2) atomicAdd(Hw + (off_s[t] + q2b[t]) * p.T + t2b[t], w[t]);
+        // (uncounted permutations add to the lane's dump word: no branches)
+        const uint32_t base = shared_addr(Hw), none = shared_addr(dump);
+        count_at<UNIT>(ok0 ? base + 4u * (uint32_t)((off_s[t] + q0b[t]) * p.T + t0b[t]) : none, w[t]);
+        count_at<UNIT>(ok1 ? base + 4u * (uint32_t)((off_m[t] + q1b[t]) * p.T + t1b[t]) : none, w[t]);
+        count_at<UNIT>(ok2 ? base + 4u * (uint32_t)((off_s[t] + q2b[t]) * p.T + t2b[t]) : none, w[t]);
         guard[t] = g;
     }
 }
@@ -1026,6 +1034,7 @@ struct TriShared {
     float box[2][6];
     float abox[6];
     int4 meta[TRI_GROUP_A];
+    unsigned int dump[32];  // counts of permutations that do not count, by lane
 };
 constexpr int TRI_DIAG_IJ = 1, TRI_CHECK_B = 2, TRI_CHECK_C = 4;
 
@@ -1034,10 +1043,10 @@ constexpr int TRI_DIAG_IJ = 1, TRI_CHECK_B = 2, TRI_CHECK_C = 4;
 
 // Runs the full binning path on n (<= 64) queued candidates, two per lane
 // (packed into the f32x2 instructions of one binning path).
-template <bool THETA_FULL, int MODE>
+template <bool THETA_FULL, int MODE, bool UNIT>
 __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, const int2* row_ij, const int2* row_ik,
                                                const float* JKd, const short* JKw, const TriParams& p, unsigned int* Hw,
-                                               RecheckQueue& q, const TriShared& S, uint32_t ia) {
+                                               RecheckQueue& q, TriShared& S, uint32_t ia) {
     const int lane = threadIdx.x & 31;
     const uint32_t e0 = lane < n ? cand[lane] : 0u;
     const uint32_t e1 = lane + 32 < n ? cand[lane + 32] : 0u;
@@ -1056,7 +1065,7 @@ __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, cons
         return;
     }
     bool guard[2];
-    triangle_full2<THETA_FULL, MODE == FAST_GEOM>(fa, wa, fb, wb, fc, wc, ww, p, Hw, guard);
+    triangle_full2<THETA_FULL, MODE == FAST_GEOM, UNIT>(fa, wa, fb, wb, fc, wc, ww, p, Hw, S.dump + lane, guard);
     const bool g0 = guard[0], g1 = guard[1];
     const uint32_t slot = S.unit.x & UNIT_SLOT_MASK;
     if (g0) push_recheck(q, slot, w0, ia, (uint32_t)(S.b0 + j0), (uint32_t)(S.c0 + k0));
@@ -1373,7 +1382,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                     if (qn >= 64) {
                         __syncwarp();
                         qn -= 64;
-                        run_candidates<THETA_FULL, MODE>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
+                        run_candidates<THETA_FULL, MODE, PRED != PRED_DDR && PRED != PRED_RDD>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
                         bn += 64;
                         __syncwarp();
                     }
@@ -1381,7 +1390,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             }
             __syncwarp();
             if (qn > 0) {
-                run_candidates<THETA_FULL, MODE>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
+                run_candidates<THETA_FULL, MODE, PRED != PRED_DDR && PRED != PRED_RDD>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
                 bn += qn;
             }
             __syncwarp();
