@@ -624,6 +624,17 @@ Binning make_binning(const tpcf_spec& sp) {
         p.t_hi = sp.axis[2].hi;
         p.t_bw = ref_bw(p.t_lo, p.t_hi, p.T);
         p.nan_zero = 0;  // no NaN reaches a counted JBJ bin (zero sides are dropped)
+        // guard bands of the fast bins (jbj_full2); binnings too fine for them
+        // take the reference's divisions for every triangle
+        auto axis_guard = [](float lo, float hi, float bw, float& scale, float& off, float& thr) {
+            const double D = std::max(fabs((double)lo), fabs((double)hi)) / (double)bw + 1.0;
+            const bool ok = D <= 65536.0 && bw >= 1e-30f;
+            scale = ok ? (float)(1.0 / (double)bw) : 1.0f;
+            off = ok ? (float)(-(double)lo / (double)bw - 0.5) : 0.0f;
+            thr = ok ? (float)(0.5 - 1e-6 * (D + 1.0)) : -1.0f;
+        };
+        axis_guard(p.q_lo, p.q_hi, p.q_bw, p.q_scale, p.q_off, p.q_thr);
+        axis_guard(p.t_lo, p.t_hi, p.t_bw, p.t_coef[0], p.t_off0, p.t_thrA);
         b.len = p.len;
         // counted: s < s_hi, s/m >= q_lo, (l - m)/s < t_hi, so
         // l < s_hi/q_lo + max(t_hi, 0) s_hi (margins cover the float roundings)

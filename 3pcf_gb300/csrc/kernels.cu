@@ -960,11 +960,14 @@ __device__ __forceinline__ void triangle_full2(const float (&a)[2], const int (&
 
 // JBJ binning of two triangles (src/3pcf_C_version_triangle_parametrization_JBJ.cc
 // distance(), :116-229): one permutation, s = shortest, q = s/m and
-// theta = (l - m)/s in float, binned as distance_to_bin does.  These are the
-// reference's float operations done exactly (IEEE division), so no guard band
-// is needed.  The s-bin comes from the shortest side's word; a triangle whose
-// weight index says its shortest side is out of range, zero or rejected, or
-// whose multiplicity is 0, adds nothing.
+// theta = (l - m)/s in float, binned as distance_to_bin does.  The coordinates
+// come from rcp.approx in packed instructions; one inside the guard band of a
+// bin edge (1e-6 of the coordinate range: the reciprocal's two ulps and the
+// roundings of either side are below 6e-7 of it) is recomputed with the
+// reference's own divisions.  The s-bin comes from the shortest side's word; a
+// triangle whose weight index says its shortest side is out of range, zero or
+// rejected, or whose multiplicity is 0, adds nothing.  (Four IEEE divisions for
+// every triangle: 20.6 ms instead of 18.5 on 5k + 5k points.)
 
 // distance_to_bin: -1 outside [lo, hi); the bin as the reference truncates it,
 // which rounding can make n at the top edge (the index then runs into the
@@ -974,20 +977,42 @@ __device__ __forceinline__ int jbj_axis_bin(float v, float lo, float hi, float b
     return __float2int_rz(__fdiv_rn(__fsub_rn(v, lo), bw));
 }
 
+template <bool UNIT>
 __device__ __forceinline__ void jbj_full2(const float (&a)[2], const int (&wa)[2], const float (&b)[2],
                                           const int (&wb)[2], const float (&c)[2], const int (&wc)[2],
-                                          const unsigned (&w)[2], const TriParams& p, unsigned int* Hw) {
+                                          const unsigned (&w)[2], const TriParams& p, unsigned int* Hw,
+                                          unsigned int* dump) {
+    float s[2], m[2], l[2];
+    int code[2];
+    bool v[2];
 #pragma unroll
     for (int t = 0; t < 2; t++) {
-        const unsigned idx = weight_index(wa[t], wb[t], wc[t]);
-        const bool v = w[t] && mask_bit(VALID_02, idx);
+        v[t] = w[t] && mask_bit(VALID_02, weight_index(wa[t], wb[t], wc[t]));
         const float lo_ab = fminf(a[t], b[t]), hi_ab = fmaxf(a[t], b[t]);
-        const float s = fminf(lo_ab, c[t]), l = fmaxf(hi_ab, c[t]), m = fmaxf(lo_ab, fminf(hi_ab, c[t]));
-        const int code = min(min(wa[t], wb[t]), wc[t]) >> 7;  // s-bin of the shortest side
-        const int i1 = jbj_axis_bin(__fdiv_rn(s, m), p.q_lo, p.q_hi, p.q_bw);
-        const int i2 = jbj_axis_bin(__fdiv_rn(__fsub_rn(l, m), s), p.t_lo, p.t_hi, p.t_bw);
-        const int x = (code * p.Q + i1) * p.T + i2;
-        if (v && i1 >= 0 && i2 >= 0 && x < p.len) atomicAdd(Hw + x, w[t]);
+        s[t] = fminf(lo_ab, c[t]);
+        l[t] = fmaxf(hi_ab, c[t]);
+        m[t] = fmaxf(lo_ab, fminf(hi_ab, c[t]));
+        code[t] = min(min(wa[t], wb[t]), wc[t]) >> 7;  // s-bin of the shortest side
+    }
+    const f32x2 S = pk2(s[0], s[1]), M = pk2(m[0], m[1]), L = pk2(l[0], l[1]);
+    const f32x2 q = mul2(S, pk2(rcp_approx(m[0]), rcp_approx(m[1])));
+    const f32x2 th = mul2(sub2(L, M), pk2(rcp_approx(s[0]), rcp_approx(s[1])));
+    int i1[2], i2[2];
+    float e1[2], e2[2];
+    magic_floor2(fma2(q, splat2(p.q_scale), splat2(p.q_off)), i1[0], i1[1], e1[0], e1[1]);
+    magic_floor2(fma2(th, splat2(p.t_coef[0]), splat2(p.t_off0)), i2[0], i2[1], e2[0], e2[1]);
+    const uint32_t base = shared_addr(Hw), none = shared_addr(dump);
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        const bool safe = fabsf(e1[t]) <= p.q_thr && fabsf(e2[t]) <= p.t_thrA;
+        const bool take = v[t] && safe && (unsigned)i1[t] < (unsigned)p.Q && (unsigned)i2[t] < (unsigned)p.T;
+        count_at<UNIT>(take ? base + 4u * (uint32_t)((code[t] * p.Q + i1[t]) * p.T + i2[t]) : none, w[t]);
+        if (v[t] && !safe) {
+            const int x1 = jbj_axis_bin(__fdiv_rn(s[t], m[t]), p.q_lo, p.q_hi, p.q_bw);
+            const int x2 = jbj_axis_bin(__fdiv_rn(__fsub_rn(l[t], m[t]), s[t]), p.t_lo, p.t_hi, p.t_bw);
+            const int x = (code[t] * p.Q + x1) * p.T + x2;
+            if (x1 >= 0 && x2 >= 0 && x < p.len) atomicAdd(Hw + x, w[t]);
+        }
     }
 }
 
@@ -1061,7 +1086,7 @@ __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, cons
     const int wc[2] = {JKw[j0 * TILE + k0], JKw[j1 * TILE + k1]};
     const unsigned ww[2] = {w0, w1};
     if (MODE == FAST_JBJ) {
-        jbj_full2(fa, wa, fb, wb, fc, wc, ww, p, Hw);
+        jbj_full2<UNIT>(fa, wa, fb, wb, fc, wc, ww, p, Hw, S.dump + lane);
         return;
     }
     bool guard[2];
