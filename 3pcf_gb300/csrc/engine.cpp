@@ -229,6 +229,7 @@ struct View {
     DevBuf<float4> box;          // tile boxes: lo at 2 t, hi at 2 t + 1
     std::vector<int32_t> h_tile_start;
     std::vector<Box> boxes;
+    double extent = 0;        // mean widest side of its tiles' boxes
     size_t upload_bytes = 0;  // host-to-device bytes of its construction
     size_t bytes() const { return pts.bytes() + tile_start.bytes() + box.bytes(); }
 };
@@ -437,6 +438,7 @@ struct Binning {
     ThreeParams three{};
     NearParams near{};
     bool near_ok = false;     // three-side: the binning suits the neighbour lists
+    bool list_ok = false;     // triangles: the same
     PairParams pair{};
     int len = 0;
     double lmax = INFINITY;   // no counted triangle/pair has a side >= lmax
@@ -581,8 +583,9 @@ Binning make_binning(const tpcf_spec& sp) {
         double tmax = std::max(fabs((double)p.t_lo), fabs((double)p.t_hi)) / (double)p.t_bw + K * pi;
         double A = 4e-6 * K + 1e-6 * tmax + 2e-6;
         p.t_thrA = (float)(0.5 - A);
-        // c-dependent part: |dc| <= 5e-7 |c| amplified by 1/sqrt(1-c^2) <= 1/sqrt(1-|c|)
-        p.t_thrB = (float)(5e-7 * K);
+        // c-dependent part: |dc| <= 7e-7 |c| (reciprocals of two sides, products, the
+        // reference's roundings: 9 x 2^-24, and a margin) amplified by 1/sqrt(1-c^2) <= 1/sqrt(1-|c|)
+        p.t_thrB = (float)(7e-7 * K);
         p.t2_off = (float)((1.0 - 3.0 * (double)p.t_lo) / (double)p.t_bw - 1.5);
         p.theta_full = (p.t_lo <= 0.f && p.t_hi >= 1.f);
         if (sp.precision == TPCF_GEOMETRY_FP64) {
@@ -663,6 +666,26 @@ Binning make_binning(const tpcf_spec& sp) {
         // (no counted separation at all below a negative upper edge)
         b.pair.reach2 = b.lmax < 0 ? 0.f : r2 < 3e38 ? nextafterf((float)r2, INFINITY) : INFINITY;
     }
+    if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) {
+        // a counted triangle has its shortest side below s_hi and its middle one
+        // below q_hi S or s_hi (JBJ: at most S / q_lo); margins cover the roundings
+        TriParams& p = b.tri;
+        const bool jbj = sp.kind == TPCF_TRIANGLE_JBJ;
+        const double q = jbj ? (p.q_lo > 0 ? 1.0 / (double)p.q_lo : INFINITY) : (double)p.q_hi;
+        const double reach = std::max((double)p.s_hi * q, jbj ? 0.0 : (double)p.s_hi) * (1 + 2e-5) + 1e-6;
+        b.list_ok = sp.prune && p.s_hi > 0 && q > 0 && reach < 1e15 && p.S <= MAX_FAST_S;
+        if (b.list_ok) {
+            p.list_r2 = nextafterf((float)(reach * reach), INFINITY);
+            p.list_q = nextafterf((float)(q * (1 + 1e-5)), INFINITY);
+            // guard bands of tri_list_bin
+            const double K = 1.0 / (3.14159 * (double)p.t_bw);
+            const double qmax = std::max(fabs((double)p.q_lo), fabs((double)p.q_hi)) / (double)p.q_bw;
+            const bool geo = sp.precision == TPCF_GEOMETRY_FP64;
+            p.list_t = jbj ? (float)(1e-6 / (double)p.t_bw) : (float)((geo ? 6e-6 : 2.2e-6) * K);
+            p.list_q_thr = geo ? p.q_thr : (float)(0.5 - (1.2e-6 * qmax + 3e-6));
+            p.list_top = jbj ? 0.f : nextafterf((float)((double)p.s_hi * (1 + 1e-5)), INFINITY);
+        }
+    }
     // device copy of the bound, rounded up so that a float side >= it is >= lmax
     if (sp.kind == TPCF_TRIANGLE_JBJ) b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
     if (sp.kind == TPCF_TRIANGLE) {
@@ -734,6 +757,7 @@ struct Lane {
     std::vector<uint64_t> plan_sig;
     uint32_t plan_rows = 0;  // rows (pairs: items) of the plan
     int plan_chunk = 0;      // pairs: tiles B per item; neighbour lists: centres per item
+    int plan_parts = 1, plan_kparts = 1;  // triangle lists: shares of a centre
     uint32_t plan_wedges = 0;  // neighbour lists: items of the wedge kernel
     // the launch sequence of the last batch, captured as a CUDA graph and
     // replayed while the batch and every buffer it touches stay the same
@@ -777,6 +801,9 @@ struct Lane {
 };
 
 // d_counters: words zeroed before every count, then the header of the plan
+// shares of centres per warp of the triangle lists at least
+constexpr uint64_t TL_WANT = 32;
+
 constexpr int CTR_WORK = 0;     // units (items) handed out
 constexpr int CTR_RECHECK = 1;  // queued guard-band triangles
 constexpr int CTR_EVAL = 2;     // evaluated (two words), binned (pairs: tile pairs; two words)
@@ -935,6 +962,11 @@ std::shared_ptr<View> build_view(const Catalog& c, int64_t begin, int64_t end, i
             }
         }
         v->boxes[t] = b;
+    }
+    for (const Box& b : v->boxes) {
+        double w = 0;
+        for (int a = 0; a < 3; a++) w = std::max(w, (double)b.hi[a] - (double)b.lo[a]);
+        v->extent += w / v->ntiles;
     }
     const auto tv3 = std::chrono::steady_clock::now();
     v->pts.reserve(pts.size());
@@ -1186,7 +1218,7 @@ size_t shape_smem(const tpcf_spec& sp, const Binning& bin, int copies, int group
 // Launch shapes worth trying for a group, the default first.  The guarded
 // triangle kernel is compiled for four CTAs per SM (its register budget);
 // the others take as many CTAs as shared memory allows, up to 8.
-std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Binning& bin, bool fp64, bool near) {
+std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Binning& bin, bool fp64, bool near, int tlist) {
     int max_smem_sm = 0, max_smem_block = 0;
     cudaDeviceGetAttribute(&max_smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
     cudaDeviceGetAttribute(&max_smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
@@ -1215,6 +1247,24 @@ std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Bi
             sh.per_sm = sh.smem + 1024 <= (size_t)max_smem_block ? 1 : 0;
             add(sh);
         }
+        return out;
+    }
+    if (tlist) {  // (tlist: output slots of the launch)
+        // as many warps per SM as the registers and the lists' shared memory
+        // allow, in CTAs of 8 to 24 warps that share histograms; groups: warps per CTA
+        for (int w : {8, 24, 12, 20, 16}) {
+            Shape sh;
+            sh.groups = w;
+            // every slot's histogram in shared memory where they take at most 24 KB of a CTA
+            sh.copies = (size_t)bin.len * 4 * tlist <= 24576 ? tlist : 1;
+            sh.smem = tri_list_smem_bytes(bin.len, sh.copies, w);
+            sh.per_sm = sh.smem + 1024 <= (size_t)max_smem_block
+                            ? std::min(TL_MAX_WARPS / w, (int)(max_smem_sm / (sh.smem + 1024))) : 0;
+            add(sh);
+        }
+        std::stable_sort(out.begin(), out.end(),
+                         [](const Shape& a, const Shape& b) { return a.per_sm * a.groups > b.per_sm * b.groups; });
+        if (out.size() > 3) out.resize(3);
         return out;
     }
     if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) {
@@ -1286,7 +1336,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     const int ncat = sp.kind == TPCF_PAIR ? 2 : 3;
     const bool pairs = sp.kind == TPCF_PAIR;
     bool tame = true;  // (asked by the double-precision geometry and the neighbour lists only)
-    if (sp.precision == TPCF_GEOMETRY_FP64 || bin.near_ok) {
+    if (sp.precision == TPCF_GEOMETRY_FP64 || bin.near_ok || bin.list_ok) {
         std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
         for (const GroupJob& g : group)
             for (int r = 0; r < ncat; r++) {
@@ -1298,13 +1348,50 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     // three-side counts from neighbour lists (see three_near_kernel)
     const char* near_env = getenv("TPCF_NEAR");
     const bool near = lists && bin.near_ok && tame && !(near_env && near_env[0] == '0') &&
-                      !shape_candidates(ctx, sp, bin, fp64, true).empty() &&
+                      !shape_candidates(ctx, sp, bin, fp64, true, 0).empty() &&
                       three_near_acc_words(bin.three.n) * group.size() <= ((size_t)1 << 27);
-    const bool items = pairs || near;  // kernels that find their tiles themselves
     const bool tri_kind = sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ;
     const bool fast_tri = tri_kind && !fp64;
     const bool fast_jbj = sp.kind == TPCF_TRIANGLE_JBJ && !fp64;  // the fast kernel's JBJ binning
     const bool geom = sp.precision == TPCF_GEOMETRY_FP64;
+    // Triangles from neighbour lists (see TriCentre) instead of tile triples:
+    //   where the tile kernel's tables leave room for one CTA beside the
+    //   histogram (50 x 16 x 25 bins, DDD+DDR+DRR+RRR twice: 5k-point cone 5.15 ->
+    //   2.0 ms, 5k-point blobs 91 -> 52 ms, 500 points 0.91 -> 0.72 ms);
+    //   where tiles are wide against s_hi (three times), so that few of a tile
+    //   triple's triangles are near (1,024 bins: 5k-point cone 1.31 -> 0.69 ms, 2k
+    //   0.41 -> 0.19 ms, 500 points 0.13 -> 0.09 ms; blobs of 500 points, whose
+    //   tiles are 6 to 20 across, the other way round: 2k 3.04 -> 3.3 ms, 10k 11.4
+    //   -> 14.4 ms);
+    //   JBJ with many centres, whose tile triples hold few shortest sides in
+    //   range (5k-point blobs 36 -> 28 ms, 2k 4.4 -> 4.7 ms).
+    // Sets of many small jobs (voxels) keep the tiles: each of a job's centres
+    // is an item here (16,500 jobs of a 20k cone 3.4 -> 8.8 ms).
+    const char* tl_env = getenv("TPCF_TRI_LISTS");
+    bool tlist = fast_tri && bin.list_ok && tame && !(tl_env && tl_env[0] == '0') &&
+                 group.size() <= (tl_env ? (size_t)1000000 : (size_t)64) &&
+                 !shape_candidates(ctx, sp, bin, fp64, false, 1).empty();
+    bool sparse = false;
+    if (tlist) {
+        uint64_t centres = 0;
+        double extent = INFINITY;
+        for (const GroupJob& g : group) {
+            int64_t n[3];
+            for (int r = 0; r < 3; r++) {
+                auto v = get_view(ctx, L, g.job->catalog[r], g.job->begin[r], g.job->end[r],
+                                  (g.job->flags & TPCF_JOB_GLOBAL_INDEX) != 0);
+                n[r] = v->n;
+                extent = std::min(extent, v->extent);
+            }
+            // (a role's points are centres once where roles share a view)
+            centres += g.spec->loop == TPCF_LOOP_SAME ? n[0] : n[0] + n[2];
+        }
+        sparse = extent > 3 * (double)bin.tri.s_hi;
+        if (!tl_env)
+            tlist = shape_candidates(ctx, sp, bin, fp64, false, 0)[0].per_sm < 2 || sparse ||
+                    (fast_jbj && centres >= 20000);
+    }
+    const bool items = pairs || near || tlist;  // kernels that find their tiles themselves
     if (group.size() > MAX_BATCH_JOBS) throw InvalidArg{"too many jobs in one batch"};
     std::vector<std::pair<const char*, double>> phases;
     auto phase = [&](const char* name) {
@@ -1374,7 +1461,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     sig.push_back((uint64_t)(uintptr_t)L.d_hist.p);
     {
         const uint64_t f[6] = {(uint64_t)sp.kind, (uint64_t)sp.prune, (uint64_t)sp.precision, (uint64_t)sp.nan_policy,
-                               (uint64_t)sp.overflow, (uint64_t)near << 2 | (uint64_t)rdd << 1 | (uint64_t)sym_three};
+                               (uint64_t)sp.overflow, (uint64_t)tlist << 3 | (uint64_t)near << 2 | (uint64_t)rdd << 1 | (uint64_t)sym_three};
         sig.insert(sig.end(), f, f + 6);
         for (int a = 0; a < 3; a++) {
             sig.push_back((uint64_t)fbits(sp.axis[a].lo) << 32 | fbits(sp.axis[a].hi));
@@ -1390,6 +1477,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         uint32_t mode;
     };
     std::vector<RoleJob> roles(group.size());
+    // triangles from neighbour lists: what is launched instead of the jobs
+    struct SubJob {
+        uint32_t range[3], mode, job;
+    };
+    std::vector<SubJob> subs;
     uint64_t units = 0;
     // reference loop size of job g
     auto job_units = [&](size_t g) {
@@ -1425,7 +1517,38 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         auto id = [&](int r) { return ranges[rg[r]].ref.id; };
         const bool ab = id(0) == id(1), bc = id(1) == id(2);
         uint32_t mode = PRED_NONE, v[3] = {rg[0], rg[1], rg[2]};
-        if (near) {
+        if (tlist) {
+            // the job's triangles by the role of their centre: each with its
+            // lists' views (one view: its unordered pairs)
+            uint32_t pred = PRED_NONE;
+            uint32_t rank[3] = {0, 1, 2};
+            auto sub = [&](int rc, int r1, int r2, bool self) {
+                SubJob sj{};
+                sj.range[0] = rg[rc], sj.range[1] = rg[r1], sj.range[2] = rg[r2];
+                sj.job = (uint32_t)g;
+                sj.mode = pred | (self ? TL_SELF : 0u) | (uint32_t)(rc | r1 << 2 | r2 << 4) << TL_ROLE_SHIFT |
+                          (rank[rc] | rank[r1] << 2 | rank[r2] << 4) << TL_RANK_SHIFT;
+                subs.push_back(sj);
+            };
+            if (ab && bc && jsp.loop == TPCF_LOOP_SAME) {
+                rank[1] = rank[2] = 0;
+                sub(0, 1, 2, true);
+            } else if (ab && !bc && jsp.loop == TPCF_LOOP_ONE) {
+                pred = PRED_DDR;
+                rank[1] = 0;
+                sub(2, 0, 1, true);
+                sub(0, 1, 2, false);
+            } else if (bc && !ab && jsp.loop == TPCF_LOOP_ONE) {
+                rank[2] = rank[1];
+                sub(0, 1, 2, true);
+                sub(1, 0, 2, false);
+            } else {
+                pred = jsp.loop == TPCF_LOOP_SAME ? PRED_SAME : jsp.loop == TPCF_LOOP_ONE ? PRED_ONE : PRED_NONE;
+                sub(0, 1, 2, false);
+                sub(1, 0, 2, false);
+                sub(2, 0, 1, false);
+            }
+        } else if (near) {
             // the centre: the point of the view that appears once, or any
             const bool ac = id(0) == id(2);
             if (ab && bc && sym_three) {
@@ -1481,7 +1604,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     }
     cudaStream_t st = L.stream;
     L.d_counters.reserve(CTR_WORDS);
-    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near);
+    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near, tlist ? (int)nslots : 0);
     const bool plan_hit = sig == L.plan_sig;
     phase("batch");
     const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
@@ -1504,6 +1627,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         L.d_acc.reserve(acc_words * accs.size());
     }
     uint32_t nwedges = L.plan_wedges;
+    int plan_parts = L.plan_parts, plan_kparts = L.plan_kparts;  // triangle lists: shares of a centre
     PlanHeader* d_header = nullptr;
     // Finds the units of the batch on the device (see plan_rows): the host
     // gives each job's number of rows.
@@ -1538,9 +1662,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         for (Range& r : ranges) r.view = get_view(ctx, L, r.key.h, r.key.b, r.key.e, r.key.gl);
         phase("views");
         CK(cudaStreamSynchronize(st));  // (a failed batch may still read the pinned buffers)
-        const size_t njobs = group.size() + nwedge_jobs + accs.size();
+        const size_t njobs = tlist ? subs.size() : group.size() + nwedge_jobs + accs.size();
         L.h_jobs.reserve(njobs);
-        L.h_rows.reserve(group.size() + nwedge_jobs + 2);
+        L.h_rows.reserve(njobs + 2);
         uint64_t rows = 0;
         plan_chunk = 0;
         if (pairs) {
@@ -1553,8 +1677,37 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             uint64_t centres = 0;
             for (const RoleJob& r : roles) centres += ranges[r.range[0]].view->n;
             plan_chunk = centres < 64ull * ctx->num_sms * 4 ? 1 : 4;
+        } else if (tlist) {
+            uint64_t centres = 0;
+            for (const SubJob& sj : subs) centres += ranges[sj.range[0]].view->n;
+            const uint64_t warps = (uint64_t)ctx->num_sms * TL_MAX_WARPS;
+            plan_chunk = centres < 64 * warps ? 1 : 4;
+            plan_parts = 1;
+            plan_kparts = 1;
+            // (J's shares first: a share of K's fills its J lists again; a sparse
+            // view's centres are light)
+            while (plan_parts * plan_kparts < (sparse ? 2 : 64) && centres * plan_parts * plan_kparts < TL_WANT * warps)
+                if (plan_parts < 16) plan_parts *= 2;
+                else plan_kparts *= 2;
+            for (size_t k = 0; k < subs.size(); k++) {
+                DevJob d{};
+                for (int r = 0; r < 3; r++) {
+                    const View& v = *ranges[subs[k].range[r]].view;
+                    d.pts[r] = v.pts.p;
+                    d.tile_start[r] = v.tile_start.p;
+                    d.box[r] = v.box.p;
+                    d.ntiles[r] = v.ntiles;
+                }
+                d.mode = subs[k].mode;
+                d.hist = L.d_hist.p + (size_t)bin.len * slot_of[subs[k].job];
+                d.weight = (unsigned long long)ranges[subs[k].range[0]].view->n | (unsigned long long)slot_of[subs[k].job] << 32;
+                L.h_jobs.p[k] = d;
+                L.h_rows.p[k] = (uint32_t)rows;
+                rows += (uint64_t)plan_parts * plan_kparts * (((uint64_t)ranges[subs[k].range[0]].view->n + plan_chunk - 1) / plan_chunk);
+                if (rows > 0xF0000000ull) throw InvalidArg{"too many points in one batch"};
+            }
         }
-        for (size_t g = 0; g < group.size(); g++) {
+        for (size_t g = 0; g < (tlist ? 0 : group.size()); g++) {
             DevJob d{};
             for (int r = 0; r < 3; r++) {
                 const View& v = *ranges[roles[g].range[r]].view;
@@ -1574,9 +1727,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             else if (d.ntiles[2] > 0) rows += (uint64_t)((d.ntiles[0] + window - 1) / window) * d.ntiles[1];
             if (rows > 0xF0000000ull) throw InvalidArg{"too many tile pairs in one batch"};
         }
-        L.h_rows.p[group.size()] = (uint32_t)rows;
+        size_t nr = tlist ? subs.size() : group.size();
+        L.h_rows.p[nr++] = (uint32_t)rows;
         nrows = (uint32_t)rows;
-        size_t nr = group.size() + 1;
         if (near) {
             // wedge jobs: pairs of sides at a point of role B (lists A, C; the
             // pairs B-C weigh the points of A) and of role C (lists A, B)
@@ -1631,13 +1784,17 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         L.plan_rows = nrows;
         L.plan_chunk = plan_chunk;
         L.plan_wedges = nwedges;
+        L.plan_parts = plan_parts;
+        L.plan_kparts = plan_kparts;
         phase("plan");
     }
     L.stats.plan_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_wall0).count();
     if (sp.kind == TPCF_TRIANGLE) ensure_acos(ctx);
     const AcosTable acos_t = sp.kind == TPCF_TRIANGLE ? acos_table(ctx) : AcosTable{};
-    uint64_t launches = (sp.kind == TPCF_TRIANGLE && !fp64) ? 2 : 1;  // counting (+ recheck)
+    // guard-band triangles are queued and recomputed (JBJ tiles: in the kernel)
+    const bool recheck = fast_tri && (!fast_jbj || tlist);
+    uint64_t launches = recheck ? 2 : 1;  // counting (+ recheck)
     const char* genv = getenv("TPCF_GRAPHS");
     const bool graphs = L.graphs_ok && !(genv && genv[0] == '0');
     L.h_hist.reserve(hist_total);
@@ -1675,9 +1832,10 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                                                  : std::max(nwork, 1u);
             if (L.slice_batches && ctx->slice_tasks > 0) slice = (unsigned int)ctx->slice_tasks;
             launches = (nwork > slice ? (nwork + slice - 1) / slice : 1) +
-                       (sp.kind == TPCF_TRIANGLE && !fp64 ? 1 : near ? (nwedges ? 2 : 1) : 0);
+                       (recheck ? 1 : near ? (nwedges ? 2 : 1) : 0);
             RecheckQueue q{};
-            if (sp.kind == TPCF_TRIANGLE && !fp64) {
+            q.hists = L.d_hist.p;
+            if (recheck) {
                 if (L.d_queue.n < queue_cap) L.drop_graph();
                 L.d_queue.reserve(queue_cap);
                 q.items = L.d_queue.p;
@@ -1703,6 +1861,10 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                 auto launch_main = [&](unsigned int t0, unsigned int n) -> cudaError_t {
                     unsigned int* counter = L.d_counters.p + CTR_WORK;
                     const UnitList ul{d_header, L.d_units.p, L.d_masks.p, t0, n};
+                    if (tlist)
+                        return launch_tri_list(L.d_jobs.p, L.d_rows.p, (int)subs.size(), t0, n, plan_chunk, plan_parts,
+                                               plan_kparts, copies,
+                                               counter, bin.tri, q, grid, sh.groups, fast_jbj ? 1 : geom ? 2 : 0, st);
                     if (fast_tri)  // (JBJ: exact without a recheck)
                         return launch_triangle_fast(L.d_jobs.p, ul, counter, bin.tri, q, grid, copies,
                                                     fast_jbj ? 1 : geom ? 2 : 0, st);
@@ -1736,8 +1898,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                                            ctx->num_sms * 8, st));
                     EQ(launch_three_expand(after + nwedge_jobs, (int)accs.size(), bin.near, st));
                 }
-                if (sp.kind == TPCF_TRIANGLE && !fp64)
-                    EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, geom ? 1 : 0, ctx->num_sms * 8, st));
+                if (recheck)
+                    EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, fast_jbj ? 1 : geom ? 2 : 0,
+                                               ctx->num_sms * 8, st));
                 EQ(cudaEventRecordWithFlags(L.ev1, st, ev_flags));
                 EQ(cudaMemcpyAsync(L.h_counters.p, L.d_counters.p, CTR_WORDS * sizeof(unsigned int),
                                    cudaMemcpyDeviceToHost, st));
@@ -1757,7 +1920,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                                           (uint64_t)(uintptr_t)acos_t.bucket, (uint64_t)acos_t.n, queue_cap,
                                           (uint64_t)grid, (uint64_t)copies, (uint64_t)sh.groups, hist_total,
                                           (uint64_t)nwork, (uint64_t)slice, (uint64_t)(uintptr_t)L.d_rows.p,
-                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk,
+                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk, (uint64_t)plan_parts << 32 | (uint64_t)plan_kparts,
                                           (uint64_t)(uintptr_t)L.d_acc.p};
                 gsig.insert(gsig.end(), extra, extra + sizeof(extra) / sizeof(extra[0]));
                 if (!L.graph || gsig != L.graph_sig) {
@@ -1801,7 +1964,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             L.stats.recheck_units = counters[CTR_RECHECK];
             memcpy(&dev_evaluated, &counters[CTR_EVAL], sizeof(dev_evaluated));
             memcpy(&dev_binned, &counters[CTR_EVAL + 2], sizeof(dev_binned));
-            if (sp.kind == TPCF_TRIANGLE && !fp64 && counters[CTR_RECHECK] > queue_cap) {
+            if (recheck && counters[CTR_RECHECK] > queue_cap) {
                 // the recheck queue overflowed: grow it and count again
                 queue_cap = (unsigned int)std::min<uint64_t>(
                     (uint64_t)counters[CTR_RECHECK] + (counters[CTR_RECHECK] >> 2) + 1024, 0xF0000000ull);
@@ -1886,7 +2049,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     // their units
     L.stats.evaluated_units = fast_tri || items ? dev_evaluated : header.evaluated;
     L.stats.binned_units = fast_tri ? dev_binned : L.stats.evaluated_units;
-    L.stats.tasks = pairs ? dev_binned : near ? nrows : header.tiles;
+    L.stats.tasks = pairs ? dev_binned : near || tlist ? nrows : header.tiles;
     L.stats.kernel_launches = launches * std::max<uint64_t>(1, tuned_runs);
     L.stats.recheck_regrows = regrows;
     L.stats.total_ms =

@@ -101,6 +101,10 @@ struct TriParams {
     float lmax;                  // sides >= lmax cannot belong to a counted triangle
     float mid_hi;                // s_hi * q_hi (rounded up): permutation 0 needs two sides below it,
                                  // permutation 1 needs all three below it
+    // neighbour lists: squared reach of a centre, limit max(q S, top) of the
+    // middle side given the shortest
+    float list_r2, list_q, list_top;
+    float list_t, list_q_thr;    // guard slope of an angle (JBJ: of theta), guard of a ratio
     // double-precision geometry: sides that are surely below s_lo / at or above
     // s_hi, the s coordinate (minus 0.5) and its guard, slope of the angle's
     float geo_s_below, geo_s_above, geo_s_inv, geo_s_off, geo_s_thr, geo_t;
@@ -165,6 +169,7 @@ struct RecheckQueue {
     uint4* items;                // {slot | weight << RECHECK_WEIGHT_SHIFT, ia, ib, ic}
     unsigned int* count;
     unsigned int cap;
+    unsigned long long* hists;      // neighbour lists: the launch's first histogram
     unsigned long long* evaluated;  // triangles of (i,j) pairs the fast kernel walked
 };
 
@@ -210,7 +215,7 @@ struct UnitList {
 cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
                                  RecheckQueue q, int grid, int hist_copies, int mode, cudaStream_t st);
 cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t,
-                                    int geom, int grid, cudaStream_t st);
+                                    int mode, int grid, cudaStream_t st);
 cudaError_t launch_triangle_fp64(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
                                  AcosTable t, int grid, int hist_copies, int mode,
                                  cudaStream_t st);  // mode: 0 FP64, 1 geometry, 2 JBJ
@@ -227,7 +232,21 @@ cudaError_t launch_acos_check(AcosTable t, uint32_t key_begin, uint32_t count, u
 cudaError_t launch_radecz_to_xyz(const double* ra, const double* dec, const double* redshift, int64_t n,
                                  const double poly[3], float* x, float* y, float* z, cudaStream_t st);
 
-// The three launches of a neighbour-list count; *dense is set where the near
+// Triangle parametrizations from neighbour lists.  Its jobs (roles: centre,
+// first list, second list; weight: the centre view's points and, from bit 32,
+// the output slot) have in
+// DevJob::mode the reference's predicate, whether both lists are one view's
+// unordered pairs, and for centre and lists two bits each of the reference's
+// role and of the rank that orders points of different views.
+constexpr int TL_MAX_WARPS = 24;  // warps per SM of its register budget
+constexpr uint32_t TL_SELF = 8u;
+constexpr int TL_ROLE_SHIFT = 4, TL_RANK_SHIFT = 10;
+cudaError_t launch_tri_list(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
+                            unsigned int nitems, int centres, int parts, int kparts, int hists, unsigned int* counter,
+                            const TriParams& p, RecheckQueue q, int grid, int warps, int mode, cudaStream_t st);
+size_t tri_list_smem_bytes(int hist_len, int hists, int warps);
+
+// The three launches of a three-side neighbour-list count; *dense is set where the near
 // tiles of a centre are too many (count with launch_three_side instead).
 cudaError_t launch_three_near(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
                               unsigned int nitems, int centres, unsigned int* counter, unsigned int* dense,

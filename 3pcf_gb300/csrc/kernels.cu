@@ -803,6 +803,12 @@ __device__ __forceinline__ void magic_bits2(f32x2 f_m, uint32_t& b0, uint32_t& b
 // points: 24 -> 18 instructions a pair).
 __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void count_at(uint32_t addr) { asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr)); }
+// A predicated 16-bit store to a 32-bit shared-memory address (no branch).
+__device__ __forceinline__ void store_if(bool ok, uint32_t addr, uint32_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u16 [%0], %1;\n\t}" ::"r"(addr),
+                 "h"((unsigned short)v), "r"((unsigned)ok)
+                 : "memory");
+}
 // UNIT: every weight is one
 template <bool UNIT>
 __device__ __forceinline__ void count_at(uint32_t addr, unsigned w) {
@@ -1016,7 +1022,7 @@ __device__ __forceinline__ void jbj_full2(const float (&a)[2], const int (&wa)[2
     }
 }
 
-__device__ __forceinline__ void push_recheck(RecheckQueue& q, uint32_t slot, unsigned w, uint32_t ia, uint32_t ib,
+__device__ __forceinline__ void push_recheck(const RecheckQueue& q, uint32_t slot, unsigned w, uint32_t ia, uint32_t ib,
                                              uint32_t ic) {
     unsigned int pos = atomicAdd(q.count, 1u);
     if (pos < q.cap) q.items[pos] = make_uint4(slot | (w << RECHECK_WEIGHT_SHIFT), ia, ib, ic);
@@ -1495,28 +1501,517 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
     }
 }
 
-// Exact recomputation of queued guard-band triangles (GEOM: of the
-// double-precision geometry).
-template <bool GEOM>
-__global__ void triangle_recheck_kernel(const DevJob* __restrict__ jobs, RecheckQueue q, TriParams p, AcosTable t) {
-    unsigned int n = *q.count;
-    if (n > q.cap) n = q.cap;
-    for (unsigned int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        uint4 it = q.items[e];
-        const DevJob& J = jobs[it.x & UNIT_SLOT_MASK];
-        unsigned w = it.x >> RECHECK_WEIGHT_SHIFT;
-        float4 pa = J.pts[0][it.y], pb = J.pts[1][it.z], pc = J.pts[2][it.w];
-        int out[3];
-        if (GEOM) tp_geom(geo_dist(pa, pb), geo_dist(pa, pc), geo_dist(pb, pc), p, out);
-        else tp_exact<false>(ref_dist<false>(pa, pb), ref_dist<false>(pa, pc), ref_dist<false>(pb, pc), p, t, out);
-        for (int k = 0; k < 3; k++)
-            if (out[k] >= 0) atomicAdd(J.hist + out[k], (unsigned long long)w);
+// ---------------------------------------------------------------------------
+// Triangle parametrizations from neighbour lists.
+//
+// Each triangle is taken at one of its points, the centre: the one opposite its
+// longest side, so that the centre's two sides are the shortest S and the
+// middle M (equal longest sides: the first of the points concerned in (rank,
+// position) order, sides compared as the reference's floats).  A counted
+// triangle has S < s_hi and M below a limit of S (q_hi S, 1/q_lo S for JBJ, or
+// s_hi): for a centre the points within s_hi ("near") make J lists, all points
+// within the largest limit K lists, and a pair (j, k) whose third side is the
+// longest is a triangle.  One warp per centre, lists of 64 in shared memory
+// filled in the order of the views' tiles and used up in turn, pairs tested
+// eight to a lane, and what passes queued and binned two to a lane.  No
+// barrier but where the CTA's shared histogram changes hands.
+//
+// Issue-bound: 14 lane-instructions a tested pair, 29 to queue what passes (of
+// 32), some 250 to fetch, test and bin one.  Against tile triples
+// (triangle_group_fast) it wins where those have few CTAs, or few near
+// triangles (run_group has the rule and the times).  Tried and left: two
+// triangles a lane in packed instructions (500 instructions a batch of 64, no
+// faster), marks kept by each lane and binned one a round instead of a queue
+// (30 % of the lanes idle: 10k-point blobs 14.3 -> 16.7 ms), 32 warps of 64
+// registers instead of 24 of 80 (17.4 against 15.3 ms), a CTA barrier per change
+// of output slot (all slots' histograms are resident where they fit).
+
+constexpr int TL_LIST = 64;  // entries of a list
+constexpr int TL_QCAP = 288;  // queued pairs: up to 31 pending + 256 of one step
+constexpr unsigned TL_SPILL = 1u << 28;
+constexpr int TL_TILES = 64;  // near tiles kept per list (more: found again at every pass)
+
+struct TriListWarp {
+    // lists J (0) and K (1)
+    float x[2][TL_LIST], y[2][TL_LIST], z[2][TL_LIST], d[2][TL_LIST];
+    int code[2][TL_LIST];
+    uint32_t pos[2][TL_LIST];
+    float lim[TL_LIST];  // J: squared limit of the middle side
+    uint16_t queue[TL_QCAP];
+    uint32_t tiles[2][TL_TILES];
+    unsigned int dump[32];
+    uint4 item;          // job, first centre, centres, part
+};
+
+size_t tri_list_smem_bytes(int hist_len, int hists, int warps) {
+    return (size_t)warps * sizeof(TriListWarp) + (size_t)hist_len * hists * 4;
+}
+
+// Which points of a view a list takes.
+constexpr int TL_NEAR = 1, TL_FAR = 2;
+
+// A bin coordinate (minus 0.5) as the bits of coordinate + MAGIC (bin =
+// bits - MAGIC_BITS) and its distance from the bin's centre.
+__device__ __forceinline__ uint32_t magic_bits(float f, float& e) {
+    const float tm = __fadd_rn(f, MAGIC);
+    e = __fsub_rn(f, __fsub_rn(tm, MAGIC));
+    return __float_as_uint(tm);
+}
+
+// The angle's coordinate of theta_fast2 for one cosine; t: 1 - |c|, y: its
+// reciprocal square root.
+__device__ __forceinline__ void theta_fast(float c, const TriParams& p, float& f, float& t, float& y) {
+    const float x = fabsf(c);
+    t = __fsub_rn(1.0f, x);
+    y = rsqrt_approx(t);
+    const float sq = __fmul_rn(t, y);
+    float P = fmaf(p.t_coef[5], x, p.t_coef[4]);
+    P = fmaf(P, x, p.t_coef[3]);
+    P = fmaf(P, x, p.t_coef[2]);
+    P = fmaf(P, x, p.t_coef[1]);
+    P = fmaf(P, x, p.t_coef[0]);
+    const float a = fmaf(sq, P, -p.t_half);
+    f = __int_as_float(__float_as_int(a) ^ (__float_as_int(c) & 0x80000000)) + p.t_off0;
+}
+
+// Bins a triangle of weight w (0: none) with sides s <= m <= l (l2: about the
+// square of l) and the s-bin codes of s and m; true where it has to be
+// recomputed exactly.  One triangle a lane: two in packed instructions took 500
+// instructions a batch of 64 here, spilled registers among them.
+//
+// s and m are the reference's floats, l2 a fused sum of the same differences.
+// With u = 2^-24 the numerator of a cosine is within 13 u of the sum of the
+// squares of the reference's and its reciprocal denominator within 8 u, so the
+// cosine within 21 u E = 1.25e-6 E, E = (s^2 + m^2 + l^2) / (2 s m): the guard
+// takes 1.5e-6 E, moves an angle by at most 1.42 times that over sqrt(1 - |c|),
+// and a cosine within twice that of +-1 is always recomputed.  Ratios of l are
+// within 15 u.  (The double-precision geometry: see triangle_full2.)
+template <int MODE>
+__device__ __forceinline__ bool tri_list_bin(float s, float m, float l2, int cs, int cm, unsigned w, const TriParams& p,
+                                             uint32_t base, uint32_t none) {
+    const bool v02 = w && (unsigned)cs < (unsigned)p.S;  // shortest side in range
+    const bool v1 = w && (unsigned)cm < (unsigned)p.S;   // middle side in range
+    const float rs = rcp_approx(s), rm = rcp_approx(m), rl = rsqrt_approx(l2), l = l2 * rl;
+    // address of (code, q bits, t bits): both MAGIC_BITS folded into the base
+    const uint32_t Q = (uint32_t)p.Q, T4 = 4u * (uint32_t)p.T;
+    const uint32_t at = base - (uint32_t)MAGIC_BITS * (T4 + 4u);
+    if (MODE == FAST_JBJ) {
+        float e1, e2;
+        const uint32_t b1 = magic_bits(fmaf(s * rm, p.q_scale, p.q_off), e1);
+        const uint32_t b2 = magic_bits(fmaf((l - m) * rs, p.t_coef[0], p.t_off0), e2);
+        // (l - m cancels: its error is 8 u l / s)
+        const bool safe = fabsf(e1) <= p.q_thr && fabsf(e2) <= fmaf(-p.list_t, l * rs, p.t_thrA);
+        const bool take = v02 && safe && b1 - MAGIC_BITS < Q && b2 - MAGIC_BITS < (uint32_t)p.T;
+        count_at<false>(take ? ((uint32_t)cs * Q + b1) * T4 + (4u * b2 + at) : none, w);
+        return v02 && !safe;
+    }
+    const float s2 = s * s, m2 = m * m;
+    const float rsq = rs * p.q_scale, rmq = rm * p.q_scale, hsm = rs * rm * 0.5f, hml = rm * rl * 0.5f;
+    const float sm2 = s2 + m2;
+    float q0e, q1e, q2e, t0e, t1e, t2e;
+    const uint32_t q0 = magic_bits(fmaf(m, rsq, p.q_off), q0e), q1 = magic_bits(fmaf(l, rmq, p.q_off), q1e),
+                   q2 = magic_bits(fmaf(l, rsq, p.q_off), q2e);
+    float f0, f1, thr0, thr1, tc0, tc1, y0, y1;
+    theta_fast((sm2 - l2) * hsm, p, f0, tc0, y0);
+    theta_fast((m2 - s2 + l2) * hml, p, f1, tc1, y1);
+    const float sum2 = sm2 + l2, E0 = sum2 * hsm, E1 = sum2 * hml;
+    constexpr float close = MODE == FAST_GEOM ? 8e-6f : 3e-6f;
+    thr0 = tc0 > close * E0 ? fmaf(-p.list_t, E0 * y0, p.t_thrA) : -1.f;
+    thr1 = tc1 > close * E1 ? fmaf(-p.list_t, E1 * y1, p.t_thrA) : -1.f;
+    bool us = true, um = true;
+    if (MODE == FAST_GEOM) {
+        float es, em;
+        magic_bits(fmaf(s, p.geo_s_inv, p.geo_s_off), es);
+        magic_bits(fmaf(m, p.geo_s_inv, p.geo_s_off), em);
+        us = fabsf(es) <= p.geo_s_thr;
+        um = fabsf(em) <= p.geo_s_thr;
+    }
+    const uint32_t t0 = magic_bits(f0, t0e), t1 = magic_bits(f1, t1e),
+                   t2 = magic_bits(p.t2_off - f0 - f1, t2e);
+    const bool u02 = fabsf(q0e) <= p.list_q_thr && fabsf(t0e) <= thr0 && fabsf(q2e) <= p.list_q_thr &&
+                     fabsf(t2e) <= thr0 + thr1 + (-0.5f - 1e-6f) && us;
+    const bool u1 = fabsf(q1e) <= p.list_q_thr && fabsf(t1e) <= thr1 && um;
+    const bool guard = (v02 && !u02) || (v1 && !u1);
+    const bool n02 = v02 && !guard, n1 = v1 && !guard;
+    const uint32_t T = (uint32_t)p.T, rs0 = (uint32_t)cs * Q, rm0 = (uint32_t)cm * Q;
+    const bool ok0 = n02 && q0 - MAGIC_BITS < Q && t0 - MAGIC_BITS < T;
+    const bool ok1 = n1 && q1 - MAGIC_BITS < Q && t1 - MAGIC_BITS < T;
+    const bool ok2 = n02 && q2 - MAGIC_BITS < Q && t2 - MAGIC_BITS < T;
+    count_at<false>(ok0 ? (rs0 + q0) * T4 + (4u * t0 + at) : none, w);
+    count_at<false>(ok1 ? (rm0 + q1) * T4 + (4u * t1 + at) : none, w);
+    count_at<false>(ok2 ? (rs0 + q2) * T4 + (4u * t2 + at) : none, w);
+    return guard;
+}
+
+// One warp's centre: its job, its point, and the running state of its lists.
+template <int MODE>
+struct TriCentre {
+    const DevJob& J;
+    const TriParams& p;
+    TriListWarp& W;
+    const RecheckQueue& rq;
+    const uint32_t base;
+    const uint32_t slot;
+    float4 c;
+    uint32_t cpos;
+    int near0, near1;  // near tiles of each list's view
+    __device__ __forceinline__ int ntl(int v) const { return v ? near1 : near0; }
+    int qn = 0;       // queued pairs
+    unsigned tested = 0, binned = 0, accounted = 0;
+    unsigned int *H, *since;  // the CTA's histograms and triangles since they were flushed
+    unsigned long long* out;  // where they are flushed to
+    int nbins;
+    int lane;
+
+    __device__ __forceinline__ TriCentre(const DevJob& J_, const TriParams& p_, TriListWarp& W_, const RecheckQueue& rq_,
+                                         unsigned int* H_, int hists, unsigned int* since_, uint32_t slot_)
+        : J(J_), p(p_), W(W_), rq(rq_),
+          base(shared_addr(H_) + (hists == 1 ? 0u : 4u * (uint32_t)(J_.weight >> 32) * (uint32_t)p_.len)), slot(slot_),
+          H(H_), since(since_), out(hists == 1 ? J_.hist : rq_.hists), nbins(hists * p_.len), lane(threadIdx.x & 31) {}
+
+    __device__ __forceinline__ bool near_box(const float4* bx) const {
+        const float4 lo = bx[0], hi = bx[1];
+        const float gx = fmaxf(0.f, fmaxf(lo.x - c.x, c.x - hi.x)), gy = fmaxf(0.f, fmaxf(lo.y - c.y, c.y - hi.y)),
+                    gz = fmaxf(0.f, fmaxf(lo.z - c.z, c.z - hi.z));
+        return (gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f) < p.list_r2;
+    }
+    // near tiles of view v (role 1 + v)
+    __device__ __forceinline__ int find_tiles(int v) {
+        int n = 0;
+        for (int t0 = 0; t0 < J.ntiles[1 + v]; t0 += 32) {
+            const bool near = t0 + lane < J.ntiles[1 + v] && near_box(J.box[1 + v] + 2 * (size_t)(t0 + lane));
+            const unsigned m = __ballot_sync(0xffffffffu, near);
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            if (near && at < TL_TILES) W.tiles[v][at] = (uint32_t)(t0 + lane);
+            n += __popc(m);
+        }
+        __syncwarp();
+        return n;
+    }
+    // Steps (half tiles) of view v before `end` (even): the tile of step s,
+    // advancing s past tiles out of reach where the near tiles are not kept; -1
+    // (s = end) where none is left.  s never goes back: an even s moves to the
+    // first half of a tile at or after it, an odd s stays.
+    __device__ __forceinline__ int tile_at(int v, int end, int& s) const {
+        if (s >= end) return -1;
+        if (ntl(v) <= TL_TILES) return (int)W.tiles[v][s >> 1];
+        if (s & 1) return s >> 1;  // (its first half found it)
+        for (int t0 = s >> 1; 2 * t0 < end; t0 += 32) {
+            const bool near = 2 * (t0 + lane) < end && near_box(J.box[1 + v] + 2 * (size_t)(t0 + lane));
+            const unsigned m = __ballot_sync(0xffffffffu, near);
+            if (m) {
+                const int t = t0 + __ffs(m) - 1;
+                s = 2 * t;
+                return t;
+            }
+        }
+        s = end;
+        return -1;
+    }
+    // Fills list h (0: J, 1: K) from view v's steps s on, with the points of
+    // `which` (near points only from step `near_from` on), until it may not
+    // hold the next step or step `end` is reached; returns the entries.
+    __device__ __forceinline__ int fill(int h, int v, int which, int near_from, int end, int& s) {
+        int n = 0;
+        for (;;) {
+            const int t = tile_at(v, end, s);
+            if (t < 0 || n + 32 > TL_LIST) break;
+            const int b0 = J.tile_start[1 + v][t] + 32 * (s & 1), b1 = J.tile_start[1 + v][t + 1];
+            const bool with_near = (which & TL_NEAR) && s >= near_from;
+            s++;
+            const uint32_t pos = (uint32_t)(b0 + lane);
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            float d = 0.f;
+            bool in = b0 + lane < b1;
+            if (in) {
+                q = J.pts[1 + v][pos];
+                const float dx = __fsub_rn(c.x, q.x), dy = __fsub_rn(c.y, q.y), dz = __fsub_rn(c.z, q.z);
+                const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                in = d2 < p.list_r2;
+                if (in) d = __fsqrt_rn(d2);
+            }
+            const float s_top = MODE == FAST_GEOM ? p.geo_s_above : p.s_hi;
+            // zero sides count nowhere (the geometry's double length may not be zero: the
+            // centre itself apart, they stay); JBJ: nor do sides below s_lo
+            if (MODE == FAST_JBJ) in = in && d >= p.s_lo && d > 0.f;
+            else if (MODE == FAST_GEOM) in = in && !(pos == cpos && J.pts[1 + v] == J.pts[0]);
+            else in = in && d > 0.f;
+            in = in && (d < s_top ? with_near : (which & TL_FAR) != 0);
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) {
+                const int at = n + __popc(m & ((1u << lane) - 1u));
+                int code = CODE16_ABOVE;
+                if (MODE == FAST_GEOM) {
+                    if (d < p.geo_s_below) code = CODE16_BELOW;
+                    else if (d < s_top) code = min(max(__float2int_rz(__fdiv_rn(__fsub_rn(d, p.s_lo), p.s_bw)), 0), p.S - 1);
+                } else if (d < p.s_lo) {
+                    code = CODE16_BELOW;
+                } else if (d < s_top) {
+                    code = __float2int_rz(__fdiv_rn(__fsub_rn(d, p.s_lo), p.s_bw));
+                }
+                W.x[h][at] = q.x;
+                W.y[h][at] = q.y;
+                W.z[h][at] = q.z;
+                W.d[h][at] = d;
+                W.code[h][at] = code;
+                W.pos[h][at] = pos;
+                if (h == 0) {
+                    const float lim = fmaxf(d * p.list_q, p.list_top);
+                    W.lim[at] = lim * lim;
+                }
+            }
+            n += __popc(m);
+        }
+        // padding to whole groups of four
+        if (h == 0 && lane < 4 && n + lane < ((n + 3) & ~3)) {
+            W.x[0][n + lane] = W.y[0][n + lane] = W.z[0][n + lane] = 0.f;
+            W.d[0][n + lane] = 0.f;
+            W.lim[n + lane] = -1.f;
+        }
+        __syncwarp();
+        return n;
+    }
+    // (rank, position) order of two points
+    static __device__ __forceinline__ bool first_of(uint32_t ra, uint32_t pa, uint32_t rb, uint32_t pb) {
+        return ra < rb || (ra == rb && pa < pb);
+    }
+    // Bins queue entries [at, at + n), n <= 32.  kh: the list that k comes from
+    // (0 in pairs of one list); vj, vk: the views of j and k.
+    __device__ __forceinline__ void run(int at, int n, int kh, int vj, int vk) {
+        __syncwarp();
+        const bool any = lane < n;
+        const uint32_t e = any ? (uint32_t)W.queue[at + lane] : 0u;
+        const int j = e & 63, k = e >> 6;
+        const float4 a = make_float4(W.x[0][j], W.y[0][j], W.z[0][j], 0.f);
+        const float4 b = make_float4(W.x[kh][k], W.y[kh][k], W.z[kh][k], 0.f);
+        const float dj = W.d[0][j], dk = W.d[kh][k];
+        const int cj = W.code[0][j], ck = W.code[kh][k];
+        const float s = fminf(dj, dk), m = fmaxf(dj, dk);
+        const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z, l2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const float m2 = m * m;
+        bool take = any && l2 > m2;
+        if (any && fabsf(l2 - m2) <= 2e-6f * m2) {
+            // too close to tell: the reference's floats
+            const float l = ref_dist<false>(a, b);
+            take = l >= m && (MODE == FAST_GEOM || l > 0.f);
+            if (take && l == m) {
+            // equal longest sides: j lies opposite k's side, k opposite j's
+            const uint32_t rc = J.mode >> TL_RANK_SHIFT & 3u, r1 = J.mode >> (TL_RANK_SHIFT + 2 + 2 * vj) & 3u,
+                           r2 = J.mode >> (TL_RANK_SHIFT + 2 + 2 * vk) & 3u;
+            if (dk == m) take = first_of(rc, cpos, r1, W.pos[0][j]);
+            if (dj == m) take = take && first_of(rc, cpos, r2, W.pos[kh][k]);
+            }
+        }
+        unsigned w = take ? 1u : 0u;
+        const uint32_t pred = J.mode & JOB_PRED_MASK;
+        if (pred != PRED_NONE && take) {
+            // keys in the reference's roles
+            int key[3] = {0, 0, 0};
+            const int kc = pkey(c), kj = pkey(J.pts[1 + vj][W.pos[0][j]]), kk = pkey(J.pts[1 + vk][W.pos[kh][k]]);
+            const uint32_t oc = J.mode >> TL_ROLE_SHIFT & 3u, o1 = J.mode >> (TL_ROLE_SHIFT + 2 + 2 * vj) & 3u,
+                           o2 = J.mode >> (TL_ROLE_SHIFT + 2 + 2 * vk) & 3u;
+#pragma unroll
+            for (int r = 0; r < 3; r++) key[r] = (uint32_t)r == oc ? kc : (uint32_t)r == o1 ? kj : (uint32_t)r == o2 ? kk : 0;
+            if (pred == PRED_DDR) w = (unsigned)(key[2] >= key[0]) + (unsigned)(key[2] >= key[1]);
+            else if (pred == PRED_SAME) w = key[0] <= key[1] && key[1] <= key[2] ? 1u : 0u;
+            else w = key[1] <= key[2] ? 1u : 0u;
+        }
+        const bool guard = tri_list_bin<MODE>(s, m, l2, min(cj, ck), max(cj, ck), w, p, base, shared_addr(W.dump + lane));
+        if (guard) {  // (positions in the job's order of views)
+            const uint32_t pj = W.pos[0][j], pk = W.pos[kh][k];
+            push_recheck(rq, slot, w, cpos, vj < vk ? pj : pk, vj < vk ? pk : pj);
+        }
+        binned += (unsigned)n;
+        __syncwarp();
+    }
+    // Tests the pairs of J's nj entries with nk entries of list kh (0: of J
+    // itself, j < k) and bins those whose third side is the longest.  vj, vk:
+    // the views of j and k (0 and 1 also where both are one).
+    __device__ __forceinline__ void pairs(int nj, int nk, int kh, int vj, int vk) {
+        const unsigned lt = (1u << lane) - 1u;
+        f32x2 X[2], Y[2], Z[2];
+        float d2[2], dm[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int k = lane + 32 * r;
+            const bool in = k < nk;
+            X[r] = splat2(in ? W.x[kh][k] : 0.f);
+            Y[r] = splat2(in ? W.y[kh][k] : 0.f);
+            Z[r] = splat2(in ? W.z[kh][k] : 0.f);
+            const float d = in ? W.d[kh][k] : 3e18f;  // (past every limit)
+            d2[r] = d * d;
+            dm[r] = d2[r] * (1.0f - 1e-5f);
+        }
+        const bool two = nk > 32;
+        const uint32_t kj = (uint32_t)lane << 6, qbase = shared_addr(W.queue);
+        tested += (unsigned)(kh == 0 ? nj * (nj - 1) / 2 : nj * nk);
+        for (int j = 0; j < nj; j += 4) {
+            const float4 x4 = *reinterpret_cast<const float4*>(W.x[0] + j), y4 = *reinterpret_cast<const float4*>(W.y[0] + j),
+                         z4 = *reinterpret_cast<const float4*>(W.z[0] + j), d4 = *reinterpret_cast<const float4*>(W.d[0] + j),
+                         l4 = *reinterpret_cast<const float4*>(W.lim + j);
+            const f32x2 xj[2] = {pk2(x4.x, x4.y), pk2(x4.z, x4.w)}, yj[2] = {pk2(y4.x, y4.y), pk2(y4.z, y4.w)},
+                        zj[2] = {pk2(z4.x, z4.y), pk2(z4.z, z4.w)}, dj[2] = {pk2(d4.x, d4.y), pk2(d4.z, d4.w)};
+            const float lj[4] = {l4.x, l4.y, l4.z, l4.w};
+            float mj[4];
+            up2(mul2(mul2(dj[0], dj[0]), splat2(1.0f - 1e-5f)), mj[0], mj[1]);
+            up2(mul2(mul2(dj[1], dj[1]), splat2(1.0f - 1e-5f)), mj[2], mj[3]);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                if (r == 1 && !two) continue;  // warp-uniform
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const f32x2 dx = sub2(xj[h], X[r]), dy = sub2(yj[h], Y[r]), dz = sub2(zj[h], Z[r]);
+                    float L2[2];
+                    up2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), L2[0], L2[1]);
+#pragma unroll
+                    for (int t = 0; t < 2; t++) {
+                        const int q = 2 * h + t;
+                        const bool ok = L2[t] >= fmaxf(mj[q], dm[r]) && d2[r] < lj[q] && (kh != 0 || j + q < lane + 32 * r);
+                        const unsigned m = __ballot_sync(0xffffffffu, ok);
+                        store_if(ok, qbase + 2u * (uint32_t)(qn + __popc(m & lt)), kj + (uint32_t)(j + q + (r << 11)));
+                        qn += __popc(m);
+                    }
+                }
+            }
+            // full batches; after the last step also the rest
+            const int least = j + 4 < nj ? 32 : 1;
+            while (qn >= least) {
+                const int n = min(qn, 32);
+                qn -= n;
+                run(qn, n, kh, vj, vk);
+            }
+        }
+        // a triangle adds at most six to one bin (three permutations, weight
+        // two): the warp that brings the CTA to 2^28 triangles empties the
+        // 32-bit counters while the others count on
+        const unsigned b1 = binned - accounted;
+        if (b1) {
+            unsigned before = 0;
+            if (lane == 0) before = atomicAdd(since, b1);
+            before = __shfl_sync(0xffffffffu, before, 0);
+            if (before < TL_SPILL && before + b1 >= TL_SPILL) {
+                for (int b = lane; b < nbins; b += 32) {
+                    const unsigned int v = atomicExch(H + b, 0u);
+                    if (v) atomicAdd(out + b, (unsigned long long)v);
+                }
+                if (lane == 0) atomicSub(since, before + b1);
+            }
+            accounted = binned;
+        }
+    }
+    // The centre's triangles: J lists of the near points of view vj, each with
+    // K lists of view vk (of one view: with itself, then with the near points
+    // after it and the far ones); of two views in both ways round, the second
+    // with far points only.  Part (q, kq) of parts x kparts takes the q-th share
+    // of J's tiles and the kq-th of K's.
+    __device__ __forceinline__ void count(uint32_t centre, int q, int parts, int kq, int kparts) {
+        cpos = centre;
+        c = J.pts[0][centre];
+        const bool self = J.mode & TL_SELF;
+        near0 = find_tiles(0);
+        near1 = self ? near0 : find_tiles(1);
+        if (!near0 || !near1) return;
+        for (int pass = 0; pass < (self ? 1 : 2); pass++) {
+            const int vj = pass, vk = self ? 0 : 1 - pass;
+            const int nt = ntl(vj) <= TL_TILES ? ntl(vj) : J.ntiles[1 + vj];
+            const int share = 2 * ((nt + parts - 1) / parts), top = min(2 * nt, (q + 1) * share);
+            const int ntk = ntl(vk) <= TL_TILES ? ntl(vk) : J.ntiles[1 + vk];
+            const int kshare = 2 * ((ntk + kparts - 1) / kparts), endk = min(2 * ntk, (kq + 1) * kshare);
+            int sj = q * share;
+            while (sj < top) {
+                const int nj = fill(0, vj, TL_NEAR, 0, top, sj);
+                if (nj == 0) continue;  // (the steps are used up)
+                int sk = kq * kshare, kh = self && kq == 0 ? 0 : 1, nk = nj;
+                for (;;) {
+                    if (kh && sk >= endk) break;
+                    if (kh) nk = fill(1, vk, pass == 0 ? TL_NEAR | TL_FAR : TL_FAR, self ? sj : 0, endk, sk);
+                    if (nk > 0) pairs(nj, nk, kh, vj, self ? 1 : vk);
+                    kh = 1;
+                }
+            }
+        }
+    }
+};
+
+// Persistent; each warp draws items: up to `centres` centres of a job, or one of
+// parts x kparts shares of a centre.  The CTA holds the histograms of all `hists`
+// output slots of the launch (job: weight >> 32) where they fit; else one, and
+// a warp whose item adds to another waits for the others at a CTA barrier,
+// where it is flushed.
+template <int MODE>
+__global__ void __launch_bounds__(TL_MAX_WARPS * 32, 1)
+tri_list_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ item_off, int njobs, unsigned int item0,
+                unsigned int nitems, int centres, int parts, int kparts, int hists, unsigned int* counter,
+                const __grid_constant__ TriParams p, const __grid_constant__ RecheckQueue rq) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    TriListWarp* const warps = reinterpret_cast<TriListWarp*>(smem);
+    const int nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned int* const H = reinterpret_cast<unsigned int*>(warps + nwarps);
+    TriListWarp& W = warps[warp];
+    __shared__ unsigned int s_since;  // triangles binned since the last flush
+    for (int b = threadIdx.x; b < hists * p.len; b += blockDim.x) H[b] = 0;
+    if (threadIdx.x == 0) s_since = 0;
+    auto draw = [&]() {
+        unsigned int t = 0;
+        if (lane == 0) t = atomicAdd(counter, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        uint4 it = make_uint4(TASK_NONE, 0, 0, 0);
+        if (t < nitems) {
+            t += item0;
+            const int slot = find_job(item_off, njobs, t);
+            const unsigned int l = t - item_off[slot], all = (unsigned)(parts * kparts), first = l / all * centres;
+            it = make_uint4((unsigned)slot, first, min((unsigned)centres, (unsigned)jobs[slot].weight - first), l % all);
+        }
+        __syncwarp();
+        if (lane == 0) W.item = it;
+        __syncwarp();
+    };
+    draw();
+    unsigned long long* cur = nullptr;
+    unsigned long long tested = 0, binned = 0;
+    for (;;) {
+        __syncthreads();  // every warp waits here with an item for another histogram, or none
+        uint32_t next = TASK_NONE;
+        for (int q = 0; q < nwarps; q++) next = min(next, warps[q].item.x);  // (TASK_NONE is the largest)
+        if (cur && (hists == 1 || next == TASK_NONE)) {
+            for (int b = threadIdx.x; b < hists * p.len; b += blockDim.x) {
+                const unsigned int v = H[b];
+                if (v) {
+                    H[b] = 0;
+                    atomicAdd((hists == 1 ? cur : rq.hists) + b, (unsigned long long)v);
+                }
+            }
+        }
+        if (next == TASK_NONE) break;  // uniform: every thread read the same words
+        cur = jobs[next].hist;
+        if (threadIdx.x == 0) s_since = 0;
+        __syncthreads();
+        for (;;) {
+            const uint4 it = W.item;
+            if (it.x == TASK_NONE || (hists == 1 && jobs[it.x].hist != cur)) break;
+            const DevJob& J = jobs[it.x];
+            TriCentre<MODE> tc(J, p, W, rq, H, hists, &s_since, it.x);
+            for (uint32_t i = 0; i < it.z; i++) tc.count(it.y + i, (int)it.w % parts, parts, (int)it.w / parts, kparts);
+            tested += tc.tested;
+            binned += tc.binned;
+            draw();
+        }
+    }
+    if (lane == 0) {
+        if (tested) atomicAdd(rq.evaluated, tested);
+        if (binned) atomicAdd(rq.evaluated + 1, binned);
     }
 }
 
-// ---------------------------------------------------------------------------
-// Triangle parametrization, plain FP64: every triangle through the exact
-// reference arithmetic with each float operation done in FP64.
+cudaError_t launch_tri_list(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
+                            unsigned int nitems, int centres, int parts, int kparts, int hists, unsigned int* counter,
+                            const TriParams& p, RecheckQueue q, int grid, int warps, int mode, cudaStream_t st) {
+    const size_t smem = tri_list_smem_bytes(p.len, hists, warps);
+    auto kern = mode == FAST_JBJ ? tri_list_kernel<FAST_JBJ> : mode == FAST_GEOM ? tri_list_kernel<FAST_GEOM>
+                                                                                 : tri_list_kernel<FAST_TP>;
+    kern<<<grid, warps * 32, smem, st>>>(jobs, item_off, njobs, item0, nitems, centres, parts, kparts, hists, counter, p, q);
+    return cudaGetLastError();
+}
 
 // JBJ shape parametrization (src/3pcf_C_version_triangle_parametrization_JBJ.cc
 // distance(), :116-229): one permutation, s = shortest, q = shortest/middle,
@@ -1553,6 +2048,34 @@ __device__ __forceinline__ int jbj_index(float dist0, float dist1, float dist2, 
     const long long idx = (long long)p.Q * p.T * i0 + (long long)p.T * i1 + i2;
     return idx < p.len ? (int)idx : -1;
 }
+
+// Exact recomputation of queued guard-band triangles (GEOM: of the
+// double-precision geometry).
+template <int MODE>
+__global__ void triangle_recheck_kernel(const DevJob* __restrict__ jobs, RecheckQueue q, TriParams p, AcosTable t) {
+    unsigned int n = *q.count;
+    if (n > q.cap) n = q.cap;
+    for (unsigned int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        uint4 it = q.items[e];
+        const DevJob& J = jobs[it.x & UNIT_SLOT_MASK];
+        unsigned w = it.x >> RECHECK_WEIGHT_SHIFT;
+        float4 pa = J.pts[0][it.y], pb = J.pts[1][it.z], pc = J.pts[2][it.w];
+        if (MODE == FAST_JBJ) {
+            const int x = jbj_index(ref_dist<false>(pa, pb), ref_dist<false>(pa, pc), ref_dist<false>(pb, pc), p);
+            if (x >= 0) atomicAdd(J.hist + x, (unsigned long long)w);
+            continue;
+        }
+        int out[3];
+        if (MODE == FAST_GEOM) tp_geom(geo_dist(pa, pb), geo_dist(pa, pc), geo_dist(pb, pc), p, out);
+        else tp_exact<false>(ref_dist<false>(pa, pb), ref_dist<false>(pa, pc), ref_dist<false>(pb, pc), p, t, out);
+        for (int k = 0; k < 3; k++)
+            if (out[k] >= 0) atomicAdd(J.hist + out[k], (unsigned long long)w);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Triangle parametrization, plain FP64: every triangle through the exact
+// reference arithmetic with each float operation done in FP64.
 
 // Arithmetic of the exact per-triangle kernel.
 enum ExactMode : int {
@@ -3001,7 +3524,9 @@ cudaError_t prepare_kernels(int device) {
                          (const void*)three_side_kernel<true, false>, (const void*)three_side_kernel<false, true>,
                          (const void*)three_side_kernel<false, false>, (const void*)three_side_grouped_kernel<true>,
                          (const void*)three_side_grouped_kernel<false>, (const void*)pair_kernel<true>,
-                         (const void*)pair_kernel<false>, (const void*)three_near_kernel, (const void*)three_wedge_kernel};
+                         (const void*)pair_kernel<false>, (const void*)three_near_kernel, (const void*)three_wedge_kernel,
+                         (const void*)tri_list_kernel<FAST_TP>, (const void*)tri_list_kernel<FAST_JBJ>,
+                         (const void*)tri_list_kernel<FAST_GEOM>};
     for (const void* f : fns) {
         cudaFuncAttributes fa;
         e = cudaFuncGetAttributes(&fa, f);
@@ -3024,10 +3549,11 @@ cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t, int geom,
+cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const TriParams& p, AcosTable t, int mode,
                                     int grid, cudaStream_t st) {
-    if (geom) triangle_recheck_kernel<true><<<grid, 128, 0, st>>>(jobs, q, p, t);
-    else triangle_recheck_kernel<false><<<grid, 128, 0, st>>>(jobs, q, p, t);
+    auto kern = mode == FAST_JBJ ? triangle_recheck_kernel<FAST_JBJ> : mode == FAST_GEOM ? triangle_recheck_kernel<FAST_GEOM>
+                                                                                         : triangle_recheck_kernel<FAST_TP>;
+    kern<<<grid, 128, 0, st>>>(jobs, q, p, t);
     return cudaGetLastError();
 }
 
