@@ -688,10 +688,12 @@ Binning make_binning(const tpcf_spec& sp) {
     }
     // device copy of the bound, rounded up so that a float side >= it is >= lmax
     if (sp.kind == TPCF_TRIANGLE_JBJ) b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
-    if (sp.kind == TPCF_TRIANGLE) {
-        b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
-        double mid = (double)b.tri.s_hi * (double)b.tri.q_hi * (1 + 1e-5) + 1e-6;
-        b.tri.mid_hi = sp.prune && b.tri.q_hi > 0 ? nextafterf((float)mid, INFINITY) : INFINITY;
+    if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) {
+        TriParams& p = b.tri;
+        p.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
+        const double q = sp.kind == TPCF_TRIANGLE ? (double)p.q_hi : p.q_lo > 0 ? 1.0 / (double)p.q_lo : 0.0;
+        const double mid = (double)p.s_hi * q * (1 + 1e-5) + 1e-6;
+        p.mid_hi = sp.prune && q > 0 && mid < 3e38 ? nextafterf((float)mid, INFINITY) : INFINITY;
     }
     return b;
 }

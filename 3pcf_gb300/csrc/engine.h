@@ -99,8 +99,8 @@ struct TriParams {
     float t2_off;                // (1 - 3 t_lo)/t_bw - 0.5 - 2*(-0.5) handled in code
     int theta_full;              // theta range covers (0,1): skip range checks
     float lmax;                  // sides >= lmax cannot belong to a counted triangle
-    float mid_hi;                // s_hi * q_hi (rounded up): permutation 0 needs two sides below it,
-                                 // permutation 1 needs all three below it
+    float mid_hi;                // s_hi * q_hi (rounded up; JBJ: s_hi / q_lo): a counted triangle has a side in the s
+                                 // range and another below it (permutation 0/2: the middle one; 1: the longest)
     // neighbour lists: squared reach of a centre, limit max(q S, top) of the
     // middle side given the shortest
     float list_r2, list_q, list_top;
