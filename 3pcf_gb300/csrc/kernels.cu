@@ -1057,6 +1057,27 @@ __device__ __forceinline__ int pkey(float4 p) { return __float_as_int(p.w); }
 // What a unit's CTA shares beside the tiles: boxes (lo, hi) of tiles B and C
 // and of all A tiles of the unit, and the resident A tiles (first point,
 // points, TRI_* flags, position of the first point in its tile).
+// floats as ints of the same order (its own inverse)
+__device__ __forceinline__ int ordered_int(float x) {
+    const int v = __float_as_int(x);
+    return v ^ ((v >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float ordered_float(int v) { return __int_as_float(v ^ ((v >> 31) & 0x7fffffff)); }
+
+// Extends a box in shared memory by those of the warp's lanes that have one.
+__device__ __forceinline__ void box_add(int* box, int lane, bool has, float4 lo, float4 hi) {
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const float l = a == 0 ? lo.x : (a == 1 ? lo.y : lo.z), h = a == 0 ? hi.x : (a == 1 ? hi.y : hi.z);
+        const int mn = __reduce_min_sync(0xffffffffu, has ? ordered_int(l) : INT_MAX);
+        const int mx = __reduce_max_sync(0xffffffffu, has ? ordered_int(h) : INT_MIN);
+        if (lane == 0) {
+            atomicMin(box + a, mn);
+            atomicMax(box + 3 + a, mx);
+        }
+    }
+}
+
 struct TriShared {
     uint4 unit;
     uint32_t mask;
@@ -1064,7 +1085,9 @@ struct TriShared {
     int next_i, end_i;  // points listed of the resident A tiles: handed out, and their number
     uint8_t list[TRI_GROUP_A * TILE];
     float box[2][6];
-    float abox[6];
+    int abox[6];         // box of the unit's listed points (of its A tiles, if they are not all resident), ordered_int
+    int nj, nk;          // points of tiles B and C listed: their number and their places in the tiles, ascending
+    uint8_t jlist[TILE], klist[TILE];
     int4 meta[TRI_GROUP_A];
     unsigned int dump[32];  // counts of permutations that do not count, by lane
 };
@@ -1100,8 +1123,8 @@ __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, cons
     triangle_full2<THETA_FULL, MODE == FAST_GEOM, UNIT>(fa, wa, fb, wb, fc, wc, ww, p, Hw, S.dump + lane, guard);
     const bool g0 = guard[0], g1 = guard[1];
     const uint32_t slot = S.unit.x & UNIT_SLOT_MASK;
-    if (g0) push_recheck(q, slot, w0, ia, (uint32_t)(S.b0 + j0), (uint32_t)(S.c0 + k0));
-    if (g1) push_recheck(q, slot, w1, ia, (uint32_t)(S.b0 + j1), (uint32_t)(S.c0 + k1));
+    if (g0) push_recheck(q, slot, w0, ia, (uint32_t)(S.b0 + S.jlist[j0]), (uint32_t)(S.c0 + S.klist[k0]));
+    if (g1) push_recheck(q, slot, w1, ia, (uint32_t)(S.b0 + S.jlist[j1]), (uint32_t)(S.c0 + S.klist[k1]));
 }
 
 // Side class for candidate filtering: 0 none (zero length or too long),
@@ -1153,7 +1176,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
     float4 *PB = P, *PC = P + TILE, *PA = P + 2 * TILE;
     // every triple of the unit has the same job and tiles B and C
     bool diag_jk;
-    int numB, numC;  // points of B and C
+    int numB, numC;  // points of B and C (that can count, once these are listed)
     {
         const DevJob& J = jobs[S.unit.x & UNIT_SLOT_MASK];
         diag_jk = (J.mode & JOB_C_FROM_B) && S.unit.z == S.unit.w;
@@ -1207,31 +1230,11 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             // first point, points (of the quarter), which j come after point i: those from i + w + 1, or all
             S.meta[threadIdx.x] = make_int4(a0 + ifrom, n, (J.mode & JOB_B_FROM_A) && a == (int)unit.z, ifrom);
         }
-        if (ch == 0 && warp == 1) {  // boxes of tiles B, C and of all A tiles
+        if (ch == 0 && warp == 1) {  // boxes of tiles B and C
             if (lane < 12) {
                 const int role = lane < 6 ? 1 : 2, f = lane % 6;
                 const float4 v = J.box[role][2 * (size_t)(role == 1 ? unit.z : unit.w) + f / 3];
                 S.box[role - 1][f] = f % 3 == 0 ? v.x : (f % 3 == 1 ? v.y : v.z);
-            }
-            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-            if ((S.mask >> lane) & 1u) {
-                const float4 al = J.box[0][2 * (size_t)(unit.y + lane)], ah = J.box[0][2 * (size_t)(unit.y + lane) + 1];
-                lo[0] = al.x, lo[1] = al.y, lo[2] = al.z;
-                hi[0] = ah.x, hi[1] = ah.y, hi[2] = ah.z;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-                    hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-                }
-            if (lane == 0) {
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    S.abox[a] = lo[a];
-                    S.abox[3 + a] = hi[a];
-                }
             }
         }
         if (threadIdx.x == 0) {
@@ -1240,60 +1243,95 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             S.b0 = tb0;
             S.c0 = tc0;
         }
+        if (ch == 0 && threadIdx.x < 6) S.abox[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
         __syncthreads();
         // The points that may be part of a counted triangle, listed by one
-        // thread each: with the lower bounds of i-j, i-k and j-k by the boxes of
-        // B and C, both i-j and i-k below lmax, and a side of the s range with
-        // another below mid_hi.  (Handed out untested, 56 % of the points of the
-        // 10k-point estimator and 77 % of those of 100 voxels cost a warp a draw
-        // and a test of its own to be dropped, and others a scan of the j by which
-        // no candidate came: kernels 11.4 -> 10.0 ms and 3.42 -> 2.56 ms.)
-        if (threadIdx.x < nr * TILE) {
-            bool keep = threadIdx.x % TILE < (unsigned)max(S.meta[threadIdx.x / TILE].y, 0);
-            if (keep) {
-                const float4 pi = PA[threadIdx.x];
-                float d2[3] = {0.f, 0.f, 0.f};  // i-j, i-k, j-k
+        // thread each: by the lower bounds of its sides, all below lmax, one in
+        // the s range and another below mid_hi.  (Handed out untested, 56 % of
+        // the points of the 10k-point estimator and 77 % of those of 100 voxels
+        // cost a warp a draw and a test of its own to be dropped, and others a
+        // scan of the j by which no candidate came: kernels 11.4 -> 10.0 ms and
+        // 3.42 -> 2.56 ms.)
+        auto possible = [&](float x2, float y2, float z2) {
+            const float lo = fminf(x2, y2), hi = fmaxf(x2, y2), in = p.s_hi * (1.0f + 1e-5f), next = p.mid_hi * (1.0f + 1e-5f);
+            return fminf(lo, z2) < in * in && fmaxf(lo, fminf(hi, z2)) < next * next && fmaxf(hi, z2) < reach2;
+        };
+        // squared distances of a point from two boxes and of these from one another
+        auto bounds2 = [&](float4 pt, auto b_lo, auto b_hi, const float* c, float& pb, float& pc, float& bc) {
+            pb = pc = bc = 0.f;
 #pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    const float v = a == 0 ? pi.x : (a == 1 ? pi.y : pi.z);
-                    const float bl = S.box[0][a], bh = S.box[0][3 + a], cl = S.box[1][a], ch_ = S.box[1][3 + a];
-                    const float gb = fmaxf(0.f, fmaxf(bl - v, v - bh)), gc = fmaxf(0.f, fmaxf(cl - v, v - ch_));
-                    const float gj = fmaxf(0.f, fmaxf(cl - bh, bl - ch_));
-                    d2[0] = fmaf(gb, gb, d2[0]);
-                    d2[1] = fmaf(gc, gc, d2[1]);
-                    d2[2] = fmaf(gj, gj, d2[2]);
-                }
-                const float lo = fminf(fminf(d2[0], d2[1]), d2[2]), hi_ij = fmaxf(d2[0], d2[1]);
-                const float mid = fmaxf(fminf(d2[0], d2[1]), fminf(hi_ij, d2[2]));
-                const float in = p.s_hi * (1.0f + 1e-5f), next = p.mid_hi * (1.0f + 1e-5f);
-                keep = hi_ij < reach2 && lo < in * in && mid < next * next;
+            for (int a = 0; a < 3; a++) {
+                const float v = a == 0 ? pt.x : (a == 1 ? pt.y : pt.z);
+                const float bl = b_lo(a), bh = b_hi(a), cl = c[a], ch = c[3 + a];
+                const float gb = fmaxf(0.f, fmaxf(bl - v, v - bh)), gc = fmaxf(0.f, fmaxf(cl - v, v - ch));
+                const float g = fmaxf(0.f, fmaxf(cl - bh, bl - ch));
+                pb = fmaf(gb, gb, pb);
+                pc = fmaf(gc, gc, pc);
+                bc = fmaf(g, g, bc);
             }
+        };
+        const bool resident = __popc(S.mask) <= TRI_GROUP_A;
+        if (threadIdx.x < nr * TILE) {
+            const float4 pi = PA[threadIdx.x];
+            float ij2, ik2, jk2;
+            bounds2(pi, [&](int a) { return S.box[0][a]; }, [&](int a) { return S.box[0][3 + a]; }, S.box[1], ij2, ik2, jk2);
+            const bool keep = (int)(threadIdx.x % TILE) < S.meta[threadIdx.x / TILE].y && possible(ij2, ik2, jk2);
             const unsigned b = __ballot_sync(0xffffffffu, keep);
             int at = 0;
             if (lane == 0 && b) at = atomicAdd(&S.end_i, __popc(b));
             at = __shfl_sync(0xffffffffu, at, 0);
             if (keep) S.list[at + __popc(b & ((1u << lane) - 1u))] = (uint8_t)threadIdx.x;
+            if (b && resident) box_add(S.abox, lane, keep, pi, pi);
+        }
+        if (ch == 0 && !resident && warp == TRI_WARPS - 1) {
+            const bool has = (S.mask >> lane) & 1u;
+            const size_t a = 2 * (size_t)(unit.y + (has ? lane : __ffs(S.mask) - 1));
+            box_add(S.abox, lane, has, J.box[0][a], J.box[0][a + 1]);
         }
         __syncthreads();
         if (S.end_i == 0) continue;
         if (!have_jk) {
             have_jk = true;
+            // The points j and k likewise, with the box of the listed i in place
+            // of the other's tile, and moved to the front of their tiles in
+            // order; their places there are j and k from here on.  (Where B and
+            // C are one tile both tests are the same, so k > j stays as it is.)
+            // A unit of 100 voxels has 14 points i on average: its 64 x 64 j-k
+            // sides cost more than its i.  (Kernel 2.56 -> 2.35 ms, 10k-point
+            // estimator 10.0 -> 9.9.)
+            if (warp < 2) {
+                float4* pts = warp == 0 ? PB : PC;
+                const float* other = S.box[1 - warp];
+                const int n = warp == 0 ? numB : numC;
+                const float4 p0 = pts[lane], p1 = pts[lane + 32];
+                auto keep = [&](float4 pt) {
+                    float pi2, jk2, io2;
+                    bounds2(pt, [&](int a) { return ordered_float(S.abox[a]); },
+                            [&](int a) { return ordered_float(S.abox[3 + a]); }, other, pi2, jk2, io2);
+                    return possible(pi2, jk2, io2);
+                };
+                const bool k0 = lane < n && keep(p0), k1 = lane + 32 < n && keep(p1);
+                const unsigned b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
+                const unsigned lt = (1u << lane) - 1u;
+                uint8_t* list = warp == 0 ? S.jlist : S.klist;
+                if (k0) {
+                    pts[__popc(b0 & lt)] = p0;
+                    list[__popc(b0 & lt)] = (uint8_t)lane;
+                }
+                if (k1) {
+                    pts[__popc(b0) + __popc(b1 & lt)] = p1;
+                    list[__popc(b0) + __popc(b1 & lt)] = (uint8_t)(lane + 32);
+                }
+                if (lane == 0) (warp == 0 ? S.nj : S.nk) = __popc(b0) + __popc(b1);
+            }
+            __syncthreads();
+            numB = S.nj;
+            numC = S.nk;
             key_k0 = pkey(PC[lane]);
             key_k1 = pkey(PC[lane + 32]);
-            // rows j of the j-k side table and their class masks, one warp per row
+            // rows j of the j-k side table and their class sets, one warp per row
             for (int j = warp; j < numB; j += TRI_WARPS) {
                 const float4 pj = PB[j];
-                float a2 = 0.f;
-#pragma unroll
-                for (int a = 0; a < 3; a++) {
-                    const float v = a == 0 ? pj.x : (a == 1 ? pj.y : pj.z);
-                    const float gap = fmaxf(0.f, fmaxf(S.abox[a] - v, v - S.abox[3 + a]));
-                    a2 = fmaf(gap, gap, a2);
-                }
-                if (a2 >= reach2) {  // no i of the group reaches j: empty masks, the row is never read
-                    if (lane < JM_WORDS) JM[lane * TILE + j] = 0ull;
-                    continue;
-                }
                 int c0 = 0, c1 = 0;
                 if (lane < numC) {
                     float d = ref_dist<false>(pj, PC[lane]);
@@ -1368,7 +1406,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 int w = tri_side_word<MODE>(d, p);
                 row_ij[j] = make_int2(__float_as_int(d), w);
                 const int c = side_class(w, d, p);
-                bool ok = c != 0 && any_k && j > j_after;
+                bool ok = c != 0 && any_k && (int)S.jlist[j] > j_after;
                 if (PRED == PRED_SAME) ok = ok && ki <= pkey(PB[j]);
                 if (!ok) return false;
                 cm = MODE == FAST_JBJ ? candidate_mask_jbj(c, nI, nM, nH, JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j])
