@@ -1081,6 +1081,7 @@ __device__ __forceinline__ void box_add(int* box, int lane, bool has, float4 lo,
 struct TriShared {
     uint4 unit;
     uint32_t mask;
+    uint32_t pred;       // loop nest of the unit's job
     int b0, c0;          // first points of tiles B and C
     int next_i, end_i;  // points listed of the resident A tiles: handed out, and their number
     uint8_t list[TRI_GROUP_A * TILE];
@@ -1168,7 +1169,13 @@ __device__ __forceinline__ unsigned long long candidate_mask_jbj(int cij, unsign
     return (nI & (mI | mM | mH)) | ((nM | nH) & mI);
 }
 
-template <int PRED, bool THETA_FULL, int MODE>
+// (UNIT: loop nests without or with a 0/1 weight; else those of two arrays.  The
+// nest itself is a value, not a template argument: five copies of the code cost
+// batches of unlike jobs, whose CTAs run different nests at a time, a fifth: 100
+// voxels 2.34 -> 1.92 ms, most of it by the second place that bins, DDD+DDR+DRR+
+// RRR of 1k points 0.465 -> 0.442.  One copy for both costs the weights of all
+// and more registers: 10k-point estimator 9.9 -> 10.5.)
+template <bool UNIT, bool THETA_FULL, int MODE>
 __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriParams& p, float4* P, float* JKd, short* JKw, int2* IJ,
                                     int2* IK, uint32_t* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
                                     RecheckQueue& q, unsigned long long& evaluated, unsigned long long& binned) {
@@ -1392,9 +1399,10 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             const unsigned long long nM = ballot64(c0 == 3, c1 == 3), nH = ballot64(c0 == 4, c1 == 4);
             const unsigned long long any_k = nB | nI | nM | nH;
             if (!any_k) continue;  // no k within reach of i (warp-uniform)
+            const uint32_t pred = S.pred;
             unsigned long long kge_i = 0;  // PRED_DDR: key_k >= key_i; PRED_RDD: key_k <= key_i
-            if (PRED == PRED_DDR) kge_i = ballot64(lane < numC && key_k0 >= ki, lane + 32 < numC && key_k1 >= ki);
-            if (PRED == PRED_RDD) kge_i = ballot64(lane < numC && key_k0 <= ki, lane + 32 < numC && key_k1 <= ki);
+            if (!UNIT && pred == PRED_DDR) kge_i = ballot64(lane < numC && key_k0 >= ki, lane + 32 < numC && key_k1 >= ki);
+            if (!UNIT && pred == PRED_RDD) kge_i = ballot64(lane < numC && key_k0 <= ki, lane + 32 < numC && key_k1 <= ki);
             // i-j sides: words for the binning path; each lane then forms the
             // candidate-k mask of its own two j's (the scan over j is lane-parallel)
             // mask of candidate k's (and of weight-2 k's) of the pair (i, j)
@@ -1407,21 +1415,21 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 row_ij[j] = make_int2(__float_as_int(d), w);
                 const int c = side_class(w, d, p);
                 bool ok = c != 0 && any_k && (int)S.jlist[j] > j_after;
-                if (PRED == PRED_SAME) ok = ok && ki <= pkey(PB[j]);
+                if (UNIT && pred == PRED_SAME) ok = ok && ki <= pkey(PB[j]);
                 if (!ok) return false;
                 cm = MODE == FAST_JBJ ? candidate_mask_jbj(c, nI, nM, nH, JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j])
                          : candidate_mask(c, nB, nI, nM, nH, JM[j], JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j]);
                 if (diag_jk) cm &= j >= 63 ? 0ull : (~0ull << (j + 1));
-                if (PRED == PRED_RDD) {
+                if (!UNIT && pred == PRED_RDD) {
                     // weight [key_j <= key_i] + [key_k <= key_i]
                     if (pkey(PB[j]) <= ki) {
                         w2 = cm & kge_i;
                     } else {
                         cm &= kge_i;
                     }
-                } else if (PRED != PRED_NONE) {
+                } else if (!UNIT || pred != PRED_NONE) {
                     const unsigned long long kge_j = JM[4 * TILE + j];
-                    if (PRED == PRED_DDR) {
+                    if (!UNIT) {
                         w2 = cm & kge_i & kge_j;  // weight 2: k >= i and k >= j
                         cm &= kge_i | kge_j;      // weight 0 otherwise
                     } else {
@@ -1448,20 +1456,19 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
             // plus j and the weight bit of two-array jobs)
             const uint32_t klo = ((uint32_t)lane << 6) | (1u << 12), khi = ((uint32_t)(lane + 32) << 6) | (1u << 12);
             int qn = 0;  // queued candidates (warp-uniform)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                unsigned live = __ballot_sync(0xffffffffu, (h ? cm1 : cm0) != 0ull);
-                const unsigned long long cmv = h ? cm1 : cm0, w2v = h ? w21 : w20;
-                while (live) {
+            unsigned live = __ballot_sync(0xffffffffu, cm0 != 0ull), live1 = __ballot_sync(0xffffffffu, cm1 != 0ull);
+            uint32_t j0 = 0;  // (one place that bins, for the code's size)
+            for (;;) {
+                if (live) {
                     const int src = __ffs(live) - 1;
                     live &= live - 1u;
-                    const uint32_t j = (uint32_t)(src + 32 * h);
-                    const unsigned lo = __shfl_sync(0xffffffffu, (unsigned)cmv, src);
-                    const unsigned hi = __shfl_sync(0xffffffffu, (unsigned)(cmv >> 32), src);
+                    const uint32_t j = (uint32_t)src + j0;
+                    const unsigned lo = __shfl_sync(0xffffffffu, (unsigned)cm0, src);
+                    const unsigned hi = __shfl_sync(0xffffffffu, (unsigned)(cm0 >> 32), src);
                     uint32_t vlo = klo + j, vhi = khi + j;
-                    if (PRED == PRED_DDR || PRED == PRED_RDD) {
-                        const unsigned w2lo = __shfl_sync(0xffffffffu, (unsigned)w2v, src);
-                        const unsigned w2hi = __shfl_sync(0xffffffffu, (unsigned)(w2v >> 32), src);
+                    if (!UNIT) {
+                        const unsigned w2lo = __shfl_sync(0xffffffffu, (unsigned)w20, src);
+                        const unsigned w2hi = __shfl_sync(0xffffffffu, (unsigned)(w20 >> 32), src);
                         vlo += (w2lo & lbit) ? (1u << 12) : 0u;
                         vhi += (w2hi & lbit) ? (1u << 12) : 0u;
                     }
@@ -1469,19 +1476,21 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                     if (lo & lbit) cand[qn + __popc(lo & lt)] = vlo;
                     if (hi & lbit) cand[qn + nlo + __popc(hi & lt)] = vhi;
                     qn += nlo + __popc(hi);
-                    if (qn >= 64) {
-                        __syncwarp();
-                        qn -= 64;
-                        run_candidates<THETA_FULL, MODE, PRED != PRED_DDR && PRED != PRED_RDD>(cand + qn, 64, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
-                        bn += 64;
-                        __syncwarp();
-                    }
+                    if (qn < 64) continue;
+                } else if (live1) {
+                    live = live1, live1 = 0;
+                    j0 = 32;
+                    cm0 = cm1, w20 = w21;
+                    continue;
+                } else if (qn == 0) {
+                    break;
                 }
-            }
-            __syncwarp();
-            if (qn > 0) {
-                run_candidates<THETA_FULL, MODE, PRED != PRED_DDR && PRED != PRED_RDD>(cand, qn, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
-                bn += qn;
+                const int n = min(qn, 64);
+                __syncwarp();
+                qn -= n;
+                run_candidates<THETA_FULL, MODE, UNIT>(cand + qn, n, row_ij, row_ik, JKd, JKw, p, Hw, q, S, ia);
+                bn += n;
+                __syncwarp();
             }
             __syncwarp();
         }
@@ -1491,17 +1500,6 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
     if (lane == 0) {
         atomicAdd(&evaluated, (unsigned long long)ev);
         atomicAdd(&binned, (unsigned long long)bn);
-    }
-}
-
-template <bool THETA_FULL, int MODE, typename... Args>
-__device__ __forceinline__ void triangle_dispatch(uint32_t pred, Args&&... args) {
-    switch (pred) {
-        case PRED_NONE: triangle_group_fast<PRED_NONE, THETA_FULL, MODE>(args...); break;
-        case PRED_DDR: triangle_group_fast<PRED_DDR, THETA_FULL, MODE>(args...); break;
-        case PRED_RDD: triangle_group_fast<PRED_RDD, THETA_FULL, MODE>(args...); break;
-        case PRED_SAME: triangle_group_fast<PRED_SAME, THETA_FULL, MODE>(args...); break;
-        default: triangle_group_fast<PRED_ONE, THETA_FULL, MODE>(args...); break;
     }
 }
 
@@ -1537,6 +1535,7 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
             const bool any = t < ul.n && ul.u0 + t < ul.header->nunits;
             S.unit = any ? ul.units[ul.u0 + t] : make_uint4(TASK_NONE, 0, 0, 0);
             S.mask = any ? ul.masks[ul.u0 + t] : 0u;
+            if (any) S.pred = jobs[S.unit.x & UNIT_SLOT_MASK].mode & JOB_PRED_MASK;
         }
         __syncthreads();
         if (S.unit.x == TASK_NONE) break;
@@ -1550,7 +1549,10 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
         cur = slot;
         since += n;
         if (n == 0) continue;  // a part without A tiles
-        triangle_dispatch<THETA_FULL, MODE>(jobs[slot].mode & JOB_PRED_MASK, jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
+        if (S.pred == PRED_DDR || S.pred == PRED_RDD)
+            triangle_group_fast<false, THETA_FULL, MODE>(jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
+        else
+            triangle_group_fast<true, THETA_FULL, MODE>(jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
     }
     if (cur >= 0) flush_hist(H, copies, p.len, jobs[cur].hist);
     __syncthreads();
