@@ -638,15 +638,11 @@ enum FastMode : int { FAST_TP = 0, FAST_JBJ = 1, FAST_GEOM = 2 };
 constexpr int TRI_WARPS = 8;
 constexpr int TRI_THREADS = TRI_WARPS * 32;
 constexpr int TRI_QCAP = 128;  // per-warp candidate queue: up to 63 pending + 64 new
-// per j of role B: bit masks over k of the classes of side j-k (B, I, M, H)
-// and of key_k >= key_j; held in shared memory as five 64-entry arrays
-// (JM_WORDS x TILE, word-major) so that lanes reading different j's do not
-// share banks
-struct JMasks {
-    unsigned long long c[4];
-    unsigned long long kge;
-};
-constexpr int JM_WORDS = 5;
+// per j of role B: the nested sets over k of the class of side j-k (SideSet)
+// and key_k >= key_j; held in shared memory as 64-entry arrays (JM_WORDS x
+// TILE, word-major) so that lanes reading different j's do not share banks
+constexpr int JM_WORDS = 6, JM_KEY = 5;
+constexpr int SET_WORDS = 5;  // the same sets of a warp's current i
 // A tiles resident at once: the tasks of a group (one job, tiles B and C
 // shared) are counted up to four at a time, their points i handed out to the
 // warps together
@@ -658,7 +654,7 @@ constexpr int TRI_GROUP_A = TRI_GROUP_A_TILES;
 // i-j and i-k rows | j-k sides | per-warp candidate queues | j-k side words
 // (16 bits) | histogram copies
 constexpr size_t TRI_SMEM_FIXED = (2 + TRI_GROUP_A) * TILE * sizeof(float4) +
-                                  JM_WORDS * TILE * sizeof(unsigned long long) + 2 * TRI_WARPS * TILE * sizeof(int2) +
+                                  (JM_WORDS * TILE + TRI_WARPS * SET_WORDS) * sizeof(unsigned long long) + 2 * TRI_WARPS * TILE * sizeof(int2) +
                                   TILE * TILE * sizeof(float) + TRI_WARPS * TRI_QCAP * sizeof(uint32_t) +
                                   TILE * TILE * sizeof(short);
 // (the plain FP64 kernel's layout -- three tiles, a j-k table of int2 and one
@@ -1128,46 +1124,63 @@ __device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, cons
     if (g1) push_recheck(q, slot, w1, ia, (uint32_t)(S.b0 + S.jlist[j1]), (uint32_t)(S.c0 + S.klist[k1]));
 }
 
-// Side class for candidate filtering: 0 none (zero length or too long),
-// 1 below s_lo, 2 in the s range, 3 above s_hi but below s_hi*q_hi, 4 from
-// s_hi*q_hi up to the largest side a counted triangle can have.
+// Side classes for candidate filtering: none (zero length or too long), X below
+// s_lo or from q_hi s_hi up, M2 and M1 from q_hi s_split and from s_hi up, I1 and
+// I2 the s range below and from s_split.  Their sets are nested by the order of
+// the numbers: all, Q without X, R without M2, I the s range, I2.
+//
+// A counted triangle has two sides one of which is an I and the other the next
+// longer one within q_hi of it (permutation 0/2: the shortest and the middle
+// one; permutation 1: the middle and the longest).  So its classes hold one of
+// the pairs I-I, I1-M1, I2-M1, I2-M2, whatever the third side is.  JBJ is
+// permutation 0 with 1/q_lo for q_hi.
+enum SideClass : int { SC_NONE = 0, SC_X = 1, SC_M2 = 2, SC_M1 = 3, SC_I1 = 4, SC_I2 = 5 };
+enum SideSet : int { SET_ALL = 0, SET_Q = 1, SET_R = 2, SET_I = 3, SET_I2 = 4 };  // class > number
+
+template <int MODE>
 __device__ __forceinline__ int side_class(int word, float d, const TriParams& p) {
     const int w = word & 127;
-    if (w >= CW_REJECT) return 0;
-    if (w == CW_BELOW) return 1;
-    if (w == CW_IN) return 2;
-    return d < p.mid_hi ? 3 : 4;
+    if (w >= CW_REJECT) return SC_NONE;
+    if (w == CW_BELOW) return MODE == FAST_JBJ ? SC_NONE : SC_X;  // (JBJ counts no triangle with such a side)
+    if (w == CW_IN) return d < p.s_split ? SC_I1 : SC_I2;
+    return d < p.mid_split ? SC_M1 : d < p.mid_hi ? SC_M2 : SC_X;
 }
 
 __device__ __forceinline__ unsigned long long ballot64(bool lo, bool hi) {
     return (unsigned long long)__ballot_sync(0xffffffffu, lo) | ((unsigned long long)__ballot_sync(0xffffffffu, hi) << 32);
 }
 
-// Candidate k's of a pair (i, j) whose side i-j has class cij, from the class
-// masks of the sides i-k (n*) and j-k (m*).  A triangle can count only through
-// permutation 0/2 (no side below s_lo, one side in the s range, at most one
-// side at/above s_hi*q_hi) or permutation 1 (no side at/above s_hi*q_hi, at
-// most one below s_lo, at most one in [s_hi, s_hi*q_hi)); these are the
-// (class_ik, class_jk) combinations that leave one of the two possible.
-__device__ __forceinline__ unsigned long long candidate_mask(int cij, unsigned long long nB, unsigned long long nI,
-                                                             unsigned long long nM, unsigned long long nH,
-                                                             unsigned long long mB, unsigned long long mI,
-                                                             unsigned long long mM, unsigned long long mH) {
-    if (cij == 2) return (nB | nI | nM | nH) & (mB | mI | mM | mH) & ~((nB | nH) & (mB | mH));
-    if (cij == 3) return (nI & (mB | mI | mM | mH)) | ((nB | nI | nM | nH) & mI);
-    return (nI & (mI | mM)) | (nM & mI);  // cij == 1 or 4
+// The nested sets of the sides of one point, lane and lane + 32, written by one
+// lane at the given stride.
+__device__ __forceinline__ unsigned long long side_sets(unsigned long long* out, int stride, int lane, int c0, int c1) {
+    const unsigned long long all = ballot64(c0 > SET_ALL, c1 > SET_ALL), q = ballot64(c0 > SET_Q, c1 > SET_Q),
+                             r = ballot64(c0 > SET_R, c1 > SET_R), i = ballot64(c0 > SET_I, c1 > SET_I),
+                             i2 = ballot64(c0 > SET_I2, c1 > SET_I2);
+    if (lane == 0) {
+        out[SET_ALL * stride] = all;
+        out[SET_Q * stride] = q;
+        out[SET_R * stride] = r;
+        out[SET_I * stride] = i;
+        out[SET_I2 * stride] = i2;
+    }
+    return all;
 }
 
-// The same for the JBJ parametrization: a triangle can count only if its
-// shortest side is in the s range, i.e. no side below s_lo and at least one
-// in range.
-__device__ __forceinline__ unsigned long long candidate_mask_jbj(int cij, unsigned long long nI, unsigned long long nM,
-                                                                 unsigned long long nH, unsigned long long mI,
-                                                                 unsigned long long mM, unsigned long long mH) {
-    if (cij == 1) return 0ull;
-    if (cij == 2) return (nI | nM | nH) & (mI | mM | mH);
-    return (nI & (mI | mM | mH)) | ((nM | nH) & mI);
+// Candidate k's of a pair (i, j) whose side i-j has class cij, from the sets of
+// the sides i-k (n) and j-k (m, at stride TILE): a class that makes a pair with
+// cij, or one of the pairs between i-k and j-k (exactly those beside M2; beside
+// X also I1-M2, beside an I or M1 they are in the first kind).  (With one class I
+// and one M 22 % more triangles of the 10k-point estimator reach the binning:
+// kernel 9.7 ms, so 8.7; without I2's set 12 % more and 9.5.)
+__device__ __forceinline__ unsigned long long candidate_mask(int cij, const unsigned long long* n, const unsigned long long* m) {
+    const int with = cij == SC_X ? SET_Q : SET_R;
+    unsigned long long cm = (n[SET_I] & m[with * TILE]) | (n[with] & m[SET_I * TILE]);
+    const int pairs = SC_M2 + SET_I2 - cij;  // the set of the classes that make a pair with cij (but X)
+    if (cij != SC_X) cm |= n[SET_ALL] & m[SET_ALL * TILE] & (n[pairs] | m[pairs * TILE]);
+    return cm;
 }
+static_assert(SC_M1 + SET_I == SC_M2 + SET_I2 && SC_I1 + SET_R == SC_M2 + SET_I2 && SC_I2 + SET_Q == SC_M2 + SET_I2,
+              "classes and the sets of those that make a pair with them");
 
 // (UNIT: loop nests without or with a 0/1 weight; else those of two arrays.  The
 // nest itself is a value, not a template argument: five copies of the code cost
@@ -1199,6 +1212,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
     int2* row_ij = IJ + warp * TILE;
     int2* row_ik = IK + warp * TILE;
     uint32_t* cand = Q + warp * TRI_QCAP;
+    unsigned long long* sets = JM + JM_WORDS * TILE + warp * SET_WORDS;
     int key_k0 = 0, key_k1 = 0;
     unsigned ev = 0, bn = 0;
     // A tiles of the unit, up to TRI_GROUP_A at a time
@@ -1345,25 +1359,19 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                     int w = tri_side_word<MODE>(d, p);
                     JKd[j * TILE + lane] = d;
                     JKw[j * TILE + lane] = (short)w;
-                    c0 = side_class(w, d, p);
+                    c0 = side_class<MODE>(w, d, p);
                 }
                 if (lane + 32 < numC) {
                     float d = ref_dist<false>(pj, PC[lane + 32]);
                     int w = tri_side_word<MODE>(d, p);
                     JKd[j * TILE + lane + 32] = d;
                     JKw[j * TILE + lane + 32] = (short)w;
-                    c1 = side_class(w, d, p);
+                    c1 = side_class<MODE>(w, d, p);
                 }
-                JMasks m;
-#pragma unroll
-                for (int c = 0; c < 4; c++) m.c[c] = ballot64(c0 == c + 1, c1 == c + 1);
+                side_sets(JM + j, TILE, lane, c0, c1);
                 const int kj = pkey(pj);
-                m.kge = ballot64(lane < numC && key_k0 >= kj, lane + 32 < numC && key_k1 >= kj);
-                if (lane == 0) {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) JM[c * TILE + j] = m.c[c];
-                    JM[4 * TILE + j] = m.kge;
-                }
+                const unsigned long long kge = ballot64(lane < numC && key_k0 >= kj, lane + 32 < numC && key_k1 >= kj);
+                if (lane == 0) JM[JM_KEY * TILE + j] = kge;
             }
             __syncthreads();
         }
@@ -1387,18 +1395,17 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 float d = ref_dist<false>(pi, PC[lane]);
                 int w = tri_side_word<MODE>(d, p);
                 row_ik[lane] = make_int2(__float_as_int(d), w);
-                c0 = side_class(w, d, p);
+                c0 = side_class<MODE>(w, d, p);
             }
             if (lane + 32 < numC) {
                 float d = ref_dist<false>(pi, PC[lane + 32]);
                 int w = tri_side_word<MODE>(d, p);
                 row_ik[lane + 32] = make_int2(__float_as_int(d), w);
-                c1 = side_class(w, d, p);
+                c1 = side_class<MODE>(w, d, p);
             }
-            const unsigned long long nB = ballot64(c0 == 1, c1 == 1), nI = ballot64(c0 == 2, c1 == 2);
-            const unsigned long long nM = ballot64(c0 == 3, c1 == 3), nH = ballot64(c0 == 4, c1 == 4);
-            const unsigned long long any_k = nB | nI | nM | nH;
+            const unsigned long long any_k = side_sets(sets, 1, lane, c0, c1);
             if (!any_k) continue;  // no k within reach of i (warp-uniform)
+            __syncwarp();
             const uint32_t pred = S.pred;
             unsigned long long kge_i = 0;  // PRED_DDR: key_k >= key_i; PRED_RDD: key_k <= key_i
             if (!UNIT && pred == PRED_DDR) kge_i = ballot64(lane < numC && key_k0 >= ki, lane + 32 < numC && key_k1 >= ki);
@@ -1413,12 +1420,11 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 float d = ref_dist<false>(pi, PB[j]);
                 int w = tri_side_word<MODE>(d, p);
                 row_ij[j] = make_int2(__float_as_int(d), w);
-                const int c = side_class(w, d, p);
+                const int c = side_class<MODE>(w, d, p);
                 bool ok = c != 0 && any_k && (int)S.jlist[j] > j_after;
                 if (UNIT && pred == PRED_SAME) ok = ok && ki <= pkey(PB[j]);
                 if (!ok) return false;
-                cm = MODE == FAST_JBJ ? candidate_mask_jbj(c, nI, nM, nH, JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j])
-                         : candidate_mask(c, nB, nI, nM, nH, JM[j], JM[TILE + j], JM[2 * TILE + j], JM[3 * TILE + j]);
+                cm = candidate_mask(c, sets, JM + j);
                 if (diag_jk) cm &= j >= 63 ? 0ull : (~0ull << (j + 1));
                 if (!UNIT && pred == PRED_RDD) {
                     // weight [key_j <= key_i] + [key_k <= key_i]
@@ -1428,7 +1434,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                         cm &= kge_i;
                     }
                 } else if (!UNIT || pred != PRED_NONE) {
-                    const unsigned long long kge_j = JM[4 * TILE + j];
+                    const unsigned long long kge_j = JM[JM_KEY * TILE + j];
                     if (!UNIT) {
                         w2 = cm & kge_i & kge_j;  // weight 2: k >= i and k >= j
                         cm &= kge_i | kge_j;      // weight 0 otherwise
@@ -1438,12 +1444,17 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                 }
                 return true;
             };
-            unsigned long long cm0, w20, cm1, w21;
-            const bool ok0 = scan_j(lane, cm0, w20);
-            const bool ok1 = scan_j(lane + 32, cm1, w21);
+            // (one copy of the scan: 100 voxels 1.99 -> 1.91 ms)
+            unsigned long long cm0 = 0, w20 = 0, cm1 = 0, w21 = 0;
+            int nok = 0;
+#pragma unroll 1
+            for (int h = 0; h < numB; h += 32) {
+                cm0 = cm1, w20 = w21;
+                nok += __popc(__ballot_sync(0xffffffffu, scan_j(lane + h, cm1, w21)));
+            }
+            if (numB <= 32) cm0 = cm1, cm1 = 0, w20 = w21;
             // walked (i, j, k): every k with a usable i-k side, for every usable j
-            ev += (unsigned)__popcll(any_k) *
-                  (unsigned)(__popc(__ballot_sync(0xffffffffu, ok0)) + __popc(__ballot_sync(0xffffffffu, ok1)));
+            ev += (unsigned)__popcll(any_k) * (unsigned)nok;
             __syncwarp();
             const uint32_t ia = (uint32_t)(meta.x + i);
             // Candidates of this i: every j with a non-empty mask in turn, expanded
@@ -1515,7 +1526,7 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
     extern __shared__ __align__(16) unsigned char smem[];
     float4* P = reinterpret_cast<float4*>(smem);
     unsigned long long* JM = reinterpret_cast<unsigned long long*>(P + (2 + TRI_GROUP_A) * TILE);
-    int2* IJ = reinterpret_cast<int2*>(JM + JM_WORDS * TILE);
+    int2* IJ = reinterpret_cast<int2*>(JM + JM_WORDS * TILE + TRI_WARPS * SET_WORDS);
     int2* IK = IJ + TRI_WARPS * TILE;
     float* JKd = reinterpret_cast<float*>(IK + TRI_WARPS * TILE);
     uint32_t* Q = reinterpret_cast<uint32_t*>(JKd + TILE * TILE);
