@@ -1347,9 +1347,12 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     bool tame = true;  // (asked by the double-precision geometry and the neighbour lists only)
     if (sp.precision == TPCF_GEOMETRY_FP64 || bin.near_ok || bin.list_ok) {
         std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
+        uint64_t seen[3] = {0, 0, 0};  // (0 is no handle: a role's catalog is often the previous job's)
         for (const GroupJob& g : group)
             for (int r = 0; r < ncat; r++) {
-                auto it = ctx->catalogs.find(g.job->catalog[r]);
+                if (g.job->catalog[r] == seen[r]) continue;
+                seen[r] = g.job->catalog[r];
+                auto it = ctx->catalogs.find(seen[r]);
                 if (it != ctx->catalogs.end()) tame = tame && it->second->tame;
             }
     }
@@ -1454,14 +1457,21 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     };
     std::vector<Range> ranges;
     std::unordered_map<RangeKey, uint32_t, RangeHash> range_at;
+    // the last range of each hash value: a batch of thousands of jobs names
+    // each of its ranges many times
+    size_t nfront = 1;
+    while (nfront < 3 * group.size() && nfront < 4096) nfront *= 2;
+    std::vector<uint32_t> front(nfront, UINT32_MAX);
     auto range_of = [&](const RangeKey& k) -> uint32_t {
-        auto ins = range_at.emplace(k, (uint32_t)ranges.size());
+        uint32_t& f = front[RangeHash{}(k) & (nfront - 1)];
+        if (f != UINT32_MAX && ranges[f].key == k) return f;
+        auto ins = range_at.try_emplace(k, (uint32_t)ranges.size());
         if (ins.second) {
             Range r{k, {}, nullptr};
             get_view(ctx, L, k.h, k.b, k.e, k.gl, &r.ref);
             ranges.push_back(std::move(r));
         }
-        return ins.first->second;
+        return f = ins.first->second;
     };
     // Signature of the batch (its binning, and each job's views, slot and loop
     // nest): a repeated batch over the same resident views reuses its plan.
@@ -2077,8 +2087,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     }
 }
 
-void validate(const tpcf_spec* sp, const tpcf_job* job) {
+// before: a spec that passed (its value is not checked again), or null
+void validate(const tpcf_spec* sp, const tpcf_job* job, const tpcf_spec* before = nullptr) {
     if (!sp || !job) throw InvalidArg{"null spec or job"};
+    const bool flags_ok = (job->flags & ~(uint32_t)TPCF_JOB_GLOBAL_INDEX) == 0 && job->reserved == 0;
+    if (before && flags_ok && memcmp(before, sp, sizeof *sp) == 0) return;
     if (sp->kind != TPCF_THREE_SIDE && sp->kind != TPCF_TRIANGLE && sp->kind != TPCF_PAIR &&
         sp->kind != TPCF_TRIANGLE_JBJ)
         throw InvalidArg{"bad kind"};
@@ -2087,7 +2100,7 @@ void validate(const tpcf_spec* sp, const tpcf_job* job) {
         throw InvalidArg{"bad precision"};
     if (sp->precision == TPCF_GEOMETRY_FP64 && sp->kind != TPCF_TRIANGLE)
         throw InvalidArg{"TPCF_GEOMETRY_FP64 is implemented for the triangle parametrization only"};
-    if ((job->flags & ~(uint32_t)TPCF_JOB_GLOBAL_INDEX) != 0 || job->reserved != 0) throw InvalidArg{"bad job flags"};
+    if (!flags_ok) throw InvalidArg{"bad job flags"};
     (void)make_binning(*sp);
 }
 
@@ -2551,7 +2564,7 @@ tpcf_status count_jobs(tpcf_ctx* ctx, const tpcf_spec* specs, const tpcf_job* jo
         CK(cudaSetDevice(ctx->device));
         std::vector<int64_t> out_len(out_index ? n_out : 0, -1);
         for (int i = 0; i < n; i++) {
-            validate(&specs[i], &jobs[i]);
+            validate(&specs[i], &jobs[i], i > 0 ? &specs[i - 1] : nullptr);
             if (out_index) {
                 const int32_t o = out_index[i];
                 if (o < 0 || o >= n_out) throw InvalidArg{"out_index out of range"};
