@@ -5,15 +5,13 @@
 //   * spatial views: a catalog range is reordered by a balanced k-d split into
 //     tiles of exactly TILE points (last tile partial), each with an
 //     axis-aligned bounding box; cached per (catalog, range);
-//   * task planning: the reference's loop nest becomes a list of tile triples
-//     (pairs).  Symmetric loop nests (DDD/RRR: i<=j<=k over one array; DRR: j<=k
-//     over one array; DDR: i,j over one array) are enumerated canonically so
-//     that each unordered set of points is visited once; everything else is
-//     enumerated as ordered tile triples with the reference's index predicate
-//     evaluated per triangle.  Tile triples whose bounding boxes prove that no
-//     triangle can reach a counted bin are skipped (exact: a rigorous lower
-//     bound on every side is compared with the largest side any counted
-//     triangle can have);
+//   * planning: the reference's loop nest becomes jobs of three views whose
+//     tile triples (pairs, centres) the device finds.  Symmetric loop nests
+//     (DDD/RRR: i<=j<=k over one array; DRR: j<=k over one array; DDR: i,j over
+//     one array) are enumerated canonically so that each unordered set of
+//     points is visited once; everything else as ordered tile triples with the
+//     reference's index predicate evaluated per triangle.  Whether triangles
+//     are counted from tiles or from neighbour lists is chosen per batch;
 //   * launches: one persistent kernel per (kind, binning, precision) group,
 //     then the exact recheck of guard-band triangles, then D2H of the counts;
 //   * glibc acosf exception table for exact theta (built from the host libm by
@@ -1087,26 +1085,10 @@ AcosTable acos_table(tpcf_ctx* ctx) {
     return t;
 }
 
-struct PlannedJob {
-    std::shared_ptr<View> v[3];
-    uint64_t loop_units = 0;
-    // Loop ONE jobs of two arrays are counted with the point of the array that
-    // appears once in role B or C and the pair array first, so that points
-    // out of reach of a tile are skipped whole (guarded kernel only):
-    //   swap 1, the D-D-R nest (A == B): roles (C, A, A), weight PRED_RDD;
-    //   swap 2, the D-R-R nest (B == C): roles (B, B, A), unordered pairs of B first.
-    int swap = 0;
-    const View* role(int r) const {
-        if (swap == 1) return r == 0 ? v[2].get() : v[0].get();
-        if (swap == 2) return r == 2 ? v[0].get() : v[1].get();
-        return v[r].get();
-    }
-};
-
-// Host worker threads for planning, started once per process (thread
-// creation would cost more than the planning work of a small batch).  run()
-// calls fn(i) for i in [0, n) on the workers and the calling thread; a run
-// that finds the pool busy (another lane planning) does its items inline.
+// Host worker threads for building views, started once per process (thread
+// creation would cost more than a small view).  run() calls fn(i) for i in
+// [0, n) on the workers and the calling thread; a run that finds the pool busy
+// does its items inline.
 class HostPool {
   public:
     static HostPool& get() {

@@ -57,12 +57,8 @@ constexpr int MAX_FAST_S = 254;
 // most A tiles in one window of the planner (one mask word)
 constexpr int MAX_WINDOW = 32;
 // weight sum (4*nBelow + nAbove, >= 32 if rejected) -> permutation validity
-constexpr unsigned VALID_ANY = 0x37u;   // shortest or middle side in range
 constexpr unsigned VALID_02 = 0x07u;    // shortest side in range (permutations 0 and 2)
 constexpr unsigned VALID_1 = 0x33u;     // middle side in range, no zero side (permutation 1)
-
-// Three-side codes: "at or above hist_max" in clean mode.
-constexpr uint32_t CODE3_CLEAN_FAR = 1u << 28;
 
 // A histogram target of one launch.
 struct DevJob {
@@ -172,10 +168,6 @@ struct RecheckQueue {
     unsigned int cap;
     unsigned long long* hists;      // neighbour lists: the launch's first histogram
     unsigned long long* evaluated;  // triangles of (i,j) pairs the fast kernel walked
-};
-
-struct LaunchStats {
-    unsigned int* error_flag;    // set by kernels on an internal invariant failure
 };
 
 // Planner: which tile triples of a launch can hold a counted triple.

@@ -1,13 +1,16 @@
 // kernels.cu -- sm_103a counting kernels.
 //
-// All kernels are persistent: a grid of (SM count x resident CTAs) pulls tile
-// tasks from a device counter.  A task names one spatial tile (<= 64 points)
-// of each role; the CTA stages the tiles' points in shared memory, computes the
-// side lengths of the tile pairs once (exactly as the reference does), and then
-// walks the triangles with one warp per point of role A, a loop over role B
-// and the 32 lanes spanning role C.  Counts go to warp-private shared
-// histograms (32-bit) that are flushed with 64-bit global atomics when the
-// task's histogram changes, after a bounded number of tasks, and at exit.
+// All kernels are persistent: a grid of (SM count x resident CTAs) draws work
+// from a device counter.  Tile kernels: a unit names one spatial tile (<= 64
+// points) of roles B and C and a set of A tiles, found by the planner kernels
+// from the views' tile boxes; the CTA stages the tiles' points in shared
+// memory, computes the side lengths of the tile pairs once (exactly as the
+// reference does), and then walks the triangles with one warp per point of
+// role A, a loop over role B and the 32 lanes spanning role C.  Neighbour-list
+// kernels: a warp or pipeline takes one point at a time, gathers the points
+// near it and counts their pairs.  Counts go to shared histograms (32-bit)
+// that are flushed with 64-bit global atomics when the histogram changes,
+// before they can run over, and at exit.
 //
 // Exactness: side lengths and their bins are computed with IEEE
 // round-to-nearest intrinsics in the reference's operation order, so they equal
@@ -661,17 +664,6 @@ constexpr size_t TRI_SMEM_FIXED = (2 + TRI_GROUP_A) * TILE * sizeof(float4) +
 // row per warp -- fits the same allocation)
 static_assert(TRI_SMEM_FIXED >= 3 * TILE * sizeof(float4) + TILE * TILE * sizeof(int2) + TRI_WARPS * TILE * sizeof(int2),
               "FP64 triangle layout");
-
-// s-bin code of one side, monotone in the side length, multiplied by Q*T
-// (used by the plain FP64 kernel).
-template <bool FP64>
-__device__ __forceinline__ int tri_side_code(float d, const TriParams& p) {
-    typedef FOps<FP64> F;
-    if (d == 0.f) return CODE_ZERO;
-    if (d < p.s_lo) return CODE_BELOW;
-    if (d >= p.s_hi) return CODE_ABOVE;
-    return __float2int_rz(F::div(F::sub(d, p.s_lo), p.s_bw)) * (p.Q * p.T);
-}
 
 // Side word of the fast kernel: code16 * 128 + class weight, 16 bits (see
 // engine.h); code16 is the s-bin itself.
