@@ -1350,17 +1350,19 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     const bool geom = sp.precision == TPCF_GEOMETRY_FP64;
     // Triangles from neighbour lists (see TriCentre) instead of tile triples:
     //   where the tile kernel's tables leave room for one CTA beside the
-    //   histogram (50 x 16 x 25 bins, DDD+DDR+DRR+RRR twice: 5k-point cone 5.15 ->
-    //   2.0 ms, 5k-point blobs 91 -> 52 ms, 500 points 0.91 -> 0.72 ms);
+    //   histogram (50 x 16 x 25 bins, DDD+DDR+DRR+RRR of two seeds: 5k-point cone
+    //   4.6 -> 2.0 ms, 5k-point blobs 76 -> 52 ms, 500 points 0.83 -> 0.72 ms;
+    //   50 x 16 x 12 bins, two CTAs: blobs 46 -> 51 ms);
     //   where tiles are wide against s_hi (three times), so that few of a tile
-    //   triple's triangles are near (1,024 bins: 5k-point cone 1.31 -> 0.69 ms, 2k
-    //   0.41 -> 0.19 ms, 500 points 0.13 -> 0.09 ms; blobs of 500 points, whose
-    //   tiles are 6 to 20 across, the other way round: 2k 3.04 -> 3.3 ms, 10k 11.4
-    //   -> 14.4 ms);
-    //   JBJ with many centres, whose tile triples hold few shortest sides in
-    //   range (5k-point blobs 36 -> 28 ms, 2k 4.4 -> 4.7 ms).
+    //   triple's triangles are near (1,024 bins: 5k-point cone 0.98 -> 0.68 ms, 2k
+    //   0.35 -> 0.19 ms, 500 points 0.14 -> 0.09 ms; blobs, whose tiles are 6 to 20
+    //   across, the other way round: 2k 2.2 -> 3.3 ms, 10k 58 -> 64 ms);
+    //   JBJ with very many centres, whose tile triples hold few shortest sides
+    //   in range (blobs of 25k points, 150,000 centres, 1244 -> 1097 ms, 15k 343 ->
+    //   338, 10k 139 -> 140, 5k 24 -> 28 ms; s/m from 0.5: 25k 179 -> 143, 10k 23.4
+    //   -> 22.9, 7k 9.9 -> 10.4).
     // Sets of many small jobs (voxels) keep the tiles: each of a job's centres
-    // is an item here (16,500 jobs of a 20k cone 3.4 -> 8.8 ms).
+    // is an item here (16,500 jobs of a 20k cone 1.9 -> 8.8 ms).
     const char* tl_env = getenv("TPCF_TRI_LISTS");
     bool tlist = fast_tri && bin.list_ok && tame && !(tl_env && tl_env[0] == '0') &&
                  group.size() <= (tl_env ? (size_t)1000000 : (size_t)64) &&
@@ -1383,7 +1385,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         sparse = extent > 3 * (double)bin.tri.s_hi;
         if (!tl_env)
             tlist = shape_candidates(ctx, sp, bin, fp64, false, 0)[0].per_sm < 2 || sparse ||
-                    (fast_jbj && centres >= 20000);
+                    (fast_jbj && centres >= 80000);
     }
     const bool items = pairs || near || tlist;  // kernels that find their tiles themselves
     if (group.size() > MAX_BATCH_JOBS) throw InvalidArg{"too many jobs in one batch"};
