@@ -606,8 +606,8 @@ def run_three_side(args):
     for _ in range(args.steps):
         eng.count_batch(sp, jobs)
         ms.append(eng.stats()["kernel_ms"])
-    units = eng.stats()["loop_units"]
-    multisets = sum(n * (n + 1) * (n + 2) // 6 for n in (len(d), len(r)))
+    st = eng.stats()
+    units = st["loop_units"]
     h64 = eng.count_batch([tpcf.make_spec(tpcf.THREE_SIDE, tpcf.LOOP_ALL, [(16, 0.0, 40.0)],
                                           precision=tpcf.PLAIN_FP64)] * 2, jobs)
     fp64_ms = eng.stats()["kernel_ms"]
@@ -633,10 +633,10 @@ def run_three_side(args):
            "triangles_per_step": units},
           ms_per_step=mean * 1e3, p50_ms=statistics.median(ms), p99_ms=float(np.percentile(ms, 99)),
           plain_fp64={"value": units / (fp64_ms / 1e3), "ms_per_step": fp64_ms, "identical": same},
-          roofline=_issue_roofline(10 * multisets / mean / 1e12, "three_side_kernel",
-                                   "10 lane-instructions per multiset of three points (the kernel visits each "
-                                   "multiset {i <= j <= k} once and counts all its orderings; %d multisets for "
-                                   "the %d ordered triples)" % (multisets, units)),
+          roofline=_issue_roofline(10 * st["evaluated_units"] / mean / 1e12, "three_near_kernel",
+                                   "10 lane-instructions per triple of points whose third side is computed (two "
+                                   "sides in range at one point; %d for the %d ordered triples, the far sides "
+                                   "by inclusion and exclusion)" % (st["evaluated_units"], units)),
           cpu_baseline=cpu)
     eng.close()
     return 0
@@ -843,7 +843,7 @@ def run_lattice(args):
            "evaluated_triangles_per_step": st["evaluated_units"], "tasks": st["tasks"],
            "counted": int(h32.sum())},
           ms_per_step=mean * 1e3, wall_ms_per_step=st["total_ms"],
-          roofline=_issue_roofline(10 * int(h32.sum()) / 6 / mean / 1e12, "three_side_grouped_kernel",
+          roofline=_issue_roofline(10 * int(h32.sum()) / 6 / mean / 1e12, "three_near_kernel",
                                    "10 lane-instructions per counted multiset of three points (all sides < 32; the "
                                    "kernel counts each multiset once for all its orderings: counted triples / 6)"),
           plain_fp64={"ms_per_step": st64["kernel_ms"], "points": int(len(sub)),
