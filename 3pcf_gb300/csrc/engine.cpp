@@ -1648,8 +1648,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         pp.s_hi2 = sq_up(bin.s_hi);
         pp.q_hi2 = sq_up(bin.q_hi);
         pp.s_lo2 = bin.s_lo > 0 ? nextafterf((float)std::min(bin.s_lo * bin.s_lo, 3e38), 0.f) : 0.f;
-        // heavy: what takes a CTA that has its SM to itself some 15 us (a line
-        // at 6000 or 8192 instead cost 1 % on 10k points and 2 % on 1k)
+        // heavy: what takes a CTA that has its SM to itself some 12 us (a line
+        // at 6000 or 8192 instead cost 1 % on 10k points and 2 % on 1k; at 1500
+        // 1k points are 4 % faster and a burst of 40 mixed jobs 8 % slower)
         pp.r = (float)(bin.lmax < 3e38 ? (sp.kind == TPCF_TRIANGLE ? std::max(0.0, bin.s_hi * bin.q_hi) : bin.lmax) : 3e38);
         pp.heavy = fast_tri ? 3000.f : 0.f;
         int rpb = 0;
