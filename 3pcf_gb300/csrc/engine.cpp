@@ -1326,8 +1326,8 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     Binning bin = make_binning(sp);
     const int ncat = sp.kind == TPCF_PAIR ? 2 : 3;
     const bool pairs = sp.kind == TPCF_PAIR;
-    bool tame = true;  // (asked by the double-precision geometry and the neighbour lists only)
-    if (sp.precision == TPCF_GEOMETRY_FP64 || bin.near_ok || bin.list_ok) {
+    bool tame = true;  // (asked by the triangle kernels and the neighbour lists only)
+    if (!pairs) {
         std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
         uint64_t seen[3] = {0, 0, 0};  // (0 is no handle: a role's catalog is often the previous job's)
         for (const GroupJob& g : group)
@@ -1339,6 +1339,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             }
     }
     const bool fp64 = !guarded_fp32(sp, bin, tame);
+    bin.tri.tame = tame;
     // three-side counts from neighbour lists (see three_near_kernel)
     const char* near_env = getenv("TPCF_NEAR");
     const bool near = lists && bin.near_ok && tame && !(near_env && near_env[0] == '0') &&

@@ -97,6 +97,7 @@ struct TriParams {
     float lmax;                  // sides >= lmax cannot belong to a counted triangle
     float mid_hi;                // s_hi * q_hi (rounded up; JBJ: s_hi / q_lo): a counted triangle has a side in the s
                                  // range and another below it (permutation 0/2: the middle one; 1: the longest)
+    int tame;                    // every coordinate of the launch is a number of ordinary size
     float s_split, mid_split;    // a side within the s range and the limit of the next longer one (rounded up)
     // neighbour lists: squared reach of a centre, limit max(q S, top) of the
     // middle side given the shortest

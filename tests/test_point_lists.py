@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import oracle
+import synth
 import tpcf
 
 pytestmark = pytest.mark.gpu
@@ -50,3 +51,16 @@ def test_limits(monkeypatch, name, spread):
             want = (oracle.triangle(c, w, axes, nan_zero=NAN == tpcf.NAN_ZERO) if kind == tpcf.TRIANGLE
                     else oracle.triangle_jbj(c, w, axes))[0]
             assert np.array_equal(got, want)
+
+
+def test_points_that_are_not_numbers():
+    """A point outside every box, whose sides are all in the s range's first
+    bin where int(NaN) is 0: no point may be left out for its distance from it."""
+    d, r = synth.blobs(50, n_blobs=2, sigma=6.0, box=40.0, seed=50), synth.uniform(70, box=60.0, seed=70)
+    d[17, 1] = r[23, 2] = np.nan
+    axes = [(8, 2.0, 10.0), (8, 1.0, 3.0), (16, 0.0, 1.0)]
+    with tpcf.Engine(0) as eng:
+        hd, hr = eng.catalog(d), eng.catalog(r)
+        s = tpcf.make_spec(tpcf.TRIANGLE, tpcf.LOOP_ONE, axes, nan_policy=tpcf.NAN_ZERO, prune=False)
+        want = oracle.triangle([r, d, r], 1, axes, nan_zero=True)[0]
+        assert np.array_equal(eng.count(s, eng.job([hr, hd, hr])), want)
