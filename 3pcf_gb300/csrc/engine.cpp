@@ -1678,10 +1678,15 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                 tile_pairs += (long long)ranges[r.range[0]].view->ntiles * ranges[r.range[1]].view->ntiles;
             plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS);
         } else if (near) {
-            // one centre per item where that balances the pipelines, else four
+            // one centre per item where that balances the pipelines, else as
+            // many as an item may have
             uint64_t centres = 0;
-            for (const RoleJob& r : roles) centres += ranges[r.range[0]].view->n;
-            plan_chunk = centres < 64ull * ctx->num_sms * 4 ? 1 : 4;
+            bool ordered = false;
+            for (const RoleJob& r : roles) {
+                centres += ranges[r.range[0]].view->n;
+                ordered = ordered || r.mode == NEAR_ORDERED;
+            }
+            plan_chunk = centres < 64ull * ctx->num_sms * 4 ? 1 : ordered ? NEAR_ITEM_ORDERED : NEAR_ITEM;
         } else if (tlist) {
             uint64_t centres = 0;
             for (const SubJob& sj : subs) centres += ranges[sj.range[0]].view->n;

@@ -153,6 +153,9 @@ enum NearClass : uint32_t {
 };
 constexpr uint32_t NEAR_CLASS_MASK = 3u;
 constexpr int NEAR_CENTRE_SHIFT = 2;
+// centres per item at most, where a batch has no NEAR_ORDERED job and where it
+// has one (see NEAR_STOP: what the 32-bit counters hold)
+constexpr int NEAR_ITEM = 4, NEAR_ITEM_ORDERED = 2;
 
 // Exact glibc-acosf exception table on the device.
 struct AcosTable {

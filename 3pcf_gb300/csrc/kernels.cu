@@ -2957,12 +2957,17 @@ __device__ __forceinline__ void near_block(const NearPipe& N, int j0, int j1, in
 // One CTA per SM of `pipes` 8-warp pipelines around one shared accumulator.  A
 // pipeline takes an item (a few centres of one tile), and waits for the others
 // at a CTA barrier when its item belongs to another job, when there is none
-// left, or when the 32-bit counters have taken 2^30 pairs; there the counters
-// are added to the job's accumulator.  An item adds at most
-// NEAR_ITEM * NEAR_MAX_POINTS^2 / 2 = 2^29 pairs, so that four pipelines stay
-// below 2^32.
-constexpr int NEAR_ITEM = 4;  // centres per item at most
-static_assert((unsigned long long)NEAR_ITEM * NEAR_MAX_POINTS * NEAR_MAX_POINTS / 2 <= (1ull << 29), "near counters");
+// left, or when the 32-bit counters have taken NEAR_STOP pairs; there the
+// counters are added to the job's accumulator.  A pipeline that draws just below
+// the line still counts its item, so the line and an item of every pipeline
+// have to stay below 2^32 counts of one word.  A centre has at most
+// NEAR_MAX_POINTS^2 / 2 pairs of one list, but NEAR_MAX_POINTS^2 of two.
+constexpr unsigned long long NEAR_STOP = 1ull << 30;
+constexpr unsigned long long near_item_pairs(int centres, bool two_lists) {
+    return (unsigned long long)centres * NEAR_MAX_POINTS * NEAR_MAX_POINTS / (two_lists ? 1 : 2);
+}
+static_assert(NEAR_STOP + TS_GROUPS_MAX * near_item_pairs(NEAR_ITEM, false) < (1ull << 32), "counters, one list");
+static_assert(NEAR_STOP + TS_GROUPS_MAX * near_item_pairs(NEAR_ITEM_ORDERED, true) < (1ull << 32), "counters, two lists");
 
 __global__ void __launch_bounds__(TS_GROUPS_MAX * TS_GROUP_THREADS, 1)
 three_near_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ item_off, int njobs, unsigned int item0,
@@ -2995,7 +3000,7 @@ three_near_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ 
         }
         if (lane == 0) {
             N.item = it;
-            N.stop = s_since >= (1ull << 30);
+            N.stop = s_since >= NEAR_STOP;
         }
     };
     draw();
