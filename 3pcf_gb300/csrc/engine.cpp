@@ -72,6 +72,9 @@ struct CudaError {
 struct InvalidArg {
     std::string msg;
 };
+struct InternalError {
+    std::string msg;
+};
 
 // ---------------------------------------------------------------------------
 // device buffers
@@ -837,6 +840,24 @@ struct GroupJob {
     bool accumulate = false;  // add into out (jobs sharing out share one device histogram)
 };
 
+// A tiles [begin, end) of a group of one job (end < 0: all)
+struct TileRange {
+    int begin = 0, end = -1;
+};
+
+// Thrown by run_group, before anything is counted, where a group's plan passes
+// its limits (see count_group); tiles: A tiles of its first job.
+struct TooLarge {
+    int tiles;
+};
+
+// Units of one plan (21 GB of unit list), and of a smaller TPCF_MAX_UNITS (tests
+// use it to have small batches counted in parts).
+uint32_t max_units() {
+    const char* e = getenv("TPCF_MAX_UNITS");
+    return e ? (uint32_t)std::min(std::max(1L, std::atol(e)), 1L << 30) : 1u << 30;
+}
+
 }  // namespace
 
 // Launch shape of a persistent kernel: warp-private histogram copies in
@@ -1319,8 +1340,9 @@ int grid_for(tpcf_ctx* ctx, const Shape& sh, uint64_t ntasks, int sm_cap) {
 }
 
 // Runs one group of jobs that share kind, binning and precision in a single
-// persistent launch.  outs[i] receives hist_len counts.
-void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool lists = true) {
+// persistent launch.  outs[i] receives hist_len counts.  lists: counts from
+// neighbour lists are allowed; part: the A tiles to count of a single job.
+void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool lists = true, TileRange part = {}) {
     auto t_wall0 = std::chrono::steady_clock::now();
     const tpcf_spec& sp = *group[0].spec;
     Binning bin = make_binning(sp);
@@ -1365,7 +1387,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     // Sets of many small jobs (voxels) keep the tiles: each of a job's centres
     // is an item here (16,500 jobs of a 20k cone 1.9 -> 8.8 ms).
     const char* tl_env = getenv("TPCF_TRI_LISTS");
-    bool tlist = fast_tri && bin.list_ok && tame && !(tl_env && tl_env[0] == '0') &&
+    bool tlist = lists && fast_tri && bin.list_ok && tame && !(tl_env && tl_env[0] == '0') &&
                  group.size() <= (tl_env ? (size_t)1000000 : (size_t)64) &&
                  !shape_candidates(ctx, sp, bin, fp64, false, 1).empty();
     bool sparse = false;
@@ -1473,6 +1495,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         }
         sig.push_back((uint64_t)bin.len);
         sig.push_back((uint64_t)group.size());
+        sig.push_back((uint64_t)(uint32_t)part.begin << 32 | (uint32_t)part.end);
     }
     // each job: its ranges in the kernel's role order, and how its tiles and
     // points are enumerated (JOB_*)
@@ -1516,7 +1539,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             n[r] = ranges[rg[r]].ref.n;
         }
         if (ncat == 2) rg[2] = rg[1];
-        units += loop_units(jsp.kind, jsp.loop, n);
+        if (part.begin == 0) units += loop_units(jsp.kind, jsp.loop, n);  // (a job's first part reports it)
         // (two ranges with one view, e.g. [0, n) and [0, -1), are the same array)
         auto id = [&](int r) { return ranges[rg[r]].ref.id; };
         const bool ab = id(0) == id(1), bc = id(1) == id(2);
@@ -1633,6 +1656,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     uint32_t nwedges = L.plan_wedges;
     int plan_parts = L.plan_parts, plan_kparts = L.plan_kparts;  // triangle lists: shares of a centre
     PlanHeader* d_header = nullptr;
+    const uint32_t unit_limit = max_units();
     // Finds the units of the batch on the device (see plan_rows): the host
     // gives each job's number of rows.
     auto plan_units = [&](size_t capacity) {
@@ -1728,6 +1752,18 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             }
             d.mode = roles[g].mode;
             d.hist = L.d_hist.p + (size_t)bin.len * slot_of[g];
+            if (part.end >= 0) {
+                // tables that begin with the first A tile; tiles B >= A then begin
+                // there as well, and tiles C >= B with them
+                d.ntiles[0] = part.end;
+                for (int r = 0; r < 3; r++) {
+                    if (r == 1 && !(d.mode & JOB_B_FROM_A)) break;
+                    if (r == 2 && !(d.mode & JOB_C_FROM_B)) break;
+                    d.tile_start[r] += part.begin;
+                    d.box[r] += 2 * (size_t)part.begin;
+                    d.ntiles[r] -= part.begin;
+                }
+            }
             L.h_jobs.p[g] = d;
             L.h_rows.p[g] = (uint32_t)rows;
             if (near) {
@@ -1789,7 +1825,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         CK(cudaMemcpyAsync(L.d_jobs.p, L.h_jobs.p, njobs * sizeof(DevJob), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(L.d_rows.p, L.h_rows.p, nr * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         L.h2d += njobs * sizeof(DevJob) + nr * sizeof(uint32_t);
-        if (!items) plan_units(std::max<size_t>(L.d_units.n, (size_t)1 << 20));
+        if (!items) plan_units(std::min<size_t>(std::max<size_t>(L.d_units.n, (size_t)1 << 20), unit_limit));
         L.plan_sig = sig;
         L.plan_rows = nrows;
         L.plan_chunk = plan_chunk;
@@ -1826,7 +1862,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     auto count_with = [&](const Shape& sh, bool allow_graph) -> float {
         const int copies = sh.copies;
         const int grid = grid_for(ctx, sh, items ? (nrows + std::max(1, sh.groups) - 1) / std::max(1, sh.groups) : UINT64_MAX, L.sm_cap);
-        for (int attempt = 0; attempt < 4; attempt++) {
+        for (int attempt = 0;; attempt++) {
+            // (the unit list and the recheck queue grow at most once each)
+            if (attempt == 4) throw InternalError{"a batch overflowed its buffers after they had been grown"};
             if (L.slice_batches && !sized) {
                 // (the header of a plan that overflowed the unit list asks for a
                 // larger one: the count below finds no units and regrows it)
@@ -1967,7 +2005,13 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             if (!items && header.nunits == 0 && header.needed > 0) {
                 // the unit list overflowed: nothing was counted; plan again into a larger one
                 L.drop_graph();
-                plan_units((size_t)header.needed + (header.needed >> 3));
+                if (header.needed > unit_limit) {
+                    L.plan_sig.clear();
+                    const int tile = ctx->tile_points;
+                    throw TooLarge{part.end < 0 ? (int)((ranges[roles[0].range[0]].ref.n + tile - 1) / tile)
+                                                : part.end - part.begin};
+                }
+                plan_units(std::min<size_t>((size_t)header.needed + (header.needed >> 3), unit_limit));
                 sized = false;
                 continue;
             }
@@ -2039,7 +2083,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     CK(cudaEventElapsedTime(&ms_main, L.ev0, L.ev_mid));
     L.stats.main_kernel_ms = ms_main;
     // JBJ compat: the reference's two extra counts in bin 0 per visited triangle
-    if (sp.kind == TPCF_TRIANGLE_JBJ && sp.overflow == TPCF_OVERFLOW_COMPAT && bin.len > 0)
+    if (sp.kind == TPCF_TRIANGLE_JBJ && sp.overflow == TPCF_OVERFLOW_COMPAT && bin.len > 0 && part.begin == 0)
         for (size_t g = 0; g < group.size(); g++) L.h_hist.p[(size_t)bin.len * slot_of[g]] += 2 * job_units(g);
     for (size_t k = 0; k < nslots; k++) {
         const GroupJob& gj = group[slot_job[k]];
@@ -2078,6 +2122,59 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     }
 }
 
+void add_stats(tpcf_stats& acc, const tpcf_stats& s) {
+    acc.kernel_ms += s.kernel_ms;
+    acc.main_kernel_ms += s.main_kernel_ms;
+    acc.binned_units += s.binned_units;
+    acc.total_ms += s.total_ms;
+    acc.loop_units += s.loop_units;
+    acc.evaluated_units += s.evaluated_units;
+    acc.recheck_units += s.recheck_units;
+    acc.recheck_regrows += s.recheck_regrows;
+    acc.tasks += s.tasks;
+    acc.kernel_launches += s.kernel_launches;
+    acc.graph_replays += s.graph_replays;
+    acc.plan_ms += s.plan_ms;
+    acc.tuned_shapes += s.tuned_shapes;
+    acc.hist_copies = s.hist_copies;
+    acc.ctas_per_sm = s.ctas_per_sm;
+}
+
+// Counts a group: in one launch, or where its plan passes the limits in parts
+// that add up -- the jobs in halves, a single job by ranges of its A tiles.
+void count_group(tpcf_ctx* ctx, Lane& L, std::vector<GroupJob> group, TileRange part = {}) {
+    int tiles = 0;
+    try {
+        run_group(ctx, L, group, part.end < 0, part);
+        return;
+    } catch (const TooLarge& e) {
+        tiles = e.tiles;
+    }
+    for (GroupJob& g : group)
+        if (!g.accumulate) {
+            int64_t len = 0;
+            tpcf_hist_len(g.spec, &len);
+            memset(g.out, 0, (size_t)len * sizeof(uint64_t));
+            g.accumulate = true;
+        }
+    tpcf_stats acc{};
+    auto half = [&](std::vector<GroupJob> jobs, TileRange r) {
+        count_group(ctx, L, std::move(jobs), r);
+        add_stats(acc, L.stats);
+    };
+    if (group.size() > 1) {
+        const auto mid = group.begin() + group.size() / 2;
+        half({group.begin(), mid}, {});
+        half({mid, group.end()}, {});
+    } else {
+        if (tiles < 2) throw InvalidArg{"too many tile triples in one batch"};
+        const int mid = part.begin + tiles / 2;
+        half(group, {part.begin, mid});
+        half(group, {mid, part.begin + tiles});
+    }
+    L.stats = acc;
+}
+
 // before: a spec that passed (its value is not checked again), or null
 void validate(const tpcf_spec* sp, const tpcf_job* job, const tpcf_spec* before = nullptr) {
     if (!sp || !job) throw InvalidArg{"null spec or job"};
@@ -2102,6 +2199,8 @@ tpcf_status guarded(tpcf_ctx* ctx, F&& f) {
         return TPCF_OK;
     } catch (const InvalidArg& e) {
         return fail(ctx, TPCF_ERR_INVALID, e.msg);
+    } catch (const InternalError& e) {
+        return fail(ctx, TPCF_ERR_INTERNAL, e.msg);
     } catch (const CudaError& e) {
         cudaGetLastError();
         if (e.e == cudaErrorMemoryAllocation) return fail(ctx, TPCF_ERR_OOM, cudaGetErrorString(e.e));
@@ -2273,7 +2372,7 @@ void worker_loop(tpcf_ctx* ctx, int lane) {
             p->t_start = t_start;
             group.push_back({&p->spec, &p->job, p->result.data(), false});
         }
-        tpcf_status st = guarded(ctx, [&] { run_group(ctx, L, group); });
+        tpcf_status st = guarded(ctx, [&] { count_group(ctx, L, group); });
         double t_done = now_ms();
         if (!ctx->trace_path.empty()) {
             double oldest = t_start;
@@ -2583,22 +2682,8 @@ tpcf_status count_jobs(tpcf_ctx* ctx, const tpcf_spec* specs, const tpcf_job* jo
                     done[k] = 1;
                 }
             Lane& L = *ctx->lanes[0];
-            run_group(ctx, L, g);
-            acc.kernel_ms += L.stats.kernel_ms;
-            acc.main_kernel_ms += L.stats.main_kernel_ms;
-            acc.binned_units += L.stats.binned_units;
-            acc.total_ms += L.stats.total_ms;
-            acc.loop_units += L.stats.loop_units;
-            acc.evaluated_units += L.stats.evaluated_units;
-            acc.recheck_units += L.stats.recheck_units;
-            acc.recheck_regrows += L.stats.recheck_regrows;
-            acc.tasks += L.stats.tasks;
-            acc.kernel_launches += L.stats.kernel_launches;
-            acc.graph_replays += L.stats.graph_replays;
-            acc.plan_ms += L.stats.plan_ms;
-            acc.tuned_shapes += L.stats.tuned_shapes;
-            acc.hist_copies = L.stats.hist_copies;
-            acc.ctas_per_sm = L.stats.ctas_per_sm;
+            count_group(ctx, L, std::move(g));
+            add_stats(acc, L.stats);
         }
         ctx->lanes[0]->stats = acc;
     });

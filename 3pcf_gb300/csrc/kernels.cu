@@ -606,7 +606,8 @@ plan_scan(uint2* block_sum, int nblocks, PlanParams pp, PlanHeader* header, uint
         const unsigned long long want = (pp.per_tile ? 2ull : 16ull) * (unsigned)pp.slots;
         const uint32_t top = pp.per_tile ? 4u : 16u;
         uint32_t parts = 1;
-        while (parts < top && th > 0 && th * parts < want) parts *= 4;
+        // (not beyond what the unit list holds)
+        while (parts < top && th > 0 && th * parts < want && th * parts * 4 + tl <= capacity) parts *= 4;
         const unsigned long long n = th * parts + tl;
         header->parts = parts;
         header->needed = (uint32_t)(n < 0xffffffffull ? n : 0xffffffffull);
