@@ -20,7 +20,7 @@ NVCC = os.path.join(CUDA, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 PROGRAMS = {"tpcf_3side": 0, "tpcf_tp": 1, "tpcf_2pcf": 2, "tpcf_jbj": 3}
 
-HEADERS = ["engine.h", "exact_acos.h"]
+HEADERS = ["engine.h", "exact_acos.h", "plan_bounds.h"]
 
 
 def _newer(target, deps):

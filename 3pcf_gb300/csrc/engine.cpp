@@ -2002,6 +2002,10 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             const unsigned int* counters = L.h_counters.p;
             L.d2h += CTR_WORDS * sizeof(unsigned int) + hist_total * sizeof(unsigned long long);
             memcpy(&header, counters + CTR_HEADER, sizeof(header));
+            if (!items && header.mismatch) {
+                L.plan_sig.clear();
+                throw InternalError{"the planner's passes found different units"};
+            }
             if (!items && header.nunits == 0 && header.needed > 0) {
                 // the unit list overflowed: nothing was counted; plan again into a larger one
                 L.drop_graph();

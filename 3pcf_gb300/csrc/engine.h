@@ -189,7 +189,7 @@ struct PlanHeader {
     uint32_t nunits;   // units to count (0 where they overflow the unit list)
     uint32_t needed;   // units found
     uint32_t parts;    // units each heavy one was cut into
-    uint32_t pad;
+    uint32_t mismatch; // not 0: the passes of the planner differed (the units are not valid)
     unsigned long long evaluated, tiles;  // triples and tile triples of the units
 };
 // row_off[j] .. row_off[j + 1]: rows (window of A tiles, tile B) of job j;

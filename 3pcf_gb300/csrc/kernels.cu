@@ -29,6 +29,7 @@
 #include "../../include/tpcf.h"
 #include "engine.h"
 #include "exact_acos.h"
+#include "plan_bounds.h"
 
 namespace tpcf {
 
@@ -291,10 +292,11 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // triangle kernel, a tile pair (B, C) with a mask of up to `window` A tiles)
 // that can hold a counted triple -- are found on the device from the views'
 // tile boxes: row (job, window of A tiles, tile B) tests every tile C.
-//   plan_count  units of each row, those of each block of rows, and totals;
-//   plan_scan   (one CTA) exclusive scan of the blocks' sums, the number of
-//               parts heavy units are cut into, the header;
-//   plan_fill   the same tests again, writing each unit to its place.
+//   plan_rows<false>  units of each row, those of each block of rows, and totals;
+//   plan_scan         (one CTA) exclusive scan of the blocks' sums, the number of
+//                     parts heavy units are cut into, the header;
+//   plan_rows<true>   the same tests again, writing each unit to its place (the
+//                     two passes have to decide alike: see plan_bounds.h).
 // Heavy units (an estimate of their triples above PlanParams::heavy) come
 // first, in job order, then the light ones in job order: a CTA flushes its
 // histogram when the job changes, and the long units are not left to the end.
@@ -325,40 +327,6 @@ int plan_blocks(uint64_t nrows, int* rows_per_block) {
     const int r = nrows <= 32768 ? PLAN_WARPS : PLAN_WARPS * 8;
     if (rows_per_block) *rows_per_block = r;
     return (int)((nrows + r - 1) / r);
-}
-
-// Lower and upper bounds of the squared side between two tile boxes; the
-// margins cover the rounding of the bounds and of the reference's sides.  A
-// lower bound that overflows stays below an infinite limit.
-__device__ __forceinline__ float2 box_bounds2(float4 al, float4 ah, float4 bl, float4 bh) {
-    const float gx = fmaxf(0.f, fmaxf(al.x - bh.x, bl.x - ah.x)), ux = fmaxf(ah.x - bl.x, bh.x - al.x);
-    const float gy = fmaxf(0.f, fmaxf(al.y - bh.y, bl.y - ah.y)), uy = fmaxf(ah.y - bl.y, bh.y - al.y);
-    const float gz = fmaxf(0.f, fmaxf(al.z - bh.z, bl.z - ah.z)), uz = fmaxf(ah.z - bl.z, bh.z - al.z);
-    return make_float2(fminf((gx * gx + gy * gy + gz * gz) * (1.0f - 4e-5f), 3.4028235e38f),
-                       (ux * ux + uy * uy + uz * uz) * (1.0f + 4e-5f) + 1e-37f);
-}
-
-// Whether a tile triple can hold a counted triangle-parametrization triangle:
-// with the three pair bounds sorted (L1<=L2<=L3 lower, U1<=U2<=U3 upper) the
-// shortest side lies in [L1,U1], the middle in [L2,U2], the longest in
-// [L3,U3]; permutations 0/2 need s_lo <= shortest < s_hi and
-// middle < q_hi*shortest, permutation 1 needs s_lo <= middle < s_hi and
-// longest < q_hi*middle.  All squared.
-__device__ __forceinline__ bool tri_possible(float2 x, float2 y, float2 z, const PlanParams& pp) {
-    const float l0 = fminf(fminf(x.x, y.x), z.x), l2 = fmaxf(fmaxf(x.x, y.x), z.x);
-    const float l1 = fmaxf(fminf(x.x, y.x), fminf(fmaxf(x.x, y.x), z.x));
-    const float u0 = fminf(fminf(x.y, y.y), z.y);
-    const float u1 = fmaxf(fminf(x.y, y.y), fminf(fmaxf(x.y, y.y), z.y));
-    return (l0 < pp.s_hi2 && u0 >= pp.s_lo2 && l1 < pp.q_hi2 * u0) ||
-           (l1 < pp.s_hi2 && u1 >= pp.s_lo2 && l2 < pp.q_hi2 * u1);
-}
-
-// Rough share of the pairs of two tiles that are within r of one another.
-__device__ __forceinline__ float near_share(float2 b, float r) {
-    const float lo = sqrtf(b.x), hi = sqrtf(fminf(b.y, 3e38f));
-    if (hi <= r) return 1.f;
-    const float f = fmaxf(r - lo, 0.f) / fmaxf(hi - lo, 1e-30f);
-    return f * f;
 }
 
 template <bool FILL>
@@ -406,9 +374,11 @@ plan_rows(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ row_off,
     for (int rr = 0; rr < per_warp; rr++) {
         const uint32_t row = row0 + (uint32_t)(warp * per_warp + rr);
         if (row >= nrows) break;
+        uint2 expect = make_uint2(0, 0);  // FILL: the places after this row's units
         if (FILL) {
             const uint2 c = row_cnt[row];
             if (c.x + c.y == 0u) continue;
+            expect = make_uint2(place.x + c.x, place.y + c.y);
         }
         const int slot = find_job(row_off, njobs, row);
         const DevJob& J = jobs[slot];
@@ -456,12 +426,8 @@ plan_rows(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ row_off,
                         const float2 ab = s_ab[warp][t], ac = box_bounds2(s_box[warp][2 * t], s_box[warp][2 * t + 1], cl, ch);
                         if (ac.x >= pp.lmax2 || (pp.tri && !tri_possible(ab, ac, bc, pp))) continue;
                         mask |= 1u << t;
-                        if (pp.heavy > 0.f) {
-                            // triangles within reach, and what walking the points i and
-                            // the j's in their reach costs in the same unit
-                            const float na = (float)s_na[warp][t], nj = (float)nb * near_share(ab, pp.r);
-                            est += na * (25.f + nj * (2.5f + (float)nc * near_share(ac, pp.r) * near_share(bc, pp.r)));
-                        }
+                        if (pp.heavy > 0.f)
+                            est = add_estimate(est, (float)s_na[warp][t], (float)nb, (float)nc, ab, ac, bc, pp.r);
                         if (!FILL) {
                             const unsigned long long na = (unsigned)s_na[warp][t], n = (unsigned)nb, k = (unsigned)nc;
                             const bool dij = from_a && a0 + t == b, djk = from_b && b == c;
@@ -527,6 +493,7 @@ plan_rows(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ row_off,
                 place.y += total >> 16;
             }
         }
+        if (FILL && lane == 0 && (place.x != expect.x || place.y != expect.y)) header->mismatch = 1u;
         if (!FILL) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
