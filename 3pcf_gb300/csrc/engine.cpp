@@ -92,6 +92,7 @@ class DeviceBlocks {
         return *d;
     }
     void* alloc(size_t bytes, size_t* cap) {
+        if (bytes > limit_.load()) throw CudaError{cudaErrorMemoryAllocation};
         int dev = 0;
         CK(cudaGetDevice(&dev));
         size_t cls = 256;
@@ -134,6 +135,8 @@ class DeviceBlocks {
             kv.second.clear();
         }
     }
+    // larger blocks are refused as if memory had run out (tests)
+    void set_limit(size_t bytes) { limit_.store(bytes); }
     void release(void* p, size_t cap) {
         if (!p) return;
         int dev = 0;
@@ -151,6 +154,7 @@ class DeviceBlocks {
   private:
     static constexpr size_t kMaxCached = (size_t)64 << 20, kMaxTotal = (size_t)2 << 30;
     std::mutex mu_;
+    std::atomic<size_t> limit_{SIZE_MAX};
     std::map<std::pair<int, size_t>, std::vector<void*>> free_;
     size_t cached_ = 0;
 };
@@ -1629,14 +1633,6 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         sig.push_back(ranges[v[2]].ref.id);
         sig.push_back((uint64_t)slot_of[g] << 32 | (uint64_t)mode << 8 | (uint64_t)jsp.loop);
     }
-    cudaStream_t st = L.stream;
-    L.d_counters.reserve(CTR_WORDS);
-    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near, tlist ? (int)nslots : 0);
-    const bool plan_hit = sig == L.plan_sig;
-    phase("batch");
-    const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
-    uint32_t nrows = L.plan_rows;   // pairs and neighbour lists: items
-    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item; neighbour lists: centres per item
     // neighbour lists: an accumulator per output slot and class of job, and the
     // wedge jobs of the reference's mode (two per job, one for a single catalog)
     std::vector<uint32_t> acc_of;
@@ -1651,8 +1647,18 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             acc_of.push_back(ins.first->second);
             if (!bin.three.clean) nwedge_jobs += roles[g].mode == NEAR_SYM ? 1 : 2;
         }
+        // (the planned jobs point into it, as into the histograms)
         L.d_acc.reserve(acc_words * accs.size());
+        sig.push_back((uint64_t)(uintptr_t)L.d_acc.p);
     }
+    cudaStream_t st = L.stream;
+    L.d_counters.reserve(CTR_WORDS);
+    const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near, tlist ? (int)nslots : 0);
+    const bool plan_hit = sig == L.plan_sig;
+    phase("batch");
+    const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
+    uint32_t nrows = L.plan_rows;   // pairs and neighbour lists: items
+    int plan_chunk = L.plan_chunk;  // pairs: tiles B per item; neighbour lists: centres per item
     uint32_t nwedges = L.plan_wedges;
     int plan_parts = L.plan_parts, plan_kparts = L.plan_kparts;  // triangle lists: shares of a centre
     PlanHeader* d_header = nullptr;
@@ -1968,8 +1974,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                                           (uint64_t)(uintptr_t)acos_t.bucket, (uint64_t)acos_t.n, queue_cap,
                                           (uint64_t)grid, (uint64_t)copies, (uint64_t)sh.groups, hist_total,
                                           (uint64_t)nwork, (uint64_t)slice, (uint64_t)(uintptr_t)L.d_rows.p,
-                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk, (uint64_t)plan_parts << 32 | (uint64_t)plan_kparts,
-                                          (uint64_t)(uintptr_t)L.d_acc.p};
+                                          (uint64_t)(uintptr_t)L.d_masks.p, (uint64_t)plan_chunk, (uint64_t)plan_parts << 32 | (uint64_t)plan_kparts};
                 gsig.insert(gsig.end(), extra, extra + sizeof(extra) / sizeof(extra[0]));
                 if (!L.graph || gsig != L.graph_sig) {
                     L.drop_graph();
@@ -2920,3 +2925,7 @@ extern "C" int32_t tpcf_debug_set_acos_exceptions(tpcf_ctx* ctx, const uint32_t*
         ctx->acos_ready = true;
     });
 }
+
+// test hook (not in the public header): device blocks above `bytes` are refused
+// as if memory had run out
+extern "C" void tpcf_debug_alloc_limit(uint64_t bytes) { DeviceBlocks::get().set_limit((size_t)bytes); }

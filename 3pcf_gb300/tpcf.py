@@ -100,6 +100,8 @@ def lib():
                                               ctypes.c_float, ctypes.c_float, ctypes.c_int32, P, P]
         L.tpcf_debug_set_acos_exceptions.restype = ctypes.c_int32
         L.tpcf_debug_set_acos_exceptions.argtypes = [P, P, P, ctypes.c_uint64]
+        L.tpcf_debug_alloc_limit.restype = None
+        L.tpcf_debug_alloc_limit.argtypes = [ctypes.c_uint64]
         L.tpcf_debug_acos_selfcheck.restype = ctypes.c_int64
         L.tpcf_debug_acos_selfcheck.argtypes = [P, ctypes.POINTER(ctypes.c_int64)]
         _LIB = L
