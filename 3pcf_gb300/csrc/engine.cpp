@@ -726,19 +726,20 @@ bool same_binning(const tpcf_spec& a, const tpcf_spec& b) {
 
 uint64_t loop_units(int kind, int loop, const int64_t n[3]) {
     typedef unsigned __int128 u128;  // sums of the loops' bounds in closed form, modulo 2^64
+    // (a range whose end lies before its begin has a negative size: its loop does not run)
     if (kind == TPCF_THREE_SIDE) return (uint64_t)n[0] * n[1] * n[2];
     if (kind == TPCF_PAIR) {
         if (loop != TPCF_LOOP_SAME) return (uint64_t)n[0] * n[1];
-        const u128 m = std::min(n[0], n[1]);  // sum over i < m of n1 - i
+        const u128 m = std::max<int64_t>(std::min(n[0], n[1]), 0);  // sum over i < m of n1 - i
         return m ? (uint64_t)(m * (u128)n[1] - m * (m - 1) / 2) : 0;
     }
     if (loop == TPCF_LOOP_ALL) return (uint64_t)n[0] * n[1] * n[2];
-    const u128 n0 = n[0], n2 = n[2], m = std::min(n[1], n[2]);
+    const u128 n0 = n[0], n2 = n[2], m = std::max<int64_t>(std::min(n[1], n[2]), 0);
     if (m == 0 || n0 == 0) return 0;
     const u128 tail = m * n2 - m * (m - 1) / 2;  // sum over j < m of n2 - j
     if (loop == TPCF_LOOP_ONE) return (uint64_t)(n0 * tail);
     // LOOP_SAME: min(n0, j + 1) points i for each j
-    const u128 p = std::min(m, n0);
+    const u128 p = n[0] > 0 ? std::min(m, n0) : 0;
     const u128 sq = (p - 1) * p * (2 * p - 1) / 6, lin = p * (p - 1) / 2;  // sums of j^2 and j over j < p
     const u128 head = p * n2 + n2 * lin - lin - sq;                        // (j + 1) (n2 - j)
     return (uint64_t)(head + n0 * (tail - (p * n2 - lin)));
