@@ -622,12 +622,16 @@ constexpr int SET_WORDS = 5;  // the same sets of a warp's current i
 #endif
 constexpr int TRI_GROUP_A = TRI_GROUP_A_TILES;
 // layout: tiles B, C and up to TRI_GROUP_A A tiles | j-class masks | per-warp
-// i-j and i-k rows | j-k sides | per-warp candidate queues | j-k side words
-// (16 bits) | histogram copies
-constexpr size_t TRI_SMEM_FIXED = (2 + TRI_GROUP_A) * TILE * sizeof(float4) +
-                                  (JM_WORDS * TILE + TRI_WARPS * SET_WORDS) * sizeof(unsigned long long) + 2 * TRI_WARPS * TILE * sizeof(int2) +
-                                  TILE * TILE * sizeof(float) + TRI_WARPS * TRI_QCAP * sizeof(uint32_t) +
-                                  TILE * TILE * sizeof(short);
+// i-j and i-k rows | j-k sides | per-warp candidate queues (16 bits) | j-k side
+// words (16 bits) | histogram copies
+constexpr size_t TRI_TABLES = (2 + TRI_GROUP_A) * TILE * sizeof(float4) +
+                              (JM_WORDS * TILE + TRI_WARPS * SET_WORDS) * sizeof(unsigned long long) + 2 * TRI_WARPS * TILE * sizeof(int2) +
+                              TILE * TILE * sizeof(float) + TRI_WARPS * TRI_QCAP * sizeof(uint16_t) +
+                              TILE * TILE * sizeof(short);
+// What the histogram does not get: fixed, so that the binnings that fit beside
+// it (up to 46,464 bins in one copy) do not change with the tables.
+constexpr size_t TRI_SMEM_FIXED = 45568;
+static_assert(TRI_TABLES <= TRI_SMEM_FIXED, "fast triangle layout");
 // (the plain FP64 kernel's layout -- three tiles, a j-k table of int2 and one
 // row per warp -- fits the same allocation)
 static_assert(TRI_SMEM_FIXED >= 3 * TILE * sizeof(float4) + TILE * TILE * sizeof(int2) + TRI_WARPS * TILE * sizeof(int2),
@@ -1056,7 +1060,7 @@ static_assert(TRI_GROUP_A * TILE <= 256 && TRI_GROUP_A * TILE <= TRI_THREADS, "o
 // Runs the full binning path on n (<= 64) queued candidates, two per lane
 // (packed into the f32x2 instructions of one binning path).
 template <bool THETA_FULL, int MODE, bool UNIT>
-__device__ __forceinline__ void run_candidates(const uint32_t* cand, int n, const int2* row_ij, const int2* row_ik,
+__device__ __forceinline__ void run_candidates(const uint16_t* cand, int n, const int2* row_ij, const int2* row_ik,
                                                const float* JKd, const short* JKw, const TriParams& p, unsigned int* Hw,
                                                RecheckQueue& q, TriShared& S, uint32_t ia) {
     const int lane = threadIdx.x & 31;
@@ -1150,7 +1154,7 @@ static_assert(SC_M1 + SET_I == SC_M2 + SET_I2 && SC_I1 + SET_R == SC_M2 + SET_I2
 // and more registers: 10k-point estimator 9.9 -> 10.5.)
 template <bool UNIT, bool THETA_FULL, int MODE>
 __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriParams& p, float4* P, float* JKd, short* JKw, int2* IJ,
-                                    int2* IK, uint32_t* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
+                                    int2* IK, uint16_t* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
                                     RecheckQueue& q, unsigned long long& evaluated, unsigned long long& binned) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float4 *PB = P, *PC = P + TILE, *PA = P + 2 * TILE;
@@ -1171,7 +1175,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
     bool have_jk = false;  // the j-k sides are in the tables
     int2* row_ij = IJ + warp * TILE;
     int2* row_ik = IK + warp * TILE;
-    uint32_t* cand = Q + warp * TRI_QCAP;
+    uint16_t* cand = Q + warp * TRI_QCAP;
     unsigned long long* sets = JM + JM_WORDS * TILE + warp * SET_WORDS;
     int key_k0 = 0, key_k1 = 0;
     unsigned ev = 0, bn = 0;
@@ -1448,8 +1452,8 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                         vhi += (w2hi & lbit) ? (1u << 12) : 0u;
                     }
                     const int nlo = __popc(lo);
-                    if (lo & lbit) cand[qn + __popc(lo & lt)] = vlo;
-                    if (hi & lbit) cand[qn + nlo + __popc(hi & lt)] = vhi;
+                    if (lo & lbit) cand[qn + __popc(lo & lt)] = (uint16_t)vlo;
+                    if (hi & lbit) cand[qn + nlo + __popc(hi & lt)] = (uint16_t)vhi;
                     qn += nlo + __popc(hi);
                     if (qn < 64) continue;
                 } else if (live1) {
@@ -1493,7 +1497,7 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
     int2* IJ = reinterpret_cast<int2*>(JM + JM_WORDS * TILE + TRI_WARPS * SET_WORDS);
     int2* IK = IJ + TRI_WARPS * TILE;
     float* JKd = reinterpret_cast<float*>(IK + TRI_WARPS * TILE);
-    uint32_t* Q = reinterpret_cast<uint32_t*>(JKd + TILE * TILE);
+    uint16_t* Q = reinterpret_cast<uint16_t*>(JKd + TILE * TILE);
     short* JKw = reinterpret_cast<short*>(Q + TRI_WARPS * TRI_QCAP);
     unsigned int* H = reinterpret_cast<unsigned int*>(JKw + TILE * TILE);
     __shared__ TriShared S;
