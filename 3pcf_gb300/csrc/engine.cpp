@@ -851,17 +851,21 @@ struct TileRange {
 };
 
 // Thrown by run_group, before anything is counted, where a group's plan passes
-// its limits (see count_group); tiles: A tiles of its first job.
+// its limits (see count_group); tiles: A tiles of its first job; lists: it was to
+// be counted from neighbour lists.
 struct TooLarge {
     int tiles;
+    bool lists;
 };
 
-// Units of one plan (21 GB of unit list), and of a smaller TPCF_MAX_UNITS (tests
-// use it to have small batches counted in parts).
-uint32_t max_units() {
-    const char* e = getenv("TPCF_MAX_UNITS");
-    return e ? (uint32_t)std::min(std::max(1L, std::atol(e)), 1L << 30) : 1u << 30;
+// The limits of one plan: its units (21 GB of unit list), its rows (4 GB of
+// counts a row) or items.  TPCF_MAX_UNITS, TPCF_MAX_ROWS: lower ones (tests use
+// them to have small batches counted in parts).
+uint32_t plan_limit(const char* env, uint32_t most) {
+    const char* e = getenv(env);
+    return e ? (uint32_t)std::min<long>(std::max(1L, std::atol(e)), most) : most;
 }
+constexpr uint32_t MAX_UNITS = 1u << 30, MAX_ROWS = 1u << 29, MAX_ITEMS = 0xF0000000u;
 
 }  // namespace
 
@@ -1663,7 +1667,14 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     uint32_t nwedges = L.plan_wedges;
     int plan_parts = L.plan_parts, plan_kparts = L.plan_kparts;  // triangle lists: shares of a centre
     PlanHeader* d_header = nullptr;
-    const uint32_t unit_limit = max_units();
+    const uint32_t unit_limit = plan_limit("TPCF_MAX_UNITS", MAX_UNITS),
+                   row_limit = plan_limit("TPCF_MAX_ROWS", items ? MAX_ITEMS : MAX_ROWS);
+    auto too_large = [&] {
+        const int tile = ctx->tile_points;
+        L.plan_sig.clear();
+        return TooLarge{part.end < 0 ? (int)((ranges[roles[0].range[0]].ref.n + tile - 1) / tile) : part.end - part.begin,
+                        near || tlist};
+    };
     // Finds the units of the batch on the device (see plan_rows): the host
     // gives each job's number of rows.
     auto plan_units = [&](size_t capacity) {
@@ -1745,7 +1756,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                 L.h_jobs.p[k] = d;
                 L.h_rows.p[k] = (uint32_t)rows;
                 rows += (uint64_t)plan_parts * plan_kparts * (((uint64_t)ranges[subs[k].range[0]].view->n + plan_chunk - 1) / plan_chunk);
-                if (rows > 0xF0000000ull) throw InvalidArg{"too many points in one batch"};
+                if (rows > row_limit) throw too_large();
             }
         }
         for (size_t g = 0; g < (tlist ? 0 : group.size()); g++) {
@@ -1778,7 +1789,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                 rows += (uint64_t)d.ntiles[0] * ((TILE + plan_chunk - 1) / plan_chunk);
             } else if (pairs) rows += (uint64_t)d.ntiles[0] * ((d.ntiles[1] + plan_chunk - 1) / plan_chunk);
             else if (d.ntiles[2] > 0) rows += (uint64_t)((d.ntiles[0] + window - 1) / window) * d.ntiles[1];
-            if (rows > 0xF0000000ull) throw InvalidArg{"too many tile pairs in one batch"};
+            if (rows > row_limit) throw too_large();
         }
         size_t nr = tlist ? subs.size() : group.size();
         L.h_rows.p[nr++] = (uint32_t)rows;
@@ -1813,7 +1824,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                     L.h_jobs.p[at] = d;
                     L.h_rows.p[nr++] = (uint32_t)w;
                     w += (uint64_t)d.ntiles[0] * 8;
-                    if (w > 0xF0000000ull) throw InvalidArg{"too many points in one batch"};
+                    if (w > row_limit) throw too_large();
                     at++;
                 }
             }
@@ -2015,12 +2026,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             if (!items && header.nunits == 0 && header.needed > 0) {
                 // the unit list overflowed: nothing was counted; plan again into a larger one
                 L.drop_graph();
-                if (header.needed > unit_limit) {
-                    L.plan_sig.clear();
-                    const int tile = ctx->tile_points;
-                    throw TooLarge{part.end < 0 ? (int)((ranges[roles[0].range[0]].ref.n + tile - 1) / tile)
-                                                : part.end - part.begin};
-                }
+                if (header.needed > unit_limit) throw too_large();
                 plan_units(std::min<size_t>((size_t)header.needed + (header.needed >> 3), unit_limit));
                 sized = false;
                 continue;
@@ -2152,14 +2158,15 @@ void add_stats(tpcf_stats& acc, const tpcf_stats& s) {
 
 // Counts a group: in one launch, or where its plan passes the limits in parts
 // that add up -- the jobs in halves, a single job by ranges of its A tiles.
-void count_group(tpcf_ctx* ctx, Lane& L, std::vector<GroupJob> group, TileRange part = {}) {
-    int tiles = 0;
+void count_group(tpcf_ctx* ctx, Lane& L, std::vector<GroupJob> group, bool lists = true, TileRange part = {}) {
+    TooLarge e;
     try {
-        run_group(ctx, L, group, part.end < 0, part);
+        run_group(ctx, L, group, lists, part);
         return;
-    } catch (const TooLarge& e) {
-        tiles = e.tiles;
+    } catch (const TooLarge& x) {
+        e = x;
     }
+    if (group.size() == 1 && e.lists) return count_group(ctx, L, std::move(group), false);
     for (GroupJob& g : group)
         if (!g.accumulate) {
             int64_t len = 0;
@@ -2169,7 +2176,7 @@ void count_group(tpcf_ctx* ctx, Lane& L, std::vector<GroupJob> group, TileRange 
         }
     tpcf_stats acc{};
     auto half = [&](std::vector<GroupJob> jobs, TileRange r) {
-        count_group(ctx, L, std::move(jobs), r);
+        count_group(ctx, L, std::move(jobs), r.end < 0 && lists, r);
         add_stats(acc, L.stats);
     };
     if (group.size() > 1) {
@@ -2177,10 +2184,10 @@ void count_group(tpcf_ctx* ctx, Lane& L, std::vector<GroupJob> group, TileRange 
         half({group.begin(), mid}, {});
         half({mid, group.end()}, {});
     } else {
-        if (tiles < 2) throw InvalidArg{"too many tile triples in one batch"};
-        const int mid = part.begin + tiles / 2;
+        if (e.tiles < 2) throw InvalidArg{"too many tile triples in one batch"};
+        const int mid = part.begin + e.tiles / 2;
         half(group, {part.begin, mid});
-        half(group, {mid, part.begin + tiles});
+        half(group, {mid, part.begin + e.tiles});
     }
     L.stats = acc;
 }

@@ -79,3 +79,47 @@ def test_a_tile_with_more_units_than_a_plan_may_have(monkeypatch):
         with pytest.raises(tpcf.EngineError) as e:
             eng.count(tpcf.make_spec(tpcf.TRIANGLE, tpcf.LOOP_SAME, TP), eng.job([h] * 3))
         assert e.value.status == -1  # TPCF_ERR_INVALID
+
+
+@pytest.mark.parametrize("name", sorted(KINDS))
+def test_more_rows_than_a_plan_may_have(monkeypatch, name):
+    _check(monkeypatch, "TPCF_MAX_ROWS", 17, *KINDS[name])
+
+
+@pytest.mark.parametrize("precision", [tpcf.GUARDED_FP32, tpcf.PLAIN_FP64])
+def test_pairs_with_more_items_than_a_plan_may_have(monkeypatch, precision):
+    monkeypatch.setenv("TPCF_TILE_POINTS", "8")
+    monkeypatch.setenv("TPCF_MAX_ROWS", "6")
+    axis = (40, 0.0, 30.0)
+    d, r = synth.lattice_mix(203, box=40.0, frac=0.5, seed=1), synth.uniform(150, box=40.0, seed=2)
+    with tpcf.Engine(0) as eng:
+        hd, hr = eng.catalog(d), eng.catalog(r)
+        cases = [([d, d], [hd, hd], tpcf.LOOP_SAME, 0), ([d, r], [hd, hr], tpcf.LOOP_ONE, 1),
+                 ([r, d], [hr, hd], tpcf.LOOP_SAME, 0), ([r, r], [hr, hr], tpcf.LOOP_ALL, 1)]
+        want = [oracle.pair(c, w, axis[1], axis[2], axis[0])[0] for c, _, _, w in cases]
+        specs = [tpcf.make_spec(tpcf.PAIR, loop, [axis], precision=precision) for _, _, loop, _ in cases]
+        jobs = [eng.job(h) for _, h, _, _ in cases]
+        for s, j, w in zip(specs, jobs, want):
+            assert np.array_equal(eng.count(s, j), w)
+            assert eng.stats()["kernel_launches"] > 4
+        assert all(np.array_equal(g, w) for g, w in zip(eng.count_batch(specs, jobs), want))
+
+
+@pytest.mark.parametrize("kind,axes,env", [(tpcf.THREE_SIDE, THREE, "TPCF_NEAR"), (tpcf.TRIANGLE, TP, "TPCF_TRI_LISTS"),
+                                           (tpcf.TRIANGLE_JBJ, JBJ, "TPCF_TRI_LISTS")])
+def test_lists_with_more_items_than_a_plan_may_have(monkeypatch, kind, axes, env):
+    """A batch of lists is halved to single jobs; one whose own lists pass the
+    limit is counted from tiles."""
+    monkeypatch.setenv("TPCF_TILE_POINTS", "8")
+    monkeypatch.setenv(env, "1")
+    d, r = synth.lattice_mix(117, box=22.0, frac=0.5, seed=1), synth.uniform(17, box=20.0, seed=2)
+    combos = [([d, r, r], 1), ([r, d, r], 1), ([d, d, d], 0), ([r, r, r], 0)]
+    want = [_want(kind, c, w, axes) for c, w in combos]
+    with tpcf.Engine(0) as eng:
+        h = {id(d): eng.catalog(d), id(r): eng.catalog(r)}
+        specs = [tpcf.make_spec(kind, tpcf.LOOP_ALL if kind == tpcf.THREE_SIDE else tpcf.LOOP_ONE if w else tpcf.LOOP_SAME,
+                                axes, nan_policy=NAN) for _, w in combos]
+        jobs = [eng.job([h[id(x)] for x in c]) for c, _ in combos]
+        for limit in (200, 2000, 20000):
+            monkeypatch.setenv("TPCF_MAX_ROWS", str(limit))
+            assert all(np.array_equal(g, w) for g, w in zip(eng.count_batch(specs, jobs), want))
