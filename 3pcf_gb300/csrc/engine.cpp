@@ -58,6 +58,7 @@ using namespace tpcf;
 namespace {
 
 thread_local std::string g_tls_error;
+std::atomic<uint64_t> g_allocations{0};  // device and page-locked blocks taken from the driver so far
 
 struct CudaError {
     cudaError_t e;
@@ -99,6 +100,7 @@ class DeviceBlocks {
         while (cls < bytes) cls <<= 1;
         if (cls > kMaxCached) {
             void* p = nullptr;
+            g_allocations++;
             CK(cudaMalloc(&p, bytes));
             *cap = bytes;
             return p;
@@ -115,6 +117,7 @@ class DeviceBlocks {
             }
         }
         void* p = nullptr;
+        g_allocations++;
         if (cudaMalloc(&p, cls) != cudaSuccess) {
             // out of memory: give the kept blocks back and try once more
             (void)cudaGetLastError();
@@ -210,6 +213,7 @@ struct PinnedBuf {
         release();
         size_t c = 4096;
         while (c < m) c <<= 1;
+        g_allocations++;
         CK(cudaMallocHost((void**)&p, c * sizeof(T)));
         n = c;
     }
@@ -2495,12 +2499,16 @@ tpcf_status tpcf_create(tpcf_ctx** out, int32_t device) {
                 L->h_counters.reserve(CTR_WORDS);
                 L->d_hist.reserve((size_t)1 << 22);
                 L->d_counters.reserve(CTR_WORDS);
+                // (three-side lists: per job of a batch of 4,096 its own, two
+                // wedge jobs and an accumulator's; 32 MB of accumulators, as of
+                // histograms)
                 L->d_jobs.reserve((size_t)1 << 16);
-                L->h_jobs.reserve(4096);
-                L->h_rows.reserve(4097);
+                L->h_jobs.reserve((size_t)1 << 14);
+                L->h_rows.reserve(((size_t)1 << 14) + 2);
                 L->d_rows.reserve((size_t)1 << 16);
-                L->d_row_cnt.reserve((size_t)1 << 20);
-                L->d_block_sum.reserve((size_t)1 << 15);
+                L->d_acc.reserve((size_t)1 << 22);
+                L->d_row_cnt.reserve((size_t)1 << 22);
+                L->d_block_sum.reserve((size_t)1 << 17);
                 L->d_units.reserve((size_t)1 << 20);
                 L->d_masks.reserve((size_t)1 << 20);
                 L->d_queue.reserve((size_t)1 << 22);
@@ -2937,3 +2945,7 @@ extern "C" int32_t tpcf_debug_set_acos_exceptions(tpcf_ctx* ctx, const uint32_t*
 // test hook (not in the public header): device blocks above `bytes` are refused
 // as if memory had run out
 extern "C" void tpcf_debug_alloc_limit(uint64_t bytes) { DeviceBlocks::get().set_limit((size_t)bytes); }
+
+// test hook (not in the public header): device and page-locked blocks taken from
+// the driver so far
+extern "C" uint64_t tpcf_debug_allocations(void) { return g_allocations.load(); }

@@ -102,6 +102,8 @@ def lib():
         L.tpcf_debug_set_acos_exceptions.argtypes = [P, P, P, ctypes.c_uint64]
         L.tpcf_debug_alloc_limit.restype = None
         L.tpcf_debug_alloc_limit.argtypes = [ctypes.c_uint64]
+        L.tpcf_debug_allocations.restype = ctypes.c_uint64
+        L.tpcf_debug_allocations.argtypes = []
         L.tpcf_debug_acos_selfcheck.restype = ctypes.c_int64
         L.tpcf_debug_acos_selfcheck.argtypes = [P, ctypes.POINTER(ctypes.c_int64)]
         _LIB = L
