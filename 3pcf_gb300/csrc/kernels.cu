@@ -1939,6 +1939,15 @@ struct TriCentre {
             accounted = binned;
         }
     }
+    // Adds the counts of work to the launch's 64-bit totals before 32 bits run
+    // over (a single centre can have more than 2^32 pairs).
+    __device__ __forceinline__ void report() {
+        if (lane == 0) {
+            if (tested) atomicAdd(rq.evaluated, (unsigned long long)tested);
+            if (binned) atomicAdd(rq.evaluated + 1, (unsigned long long)binned);
+        }
+        tested = binned = accounted = 0;
+    }
     // The centre's triangles: J lists of the near points of view vj, each with
     // K lists of view vk (of one view: with itself, then with the near points
     // after it and the far ones); of two views in both ways round, the second
@@ -1966,6 +1975,7 @@ struct TriCentre {
                     if (kh && sk >= endk) break;
                     if (kh) nk = fill(1, vk, pass == 0 ? TL_NEAR | TL_FAR : TL_FAR, self ? sj : 0, endk, sk);
                     if (nk > 0) pairs(nj, nk, kh, vj, self ? 1 : vk);
+                    if ((tested | binned) >> 31) report();
                     kh = 1;
                 }
             }
