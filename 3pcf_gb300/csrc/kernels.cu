@@ -1570,6 +1570,10 @@ constexpr int TL_LIST = 64;  // entries of a list
 constexpr int TL_QCAP = 288;  // queued pairs: up to 31 pending + 256 of one step
 constexpr unsigned TL_SPILL = 1u << 28;
 constexpr int TL_TILES = 64;  // near tiles kept per list (more: found again at every pass)
+// Margin of compared squares beside their relative ones: subnormal squares (the
+// smallest number is 1.4e-45) have lost bits, in other places in the reference's
+// sums than in the fused ones here.
+constexpr float TL_TINY2 = 2e-38f;
 
 struct TriListWarp {
     // lists J (0) and K (1)
@@ -1797,7 +1801,7 @@ struct TriCentre {
                 W.pos[h][at] = pos;
                 if (h == 0) {
                     const float lim = fmaxf(d * p.list_q, p.list_top);
-                    W.lim[at] = lim * lim;
+                    W.lim[at] = fmaf(lim, lim, TL_TINY2);
                 }
             }
             n += __popc(m);
@@ -1830,7 +1834,7 @@ struct TriCentre {
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z, l2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
         const float m2 = m * m;
         bool take = any && l2 > m2;
-        if (any && fabsf(l2 - m2) <= 2e-6f * m2) {
+        if (any && fabsf(l2 - m2) <= fmaf(2e-6f, m2, TL_TINY2)) {
             // too close to tell: the reference's floats
             const float l = ref_dist<false>(a, b);
             take = l >= m && (MODE == FAST_GEOM || l > 0.f);
@@ -1856,7 +1860,9 @@ struct TriCentre {
             else if (pred == PRED_SAME) w = key[0] <= key[1] && key[1] <= key[2] ? 1u : 0u;
             else w = key[1] <= key[2] ? 1u : 0u;
         }
-        const bool guard = tri_list_bin<MODE>(s, m, l2, min(cj, ck), max(cj, ck), w, p, base, shared_addr(W.dump + lane));
+        // (a longest side whose square may have lost bits to underflow: 0 is in every band)
+        const bool guard = tri_list_bin<MODE>(s, m, l2 < 1e-36f ? 0.f : l2, min(cj, ck), max(cj, ck), w, p, base,
+                                              shared_addr(W.dump + lane));
         if (guard) {  // (positions in the job's order of views)
             const uint32_t pj = W.pos[0][j], pk = W.pos[kh][k];
             push_recheck(rq, slot, w, cpos, vj < vk ? pj : pk, vj < vk ? pk : pj);
@@ -1880,7 +1886,7 @@ struct TriCentre {
             Z[r] = splat2(in ? W.z[kh][k] : 0.f);
             const float d = in ? W.d[kh][k] : 3e18f;  // (past every limit)
             d2[r] = d * d;
-            dm[r] = d2[r] * (1.0f - 1e-5f);
+            dm[r] = fmaf(d2[r], 1.0f - 1e-5f, -TL_TINY2);
         }
         const bool two = nk > 32;
         const uint32_t kj = (uint32_t)lane << 6, qbase = shared_addr(W.queue);
@@ -1893,8 +1899,9 @@ struct TriCentre {
                         zj[2] = {pk2(z4.x, z4.y), pk2(z4.z, z4.w)}, dj[2] = {pk2(d4.x, d4.y), pk2(d4.z, d4.w)};
             const float lj[4] = {l4.x, l4.y, l4.z, l4.w};
             float mj[4];
-            up2(mul2(mul2(dj[0], dj[0]), splat2(1.0f - 1e-5f)), mj[0], mj[1]);
-            up2(mul2(mul2(dj[1], dj[1]), splat2(1.0f - 1e-5f)), mj[2], mj[3]);
+            const f32x2 part = splat2(1.0f - 1e-5f), tiny = splat2(-TL_TINY2);
+            up2(fma2(mul2(dj[0], dj[0]), part, tiny), mj[0], mj[1]);
+            up2(fma2(mul2(dj[1], dj[1]), part, tiny), mj[2], mj[3]);
 #pragma unroll
             for (int r = 0; r < 2; r++) {
                 if (r == 1 && !two) continue;  // warp-uniform
