@@ -51,6 +51,7 @@
 #include <thread>
 #include <tuple>
 #include <unordered_map>
+#include <unordered_set>
 #include <vector>
 
 using namespace tpcf;
@@ -931,9 +932,13 @@ struct tpcf_ctx {
     int slice_tasks = 0;       // tasks per slice (0: at least 8 per CTA and at most 64 slices)
     int group_tasks = 0;       // A tiles per row of the planner, sharing one j-k table (0: by the batch)
     int64_t inflight_bytes = 0;  // device bytes of batches running on serving lanes
-    // autotuner: launch shape per batch signature
+    // share of the pairs of two catalog ranges within a reach (see pair_share; under view_mu)
+    std::map<std::tuple<uint64_t, int64_t, int64_t, uint64_t, int64_t, int64_t, float>, double> shares;
+    // autotuner: launch shape per batch signature, and the batches whose
+    // neighbour lists the device refused (counted from tiles)
     std::mutex tune_mu;
     std::map<uint64_t, Shape> tuned;
+    std::unordered_set<uint64_t> refused;
 };
 
 namespace {
@@ -1352,6 +1357,81 @@ int grid_for(tpcf_ctx* ctx, const Shape& sh, uint64_t ntasks, int sm_cap) {
     return (int)g;
 }
 
+// Share of the pairs of catalog ranges a and b within `reach`, from 16 points
+// spread over a and 256 over b (kept: catalogs do not change); at least half a
+// pair of the sample.  Called with ctx->view_mu held.
+double pair_share(tpcf_ctx* ctx, const tpcf_job& job, int ra, int rb, const int64_t n[3], float reach) {
+    auto key = std::make_tuple(job.catalog[ra], job.begin[ra], n[ra], job.catalog[rb], job.begin[rb], n[rb], reach);
+    auto hit = ctx->shares.find(key);
+    if (hit != ctx->shares.end()) return hit->second;
+    const Catalog &A = *ctx->catalogs.at(job.catalog[ra]), &B = *ctx->catalogs.at(job.catalog[rb]);
+    const int64_t sa = std::min<int64_t>(16, n[ra]), sb = std::min<int64_t>(256, n[rb]);
+    int within = 0;
+    for (int64_t i = 0; i < sa; i++) {
+        const int64_t p = job.begin[ra] + i * n[ra] / sa;
+        for (int64_t j = 0; j < sb; j++) {
+            const int64_t q = job.begin[rb] + j * n[rb] / sb;
+            if (p == q && job.catalog[ra] == job.catalog[rb]) continue;
+            const float dx = A.x[p] - B.x[q], dy = A.y[p] - B.y[q], dz = A.z[p] - B.z[q];
+            within += dx * dx + dy * dy + dz * dz < reach * reach;
+        }
+    }
+    if (ctx->shares.size() >= 65536) ctx->shares.clear();
+    return ctx->shares[key] = std::max(0.5, (double)within) / (double)std::max<int64_t>(1, sa * sb);
+}
+
+// Whether neighbour lists count a three-side batch sooner than tiles, from the
+// shares of its pairs below hist_max.  Times measured on uniform points in a
+// box of 100, 300 to 4,000 of them, and the 150k-point lattice:
+//   lists: 0.82 ps a pair of a list, and beside what a tile launch needs anyway
+//     5 us for two more launches and 0.5 ns an accumulator word, in the reference's
+//     mode 16 us for the wedges;
+//   tiles, reference's mode: 0.5 ps a triple (multiset of one catalog), 0.8 ps
+//     where a CTA's pipelines share a histogram; clean mode: 1.9 ps a triple with
+//     two sides in range and 27 ns a tile triple in reach.
+// (4,000 points, one catalog, 16 bins to hist_max 180, 90 and 60: lists 8.8, 6.2
+// and 1.9 ms, tiles 5.3 each; three catalogs 53, 38 and 12, tiles 32; 32 bins to
+// 180: 8.9 and 8.2.  1,000 points, clean, 32 bins to 10: 40 and 23 us.)
+bool near_pays(tpcf_ctx* ctx, const Binning& bin, const std::vector<GroupJob>& group, bool shared_hist) {
+    const float reach = bin.three.hi;
+    const bool clean = bin.three.clean;
+    double lists = 0, tiles = 0;
+    std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
+    const size_t step = (group.size() + 31) / 32;  // (a sample of a large set)
+    for (size_t g = 0; g < group.size(); g += step) {
+        const tpcf_job& job = *group[g].job;
+        int64_t n[3];
+        for (int r = 0; r < 3; r++) {
+            auto it = ctx->catalogs.find(job.catalog[r]);
+            if (it == ctx->catalogs.end()) return true;  // (refused where its view is looked up)
+            const int64_t all = it->second->n, end = job.end[r] < 0 ? all : job.end[r];
+            if (job.begin[r] < 0 || job.begin[r] > end || end > all) return true;
+            n[r] = end - job.begin[r];
+        }
+        if (n[0] == 0 || n[1] == 0 || n[2] == 0) continue;
+        auto same = [&](int a, int b) {
+            return job.catalog[a] == job.catalog[b] && job.begin[a] == job.begin[b] && n[a] == n[b];
+        };
+        // centre and list roles, and the orderings that one pair stands for
+        const bool ab = same(0, 1), bc = same(1, 2), ac = same(0, 2);
+        const int c = bc ? 0 : ac ? 1 : ab ? 2 : 0, l1 = c == 0 ? 1 : 0, l2 = c == 2 ? 1 : 2;
+        const double sym = ab && bc ? 6 : 1, half = ab && bc ? 6 : ab || bc || ac ? 2 : 1;
+        double pairs = (double)n[c] / half, near_tiles = 1;
+        for (int l : {l1, l2}) {
+            const double f = pair_share(ctx, job, c, l, n, reach);
+            pairs *= f * (double)n[l];
+            // tiles of 64 points are cbrt(64) mean separations wide
+            near_tiles *= std::min(1.0, f * pow(1 + cbrt(64 * 4.19 / (f * (double)n[l])), 3));
+        }
+        const double triples = (double)n[0] * (double)n[1] * (double)n[2] / sym;
+        lists += 0.82e-12 * pairs;
+        tiles += clean ? 1.9e-12 * pairs * half / sym + 27e-9 * near_tiles * triples / (TILE * TILE * TILE)
+                       : (shared_hist ? 0.8e-12 : 0.5e-12) * triples;
+    }
+    const double scale = (double)step;
+    return lists * scale + 0.5e-9 * (double)three_near_acc_words(bin.three.n) + (clean ? 5e-6 : 21e-6) < tiles * scale;
+}
+
 // Runs one group of jobs that share kind, binning and precision in a single
 // persistent launch.  outs[i] receives hist_len counts.  lists: counts from
 // neighbour lists are allowed; part: the A tiles to count of a single job.
@@ -1377,9 +1457,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     bin.tri.tame = tame;
     // three-side counts from neighbour lists (see three_near_kernel)
     const char* near_env = getenv("TPCF_NEAR");
-    const bool near = lists && bin.near_ok && tame && !(near_env && near_env[0] == '0') &&
-                      !shape_candidates(ctx, sp, bin, fp64, true, 0).empty() &&
-                      three_near_acc_words(bin.three.n) * group.size() <= ((size_t)1 << 27);
+    bool near = lists && bin.near_ok && tame && !(near_env && near_env[0] == '0') &&
+                !shape_candidates(ctx, sp, bin, fp64, true, 0).empty() &&
+                three_near_acc_words(bin.three.n) * group.size() <= ((size_t)1 << 27);
+    if (near && !near_env)
+        near = near_pays(ctx, bin, group, shape_candidates(ctx, sp, bin, fp64, false, 0)[0].groups > 0);
     const bool tri_kind = sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ;
     const bool fast_tri = tri_kind && !fp64;
     const bool fast_jbj = sp.kind == TPCF_TRIANGLE_JBJ && !fp64;  // the fast kernel's JBJ binning
@@ -1664,6 +1746,16 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     L.d_counters.reserve(CTR_WORDS);
     const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near, tlist ? (int)nslots : 0);
     const bool plan_hit = sig == L.plan_sig;
+    uint64_t key = 1469598103934665603ull;  // of the batch, in what is remembered of it
+    for (uint64_t v : sig) key = (key ^ v) * 1099511628211ull;
+    if (near) {
+        bool refused = false;
+        {
+            std::lock_guard<std::mutex> tlk(ctx->tune_mu);
+            refused = ctx->refused.count(key) > 0;
+        }
+        if (refused) return run_group(ctx, L, group, false);
+    }
     phase("batch");
     const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
     uint32_t nrows = L.plan_rows;   // pairs and neighbour lists: items
@@ -1964,9 +2056,10 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                 EQ(cudaEventRecordWithFlags(L.ev_mid, st, ev_flags));
                 if (near) {
                     const DevJob* after = L.d_jobs.p + group.size();
-                    EQ(launch_three_wedges(after, L.d_rows.p + group.size() + 1, (int)nwedge_jobs, nwedges, bin.near,
-                                           ctx->num_sms * 8, st));
-                    EQ(launch_three_expand(after + nwedge_jobs, (int)accs.size(), bin.near, st));
+                    const unsigned int* dense = L.d_counters.p + CTR_DENSE;
+                    EQ(launch_three_wedges(after, L.d_rows.p + group.size() + 1, (int)nwedge_jobs, nwedges, dense,
+                                           bin.near, ctx->num_sms * 8, st));
+                    EQ(launch_three_expand(after + nwedge_jobs, (int)accs.size(), dense, bin.near, st));
                 }
                 if (recheck)
                     EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, fast_jbj ? 1 : geom ? 2 : 0,
@@ -2056,8 +2149,6 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     // else the default.  A batch that repeats (its plan was cached) and has no
     // tuned shape yet is counted once with every candidate shape -- each count
     // is exact -- and the fastest is kept for the next calls.
-    uint64_t key = 1469598103934665603ull;
-    for (uint64_t v : sig) key = (key ^ v) * 1099511628211ull;
     const char* tenv = getenv("TPCF_AUTOTUNE");
     const bool autotune = !(tenv && tenv[0] == '0');
     Shape shape = cands[0];
@@ -2091,7 +2182,13 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         count_with(shape, graphs && (plan_hit || (pl_env && pl_env[0] == '0')));
     }
     if (near && L.h_counters.p[CTR_DENSE]) {
-        // a centre with more near tiles than a list holds: by tile triples
+        // a centre with more near tiles than a list holds: by tile triples, now
+        // and whenever the batch comes again
+        {
+            std::lock_guard<std::mutex> tlk(ctx->tune_mu);
+            if (ctx->refused.size() >= 65536) ctx->refused.clear();
+            ctx->refused.insert(key);
+        }
         run_group(ctx, L, group, false);
         return;
     }

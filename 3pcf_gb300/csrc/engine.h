@@ -244,13 +244,15 @@ cudaError_t launch_tri_list(const DevJob* jobs, const uint32_t* item_off, int nj
 size_t tri_list_smem_bytes(int hist_len, int hists, int warps);
 
 // The three launches of a three-side neighbour-list count; *dense is set where the near
-// tiles of a centre are too many (count with launch_three_side instead).
+// tiles of a centre are too many (count with launch_three_side instead): no more
+// is counted then.
 cudaError_t launch_three_near(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int item0,
                               unsigned int nitems, int centres, unsigned int* counter, unsigned int* dense,
                               unsigned long long* work, const NearParams& p, int grid, int pipes, cudaStream_t st);
 cudaError_t launch_three_wedges(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int nitems,
-                                const NearParams& p, int grid, cudaStream_t st);
-cudaError_t launch_three_expand(const DevJob* accs, int naccs, const NearParams& p, cudaStream_t st);
+                                const unsigned int* dense, const NearParams& p, int grid, cudaStream_t st);
+cudaError_t launch_three_expand(const DevJob* accs, int naccs, const unsigned int* dense, const NearParams& p,
+                                cudaStream_t st);
 size_t three_near_acc_words(int n);
 size_t three_near_smem_bytes(int n, int pipes);
 
