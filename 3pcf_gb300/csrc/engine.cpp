@@ -1240,7 +1240,7 @@ class HostPool {
 void parallel_items(size_t n, const std::function<void(size_t)>& fn) { HostPool::get().run(n, fn); }
 
 size_t shape_smem(const tpcf_spec& sp, const Binning& bin, int copies, int groups) {
-    if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) return triangle_smem_bytes(bin.len, copies);
+    if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) return triangle_smem_bytes(bin.len, copies, sp.kind == TPCF_TRIANGLE_JBJ);
     if (sp.kind == TPCF_THREE_SIDE) return three_side_smem_bytes(bin.three, copies, groups);
     return pair_smem_bytes(bin.len, copies);
 }

@@ -257,7 +257,7 @@ size_t three_near_acc_words(int n);
 size_t three_near_smem_bytes(int n, int pipes);
 
 // shared-memory bytes of a launch (for occupancy / admission)
-size_t triangle_smem_bytes(int hist_len, int hist_copies);
+size_t triangle_smem_bytes(int hist_len, int hist_copies, bool jbj);
 size_t three_side_smem_bytes(const ThreeParams& p, int hist_copies, int groups);
 size_t pair_smem_bytes(int hist_len, int hist_copies);
 void pair_guard(PairParams& p);  // from p.n, lo, hi, bw

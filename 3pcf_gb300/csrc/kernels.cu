@@ -622,19 +622,26 @@ constexpr int SET_WORDS = 5;  // the same sets of a warp's current i
 #endif
 constexpr int TRI_GROUP_A = TRI_GROUP_A_TILES;
 // layout: tiles B, C and up to TRI_GROUP_A A tiles | j-class masks | per-warp
-// i-j and i-k rows | j-k sides | per-warp candidate queues (16 bits) | j-k side
-// words (16 bits) | histogram copies
-constexpr size_t TRI_TABLES = (2 + TRI_GROUP_A) * TILE * sizeof(float4) +
-                              (JM_WORDS * TILE + TRI_WARPS * SET_WORDS) * sizeof(unsigned long long) + 2 * TRI_WARPS * TILE * sizeof(int2) +
-                              TILE * TILE * sizeof(float) + TRI_WARPS * TRI_QCAP * sizeof(uint16_t) +
-                              TILE * TILE * sizeof(short);
-// What the histogram does not get: fixed, so that the binnings that fit beside
-// it (up to 46,464 bins in one copy) do not change with the tables.
-constexpr size_t TRI_SMEM_FIXED = 45568;
-static_assert(TRI_TABLES <= TRI_SMEM_FIXED, "fast triangle layout");
+// i-j and i-k rows | j-k sides | per-warp candidate queues | j-k side words
+// (16 bits) | histogram copies
+constexpr size_t tri_tables(size_t queue_entry) {
+    return (2 + TRI_GROUP_A) * TILE * sizeof(float4) +
+           (JM_WORDS * TILE + TRI_WARPS * SET_WORDS) * sizeof(unsigned long long) + 2 * TRI_WARPS * TILE * sizeof(int2) +
+           TILE * TILE * sizeof(float) + TRI_WARPS * TRI_QCAP * queue_entry + TILE * TILE * sizeof(short);
+}
+// Queue entries (14 bits) take 32 bits (10k-point estimator 13.8 ms, with 16 bits
+// 14.0), but 16 for JBJ (whose four copies of 640 bins let four CTAs share an SM
+// then: 5k + 5k points 14.4 ms, else 15.8) and beside the largest histograms: a
+// launch has 227 KB less 1 KB for static shared memory, and up to 46,464 bins
+// must fit.
+constexpr int TRI_WIDE_QUEUE_BINS = 46256;
+constexpr bool tri_wide_queue(int hist_len, bool jbj) { return !jbj && hist_len <= TRI_WIDE_QUEUE_BINS; }
+constexpr size_t TRI_SMEM_WIDE = tri_tables(sizeof(uint32_t)), TRI_SMEM_NARROW = 45568;
+static_assert(TRI_SMEM_WIDE + 4 * TRI_WIDE_QUEUE_BINS <= 226 * 1024 && TRI_SMEM_NARROW + 4 * 46464 <= 226 * 1024 &&
+              tri_tables(sizeof(uint16_t)) <= TRI_SMEM_NARROW, "fast triangle layout");
 // (the plain FP64 kernel's layout -- three tiles, a j-k table of int2 and one
 // row per warp -- fits the same allocation)
-static_assert(TRI_SMEM_FIXED >= 3 * TILE * sizeof(float4) + TILE * TILE * sizeof(int2) + TRI_WARPS * TILE * sizeof(int2),
+static_assert(TRI_SMEM_NARROW >= 3 * TILE * sizeof(float4) + TILE * TILE * sizeof(int2) + TRI_WARPS * TILE * sizeof(int2),
               "FP64 triangle layout");
 
 // Side word of the fast kernel: code16 * 128 + class weight, 16 bits (see
@@ -1059,8 +1066,8 @@ static_assert(TRI_GROUP_A * TILE <= 256 && TRI_GROUP_A * TILE <= TRI_THREADS, "o
 
 // Runs the full binning path on n (<= 64) queued candidates, two per lane
 // (packed into the f32x2 instructions of one binning path).
-template <bool THETA_FULL, int MODE, bool UNIT>
-__device__ __forceinline__ void run_candidates(const uint16_t* cand, int n, const int2* row_ij, const int2* row_ik,
+template <bool THETA_FULL, int MODE, bool UNIT, typename Entry>
+__device__ __forceinline__ void run_candidates(const Entry* cand, int n, const int2* row_ij, const int2* row_ik,
                                                const float* JKd, const short* JKw, const TriParams& p, unsigned int* Hw,
                                                RecheckQueue& q, TriShared& S, uint32_t ia) {
     const int lane = threadIdx.x & 31;
@@ -1152,9 +1159,9 @@ static_assert(SC_M1 + SET_I == SC_M2 + SET_I2 && SC_I1 + SET_R == SC_M2 + SET_I2
 // voxels 2.34 -> 1.92 ms, most of it by the second place that bins, DDD+DDR+DRR+
 // RRR of 1k points 0.465 -> 0.442.  One copy for both costs the weights of all
 // and more registers: 10k-point estimator 9.9 -> 10.5.)
-template <bool UNIT, bool THETA_FULL, int MODE>
+template <bool UNIT, bool THETA_FULL, int MODE, typename Entry>
 __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriParams& p, float4* P, float* JKd, short* JKw, int2* IJ,
-                                    int2* IK, uint16_t* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
+                                    int2* IK, Entry* Q, unsigned long long* JM, TriShared& S, unsigned int* Hw,
                                     RecheckQueue& q, unsigned long long& evaluated, unsigned long long& binned) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float4 *PB = P, *PC = P + TILE, *PA = P + 2 * TILE;
@@ -1175,7 +1182,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
     bool have_jk = false;  // the j-k sides are in the tables
     int2* row_ij = IJ + warp * TILE;
     int2* row_ik = IK + warp * TILE;
-    uint16_t* cand = Q + warp * TRI_QCAP;
+    Entry* cand = Q + warp * TRI_QCAP;
     unsigned long long* sets = JM + JM_WORDS * TILE + warp * SET_WORDS;
     int key_k0 = 0, key_k1 = 0;
     unsigned ev = 0, bn = 0;
@@ -1452,8 +1459,8 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
                         vhi += (w2hi & lbit) ? (1u << 12) : 0u;
                     }
                     const int nlo = __popc(lo);
-                    if (lo & lbit) cand[qn + __popc(lo & lt)] = (uint16_t)vlo;
-                    if (hi & lbit) cand[qn + nlo + __popc(hi & lt)] = (uint16_t)vhi;
+                    if (lo & lbit) cand[qn + __popc(lo & lt)] = (Entry)vlo;
+                    if (hi & lbit) cand[qn + nlo + __popc(hi & lt)] = (Entry)vhi;
                     qn += nlo + __popc(hi);
                     if (qn < 64) continue;
                 } else if (live1) {
@@ -1487,7 +1494,7 @@ __device__ void triangle_group_fast(const DevJob* __restrict__ jobs, const TriPa
 #endif
 // Persistent over the plan's units: tiles B and C of a job with a mask of A
 // tiles.
-template <bool THETA_FULL, int MODE>
+template <bool THETA_FULL, int MODE, typename Entry>
 __global__ void __launch_bounds__(TRI_THREADS, TRI_MIN_BLOCKS)
 triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int* counter, TriParams p, RecheckQueue q,
                      int copies) {
@@ -1497,7 +1504,7 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
     int2* IJ = reinterpret_cast<int2*>(JM + JM_WORDS * TILE + TRI_WARPS * SET_WORDS);
     int2* IK = IJ + TRI_WARPS * TILE;
     float* JKd = reinterpret_cast<float*>(IK + TRI_WARPS * TILE);
-    uint16_t* Q = reinterpret_cast<uint16_t*>(JKd + TILE * TILE);
+    Entry* Q = reinterpret_cast<Entry*>(JKd + TILE * TILE);
     short* JKw = reinterpret_cast<short*>(Q + TRI_WARPS * TRI_QCAP);
     unsigned int* H = reinterpret_cast<unsigned int*>(JKw + TILE * TILE);
     __shared__ TriShared S;
@@ -1529,9 +1536,9 @@ triangle_fast_kernel(const DevJob* __restrict__ jobs, UnitList ul, unsigned int*
         since += n;
         if (n == 0) continue;  // a part without A tiles
         if (S.pred == PRED_DDR || S.pred == PRED_RDD)
-            triangle_group_fast<false, THETA_FULL, MODE>(jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
+            triangle_group_fast<false, THETA_FULL, MODE, Entry>(jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
         else
-            triangle_group_fast<true, THETA_FULL, MODE>(jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
+            triangle_group_fast<true, THETA_FULL, MODE, Entry>(jobs, p, P, JKd, JKw, IJ, IK, Q, JM, S, Hw, q, ev, bn);
     }
     if (cur >= 0) flush_hist(H, copies, p.len, jobs[cur].hist);
     __syncthreads();
@@ -3539,7 +3546,9 @@ __global__ void acos_check_kernel(AcosTable t, uint32_t key_begin, uint32_t coun
 // ---------------------------------------------------------------------------
 // Launchers
 
-size_t triangle_smem_bytes(int hist_len, int copies) { return TRI_SMEM_FIXED + (size_t)hist_len * copies * 4; }
+size_t triangle_smem_bytes(int hist_len, int copies, bool jbj) {
+    return (tri_wide_queue(hist_len, jbj) ? TRI_SMEM_WIDE : TRI_SMEM_NARROW) + (size_t)hist_len * copies * 4;
+}
 size_t three_side_smem_bytes(const ThreeParams& p, int copies, int groups) {
     // groups > 0: the grouped kernel (one histogram); else 8-warp CTAs with
     // 'copies' copies (0: the global histogram)
@@ -3583,8 +3592,12 @@ cudaError_t prepare_kernels(int device) {
     int optin = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (e != cudaSuccess) return e;
-    const void* fns[] = {(const void*)triangle_fast_kernel<true, FAST_TP>, (const void*)triangle_fast_kernel<false, FAST_TP>,
-                         (const void*)triangle_fast_kernel<false, FAST_JBJ>, (const void*)triangle_fast_kernel<false, FAST_GEOM>,
+    const void* fns[] = {(const void*)triangle_fast_kernel<true, FAST_TP, uint32_t>,
+                         (const void*)triangle_fast_kernel<false, FAST_TP, uint32_t>,
+                         (const void*)triangle_fast_kernel<false, FAST_GEOM, uint32_t>,
+                         (const void*)triangle_fast_kernel<false, FAST_TP, uint16_t>,
+                         (const void*)triangle_fast_kernel<false, FAST_JBJ, uint16_t>,
+                         (const void*)triangle_fast_kernel<false, FAST_GEOM, uint16_t>,
                          (const void*)triangle_fp64_kernel<MODE_FP64>, (const void*)triangle_fp64_kernel<MODE_GEOM>,
                          (const void*)triangle_fp64_kernel<MODE_JBJ>, (const void*)three_side_kernel<true, true>,
                          (const void*)three_side_kernel<true, false>, (const void*)three_side_kernel<false, true>,
@@ -3606,11 +3619,13 @@ cudaError_t prepare_kernels(int device) {
 
 cudaError_t launch_triangle_fast(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
                                  RecheckQueue q, int grid, int copies, int mode, cudaStream_t st) {
-    size_t smem = triangle_smem_bytes(p.len, copies);
-    auto kern = mode == FAST_JBJ    ? triangle_fast_kernel<false, FAST_JBJ>
-                : mode == FAST_GEOM ? triangle_fast_kernel<false, FAST_GEOM>
-                : p.theta_full      ? triangle_fast_kernel<true, FAST_TP>
-                                    : triangle_fast_kernel<false, FAST_TP>;
+    const size_t smem = triangle_smem_bytes(p.len, copies, mode == FAST_JBJ);
+    const bool wide = tri_wide_queue(p.len, false);
+    auto kern = mode == FAST_JBJ    ? triangle_fast_kernel<false, FAST_JBJ, uint16_t>
+                : mode == FAST_GEOM ? (wide ? triangle_fast_kernel<false, FAST_GEOM, uint32_t> : triangle_fast_kernel<false, FAST_GEOM, uint16_t>)
+                : !wide             ? triangle_fast_kernel<false, FAST_TP, uint16_t>
+                : p.theta_full      ? triangle_fast_kernel<true, FAST_TP, uint32_t>
+                                    : triangle_fast_kernel<false, FAST_TP, uint32_t>;
     kern<<<grid, TRI_THREADS, smem, st>>>(jobs, ul, counter, p, q, copies);
     return cudaGetLastError();
 }
@@ -3625,7 +3640,7 @@ cudaError_t launch_triangle_recheck(const DevJob* jobs, RecheckQueue q, const Tr
 
 cudaError_t launch_triangle_fp64(const DevJob* jobs, UnitList ul, unsigned int* counter, const TriParams& p,
                                  AcosTable t, int grid, int copies, int mode, cudaStream_t st) {
-    size_t smem = triangle_smem_bytes(p.len, copies);
+    const size_t smem = triangle_smem_bytes(p.len, copies, mode == MODE_JBJ);
     auto kern = mode == MODE_GEOM ? triangle_fp64_kernel<MODE_GEOM>
                 : mode == MODE_JBJ  ? triangle_fp64_kernel<MODE_JBJ>
                                     : triangle_fp64_kernel<MODE_FP64>;

@@ -31,6 +31,10 @@ def test_the_largest(monkeypatch, lists):
         for precision in (tpcf.GUARDED_FP32, tpcf.PLAIN_FP64):
             s = tpcf.make_spec(tpcf.TRIANGLE, tpcf.LOOP_SAME, MOST, precision=precision, nan_policy=NAN)
             assert np.array_equal(eng.count(s, j), want)
+        # FP64 geometry, also by the exhaustive kernel (coordinates past 1e15)
+        far = np.concatenate([d, np.array([[2e15, 2e15, 2e15]], np.float32)])
+        s = tpcf.make_spec(tpcf.TRIANGLE, tpcf.LOOP_SAME, MOST, precision=tpcf.GEOMETRY_FP64, nan_policy=NAN)
+        assert np.array_equal(eng.count(s, j), eng.count(s, eng.job([eng.catalog(far)] * 3)))
         s = tpcf.make_spec(tpcf.TRIANGLE_JBJ, tpcf.LOOP_SAME, JBJ)
         assert np.array_equal(eng.count(s, j), oracle.triangle_jbj([d] * 3, 0, JBJ)[0])
         with pytest.raises(tpcf.EngineError) as e:
