@@ -1779,6 +1779,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         PlanParams pp{};
         pp.window = window;
         pp.per_tile = fast_tri ? 0 : 1;
+        // (A part makes the unit's j-k table again.  That is most of the work where
+        // sides are computed in FP64, or where clean mode leaves few triples:
+        // three-side DDD+DRR of 400 points in plain FP64 0.57 ms whole, 0.83 cut; a
+        // clean D-D-R of 1,000 points, hist_max a tenth of the box, 31 and 42 us.)
+        pp.max_parts = fast_tri ? 16 : sp.kind == TPCF_THREE_SIDE && (fp64 || bin.three.clean) ? 1 : 4;
         pp.tri = bin.tri_prune ? 1 : 0;
         pp.slots = grid_for(ctx, cands[0], UINT64_MAX, L.sm_cap) * std::max(1, cands[0].groups);
         const double l2 = bin.lmax * bin.lmax;

@@ -179,6 +179,7 @@ struct PlanParams {
     int window;        // A tiles per row (at most MAX_WINDOW)
     int per_tile;      // 1: a unit per A tile; 0: a unit per row and tile C, its A tiles as a mask
     int tri;           // test the s and q ranges on the triple's side bounds
+    int max_parts;     // parts a heavy unit may be cut into: 1, 4 or (per_tile == 0) 16
     int slots;         // CTAs (pipelines) that will share the units
     float lmax2;       // squared: no counted triple has a side at or above it (infinite: no pruning)
     float s_lo2, s_hi2, q_hi2;

@@ -571,7 +571,7 @@ plan_scan(uint2* block_sum, int nblocks, PlanParams pp, PlanHeader* header, uint
         // 0.51 ms cut to them; 10k points have enough whole units.)
         // (single tile triples cost alike: two per CTA are enough)
         const unsigned long long want = (pp.per_tile ? 2ull : 16ull) * (unsigned)pp.slots;
-        const uint32_t top = pp.per_tile ? 4u : 16u;
+        const uint32_t top = (uint32_t)pp.max_parts;
         uint32_t parts = 1;
         // (not beyond what the unit list holds)
         while (parts < top && th > 0 && th * parts < want && th * parts * 4 + tl <= capacity) parts *= 4;
