@@ -1819,7 +1819,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
             long long tile_pairs = 0;
             for (const RoleJob& r : roles)
                 tile_pairs += (long long)ranges[r.range[0]].view->ntiles * ranges[r.range[1]].view->ntiles;
-            plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS);
+            plan_chunk = pair_chunk(tile_pairs, ctx->num_sms * PAIR_CTAS, fp64);
         } else if (near) {
             // one centre per item where that balances the pipelines, else as
             // many as an item may have

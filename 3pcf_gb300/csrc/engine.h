@@ -262,7 +262,7 @@ size_t triangle_smem_bytes(int hist_len, int hist_copies, bool jbj);
 size_t three_side_smem_bytes(const ThreeParams& p, int hist_copies, int groups);
 size_t pair_smem_bytes(int hist_len, int hist_copies);
 void pair_guard(PairParams& p);  // from p.n, lo, hi, bw
-int pair_chunk(long long tile_pairs, int ctas);
+int pair_chunk(long long tile_pairs, int ctas, bool fp64);
 
 }  // namespace tpcf
 #endif

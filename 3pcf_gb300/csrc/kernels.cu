@@ -3575,8 +3575,12 @@ void pair_guard(PairParams& p) {
 
 // Tiles B per item of the pair kernels: as many as leave eight items to every
 // resident CTA, at least one for each of its warps (an item's tile A is staged
-// once, but the items are what balances the CTAs).
-int pair_chunk(long long tile_pairs, int ctas) {
+// once, but the items are what balances the CTAs).  One where there are few tile
+// pairs for the CTAs, whose warps then share the points of tile A (1,500 points,
+// DD + DR: 21 us with eight, 12 with one), and in FP64, where a tile pair is 30 us
+// (6,000 points 2.0 and 1.0 ms).
+int pair_chunk(long long tile_pairs, int ctas, bool fp64) {
+    if (fp64 || tile_pairs < 2ll * ctas) return 1;
     int chunk = PR_CHUNK_MAX;
     while (chunk > PR_WARPS && tile_pairs / chunk < 8ll * ctas) chunk /= 2;
     return chunk;
@@ -3854,7 +3858,7 @@ extern "C" int32_t tpcf_pair_count_noalloc(const float* x0, const float* y0, con
                 cudaSuccess)
                 return own_error();
         }
-        const int slots = sms * PAIR_CTAS, chunk = pair_chunk((long long)ntA * ntB, slots);
+        const int slots = sms * PAIR_CTAS, chunk = pair_chunk((long long)ntA * ntB, slots, false);
         const int nbc = (ntB + chunk - 1) / chunk;
         const int grid = (int)std::min<long long>((long long)ntA * nbc, slots);
         pair_kernel_noalloc<<<grid, PR_THREADS, smem, st>>>(x0, y0, z0, (int)n0, x1, y1, z1, (int)n1, same ? 1 : 0,
