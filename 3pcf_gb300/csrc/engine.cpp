@@ -1381,21 +1381,23 @@ double pair_share(tpcf_ctx* ctx, const tpcf_job& job, int ra, int rb, const int6
 }
 
 // Whether neighbour lists count a three-side batch sooner than tiles, from the
-// shares of its pairs below hist_max.  Times measured on uniform points in a
-// box of 100, 300 to 4,000 of them, and the 150k-point lattice:
-//   lists: 0.82 ps a pair of a list, and beside what a tile launch needs anyway
-//     5 us for two more launches and 0.5 ns an accumulator word, in the reference's
-//     mode 16 us for the wedges;
+// shares of its pairs below hist_max.  Times beyond those of any launch, measured
+// on uniform points (60 to 6,000 in boxes of 100 to 400) and the 150k-point lattice:
+//   lists: 0.82 ps a pair of a list; 13 us and 0.5 ns an accumulator word, for
+//     every further job 3 us and 1 ns a word; in the reference's mode 8 us for the
+//     wedges;
 //   tiles, reference's mode: 0.5 ps a triple (multiset of one catalog), 0.8 ps
 //     where a CTA's pipelines share a histogram; clean mode: 1.9 ps a triple with
-//     two sides in range and 27 ns a tile triple in reach.
-// (4,000 points, one catalog, 16 bins to hist_max 180, 90 and 60: lists 8.8, 6.2
-// and 1.9 ms, tiles 5.3 each; three catalogs 53, 38 and 12, tiles 32; 32 bins to
-// 180: 8.9 and 8.2.  1,000 points, clean, 32 bins to 10: 40 and 23 us.)
+//     two sides in range, 8 ns a tile triple in reach, and a unit's own time, 0.7 us
+//     (shared histogram 1.5) a neighbour of its points.
+// (4,000 points, one catalog, 16 bins to hist_max 180, 90 and 60 in a box of 100:
+// lists 8.8, 6.2 and 1.9 ms, tiles 5.3 each; three catalogs 53, 38 and 12, tiles 32;
+// 32 bins to 180: 8.9 and 8.2.  Clean, calls: 700 points, 32 bins to 32, lists 99 us,
+// tiles 182; 1,500 in a box of 200 and two jobs 166 and 143; 300 to 12 91 and 78.)
 bool near_pays(tpcf_ctx* ctx, const Binning& bin, const std::vector<GroupJob>& group, bool shared_hist) {
     const float reach = bin.three.hi;
     const bool clean = bin.three.clean;
-    double lists = 0, tiles = 0;
+    double lists = 0, tiles = 0, neighbours = 0;
     std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
     const size_t step = (group.size() + 31) / 32;  // (a sample of a large set)
     for (size_t g = 0; g < group.size(); g += step) {
@@ -1420,16 +1422,19 @@ bool near_pays(tpcf_ctx* ctx, const Binning& bin, const std::vector<GroupJob>& g
         for (int l : {l1, l2}) {
             const double f = pair_share(ctx, job, c, l, n, reach);
             pairs *= f * (double)n[l];
+            neighbours = std::max(neighbours, f * (double)n[l]);
             // tiles of 64 points are cbrt(64) mean separations wide
             near_tiles *= std::min(1.0, f * pow(1 + cbrt(64 * 4.19 / (f * (double)n[l])), 3));
         }
         const double triples = (double)n[0] * (double)n[1] * (double)n[2] / sym;
         lists += 0.82e-12 * pairs;
-        tiles += clean ? 1.9e-12 * pairs * half / sym + 27e-9 * near_tiles * triples / (TILE * TILE * TILE)
+        tiles += clean ? 1.9e-12 * pairs * half / sym + 8e-9 * near_tiles * triples / (TILE * TILE * TILE)
                        : (shared_hist ? 0.8e-12 : 0.5e-12) * triples;
     }
-    const double scale = (double)step;
-    return lists * scale + 0.5e-9 * (double)three_near_acc_words(bin.three.n) + (clean ? 5e-6 : 21e-6) < tiles * scale;
+    const double words = (double)three_near_acc_words(bin.three.n), jobs = (double)group.size();
+    lists = lists * (double)step + 13e-6 + 0.5e-9 * words + (jobs - 1) * (3e-6 + 1e-9 * words) + (clean ? 0 : 8e-6);
+    tiles = tiles * (double)step + (clean ? (shared_hist ? 1.5e-6 : 0.7e-6) * neighbours : 0);
+    return lists < tiles;
 }
 
 // Runs one group of jobs that share kind, binning and precision in a single

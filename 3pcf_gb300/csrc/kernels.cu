@@ -3577,7 +3577,7 @@ void pair_guard(PairParams& p) {
 // resident CTA, at least one for each of its warps (an item's tile A is staged
 // once, but the items are what balances the CTAs).  One where there are few tile
 // pairs for the CTAs, whose warps then share the points of tile A (1,500 points,
-// DD + DR: 21 us with eight, 12 with one), and in FP64, where a tile pair is 30 us
+// DD + DR: 21 us with eight, 17 with one), and in FP64, where a tile pair is 30 us
 // (6,000 points 2.0 and 1.0 ms).
 int pair_chunk(long long tile_pairs, int ctas, bool fp64) {
     if (fp64 || tile_pairs < 2ll * ctas) return 1;

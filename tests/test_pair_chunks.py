@@ -1,5 +1,5 @@
 """Pair counts at catalog sizes on both sides of each number of tiles B per item
-(1 below 1,520 tile pairs, 8, 16 and 32 from some 12,000, 97,000 and 195,000 on),
+(1 below 1,520 tile pairs, 8 above, 16 and 32 from some 97,000 and 195,000 on),
 against the plain FP64 kernel, whose items have one, through both pair entry
 points.  Integer histograms: tolerance 0."""
 import numpy as np

@@ -38,6 +38,25 @@ def test_rule(monkeypatch, overflow, n, hi, bins, tiles):
     assert got.sum() > 0
 
 
+@pytest.mark.parametrize("overflow", [tpcf.OVERFLOW_COMPAT, tpcf.OVERFLOW_CLEAN])
+def test_sets_of_small_jobs_go_to_the_tiles(monkeypatch, overflow):
+    """Every job of such a set would make a launch's CTAs change accumulators."""
+    d = synth.uniform(20000, box=200.0, seed=7)
+    begin = np.random.default_rng(1).integers(0, 19900, (50, 3))
+    tasks = {}
+    with tpcf.Engine(0) as eng:
+        h = eng.catalog(d)
+        jobs = [eng.job([h] * 3, [(int(x), int(x) + 100) for x in b]) for b in begin]
+        res = []
+        for env in (None, "0", "1"):
+            if env:
+                monkeypatch.setenv("TPCF_NEAR", env)
+            res.append(eng.count_batch([_spec(overflow, (16, 0.0, 32.0))] * len(jobs), jobs))
+            tasks[env] = eng.stats()["tasks"]
+        assert all(np.array_equal(a, b) and np.array_equal(a, c) for a, b, c in zip(*res))
+    assert tasks[None] == tasks["0"] != tasks["1"]
+
+
 def test_refused_lists_are_not_tried_again(monkeypatch):
     """Tiles of eight points: 290 near tiles, more than are listed."""
     monkeypatch.setenv("TPCF_TILE_POINTS", "8")
