@@ -730,24 +730,23 @@ bool same_binning(const tpcf_spec& a, const tpcf_spec& b) {
 // loop units (the reference's numcalc / fake_tot)
 
 uint64_t loop_units(int kind, int loop, const int64_t n[3]) {
-    typedef unsigned __int128 u128;  // sums of the loops' bounds in closed form, modulo 2^64
-    // (a range whose end lies before its begin has a negative size: its loop does not run)
-    if (kind == TPCF_THREE_SIDE) return (uint64_t)n[0] * n[1] * n[2];
-    if (kind == TPCF_PAIR) {
-        if (loop != TPCF_LOOP_SAME) return (uint64_t)n[0] * n[1];
-        const u128 m = std::max<int64_t>(std::min(n[0], n[1]), 0);  // sum over i < m of n1 - i
-        return m ? (uint64_t)(m * (u128)n[1] - m * (m - 1) / 2) : 0;
-    }
-    if (loop == TPCF_LOOP_ALL) return (uint64_t)n[0] * n[1] * n[2];
-    const u128 n0 = n[0], n2 = n[2], m = std::max<int64_t>(std::min(n[1], n[2]), 0);
-    if (m == 0 || n0 == 0) return 0;
-    const u128 tail = m * n2 - m * (m - 1) / 2;  // sum over j < m of n2 - j
-    if (loop == TPCF_LOOP_ONE) return (uint64_t)(n0 * tail);
+    if (kind == TPCF_THREE_SIDE || (kind != TPCF_PAIR && loop == TPCF_LOOP_ALL)) return (uint64_t)n[0] * n[1] * n[2];
+    if (kind == TPCF_PAIR && loop != TPCF_LOOP_SAME) return (uint64_t)n[0] * n[1];
+    // Sums of the loops' bounds in closed form, modulo 2^64.  (A range whose end
+    // lies before its begin has a negative size: its loop does not run.)
+    const uint64_t last = kind == TPCF_PAIR ? n[1] : n[2];
+    const int64_t outer = kind == TPCF_PAIR ? std::min(n[0], n[1]) : std::min(n[1], n[2]);
+    if (outer <= 0) return 0;
+    const uint64_t m = outer, tail = m * last - m * (m - 1) / 2;  // sum over j < m of last - j
+    if (kind == TPCF_PAIR) return tail;
+    const uint64_t n0 = n[0];
+    if (loop == TPCF_LOOP_ONE) return n0 * tail;
     // LOOP_SAME: min(n0, j + 1) points i for each j
-    const u128 p = n[0] > 0 ? std::min(m, n0) : 0;
-    const u128 sq = (p - 1) * p * (2 * p - 1) / 6, lin = p * (p - 1) / 2;  // sums of j^2 and j over j < p
-    const u128 head = p * n2 + n2 * lin - lin - sq;                        // (j + 1) (n2 - j)
-    return (uint64_t)(head + n0 * (tail - (p * n2 - lin)));
+    const uint64_t p = n[0] > 0 ? std::min(m, n0) : 0;
+    const uint64_t lin = p ? p * (p - 1) / 2 : 0;                                  // sums of j and j^2 over j < p
+    const uint64_t sq = lin % 3 == 0 ? lin / 3 * (2 * p - 1) : lin * ((2 * p - 1) / 3);
+    const uint64_t head = p * last + last * lin - lin - sq;                        // (j + 1) (last - j)
+    return head + n0 * (tail - (p * last - lin));
 }
 
 // ---------------------------------------------------------------------------
@@ -889,6 +888,7 @@ struct Shape {
 struct tpcf_ctx {
     int device = 0;
     int num_sms = 0;
+    int max_smem_sm = 0, max_smem_block = 0;  // shared memory of an SM, most of a block
     std::recursive_mutex mu;      // serialises the synchronous API (lane 0)
     std::recursive_mutex view_mu; // catalogs and spatial views
     std::mutex acos_mu;
@@ -1249,9 +1249,7 @@ size_t shape_smem(const tpcf_spec& sp, const Binning& bin, int copies, int group
 // triangle kernel is compiled for four CTAs per SM (its register budget);
 // the others take as many CTAs as shared memory allows, up to 8.
 std::vector<Shape> shape_candidates(tpcf_ctx* ctx, const tpcf_spec& sp, const Binning& bin, bool fp64, bool near, int tlist) {
-    int max_smem_sm = 0, max_smem_block = 0;
-    cudaDeviceGetAttribute(&max_smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
-    cudaDeviceGetAttribute(&max_smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    const int max_smem_sm = ctx->max_smem_sm, max_smem_block = ctx->max_smem_block;
     auto fit = [&](int copies, int cap_per_sm, int groups = 0) {
         Shape sh;
         sh.copies = copies;
@@ -1355,6 +1353,19 @@ int grid_for(tpcf_ctx* ctx, const Shape& sh, uint64_t ntasks, int sm_cap) {
     uint64_t g = (uint64_t)sms * sh.per_sm;
     if (g > ntasks) g = std::max<uint64_t>(ntasks, 1);
     return (int)g;
+}
+
+// Hash of a batch's signature: four chains side by side (one chain of 66,000
+// multiplications, the signature of 16,500 voxel jobs, is 0.1 ms).
+uint64_t batch_key(const std::vector<uint64_t>& sig) {
+    uint64_t h[4] = {1469598103934665603ull, 0x9E3779B97F4A7C15ull, 0xC2B2AE3D27D4EB4Full, 0x165667B19E3779F9ull};
+    size_t i = 0;
+    for (; i + 4 <= sig.size(); i += 4)
+        for (int k = 0; k < 4; k++) h[k] = (h[k] ^ sig[i + k]) * 1099511628211ull;
+    for (; i < sig.size(); i++) h[0] = (h[0] ^ sig[i]) * 1099511628211ull;
+    uint64_t key = sig.size();
+    for (uint64_t x : h) key = (key ^ x) * 1099511628211ull;
+    return key;
 }
 
 // Share of the pairs of catalog ranges a and b within `reach`, from 16 points
@@ -1751,8 +1762,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     L.d_counters.reserve(CTR_WORDS);
     const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near, tlist ? (int)nslots : 0);
     const bool plan_hit = sig == L.plan_sig;
-    uint64_t key = 1469598103934665603ull;  // of the batch, in what is remembered of it
-    for (uint64_t v : sig) key = (key ^ v) * 1099511628211ull;
+    const uint64_t key = batch_key(sig);  // of the batch, in what is remembered of it
     if (near) {
         bool refused = false;
         {
@@ -2564,6 +2574,8 @@ tpcf_status tpcf_create(tpcf_ctx** out, int32_t device) {
         ctx->device = device;
         CK(cudaSetDevice(device));
         CK(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device));
+        CK(cudaDeviceGetAttribute(&ctx->max_smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+        CK(cudaDeviceGetAttribute(&ctx->max_smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         CK(prepare_kernels(device));
         const char* tp = getenv("TPCF_TILE_POINTS");
         if (tp) ctx->tile_points = std::max(8, std::min(TILE, atoi(tp)));
