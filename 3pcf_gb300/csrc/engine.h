@@ -33,27 +33,20 @@ constexpr uint32_t UNIT_QUARTER = 1u << 24;
 // recheck queue item .x: job slot | weight << 22
 constexpr int RECHECK_WEIGHT_SHIFT = 22;
 
-// Per-side word of the triangle kernels: word = code * 128 + class_weight.
-// code is the side's s-bin times Q*T (monotone in the side length, so the
-// codes of the shortest and middle side are the min and median of the three
-// words, >> 7); the special codes below keep that order.  class_weight counts
-// side classes so that the sum of a triangle's three weights tells whether any
-// permutation can be counted: below s_lo: 4, at/above s_hi (or rounding to bin
-// S): 1, in range: 0, zero length or at/above the largest side a counted
-// triangle can have: 32 (rejects the triangle).
-constexpr int CODE_ZERO = -(1 << 23);   // side length exactly 0
-constexpr int CODE_BELOW = -(1 << 22);  // 0 < side < s_lo
-constexpr int CODE_ABOVE = (1 << 22);   // side >= s_hi
-constexpr int CW_IN = 0, CW_ABOVE = 1, CW_BELOW = 4, CW_REJECT = 32;
-constexpr int MAX_TRI_BINS = (1 << 22) - 1;  // S*Q*T limit of the triangle kernel encodings
-// The fast (guarded FP32) kernel's side words fit 16 bits, so that its j-k
-// table holds them in two bytes: word = code16 * 128 + class_weight with
-// code16 the side's s-bin itself (the kernel multiplies by Q*T) and the
-// special codes below, in the same order as above.  It takes binnings of at
+// Per-side word of the fast triangle kernel: word = code16 * 128 + class_weight,
+// in 16 bits, so that its j-k table holds it in two bytes.  code16 is the side's
+// s-bin (monotone in the side length, so that those of the shortest and middle
+// side are the min and median of the three words, >> 7; the kernel multiplies by
+// Q*T); the special codes below keep that order.  The kernel takes binnings of at
 // most MAX_FAST_S s bins (b == S, rounding at the top edge, stays below
-// CODE16_ABOVE).
+// CODE16_ABOVE).  class_weight counts side classes so that the sum of a
+// triangle's three weights tells whether any permutation can be counted: below
+// s_lo: 4, at/above s_hi (or rounding to bin S): 1, in range: 0, zero length or
+// at/above the largest side a counted triangle can have: 32 (rejects the triangle).
 constexpr int CODE16_ZERO = -2, CODE16_BELOW = -1, CODE16_ABOVE = 255;
+constexpr int CW_IN = 0, CW_ABOVE = 1, CW_BELOW = 4, CW_REJECT = 32;
 constexpr int MAX_FAST_S = 254;
+constexpr int MAX_TRI_BINS = (1 << 22) - 1;  // S*Q*T limit of the triangle kernels
 // most A tiles in one window of the planner (one mask word)
 constexpr int MAX_WINDOW = 32;
 // weight sum (4*nBelow + nAbove, >= 32 if rejected) -> permutation validity

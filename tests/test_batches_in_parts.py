@@ -89,7 +89,7 @@ def test_more_rows_than_a_plan_may_have(monkeypatch, name):
 @pytest.mark.parametrize("precision", [tpcf.GUARDED_FP32, tpcf.PLAIN_FP64])
 def test_pairs_with_more_items_than_a_plan_may_have(monkeypatch, precision):
     monkeypatch.setenv("TPCF_TILE_POINTS", "8")
-    monkeypatch.setenv("TPCF_MAX_ROWS", "6")
+    monkeypatch.setenv("TPCF_MAX_ROWS", "60")  # (items of one tile pair)
     axis = (40, 0.0, 30.0)
     d, r = synth.lattice_mix(203, box=40.0, frac=0.5, seed=1), synth.uniform(150, box=40.0, seed=2)
     with tpcf.Engine(0) as eng:
