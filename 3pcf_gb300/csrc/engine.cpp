@@ -454,6 +454,7 @@ struct Binning {
     double lmax = INFINITY;   // no counted triangle/pair has a side >= lmax
     bool tri_prune = false;   // triangle: test the s and q ranges on tile-triple side bounds
     double s_lo = 0, s_hi = 0, q_hi = 0;
+    double lmin_pair = 0;     // pairs: no counted pair has d < lmin_pair
 };
 
 // Whether a job of this spec runs in the guarded FP32 kernels.  The fast
@@ -696,6 +697,7 @@ Binning make_binning(const tpcf_spec& sp) {
         }
     }
     // device copy of the bound, rounded up so that a float side >= it is >= lmax
+    if (sp.kind == TPCF_TRIANGLE_JBJ) b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
     if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) {
         TriParams& p = b.tri;
         p.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
@@ -817,10 +819,10 @@ struct Lane {
     }
 };
 
+// d_counters: words zeroed before every count, then the header of the plan
 // shares of centres per warp of the triangle lists at least
 constexpr uint64_t TL_WANT = 32;
 
-// d_counters: words zeroed before every count, then the header of the plan
 constexpr int CTR_WORK = 0;     // units (items) handed out
 constexpr int CTR_RECHECK = 1;  // queued guard-band triangles
 constexpr int CTR_EVAL = 2;     // evaluated (two words), binned (pairs: tile pairs; two words)
@@ -1492,11 +1494,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     //   JBJ with very many centres, whose tile triples hold few shortest sides
     //   in range (blobs of 25k points, 150,000 centres, 1244 -> 1097 ms, 15k 343 ->
     //   338, 10k 139 -> 140, 5k 24 -> 28 ms; s/m from 0.5: 25k 179 -> 143, 10k 23.4
-    //   -> 22.9, 7k 9.9 -> 10.4).  The number of centres stands in for how few of a
-    //   tile triple's triangles are near, which depends on the field: of uniform
-    //   points the lists are sooner from 5k on (14k in a box of 100 114 -> 74 ms, 5k
-    //   9.0 -> 4.6), of many small blobs not at 25k (500 points a blob, 14k 44 ->
-    //   57, 25k 164 -> 171).
+    //   -> 22.9, 7k 9.9 -> 10.4).
     // Sets of many small jobs (voxels) keep the tiles: each of a job's centres
     // is an item here (16,500 jobs of a 20k cone 1.9 -> 8.8 ms).
     const char* tl_env = getenv("TPCF_TRI_LISTS");
@@ -1774,7 +1772,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
         if (refused) return run_group(ctx, L, group, false);
     }
     phase("batch");
-    const int window = ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW) : (group.size() > 64 ? 16 : 4);
+    // (plain FP64 one A tile at a time, so that CTAs side by side take unlike tiles B
+    // and C: three-side DDD+DRR of 400 points 0.65 -> 0.55 ms)
+    const int window = fp64                   ? 1
+                       : ctx->group_tasks > 0 ? std::min(ctx->group_tasks, MAX_WINDOW)
+                                              : (group.size() > 64 ? 16 : 4);
     uint32_t nrows = L.plan_rows;   // pairs and neighbour lists: items
     int plan_chunk = L.plan_chunk;  // pairs: tiles B per item; neighbour lists: centres per item
     uint32_t nwedges = L.plan_wedges;
