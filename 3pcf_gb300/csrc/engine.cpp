@@ -1392,23 +1392,27 @@ double pair_share(tpcf_ctx* ctx, const tpcf_job& job, int ra, int rb, const int6
 }
 
 // Whether neighbour lists count a three-side batch sooner than tiles, from the
-// shares of its pairs below hist_max.  Times beyond those of any launch, measured
-// on uniform points (60 to 6,000 in boxes of 100 to 400) and the 150k-point lattice:
-//   lists: 0.82 ps a pair of a list; 13 us and 0.5 ns an accumulator word, for
-//     every further job 3 us and 1 ns a word; in the reference's mode 8 us for the
-//     wedges;
-//   tiles, reference's mode: 0.5 ps a triple (multiset of one catalog), 0.8 ps
-//     where a CTA's pipelines share a histogram; clean mode: 1.9 ps a triple with
-//     two sides in range, 8 ns a tile triple in reach, and a unit's own time, 0.7 us
-//     (shared histogram 1.5) a neighbour of its points.
+// shares of its pairs below hist_max.  The coefficients fit the calls' times beyond
+// those of any launch, over 950 batches counted both ways (uniform points, clumps
+// and sets of small ranges; 60 to 4,000 points, 1 to 1,000 jobs, 1 to 32 bins); the
+// rule's choice takes 0.6 % longer than the better of the two on average.
+//   Lists: 0.82 ps a pair of a list.  Reference's mode: 4 us and 0.5 ns an
+//     accumulator word, for every further job 3 us and 0.4 ns a word, 0.25 us a
+//     neighbour of a centre; clean: 1.7 us and 1.15 ns, 7 us and 0.5 ns.
+//   Tiles, reference's mode: 0.5 ps a triple (multiset of one catalog), 0.8 ps where
+//     a CTA's pipelines share a histogram, and for a multiset accumulator 36 us and
+//     1.5 ns a word; clean: 4 ps a triple with two sides in range, 17 ns a tile
+//     triple in reach, and a unit's own time, 1.1 us (shared histogram 1.8) a
+//     neighbour of its points; for every further job 0.05 ns a word.
 // (4,000 points, one catalog, 16 bins to hist_max 180, 90 and 60 in a box of 100:
-// lists 8.8, 6.2 and 1.9 ms, tiles 5.3 each; three catalogs 53, 38 and 12, tiles 32;
-// 32 bins to 180: 8.9 and 8.2.  Clean, calls: 700 points, 32 bins to 32, lists 99 us,
-// tiles 182; 1,500 in a box of 200 and two jobs 166 and 143; 300 to 12 91 and 78.)
+// lists 8.8, 6.2 and 1.9 ms, tiles 5.3 each; three catalogs 53, 38 and 12, tiles 32.
+// Clean, 32 bins: 700 points to 32 lists 99 us, tiles 182; 300 to 12 91 and 78; 300
+// jobs of 100 points 4.8 and 0.35 ms.)
 bool near_pays(tpcf_ctx* ctx, const Binning& bin, const std::vector<GroupJob>& group, bool shared_hist) {
     const float reach = bin.three.hi;
     const bool clean = bin.three.clean;
-    double lists = 0, tiles = 0, neighbours = 0;
+    const double words = (double)three_near_acc_words(bin.three.n), more = (double)group.size() - 1;
+    double pairs = 0, triples = 0, usable = 0, near_triples = 0, neighbours = 0, multisets = 0;
     std::lock_guard<std::recursive_mutex> vlk(ctx->view_mu);
     const size_t step = (group.size() + 31) / 32;  // (a sample of a large set)
     for (size_t g = 0; g < group.size(); g += step) {
@@ -1425,26 +1429,33 @@ bool near_pays(tpcf_ctx* ctx, const Binning& bin, const std::vector<GroupJob>& g
         auto same = [&](int a, int b) {
             return job.catalog[a] == job.catalog[b] && job.begin[a] == job.begin[b] && n[a] == n[b];
         };
-        // centre and list roles, and the orderings that one pair stands for
+        // centre and list roles, and the ordered triples of one that is counted
         const bool ab = same(0, 1), bc = same(1, 2), ac = same(0, 2);
         const int c = bc ? 0 : ac ? 1 : ab ? 2 : 0, l1 = c == 0 ? 1 : 0, l2 = c == 2 ? 1 : 2;
-        const double sym = ab && bc ? 6 : 1, half = ab && bc ? 6 : ab || bc || ac ? 2 : 1;
-        double pairs = (double)n[c] / half, near_tiles = 1;
+        const double by_tiles = ab && bc ? 6 : 1, by_lists = ab && bc ? 6 : ab || bc || ac ? 2 : 1;
+        double ordered = (double)n[c], reached = 1;  // triples with two sides in range; share of tile triples in reach
         for (int l : {l1, l2}) {
-            const double f = pair_share(ctx, job, c, l, n, reach);
-            pairs *= f * (double)n[l];
-            neighbours = std::max(neighbours, f * (double)n[l]);
+            const double near = (double)n[l] * pair_share(ctx, job, c, l, n, reach);
+            ordered *= near;
+            neighbours = std::max(neighbours, near);
             // tiles of 64 points are cbrt(64) mean separations wide
-            near_tiles *= std::min(1.0, f * pow(1 + cbrt(64 * 4.19 / (f * (double)n[l])), 3));
+            reached *= std::min(1.0, near / (double)n[l] * pow(1 + cbrt(64 * 4.19 / near), 3));
         }
-        const double triples = (double)n[0] * (double)n[1] * (double)n[2] / sym;
-        lists += 0.82e-12 * pairs;
-        tiles += clean ? 1.9e-12 * pairs * half / sym + 8e-9 * near_tiles * triples / (TILE * TILE * TILE)
-                       : (shared_hist ? 0.8e-12 : 0.5e-12) * triples;
+        const double t = (double)step * (double)n[0] * (double)n[1] * (double)n[2] / by_tiles;
+        pairs += (double)step * ordered / by_lists;
+        usable += (double)step * ordered / by_tiles;
+        triples += t;
+        near_triples += reached * t / (TILE * TILE * TILE);
+        if (ab && bc) multisets += (double)step;
     }
-    const double words = (double)three_near_acc_words(bin.three.n), jobs = (double)group.size();
-    lists = lists * (double)step + 13e-6 + 0.5e-9 * words + (jobs - 1) * (3e-6 + 1e-9 * words) + (clean ? 0 : 8e-6);
-    tiles = tiles * (double)step + (clean ? (shared_hist ? 1.5e-6 : 0.7e-6) * neighbours : 0);
+    double lists = 0.82e-12 * pairs, tiles = 0.05e-9 * words * more;
+    if (clean) {
+        lists += 1.7e-6 + 1.15e-9 * words + more * (7e-6 + 0.5e-9 * words);
+        tiles += 4e-12 * usable + 17e-9 * near_triples + (shared_hist ? 1.8e-6 : 1.1e-6) * std::min(64.0, neighbours);
+    } else {
+        lists += 4e-6 + 0.5e-9 * words + more * (3e-6 + 0.4e-9 * words) + 0.25e-6 * std::min(150.0, neighbours);
+        tiles += (shared_hist ? 0.8e-12 : 0.5e-12) * triples + std::min(3.0, multisets) * (36e-6 + 1.5e-9 * words);
+    }
     return lists < tiles;
 }
 

@@ -21,6 +21,7 @@ def _spec(overflow, axis, precision=tpcf.GUARDED_FP32):
     (1000, 180.0, 16, {tpcf.OVERFLOW_COMPAT: True, tpcf.OVERFLOW_CLEAN: False}),
     (1000, 40.0, 16, {tpcf.OVERFLOW_COMPAT: False, tpcf.OVERFLOW_CLEAN: False}),
     (1000, 8.0, 32, {tpcf.OVERFLOW_COMPAT: False, tpcf.OVERFLOW_CLEAN: True}),
+    (300, 40.0, 16, {tpcf.OVERFLOW_COMPAT: False, tpcf.OVERFLOW_CLEAN: False}),
 ])
 def test_rule(monkeypatch, overflow, n, hi, bins, tiles):
     d = synth.uniform(n, box=100.0, seed=n)
