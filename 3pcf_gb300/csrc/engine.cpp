@@ -454,7 +454,6 @@ struct Binning {
     double lmax = INFINITY;   // no counted triangle/pair has a side >= lmax
     bool tri_prune = false;   // triangle: test the s and q ranges on tile-triple side bounds
     double s_lo = 0, s_hi = 0, q_hi = 0;
-    double lmin_pair = 0;     // pairs: no counted pair has d < lmin_pair
 };
 
 // Whether a job of this spec runs in the guarded FP32 kernels.  The fast
@@ -697,7 +696,6 @@ Binning make_binning(const tpcf_spec& sp) {
         }
     }
     // device copy of the bound, rounded up so that a float side >= it is >= lmax
-    if (sp.kind == TPCF_TRIANGLE_JBJ) b.tri.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
     if (sp.kind == TPCF_TRIANGLE || sp.kind == TPCF_TRIANGLE_JBJ) {
         TriParams& p = b.tri;
         p.lmax = b.lmax < 3e38 ? nextafterf((float)b.lmax, INFINITY) : INFINITY;
@@ -708,7 +706,9 @@ Binning make_binning(const tpcf_spec& sp) {
         };
         p.mid_hi = limit((double)p.s_hi);
         // the split lets the fewest triangles through to the binning on
-        // clustered data (77 to 83 % for splits at 0.6 to 0.8 of s_hi)
+        // clustered data (77 to 83 % for splits at 0.6 to 0.8 of s_hi; of the
+        // benchmark's binning -- other binnings take the same, JBJ included, where
+        // another share might let fewer through)
         p.s_split = std::max(p.s_lo, 0.72f * p.s_hi);
         p.mid_split = std::max(p.s_hi, limit((double)p.s_split));
     }
@@ -819,10 +819,10 @@ struct Lane {
     }
 };
 
-// d_counters: words zeroed before every count, then the header of the plan
 // shares of centres per warp of the triangle lists at least
 constexpr uint64_t TL_WANT = 32;
 
+// d_counters: words zeroed before every count, then the header of the plan
 constexpr int CTR_WORK = 0;     // units (items) handed out
 constexpr int CTR_RECHECK = 1;  // queued guard-band triangles
 constexpr int CTR_EVAL = 2;     // evaluated (two words), binned (pairs: tile pairs; two words)
@@ -1505,7 +1505,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     //   JBJ with very many centres, whose tile triples hold few shortest sides
     //   in range (blobs of 25k points, 150,000 centres, 1244 -> 1097 ms, 15k 343 ->
     //   338, 10k 139 -> 140, 5k 24 -> 28 ms; s/m from 0.5: 25k 179 -> 143, 10k 23.4
-    //   -> 22.9, 7k 9.9 -> 10.4).
+    //   -> 22.9, 7k 9.9 -> 10.4).  The number of centres stands in for how few of a
+    //   tile triple's triangles are near, which depends on the field: of uniform
+    //   points the lists are sooner from 5k on (14k in a box of 100 114 -> 74 ms, 5k
+    //   9.0 -> 4.6), of many small blobs not at 25k (500 points a blob, 14k 44 ->
+    //   57, 25k 164 -> 171).
     // Sets of many small jobs (voxels) keep the tiles: each of a job's centres
     // is an item here (16,500 jobs of a 20k cone 1.9 -> 8.8 ms).
     const char* tl_env = getenv("TPCF_TRI_LISTS");
