@@ -595,6 +595,15 @@ Binning make_binning(const tpcf_spec& sp) {
         // c-dependent part: |dc| <= 7e-7 |c| (reciprocals of two sides, products, the
         // reference's roundings: 9 x 2^-24, and a margin) amplified by 1/sqrt(1-c^2) <= 1/sqrt(1-|c|)
         p.t_thrB = (float)(7e-7 * K);
+        // A cosine that the reference rounds beyond +-1 gives it NaN, which has a bin
+        // of its own or none.  Where the angles 0 and pi lie on bin edges, as with
+        // [0, 1), the bands hold every such triangle; else the band takes in the
+        // whole bin as the cosine comes within 7e-7 of +-1.
+        auto at_edge = [&](double angle) {
+            const double x = (angle / pi_ref - (double)p.t_lo) / (double)p.t_bw;
+            return fabs(x - nearbyint(x)) <= 1e-4 * K;
+        };
+        if (!at_edge(0) || !at_edge(pi)) p.t_thrB = (float)std::max(7e-7 * K, 4.2e-4);
         p.t2_off = (float)((1.0 - 3.0 * (double)p.t_lo) / (double)p.t_bw - 1.5);
         p.theta_full = (p.t_lo <= 0.f && p.t_hi >= 1.f);
         if (sp.precision == TPCF_GEOMETRY_FP64) {
