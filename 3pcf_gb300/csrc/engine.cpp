@@ -2112,10 +2112,9 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
                 EQ(cudaEventRecordWithFlags(L.ev_mid, st, ev_flags));
                 if (near) {
                     const DevJob* after = L.d_jobs.p + group.size();
-                    const unsigned int* dense = L.d_counters.p + CTR_DENSE;
-                    EQ(launch_three_wedges(after, L.d_rows.p + group.size() + 1, (int)nwedge_jobs, nwedges, dense,
-                                           bin.near, ctx->num_sms * 8, st));
-                    EQ(launch_three_expand(after + nwedge_jobs, (int)accs.size(), dense, bin.near, st));
+                    EQ(launch_three_wedges(after, L.d_rows.p + group.size() + 1, (int)nwedge_jobs, nwedges,
+                                           L.d_counters.p + CTR_DENSE, bin.near, ctx->num_sms * 8, st));
+                    EQ(launch_three_expand(after + nwedge_jobs, (int)accs.size(), bin.near, st));
                 }
                 if (recheck)
                     EQ(launch_triangle_recheck(L.d_jobs.p, q, bin.tri, acos_t, fast_jbj ? 1 : geom ? 2 : 0,

@@ -245,8 +245,7 @@ cudaError_t launch_three_near(const DevJob* jobs, const uint32_t* item_off, int 
                               unsigned long long* work, const NearParams& p, int grid, int pipes, cudaStream_t st);
 cudaError_t launch_three_wedges(const DevJob* jobs, const uint32_t* item_off, int njobs, unsigned int nitems,
                                 const unsigned int* dense, const NearParams& p, int grid, cudaStream_t st);
-cudaError_t launch_three_expand(const DevJob* accs, int naccs, const unsigned int* dense, const NearParams& p,
-                                cudaStream_t st);
+cudaError_t launch_three_expand(const DevJob* accs, int naccs, const NearParams& p, cudaStream_t st);
 size_t three_near_acc_words(int n);
 size_t three_near_smem_bytes(int n, int pipes);
 

@@ -2984,8 +2984,12 @@ three_near_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ 
     if (threadIdx.x == 0) s_since = s_pairs = 0;
     auto draw = [&]() {  // by the pipeline's first warp; nothing more once the launch is refused
         if (warp != 0) return;
-        unsigned int t = TASK_NONE;
-        if (lane == 0 && *(volatile unsigned int*)dense == 0u) t = atomicAdd(counter, 1u);
+        unsigned int t = 0;
+        if (lane == 0) {  // (both on their way together: an item after the refusal is left undone)
+            const unsigned int refused = *(volatile unsigned int*)dense;
+            t = atomicAdd(counter, 1u);
+            if (refused) t = TASK_NONE;
+        }
         t = __shfl_sync(0xffffffffu, t, 0);
         uint4 it = make_uint4(TASK_NONE, 0, 0, 0);
         if (t < nitems) {
@@ -3177,7 +3181,7 @@ size_t three_wedge_smem_bytes(int n) { return (size_t)TS_WARPS * 2 * (n + 1) * s
 __global__ void __launch_bounds__(TS_GROUP_THREADS)
 three_wedge_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ item_off, int njobs,
                    unsigned int nitems, const unsigned int* __restrict__ dense, NearParams p) {
-    if (*dense) return;
+    const unsigned int refused = *dense;
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned int* const H = reinterpret_cast<unsigned int*>(smem);  // [warp][list][code]
     __shared__ int s_job;
@@ -3189,6 +3193,7 @@ three_wedge_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__
             if (lane == 0) s_job = slot;
         }
         for (int b = threadIdx.x; b < TS_WARPS * 2 * m; b += blockDim.x) H[b] = 0;
+        if (refused) return;  // (by the launch before this one: the same for all threads)
         __syncthreads();
         const DevJob& J = jobs[s_job];
         const unsigned int l = t - item_off[s_job];
@@ -3238,9 +3243,7 @@ three_wedge_kernel(const DevJob* __restrict__ jobs, const uint32_t* __restrict__
 // Expands accumulators (job: its hist) into the histograms (its aux): the
 // orderings of each multiset, and in the reference's mode the triples with
 // sides at or above hist_max.
-__global__ void __launch_bounds__(256)
-three_expand_kernel(const DevJob* __restrict__ accs, const unsigned int* __restrict__ dense, NearParams p) {
-    if (*dense) return;
+__global__ void __launch_bounds__(256) three_expand_kernel(const DevJob* __restrict__ accs, NearParams p) {
     const DevJob& A = accs[blockIdx.y];
     const uint32_t cls = A.mode & NEAR_CLASS_MASK, centre = A.mode >> NEAR_CENTRE_SHIFT;
     const int n = p.n, m = n + 1, m3 = m * m * m, z = p.zcode, F = n + 1;
@@ -3316,13 +3319,12 @@ cudaError_t launch_three_wedges(const DevJob* jobs, const uint32_t* item_off, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_three_expand(const DevJob* accs, int naccs, const unsigned int* dense, const NearParams& p,
-                                cudaStream_t st) {
+cudaError_t launch_three_expand(const DevJob* accs, int naccs, const NearParams& p, cudaStream_t st) {
     const int m = p.n + 1, words = m * m * m + 2 * m * m + m;
     // (at most 65535 accumulators a launch)
     for (int a = 0; a < naccs; a += 65535) {
         const dim3 grid(std::min(32, (words + 255) / 256), std::min(65535, naccs - a));
-        three_expand_kernel<<<grid, 256, 0, st>>>(accs + a, dense, p);
+        three_expand_kernel<<<grid, 256, 0, st>>>(accs + a, p);
     }
     return cudaGetLastError();
 }
