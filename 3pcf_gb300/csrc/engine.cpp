@@ -1794,8 +1794,11 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     L.d_counters.reserve(CTR_WORDS);
     const std::vector<Shape> cands = shape_candidates(ctx, sp, bin, fp64, near, tlist ? (int)nslots : 0);
     const bool plan_hit = sig == L.plan_sig;
-    const uint64_t key = batch_key(sig);  // of the batch, in what is remembered of it
+    // of the batch, in what is remembered of it (without lists it is asked for only
+    // when the plan is under way on the device)
+    uint64_t key = 0;
     if (near) {
+        key = batch_key(sig);
         bool refused = false;
         {
             std::lock_guard<std::mutex> tlk(ctx->tune_mu);
@@ -2208,6 +2211,7 @@ void run_group(tpcf_ctx* ctx, Lane& L, const std::vector<GroupJob>& group, bool 
     const bool autotune = !(tenv && tenv[0] == '0');
     Shape shape = cands[0];
     uint64_t tuned_runs = 0;
+    if (!near) key = batch_key(sig);
     {
         std::lock_guard<std::mutex> tlk(ctx->tune_mu);
         auto it = ctx->tuned.find(key);
